@@ -83,6 +83,13 @@ static_assert(offsetof(rg_mb_out, luma) % 4 == 0 && offsetof(rg_mb_out, chroma_d
               "record levels written by words");
 static_assert(offsetof(Smem, pred_y) % 8 == 0 && offsetof(Smem, tmp_y) % 8 == 0, "16x16 predictions written 8 bytes per lane");
 
+// Every kernel of this file runs one warp per block, and its shared memory has this one name: the
+// functions below address it directly (shared-memory loads at constant offsets) instead of through
+// a reference, which a call turns into a generic address -- a 64-bit pointer in registers and loads
+// that resolve their memory space as they run.
+__shared__ Smem sm;
+__device__ __forceinline__ uint8_t* sm_at(int off) { return (uint8_t*)&sm + off; }
+
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 __device__ __forceinline__ MbInfo ld_info(const MbInfo* p) {
   int4 v = *(const int4*)p;
@@ -200,7 +207,11 @@ __device__ __forceinline__ void idct8_1d(const int* d, int* o) {
   o[4] = (int)(b6 - b1); o[5] = (int)(b4 - b3); o[6] = (int)(b2 - b5); o[7] = (int)(b0 - b7);
 }
 // SATD of a 4x4 block (metrics.rs:705, halved).
-__device__ __noinline__ uint32_t satd4(const uint8_t* a, int sa, const uint8_t* b, int sb) {
+// Byte offsets of the two blocks in Smem, rows of 16 samples.
+__device__ __noinline__ uint32_t satd4(int off_a, int off_b) {
+  const uint8_t* a = sm_at(off_a);
+  const uint8_t* b = sm_at(off_b);
+  constexpr int sa = 16, sb = 16;
   int t[4][4];
 #pragma unroll
   for (int y = 0; y < 4; y++) {
@@ -242,7 +253,7 @@ __device__ __forceinline__ int inv4_pass(int v, int step, int i) {
 // ---------------------------------------------------------------------------------------------
 // Half-sample window (h264_enc.rs:747 hpel_window, :803 hpel_window_centre): integer origin
 // (ox, oy); plane coordinate (r, c) is the sample at (ox + c, oy + r).
-__device__ __noinline__ void stage_window(const uint8_t* ref, int stride, int ox, int oy, Smem& sm) {
+__device__ __noinline__ void stage_window(const uint8_t* ref, int stride, int ox, int oy) {
   int lane = lane_id();
   // 23 rows x 6 words: five words per lane, all loads issued before the first use
   uint32_t lo[5], hi[5], sh[5];
@@ -267,7 +278,7 @@ __device__ __noinline__ void stage_window(const uint8_t* ref, int stride, int ox
   __syncwarp();
 }
 // need: bit 0 b plane (h), bit 1 h plane (v), bit 2 j plane (c)
-__device__ __noinline__ void build_hpel(Smem& sm, int need) {
+__device__ __noinline__ void build_hpel(int need) {
   int lane = lane_id();
   if (need & 5) {
     for (int i = lane; i < 23 * 18; i += 32) {
@@ -306,16 +317,15 @@ __device__ __forceinline__ int planes_needed(int fx, int fy) {
 // Quarter-sample prediction of the 16x16 block whose integer position is (wx, wy) in window
 // coordinates: one window plane, or the rounded average of two (window_src, enc.rs:1395; equal
 // to h264_luma_mc_scalar, h264_mc.rs:148, by enc.rs:4030). Returns the two source rows' bases.
+// (byte offsets in Smem).
 struct QSrc {
-  const uint8_t* a;
-  const uint8_t* b;
-  int sa, sb, avg;
+  int a, b, sa, sb, avg;
 };
-__device__ __noinline__ QSrc qpel_src(const Smem& sm, int wx, int wy, int fx, int fy) {
-  const uint8_t* G = &sm.win[(wy + 2) * 24 + wx + 2];
-  const uint8_t* B = &sm.hph[wy * 20 + wx];
-  const uint8_t* V = &sm.hpv[wy * 20 + wx];
-  const uint8_t* J = &sm.hpj[wy * 20 + wx];
+__device__ __noinline__ QSrc qpel_src(int wx, int wy, int fx, int fy) {
+  const int G = (int)offsetof(Smem, win) + (wy + 2) * 24 + wx + 2;
+  const int B = (int)offsetof(Smem, hph) + wy * 20 + wx;
+  const int V = (int)offsetof(Smem, hpv) + wy * 20 + wx;
+  const int J = (int)offsetof(Smem, hpj) + wy * 20 + wx;
   switch (fx | (fy << 2)) {
     case 0: return {G, G, 24, 24, 0};
     case 1: return {G, B, 24, 20, 1};
@@ -346,9 +356,9 @@ __device__ __forceinline__ uint2 lds8(const uint8_t* p) {
 // This lane's 8 prediction samples (row lane/2, columns 8 (lane&1) ..) packed in two words.
 __device__ __forceinline__ uint2 qpel8(const QSrc& q) {
   int lane = lane_id(), i = lane >> 1, j0 = (lane & 1) * 8;
-  uint2 a = lds8(q.a + i * q.sa + j0);
+  uint2 a = lds8(sm_at(q.a + i * q.sa + j0));
   if (!q.avg) return a;
-  uint2 b = lds8(q.b + i * q.sb + j0);
+  uint2 b = lds8(sm_at(q.b + i * q.sb + j0));
   return make_uint2(__vavgu4(a.x, b.x), __vavgu4(a.y, b.y));
 }
 // Cost of a full-pel position (mx, my): the warp's SAD of the 16x16 block (this lane's 8 source
@@ -359,15 +369,15 @@ __device__ __noinline__ uint32_t fullpel_cost(uint2 sv, uint2 r, int mx, int my,
 }
 // This lane's SAD against the quarter-sample prediction at window position (wx, wy), phase
 // (fx, fy): shared by the candidates of the sub-pel search.
-__device__ __noinline__ uint32_t qpel_sad(const Smem& sm, uint2 sv, int wx, int wy, int fx, int fy) {
-  return vsad8(sv, qpel8(qpel_src(sm, wx, wy, fx, fy)));
+__device__ __noinline__ uint32_t qpel_sad(uint2 sv, int wx, int wy, int fx, int fy) {
+  return vsad8(sv, qpel8(qpel_src(wx, wy, fx, fy)));
 }
-__device__ __forceinline__ uint2 src8(const Smem& sm) {
+__device__ __forceinline__ uint2 src8() {
   int lane = lane_id();
   return *(const uint2*)&sm.src_y[(lane >> 1) * 16 + (lane & 1) * 8];
 }
 // Prediction of the 16x16 block displaced by mv into pred_y (enc.rs:1058 mc_luma).
-__device__ __noinline__ void mc_luma16(const uint8_t* ref, int stride, int x0, int y0, int mvx, int mvy, Smem& sm) {
+__device__ __noinline__ void mc_luma16(const uint8_t* ref, int stride, int x0, int y0, int mvx, int mvy) {
   int ix = x0 + (mvx >> 2), iy = y0 + (mvy >> 2), fx = mvx & 3, fy = mvy & 3;
   int lane = lane_id();
   if ((fx | fy) == 0) {
@@ -376,14 +386,14 @@ __device__ __noinline__ void mc_luma16(const uint8_t* ref, int stride, int x0, i
     __syncwarp();
     return;
   }
-  stage_window(ref, stride, ix, iy, sm);
-  build_hpel(sm, planes_needed(fx, fy));
-  uint2 v = qpel8(qpel_src(sm, 0, 0, fx, fy));
+  stage_window(ref, stride, ix, iy);
+  build_hpel(planes_needed(fx, fy));
+  uint2 v = qpel8(qpel_src(0, 0, fx, fy));
   *(uint2*)&sm.pred_y[(lane >> 1) * 16 + (lane & 1) * 8] = v;
   __syncwarp();
 }
 // Chroma prediction of both planes (h264_enc.rs:1279 chroma_mc_8x8_x2_scalar; enc.rs:1082).
-__device__ __noinline__ void mc_chroma8(const uint8_t* ru, const uint8_t* rv, int stride, int mbx, int mby, int mvx, int mvy, Smem& sm) {
+__device__ __noinline__ void mc_chroma8(const uint8_t* ru, const uint8_t* rv, int stride, int mbx, int mby, int mvx, int mvy) {
   int lane = lane_id();
   int cx = mbx * 8 + (mvx >> 3), cy = mby * 8 + (mvy >> 3), fx = mvx & 7, fy = mvy & 7;
   int wa = (8 - fx) * (8 - fy), wb = fx * (8 - fy), wc = (8 - fx) * fy, wd = fx * fy;
@@ -418,13 +428,13 @@ constexpr unsigned long long kZigzagIndex4 = 0xfea9db83c7426510ull;
 // Forward 4x4 core transform (fixed.rs:104, int16 output) and quantisation of `nblocks` 4x4
 // residual blocks (src - pred): luma blocks in decoding order (chroma = false) or the eight chroma
 // blocks, U then V (chroma = true). Lane = coefficient (raster p = lane & 15); half-warp h takes
-// block 2 it + h, two blocks per step. Levels go to out[16 b + p]; the raw DC of each block to
-// dc_raw[b] when given. Lane b then holds block b's: any level (among zig-zag indices >= first),
-// any |level| > 1 (same), and the decimation score of its zig-zag levels from index `first`
-// (enc.rs:559 decimate_score without its |level| > 1 rule; the caller applies it).
-__device__ __noinline__ void quant4x4_blocks(Smem& sm, bool chroma, int nblocks, int first, int qp, uint32_t shift,
-                                             uint32_t bias, int16_t* out, int16_t* dc_raw, int& my_nz, int& my_big,
-                                             int& my_score) {
+// block 2 it + h, two blocks per step. Levels go to sm.coef / sm.ccoef [16 b + p]; the raw DC of each
+// chroma block to sm.cdcraw[b]. Lane b returns block b's: bit 0 any level (among zig-zag indices >=
+// first), bit 1 any |level| > 1 (same), and from bit 2 the decimation score of its zig-zag levels
+// from index `first` (enc.rs:559 decimate_score without its |level| > 1 rule; the caller applies it).
+__device__ __noinline__ uint32_t quant4x4_blocks(bool chroma, int nblocks, int first, int qp, uint32_t shift, uint32_t bias) {
+  int16_t* const out = chroma ? sm.ccoef : sm.coef;
+  int my_nz, my_big, my_score;
   int lane = lane_id(), p = lane & 15, h = lane >> 4, xl = p & 3, yl = p >> 2;
   int zi = (int)((kZigzagIndex4 >> (4 * p)) & 15);
   uint32_t mf = c_mf4[qp % 6][pos4(p)];
@@ -448,7 +458,7 @@ __device__ __noinline__ void quant4x4_blocks(Smem& sm, bool chroma, int nblocks,
     }
     int d = (int)s[yl * stride + xl] - (int)pr[yl * stride + xl];
     int c = (int16_t)fwd4_pass(fwd4_pass(d, 1, xl), 4, yl);
-    if (dc_raw && p == 0) dc_raw[b] = (int16_t)c;
+    if (chroma && p == 0) sm.cdcraw[b] = (int16_t)c;
     int l = quant_level(c, mf, bias, shift);
     out[b * 16 + p] = (int16_t)l;
     bool nz = l != 0 && counted;
@@ -472,16 +482,17 @@ __device__ __noinline__ void quant4x4_blocks(Smem& sm, bool chroma, int nblocks,
     }
   }
   __syncwarp();
+  return (uint32_t)my_nz | ((uint32_t)my_big << 1) | ((uint32_t)my_score << 2);
 }
 
 // Luma 4x4 residual of pred_y, quantised (inter) and decimated into sm.coef
-// (enc.rs:1810 quant_luma_4x4_inter). Returns cbp; lanes 0..15 report block lane's "any level".
-__device__ __noinline__ int luma4x4_inter(int qp, Smem& sm, uint32_t* nz_lane_out) {
+// (enc.rs:1810 quant_luma_4x4_inter). Returns cbp.
+__device__ __noinline__ int luma4x4_inter(int qp) {
   int lane = lane_id();
   uint32_t shift, bias;
   quant4_params(qp, false, shift, bias);
-  int my_nz, my_big, my_score;
-  quant4x4_blocks(sm, false, 16, 0, qp, shift, bias, sm.coef, nullptr, my_nz, my_big, my_score);
+  const uint32_t mine = quant4x4_blocks(false, 16, 0, qp, shift, bias);
+  int my_nz = mine & 1, my_big = (mine >> 1) & 1, my_score = mine >> 2;
   // per-8x8 aggregates (lanes 4g..4g+3)
   int g_nz = my_nz | __shfl_xor_sync(FULL, my_nz, 1);
   g_nz |= __shfl_xor_sync(FULL, g_nz, 2);
@@ -506,13 +517,13 @@ __device__ __noinline__ int luma4x4_inter(int qp, Smem& sm, uint32_t* nz_lane_ou
   for (int k = 0; k < 4; k++)
     if (!((cbp >> k) & 1)) ((uint32_t*)sm.coef)[lane + 32 * k] = 0u;
   __syncwarp();
-  if (nz_lane_out) *nz_lane_out = (lane < 16 && ((cbp >> (lane >> 2)) & 1)) ? (uint32_t)my_nz : 0u;
   return cbp;
 }
 
-// The 1-D forward 8x8 transform in place on p[0], p[stride], ..., p[7 * stride] (row and column
+// The 1-D forward 8x8 transform in place on sm.t8[at], [at + stride], ..., [at + 7 * stride] (row and column
 // passes share it).
-__device__ __noinline__ void fdct8_inplace(int* p, int stride) {
+__device__ __noinline__ void fdct8_inplace(int at, int stride) {
+  int* p = &sm.t8[at];
   int a[8], o[8];
 #pragma unroll
   for (int k = 0; k < 8; k++) a[k] = p[k * stride];
@@ -533,8 +544,8 @@ __device__ __forceinline__ int zigzag8(int y, int x) {
 // (enc.rs:2041 quant_luma_8x8_inter). Lanes 8b..8b+7 own block b: a row each in the first pass,
 // column q each in the second. The decimation score of a block comes from the bitmask of its
 // nonzero zig-zag positions (run of zeros below each, weights 3 / 2 / 1 / 0 for runs of
-// 0-3 / 4-11 / 12-23 / longer, enc.rs:559 with the 8x8 table). Returns cbp; *nnz8 = count.
-__device__ __noinline__ int luma8x8_inter(int qp, Smem& sm, uint32_t* nnz8) {
+// 0-3 / 4-11 / 12-23 / longer, enc.rs:559 with the 8x8 table). Returns cbp | nonzero levels << 4.
+__device__ __noinline__ uint32_t luma8x8_inter(int qp) {
   int lane = lane_id();
   int b = lane >> 3, q = lane & 7;
   int bx = (b & 1) * 8, by = (b >> 1) * 8;
@@ -545,14 +556,14 @@ __device__ __noinline__ int luma8x8_inter(int qp, Smem& sm, uint32_t* nnz8) {
     int off = (by + q) * 16 + bx + x;
     sm.t8[b * 64 + q * 8 + x] = (int)sm.src_y[off] - (int)sm.pred_y[off];
   }
-  fdct8_inplace(&sm.t8[b * 64 + q * 8], 1);
+  fdct8_inplace(b * 64 + q * 8, 1);
   __syncwarp();
   uint32_t mf6[6];
 #pragma unroll
   for (int k = 0; k < 6; k++) mf6[k] = c_mf8[qp % 6][k];
   int any = 0, big = 0;
   unsigned long long zmask = 0;
-  fdct8_inplace(&sm.t8[b * 64 + q], 8);  // column q; then quantisation row by row
+  fdct8_inplace(b * 64 + q, 8);  // column q; then quantisation row by row
 #pragma unroll 1
   for (int y = 0; y < 8; y++) {
     int i = y * 8 + q, cls = pos8(i);
@@ -600,19 +611,23 @@ __device__ __noinline__ int luma8x8_inter(int qp, Smem& sm, uint32_t* nnz8) {
     cnt = __popcll(zmask) * (q == 0);
   }
   __syncwarp();
-  *nnz8 = wsum(cnt);
-  return cbp;
+  return (uint32_t)cbp | (wsum(cnt) << 4);
 }
 
 // Chroma residual of pred_u/pred_v (enc.rs:1899 quant_chroma): lanes 0..7 own block
 // (plane = lane / 4, b = lane % 4). Levels into sm.ccoef (raster), DC levels into sm.cdc.
-// Outputs per plane: AC present and AC decimation score. Lanes 0..31 all return the values.
-__device__ __noinline__ void chroma_quant(int qpc, bool intra, Smem& sm, uint32_t ac_any[2], uint32_t ac_score[2]) {
+// Returns, in every lane and per plane: AC present and AC decimation score.
+struct ChromaAc {
+  uint32_t w;  // byte p: the score of plane p (at most 4 x 45); bits 16, 17: AC present
+  __device__ __forceinline__ bool any(int p) const { return (w >> (16 + p)) & 1u; }
+  __device__ __forceinline__ uint32_t score(int p) const { return (w >> (8 * p)) & 255u; }
+};
+__device__ __noinline__ ChromaAc chroma_quant(int qpc, bool intra) {
   int lane = lane_id();
   uint32_t shift, bias;
   quant4_params(qpc, intra, shift, bias);
-  int ac, big, sc;
-  quant4x4_blocks(sm, true, 8, 1, qpc, shift, bias, sm.ccoef, sm.cdcraw, ac, big, sc);
+  const uint32_t mine = quant4x4_blocks(true, 8, 1, qpc, shift, bias);
+  int ac = mine & 1, big = (mine >> 1) & 1, sc = mine >> 2;
   uint32_t my_ac = lane < 8 ? (uint32_t)ac : 0u;
   uint32_t my_score = lane < 8 ? (big ? 9u : (uint32_t)sc) : 0u;  // decimate_score's |level| > 1 rule
   __syncwarp();
@@ -632,13 +647,12 @@ __device__ __noinline__ void chroma_quant(int qpc, bool intra, Smem& sm, uint32_
   pa |= __shfl_xor_sync(FULL, pa, 2);
   uint32_t ps = my_score + __shfl_xor_sync(FULL, my_score, 1);
   ps += __shfl_xor_sync(FULL, ps, 2);
-  ac_any[0] = __shfl_sync(FULL, pa, 0);
-  ac_any[1] = __shfl_sync(FULL, pa, 4);
-  ac_score[0] = __shfl_sync(FULL, ps, 0);
-  ac_score[1] = __shfl_sync(FULL, ps, 4);
+  const uint32_t both = ps | (pa << 16);
+  const uint32_t u = __shfl_sync(FULL, both, 0), v = __shfl_sync(FULL, both, 4);
   __syncwarp();
+  return ChromaAc{(u & 0x100ffu) | ((v & 0xffu) << 8) | ((v & 0x10000u) << 1)};
 }
-__device__ __forceinline__ bool chroma_dc_any(const Smem& sm) {
+__device__ __forceinline__ bool chroma_dc_any() {
   bool a = false;
 #pragma unroll
   for (int i = 0; i < 8; i++) a |= sm.cdc[i] != 0;
@@ -648,7 +662,7 @@ __device__ __forceinline__ bool chroma_dc_any(const Smem& sm) {
 // Adds the dequantised chroma residual to pred_u / pred_v (enc.rs:1992 recon_chroma): the DC of
 // each block from the 2x2 inverse (h264.rs:1674 dequantize_idct_chroma_dc2x2), its AC dequantised
 // when cbpc == 2, then the inverse core transform. Lane = coefficient, two blocks per step.
-__device__ __noinline__ void chroma_recon(int qpc, int cbpc, Smem& sm) {
+__device__ __noinline__ void chroma_recon(int qpc, int cbpc) {
   if (cbpc == 0) return;
   int lane = lane_id(), p = lane & 15, h = lane >> 4, xl = p & 3, yl = p >> 2;
   int qmul = (c_dq4[qpc % 6][0] * 16) << (qpc / 6 + 2);
@@ -671,9 +685,10 @@ __device__ __noinline__ void chroma_recon(int qpc, int cbpc, Smem& sm) {
 // Raster position of each 4x4 zig-zag index, 4 bits per index (frame scan, Table 8-12).
 constexpr unsigned long long kScan4Packed = 0xfeb7adc963258410ull;
 
-// The 1-D inverse 8x8 transform in place on p[0], p[stride], ..., p[7 * stride] (rows and columns
+// The 1-D inverse 8x8 transform in place on sm.t8[at], [at + stride], ..., [at + 7 * stride] (rows and columns
 // of the 8x8 reconstruction share it).
-__device__ __noinline__ void idct8_inplace(int* p, int stride) {
+__device__ __noinline__ void idct8_inplace(int at, int stride) {
+  int* p = &sm.t8[at];
   int d[8], o[8];
 #pragma unroll
   for (int k = 0; k < 8; k++) d[k] = p[k * stride];
@@ -685,7 +700,7 @@ __device__ __noinline__ void idct8_inplace(int* p, int stride) {
 // Adds the dequantised 8x8 residual of the coded blocks of sm.coef8 to pred_y (enc.rs:2013
 // recon_8x8: dequantize_block8x8, h264.rs:1403, then h264_idct8_add, h264_idct.rs:207).
 // Lanes 8b..8b+7 own block b: row q, then column q.
-__device__ __noinline__ void recon_luma8x8(Smem& sm, int qp, int cbp) {
+__device__ __noinline__ void recon_luma8x8(int qp, int cbp) {
   int lane = lane_id(), b = lane >> 3, q = lane & 7;
   bool coded = (cbp >> b) & 1;
   int qdiv = qp / 6, rem = qp % 6;
@@ -701,11 +716,11 @@ __device__ __noinline__ void recon_luma8x8(Smem& sm, int qp, int cbp) {
       int dv = qdiv >= 2 ? l * (v << (qdiv - 2)) : ((l * v + (1 << (1 - qdiv))) >> (2 - qdiv));
       sm.t8[b * 64 + i] = clamp_i16(dv);
     }
-    idct8_inplace(&sm.t8[b * 64 + q * 8], 1);
+    idct8_inplace(b * 64 + q * 8, 1);
   }
   __syncwarp();
   if (coded) {
-    idct8_inplace(&sm.t8[b * 64 + q], 8);
+    idct8_inplace(b * 64 + q, 8);
     int bx = (b & 1) * 8, by = (b >> 1) * 8;
 #pragma unroll 1
     for (int y = 0; y < 8; y++) {
@@ -719,7 +734,7 @@ __device__ __noinline__ void recon_luma8x8(Smem& sm, int qp, int cbp) {
 
 // Adds the dequantised luma 4x4 residual of the coded 8x8 groups of sm.coef to pred_y
 // (enc.rs:1978 recon_luma_4x4). Lane = coefficient, two blocks per step.
-__device__ __noinline__ void recon_luma4x4(Smem& sm, int qp, int cbp) {
+__device__ __noinline__ void recon_luma4x4(int qp, int cbp) {
   int lane = lane_id(), p = lane & 15, h = lane >> 4, xl = p & 3, yl = p >> 2;
   int dqs = (int)c_dq4[qp % 6][pos4(p)] << (qp / 6);
 #pragma unroll 1
@@ -740,7 +755,7 @@ __device__ __noinline__ void recon_luma4x4(Smem& sm, int qp, int cbp) {
 // Intra prediction (h264.rs:1715 predict_intra_16x16_scalar, :1967 chroma; enc.rs:1561,1586)
 // Plane-mode parameters; called by the whole warp: lanes 0..7 take the terms of H
 // ((q + 1) (top[8 + q] - top[6 - q])), lanes 8..15 those of V down the left column.
-__device__ void plane16_params(const Smem& sm, bool ht, bool hl, int tl, int& pa, int& pb, int& pc) {
+__device__ void plane16_params(bool ht, bool hl, int tl, int& pa, int& pb, int& pc) {
   int lane = lane_id(), q = lane & 7;
   int term = 0;
   if (lane < 16) {
@@ -757,7 +772,7 @@ __device__ void plane16_params(const Smem& sm, bool ht, bool hl, int tl, int& pa
 }
 // DC of the 16x16 prediction; called by the whole warp: lane q < 16 adds top[q], lane 16 + q
 // left[q] (both sums below 2^16, one reduction).
-__device__ __forceinline__ int dc16(const Smem& sm, bool ht, bool hl) {
+__device__ __forceinline__ int dc16(bool ht, bool hl) {
   int lane = lane_id();
   uint32_t v = lane < 16 ? (ht ? (uint32_t)sm.top[lane] : 0u) : (hl ? (uint32_t)sm.left[lane - 16] << 16 : 0u);
   uint32_t both = wsum(v), st = both & 0xffffu, sl = both >> 16;
@@ -766,13 +781,13 @@ __device__ __forceinline__ int dc16(const Smem& sm, bool ht, bool hl) {
   if (hl) return (int)((sl + 8) >> 4);
   return 128;
 }
-__device__ __noinline__ void pred16_into(int mode, Smem& sm, uint8_t* dst, bool ht, bool hl, int tl) {
+__device__ __noinline__ void pred16_into(int mode, int dst, bool ht, bool hl, int tl) {
   int lane = lane_id();
   int y = lane >> 1, x0 = (lane & 1) * 8;
-  uint8_t* o = dst + y * 16 + x0;  // this lane's 8 samples (8-byte aligned)
+  uint8_t* o = sm_at(dst + y * 16 + x0);  // this lane's 8 samples (8-byte aligned)
   if (mode == 3) {
     int pa, pb, pc;
-    plane16_params(sm, ht, hl, tl, pa, pb, pc);
+    plane16_params(ht, hl, tl, pa, pb, pc);
     uint32_t w[2] = {0u, 0u};
 #pragma unroll
     for (int k = 0; k < 8; k++)
@@ -783,17 +798,21 @@ __device__ __noinline__ void pred16_into(int mode, Smem& sm, uint8_t* dst, bool 
     if (mode == 0) {
       v = ht ? lds8(&sm.top[x0]) : make_uint2(0x80808080u, 0x80808080u);
     } else {
-      uint32_t b = mode == 1 ? (hl ? sm.left[y] : 128u) : (uint32_t)dc16(sm, ht, hl);
+      uint32_t b = mode == 1 ? (hl ? sm.left[y] : 128u) : (uint32_t)dc16(ht, hl);
       v = make_uint2(b * 0x01010101u, b * 0x01010101u);
     }
     *(uint2*)o = v;
   }
   __syncwarp();
 }
-// Intra 16x16 analysis (enc.rs:1637 analyse_i16_edges): SATD per mode; returns best mode.
-__device__ __noinline__ int analyse_i16(Smem& sm, bool ht, bool hl, int tl, uint32_t* best_cost) {
+// Intra 16x16 analysis (enc.rs:1637 analyse_i16_edges): SATD per mode; the best mode and its cost.
+struct I16Fit {
+  int mode;
+  uint32_t cost;
+};
+__device__ __noinline__ I16Fit analyse_i16(bool ht, bool hl, int tl) {
   int lane = lane_id();
-  int dc = dc16(sm, ht, hl);
+  int dc = dc16(ht, hl);
   uint32_t sv = 0, sh = 0, sd = 0;
   if (lane < 16) {
     int bx = lane & 3, by = lane >> 2;
@@ -835,20 +854,19 @@ __device__ __noinline__ int analyse_i16(Smem& sm, bool ht, bool hl, int tl, uint
   if (ht && sv < best) { best = sv; mode = 0; }
   if (hl && sh < best) { best = sh; mode = 1; }
   if (ht && hl) {
-    pred16_into(3, sm, sm.tmp_y, ht, hl, tl);
+    pred16_into(3, (int)offsetof(Smem, tmp_y), ht, hl, tl);
     uint32_t s = 0;
     if (lane < 16) {
       int bx = lane & 3, by = lane >> 2;
-      s = satd4(&sm.src_y[by * 64 + bx * 4], 16, &sm.tmp_y[by * 64 + bx * 4], 16);
+      s = satd4((int)offsetof(Smem, src_y) + by * 64 + bx * 4, (int)offsetof(Smem, tmp_y) + by * 64 + bx * 4);
     }
     s = wsum(s) >> 1;
     if (s < best) { best = s; mode = 3; }
   }
-  *best_cost = best;
-  return mode;
+  return I16Fit{mode, best};
 }
 // Chroma intra prediction sample of mode for plane p at (x, y).
-__device__ __forceinline__ int predc_sample(int mode, const Smem& sm, int p, bool ht, bool hl, int tl, int x, int y,
+__device__ __forceinline__ int predc_sample(int mode, int p, bool ht, bool hl, int tl, int x, int y,
                                             const int* dcv, int pa, int pb, int pc) {
   switch (mode) {
     case 0: return dcv[(y >> 2) * 2 + (x >> 2)];
@@ -860,7 +878,7 @@ __device__ __forceinline__ int predc_sample(int mode, const Smem& sm, int p, boo
 // DC and plane parameters of plane p's chroma prediction; called by the whole warp with p =
 // lane / 16. In each half-warp lanes 0..7 hold top[0..7], lanes 8..15 left[0..7] (DC sums of four
 // by two butterflies), then lanes 0..3 the terms of H, lanes 4..7 those of V.
-__device__ void chroma_pred_params(const Smem& sm, int p, bool ht, bool hl, int tl, int* dcv, int& pa, int& pb, int& pc) {
+__device__ void chroma_pred_params(int p, bool ht, bool hl, int tl, int* dcv, int& pa, int& pb, int& pc) {
   const uint8_t* t = sm.ctop[p];
   const uint8_t* l = sm.cleft[p];
   int lane = lane_id(), j = lane & 15, base = lane & 16;
@@ -890,12 +908,17 @@ __device__ void chroma_pred_params(const Smem& sm, int p, bool ht, bool hl, int 
   pb = (17 * H + 16) >> 5;
   pc = (17 * V + 16) >> 5;
 }
+// The sample diagonally above-left of the macroblock in each plane (128 when absent).
+struct Corner {
+  int y, u, v;
+};
 // Intra chroma mode by SAD (enc.rs:1526 analyse_chroma_intra); best prediction into pred_u/v.
-__device__ __noinline__ int analyse_chroma(Smem& sm, bool ht, bool hl, const int* ctl) {
+__device__ __noinline__ int analyse_chroma(bool ht, bool hl, Corner k0) {
   int lane = lane_id();
   int plane = lane >> 4, idx = (lane & 15) * 4, y = idx >> 3, x0 = idx & 7;
+  const int plane_tl = plane ? k0.v : k0.u;
   int dcv[4], pa, pb, pc;
-  chroma_pred_params(sm, plane, ht, hl, ctl[plane], dcv, pa, pb, pc);
+  chroma_pred_params(plane, ht, hl, plane_tl, dcv, pa, pb, pc);
   const uint8_t* s = (plane ? sm.src_v : sm.src_u) + y * 8 + x0;
   uint32_t best = UMAX;
   int bm = 0;
@@ -904,13 +927,13 @@ __device__ __noinline__ int analyse_chroma(Smem& sm, bool ht, bool hl, const int
     if (!ok) continue;
     uint32_t sad = 0;
 #pragma unroll
-    for (int k = 0; k < 4; k++) sad += abs((int)s[k] - predc_sample(mode, sm, plane, ht, hl, ctl[plane], x0 + k, y, dcv, pa, pb, pc));
+    for (int k = 0; k < 4; k++) sad += abs((int)s[k] - predc_sample(mode, plane, ht, hl, plane_tl, x0 + k, y, dcv, pa, pb, pc));
     uint32_t cost = wsum(sad) + (mode == 0 ? 0u : 8u);
     if (cost < best) { best = cost; bm = mode; }
   }
   uint8_t* out = (plane ? sm.pred_v : sm.pred_u) + y * 8 + x0;
 #pragma unroll
-  for (int k = 0; k < 4; k++) out[k] = (uint8_t)predc_sample(bm, sm, plane, ht, hl, ctl[plane], x0 + k, y, dcv, pa, pb, pc);
+  for (int k = 0; k < 4; k++) out[k] = (uint8_t)predc_sample(bm, plane, ht, hl, plane_tl, x0 + k, y, dcv, pa, pb, pc);
   __syncwarp();
   return bm;
 }
@@ -958,7 +981,7 @@ struct Ctx {
 
 // Loads the source macroblock, replicating the last row / column past the picture edges
 // (enc.rs:400 MbSrc::load, h264.rs:3660 extract_mb_planes).
-__device__ __noinline__ void load_source(const Ctx c, Smem& sm) {
+__device__ __noinline__ void load_source(const Ctx c) {
   const FrameParams& fp = *c.fp;
   int lane = lane_id();
   int W = fp.width, H = fp.height, cw = (W + 1) >> 1, ch = (H + 1) >> 1;
@@ -975,8 +998,9 @@ __device__ __noinline__ void load_source(const Ctx c, Smem& sm) {
   for (int k = 0; k < 4; k++) dst[k] = __ldg(crow + min(c.mbx * 8 + c0 + k, cw - 1));
   __syncwarp();
 }
-// Intra edges from the unfiltered reconstruction of this picture (enc.rs:1459-1521).
-__device__ __noinline__ void load_edges(const Ctx c, Smem& sm, bool want_topright, int& tl, int* ctl) {
+// Intra edges from the unfiltered reconstruction of this picture (enc.rs:1459-1521) into shared
+// memory; returns the samples at the corner.
+__device__ __noinline__ Corner load_edges(const Ctx c, bool want_topright) {
   const FrameParams& fp = *c.fp;
   int lane = lane_id();
   const uint8_t* Y = c.sd->cur_y;
@@ -994,18 +1018,20 @@ __device__ __noinline__ void load_edges(const Ctx c, Smem& sm, bool want_toprigh
     if (ht) sm.ctop[p][k] = ldcg_u8(P + (long)(cy0 - 1) * fp.stride_c + cx0 + k);
     if (hl) sm.cleft[p][k] = ldcg_u8(P + (long)(cy0 + k) * fp.stride_c + cx0 - 1);
   }
-  tl = (ht && hl) ? ldcg_u8(Y + (long)(y0 - 1) * fp.stride_y + x0 - 1) : 128;
-  ctl[0] = (ht && hl) ? ldcg_u8(c.sd->cur_u + (long)(cy0 - 1) * fp.stride_c + cx0 - 1) : 128;
-  ctl[1] = (ht && hl) ? ldcg_u8(c.sd->cur_v + (long)(cy0 - 1) * fp.stride_c + cx0 - 1) : 128;
+  Corner k;
+  k.y = (ht && hl) ? ldcg_u8(Y + (long)(y0 - 1) * fp.stride_y + x0 - 1) : 128;
+  k.u = (ht && hl) ? ldcg_u8(c.sd->cur_u + (long)(cy0 - 1) * fp.stride_c + cx0 - 1) : 128;
+  k.v = (ht && hl) ? ldcg_u8(c.sd->cur_v + (long)(cy0 - 1) * fp.stride_c + cx0 - 1) : 128;
   __syncwarp();
+  return k;
 }
 
-// Stores the reconstruction of pred_y/u/v (or tmp_y for luma) into the current picture.
-__device__ __noinline__ void store_recon(const Ctx c, const uint8_t* ly, Smem& sm) {
+// Stores the reconstruction of pred_y/u/v (or tmp_y for luma: its byte offset in Smem) into the current picture.
+__device__ __noinline__ void store_recon(const Ctx c, int ly) {
   const FrameParams& fp = *c.fp;
   int lane = lane_id();
   int y = lane >> 1, x = (lane & 1) * 8;
-  uint2 v = *(const uint2*)&ly[y * 16 + x];
+  uint2 v = *(const uint2*)sm_at(ly + y * 16 + x);
   *(uint2*)(c.sd->cur_y + (long)(c.mby * 16 + y) * fp.stride_y + c.mbx * 16 + x) = v;
   if (c.sd->unf_y) {
     int cw = fp.mb_w * 16;
@@ -1025,7 +1051,7 @@ __device__ __noinline__ void store_recon(const Ctx c, const uint8_t* ly, Smem& s
 // The chroma levels of the record, a word (two zig-zag levels) per lane and store: word w of the
 // AC levels holds slots 2 (w & 7), 2 (w & 7) + 1 of block w / 8 (plane * 4 + block); slot 0 (the
 // DC position) stays 0. Lanes 0..3 write the DC levels.
-__device__ __noinline__ void record_chroma(rg_mb_out* rec, Smem& sm, int cbpc) {
+__device__ __noinline__ void record_chroma(rg_mb_out* rec, int cbpc) {
   int lane = lane_id();
 #pragma unroll 1
   for (int k = 0; k < 2; k++) {
@@ -1042,7 +1068,7 @@ __device__ __noinline__ void record_chroma(rg_mb_out* rec, Smem& sm, int cbpc) {
 // The 4x4 luma levels of the record in zig-zag order, a word per lane and store: word w holds
 // levels 2 (w & 7), 2 (w & 7) + 1 of block w / 8; lanes 8j..8j+7 of step k cover block 4k + j.
 // Returns the blocks holding levels (bit b: block b).
-__device__ __noinline__ uint16_t record_luma4x4(rg_mb_out* rec, const Smem& sm) {
+__device__ __noinline__ uint16_t record_luma4x4(rg_mb_out* rec) {
   int lane = lane_id();
   uint32_t nz = 0;
 #pragma unroll 1
@@ -1075,7 +1101,7 @@ __device__ __noinline__ void record_header(rg_mb_out* rec, int type, int i16_mod
   rec->nz_mask = nz;
   rec->reserved1 = 0;
 }
-__device__ __noinline__ void write_info(const Ctx c, int flags, int cbpl, int mvx, int mvy, int ref, uint16_t nz, const uint8_t* i4m) {
+__device__ __noinline__ void write_info(const Ctx c, int flags, int cbpl, int mvx, int mvy, int ref, uint16_t nz, bool i4) {
   MbInfo inf;
   inf.mv[0] = (int16_t)mvx;
   inf.mv[1] = (int16_t)mvy;
@@ -1090,19 +1116,19 @@ __device__ __noinline__ void write_info(const Ctx c, int flags, int cbpl, int mv
     // bottom row blocks (x = k, y = 3) and right column blocks (x = 3, y = k), decoding order
     int bb = ((3 >> 1) << 3) | ((k >> 1) << 2) | ((3 & 1) << 1) | (k & 1);
     int br = ((k >> 1) << 3) | ((3 >> 1) << 2) | ((k & 1) << 1) | (3 & 1);
-    inf.i4_bottom |= (uint16_t)((i4m ? i4m[bb] : 2) << (4 * k));
-    inf.i4_right |= (uint16_t)((i4m ? i4m[br] : 2) << (4 * k));
+    inf.i4_bottom |= (uint16_t)((i4 ? sm.i4m[bb] : 2) << (4 * k));
+    inf.i4_right |= (uint16_t)((i4 ? sm.i4m[br] : 2) << (4 * k));
   }
   inf.pad_ = 0;
   c.sd->info[c.mb] = inf;
 }
 
 // I16x16 coding and reconstruction (enc.rs:3587 code_i16) with prediction mode `mode`.
-__device__ __noinline__ void code_i16(const Ctx c, Smem& sm, int mode, bool ht, bool hl, int tl, const int* ctl) {
+__device__ __noinline__ void code_i16(const Ctx c, int mode, bool ht, bool hl, Corner k0) {
   int lane = lane_id();
   int qp = c.sd->qp, qpc = c.sd->qpc;
-  pred16_into(mode, sm, sm.pred_y, ht, hl, tl);
-  int cmode = analyse_chroma(sm, ht, hl, ctl);
+  pred16_into(mode, (int)offsetof(Smem, pred_y), ht, hl, k0.y);
+  int cmode = analyse_chroma(ht, hl, k0);
   uint32_t shift, bias;
   quant4_params(qp, true, shift, bias);
   uint32_t my_ac = 0, my_nz = 0;
@@ -1177,9 +1203,8 @@ __device__ __noinline__ void code_i16(const Ctx c, Smem& sm, int mode, bool ht, 
       sm.ldcr[12 + i] = (int16_t)(((z0 - z3) * qmul + 128) >> 8);
     }
   }
-  uint32_t ac_any[2], ac_sc[2];
-  chroma_quant(qpc, true, sm, ac_any, ac_sc);
-  int cbpc = (ac_any[0] | ac_any[1]) ? 2 : (chroma_dc_any(sm) ? 1 : 0);
+  const ChromaAc ac = chroma_quant(qpc, true);
+  int cbpc = (ac.any(0) || ac.any(1)) ? 2 : (chroma_dc_any() ? 1 : 0);
   __syncwarp();
   // record
   rg_mb_out* rec = c.sd->rec + c.mb;
@@ -1191,7 +1216,7 @@ __device__ __noinline__ void code_i16(const Ctx c, Smem& sm, int mode, bool ht, 
     rec->i4_modes[lane] = 2;
   }
   nzm = (uint16_t)__ballot_sync(FULL, lane < 16 && cbpl && my_ac);
-  record_chroma(rec, sm, cbpc);
+  record_chroma(rec, cbpc);
   if (lane == 0) record_header(rec, RG_MB_I16X16, mode, cmode, cbpl | (cbpc << 4), 0, qp, 0, 0, 0, 0, nzm);
   // reconstruction
   if (lane < 16) {
@@ -1213,9 +1238,9 @@ __device__ __noinline__ void code_i16(const Ctx c, Smem& sm, int mode, bool ht, 
       }
   }
   __syncwarp();
-  chroma_recon(qpc, cbpc, sm);
-  store_recon(c, sm.pred_y, sm);
-  if (lane == 0) write_info(c, kFlagIntra, cbpl, 0, 0, -1, nzm, nullptr);
+  chroma_recon(qpc, cbpc);
+  store_recon(c, (int)offsetof(Smem, pred_y));
+  if (lane == 0) write_info(c, kFlagIntra, cbpl, 0, 0, -1, nzm, false);
 }
 
 // I4x4 analysis (enc.rs:3336 analyse_i4): sixteen blocks in decoding order, each choosing among
@@ -1223,11 +1248,11 @@ __device__ __noinline__ void code_i16(const Ctx c, Smem& sm, int mode, bool ht, 
 // reconstructing before the next block. Per block the warp gathers the edge samples (lane k ->
 // Q[k]), builds all nine predictions (lane -> pixel, the two half-warps taking even / odd modes),
 // costs the modes (lane -> mode), and transforms the chosen residual with shuffles (lane ->
-// coefficient). Gives up (false) as soon as the running cost reaches `budget`.
+// coefficient). Returns the luma coded block pattern, or -1 as soon as the running cost reaches `budget`.
 // kMask: only the modes of masks[b] (bit m: Intra4x4PredMode m) that are available at block b are
 // tried -- DC alone when none is (the learned form); the plain form tries every available mode.
 template <bool kMask>
-__device__ __noinline__ bool analyse_i4(const Ctx c, Smem& sm, uint32_t budget, bool ht_mb, bool hl_mb, int tl_mb, int* cbpl_out,
+__device__ __noinline__ int analyse_i4(const Ctx c, uint32_t budget, bool ht_mb, bool hl_mb, int tl_mb,
                                         const uint16_t* masks) {
   const FrameParams& fp = *c.fp;
   int lane = lane_id();
@@ -1325,7 +1350,7 @@ __device__ __noinline__ bool analyse_i4(const Ctx c, Smem& sm, uint32_t budget, 
     }
     int bm = (int)(key & 15);
     total += key >> 4;
-    if (total >= budget) return false;
+    if (total >= budget) return -1;
     if (lane == 0) sm.i4m[b] = (uint8_t)bm;
     // residual transform and quantisation, lane p -> coefficient p (raster); the chosen mode's
     // sample p is in lane 16 (bm & 1) + p
@@ -1352,50 +1377,46 @@ __device__ __noinline__ bool analyse_i4(const Ctx c, Smem& sm, uint32_t budget, 
     if (lane < 16) sm.tmp_y[(py + yl) * 16 + px + xl] = (uint8_t)rec;
     __syncwarp();
   }
-  *cbpl_out = cbpl;
-  return true;
+  return cbpl;
 }
 
-__device__ __noinline__ void code_i4(const Ctx c, Smem& sm, int cbpl, bool ht, bool hl, const int* ctl) {
+__device__ __noinline__ void code_i4(const Ctx c, int cbpl, bool ht, bool hl, Corner k0) {
   int lane = lane_id();
   int qpc = c.sd->qpc;
-  int cmode = analyse_chroma(sm, ht, hl, ctl);
-  uint32_t ac_any[2], ac_sc[2];
-  chroma_quant(qpc, true, sm, ac_any, ac_sc);
-  int cbpc = (ac_any[0] | ac_any[1]) ? 2 : (chroma_dc_any(sm) ? 1 : 0);
+  int cmode = analyse_chroma(ht, hl, k0);
+  const ChromaAc ac = chroma_quant(qpc, true);
+  int cbpc = (ac.any(0) || ac.any(1)) ? 2 : (chroma_dc_any() ? 1 : 0);
   rg_mb_out* rec = c.sd->rec + c.mb;
-  uint16_t nzm = record_luma4x4(rec, sm);
+  uint16_t nzm = record_luma4x4(rec);
   if (lane < 16) {
     rec->luma_dc[lane] = 0;
     rec->i4_modes[lane] = sm.i4m[lane];
   }
-  record_chroma(rec, sm, cbpc);
+  record_chroma(rec, cbpc);
   if (lane == 0) record_header(rec, RG_MB_I4X4, 0, cmode, cbpl | (cbpc << 4), 0, c.sd->qp, 0, 0, 0, 0, nzm);
-  chroma_recon(qpc, cbpc, sm);
-  store_recon(c, sm.tmp_y, sm);
-  if (lane == 0) write_info(c, kFlagIntra, cbpl, 0, 0, -1, nzm, sm.i4m);
+  chroma_recon(qpc, cbpc);
+  store_recon(c, (int)offsetof(Smem, tmp_y));
+  if (lane == 0) write_info(c, kFlagIntra, cbpl, 0, 0, -1, nzm, true);
 }
 
 // One macroblock of an I slice (enc.rs:3311 code_intra).
-__device__ __noinline__ void analyse_intra_mb(const Ctx c, Smem& sm) {
-  int tl, ctl[2];
-  load_edges(c, sm, true, tl, ctl);
+__device__ __noinline__ void analyse_intra_mb(const Ctx c) {
+  const Corner k0 = load_edges(c, true);
   bool ht = c.mby > 0, hl = c.mbx > 0;
   uint32_t lambda = c_lambda[c.sd->qp];
-  uint32_t i16c;
-  int i16m = analyse_i16(sm, ht, hl, tl, &i16c);
-  if (i16c > 40 * lambda) {
-    int cbpl;
-    if (analyse_i4<false>(c, sm, i16c + lambda * 4, ht, hl, tl, &cbpl, nullptr)) {
-      code_i4(c, sm, cbpl, ht, hl, ctl);
+  const I16Fit fit16 = analyse_i16(ht, hl, k0.y);
+  if (fit16.cost > 40 * lambda) {
+    const int cbpl = analyse_i4<false>(c, fit16.cost + lambda * 4, ht, hl, k0.y, nullptr);
+    if (cbpl >= 0) {
+      code_i4(c, cbpl, ht, hl, k0);
       return;
     }
   }
-  code_i16(c, sm, i16m, ht, hl, tl, ctl);
+  code_i16(c, fit16.mode, ht, hl, k0);
 }
 
 // Codes P_Skip with vector mv; prediction already in pred_y / pred_u / pred_v.
-__device__ __noinline__ void code_skip(const Ctx c, Smem& sm, int mvx, int mvy) {
+__device__ __noinline__ void code_skip(const Ctx c, int mvx, int mvy) {
   int lane = lane_id();
   rg_mb_out* rec = c.sd->rec + c.mb;
   if (lane < 16) {
@@ -1411,21 +1432,21 @@ __device__ __noinline__ void code_skip(const Ctx c, Smem& sm, int mvx, int mvy) 
   }
   if (lane == 0) {
     record_header(rec, RG_MB_P_SKIP, 0, 0, 0, 0, c.sd->qp, mvx, mvy, 0, 0, 0);
-    write_info(c, kFlagSkip, 0, mvx, mvy, 0, 0, nullptr);
+    write_info(c, kFlagSkip, 0, mvx, mvy, 0, 0, false);
   }
-  store_recon(c, sm.pred_y, sm);
+  store_recon(c, (int)offsetof(Smem, pred_y));
 }
 
 // Probe of the skip residual (enc.rs:2163 probe_skip_luma): no level above 1 and a total
 // decimation score below 6.
-__device__ __noinline__ bool probe_skip_luma(int qp, Smem& sm) {
+__device__ __noinline__ bool probe_skip_luma(int qp) {
   int lane = lane_id();
   uint32_t shift, bias;
   quant4_params(qp, false, shift, bias);
-  int nz, big, sc;  // levels go to sm.coef as scratch: a skipped macroblock records none
-  quant4x4_blocks(sm, false, 16, 0, qp, shift, bias, sm.coef, nullptr, nz, big, sc);
-  uint32_t b = wor(lane < 16 ? (uint32_t)big : 0u);
-  uint32_t score = wsum(lane < 16 ? (uint32_t)sc : 0u);
+  // levels go to sm.coef as scratch: a skipped macroblock records none
+  const uint32_t mine = quant4x4_blocks(false, 16, 0, qp, shift, bias);
+  uint32_t b = wor(lane < 16 ? mine & 2u : 0u);
+  uint32_t score = wsum(lane < 16 ? mine >> 2 : 0u);
   return !b && score < 6;
 }
 
@@ -1496,9 +1517,9 @@ __device__ __forceinline__ bool wait_seen(const int* p, int need, int& seen, int
   seen = v;
   return true;
 }
-// Makes this warp's global writes visible, then publishes v.
+// Publishes v after this warp's global writes: the warp barrier orders every lane's writes before lane
+// 0's release store, which is cumulative over them.
 __device__ __forceinline__ void publish(int* p, int v) {
-  __threadfence();
   __syncwarp();
   if (lane_id() == 0) st_release(p, v);
 }
@@ -1517,7 +1538,7 @@ struct PipeWait {
 // One macroblock of a P slice (enc.rs:3011 code_p_mb). In the pipelined mode (pw != null) it
 // first waits for the reference frame to be final over every sample its search can read; when
 // a wait gives up it returns with pw->failed set and writes nothing.
-__device__ __noinline__ void analyse_p_mb(const Ctx c, Smem& sm, PipeWait* pw) {
+__device__ __noinline__ void analyse_p_mb(const Ctx c, PipeWait* pw) {
   const FrameParams& fp = *c.fp;
   const StreamDev& sd = *c.sd;
   int lane = lane_id();
@@ -1552,7 +1573,7 @@ __device__ __noinline__ void analyse_p_mb(const Ctx c, Smem& sm, PipeWait* pw) {
   }
   int ps0 = mvp0, ps1 = mvp1;
   if (mbx == 0 || mby == 0 || (lref == 0 && a0 == 0 && a1 == 0) || (tref == 0 && b0 == 0 && b1 == 0)) { ps0 = 0; ps1 = 0; }
-  load_source(c, sm);
+  load_source(c);
   int qpc = c.sd->qpc;
   // co-located vector of the previous picture: a search candidate (enc.rs:3094)
   if (pw && !wait_seen(pw->ana_prev + mby, mbx + 1, pw->seen_ana, pw->error, pw->timeout_ns)) {
@@ -1592,8 +1613,8 @@ __device__ __noinline__ void analyse_p_mb(const Ctx c, Smem& sm, PipeWait* pw) {
 
   // 1. skip probe (enc.rs:2906 try_p_skip)
   if (ps0 >= bmin0 && ps0 <= bmax0 && ps1 >= bmin1 && ps1 <= bmax1) {
-    mc_luma16(sd.ref_y, fp.stride_y, x0, y0, ps0, ps1, sm);
-    uint2 s = src8(sm), p = *(const uint2*)&sm.pred_y[(lane >> 1) * 16 + (lane & 1) * 8];
+    mc_luma16(sd.ref_y, fp.stride_y, x0, y0, ps0, ps1);
+    uint2 s = src8(), p = *(const uint2*)&sm.pred_y[(lane >> 1) * 16 + (lane & 1) * 8];
     uint32_t sad = wsum(vsad8(s, p));
     if (sad < c.sd->sb_probe) {
       bool lz = sad <= c.sd->sb_luma;
@@ -1607,9 +1628,9 @@ __device__ __noinline__ void analyse_p_mb(const Ctx c, Smem& sm, PipeWait* pw) {
         }
         lz = wsum(ssd) <= c.sd->sb_luma_ssd;
       }
-      if (!lz) lz = probe_skip_luma(qp, sm);
+      if (!lz) lz = probe_skip_luma(qp);
       if (lz) {
-        mc_chroma8(sd.ref_u, sd.ref_v, fp.stride_c, mbx, mby, ps0, ps1, sm);
+        mc_chroma8(sd.ref_u, sd.ref_v, fp.stride_c, mbx, mby, ps0, ps1);
         // per plane SAD / SSD bounds (lanes 0..15 U, 16..31 V, 4 samples each)
         int plane = lane >> 4, idx = (lane & 15) * 4;
         const uint8_t* ss = (plane ? sm.src_v : sm.src_u) + idx;
@@ -1623,12 +1644,11 @@ __device__ __noinline__ void analyse_p_mb(const Ctx c, Smem& sm, PipeWait* pw) {
         bool zv = sad_v <= c.sd->sb_chroma || ssd_v <= c.sd->sb_chroma_ssd;
         bool cz = zu && zv;
         if (!cz) {
-          uint32_t ac_any[2], ac_sc[2];
-          chroma_quant(qpc, false, sm, ac_any, ac_sc);
-          cz = !chroma_dc_any(sm) && ac_sc[0] < 7 && ac_sc[1] < 7;
+          const ChromaAc ac = chroma_quant(qpc, false);
+          cz = !chroma_dc_any() && ac.score(0) < 7 && ac.score(1) < 7;
         }
         if (cz) {
-          code_skip(c, sm, ps0, ps1);
+          code_skip(c, ps0, ps1);
           return;
         }
       }
@@ -1641,7 +1661,7 @@ __device__ __noinline__ void analyse_p_mb(const Ctx c, Smem& sm, PipeWait* pw) {
   // candidates in order: predictor, zero, left (if any), top (if any), co-located of the previous
   // picture -- five fixed slots, the left / top ones skipped when absent
   int imin0 = (bmin0 + 3) >> 2, imin1 = (bmin1 + 3) >> 2, imax0 = bmax0 >> 2, imax1 = bmax1 >> 2;
-  uint2 sv = src8(sm);
+  uint2 sv = src8();
   const uint8_t* base = ref + (long)(y0 + (lane >> 1)) * stride + x0 + (lane & 1) * 8;
   int best0 = 0, best1 = 0;
   uint32_t best_cost = UMAX;
@@ -1710,8 +1730,8 @@ __device__ __noinline__ void analyse_p_mb(const Ctx c, Smem& sm, PipeWait* pw) {
     } else {
       // sub-pel refinement over a half-sample window around the full-pel best (enc.rs:1283)
       int bxp = x0 + best0, byp = y0 + best1;
-      stage_window(ref, stride, bxp - 1, byp - 1, sm);
-      build_hpel(sm, 7);
+      stage_window(ref, stride, bxp - 1, byp - 1);
+      build_hpel(7);
       int q0 = fm0, q1 = fm1;
       uint32_t bc = best_cost;
 #pragma unroll 1
@@ -1726,7 +1746,7 @@ __device__ __noinline__ void analyse_p_mb(const Ctx c, Smem& sm, PipeWait* pw) {
           for (int k = 0; k < 4; k++) {
             int cx = f0 + dd[k][0], cy = f1 + dd[k][1];
             bool ok = abs(cx - fm0) <= 3 && abs(cy - fm1) <= 3 && cx >= bmin0 && cx <= bmax0 && cy >= bmin1 && cy <= bmax1;
-            uint32_t s = ok ? qpel_sad(sm, sv, (cx >> 2) - best0 + 1, (cy >> 2) - best1 + 1, cx & 3, cy & 3) : 0u;
+            uint32_t s = ok ? qpel_sad(sv, (cx >> 2) - best0 + 1, (cy >> 2) - best1 + 1, cx & 3, cy & 3) : 0u;
             s = wsum(s);
             cc[k] = ok ? s + mvd_cost(cx - mvp0, lambda) + mvd_cost(cy - mvp1, lambda) : UMAX;
           }
@@ -1737,7 +1757,7 @@ __device__ __noinline__ void analyse_p_mb(const Ctx c, Smem& sm, PipeWait* pw) {
         }
       }
       mv0 = q0; mv1 = q1;
-      uint2 v = qpel8(qpel_src(sm, (q0 >> 2) - best0 + 1, (q1 >> 2) - best1 + 1, q0 & 3, q1 & 3));
+      uint2 v = qpel8(qpel_src((q0 >> 2) - best0 + 1, (q1 >> 2) - best1 + 1, q0 & 3, q1 & 3));
       *(uint2*)&sm.pred_y[(lane >> 1) * 16 + (lane & 1) * 8] = v;
       __syncwarp();
     }
@@ -1747,26 +1767,23 @@ __device__ __noinline__ void analyse_p_mb(const Ctx c, Smem& sm, PipeWait* pw) {
   uint32_t inter_satd = 0;
   if (lane < 16) {
     int bx = lane & 3, by = lane >> 2;
-    inter_satd = satd4(&sm.src_y[by * 64 + bx * 4], 16, &sm.pred_y[by * 64 + bx * 4], 16);
+    inter_satd = satd4((int)offsetof(Smem, src_y) + by * 64 + bx * 4, (int)offsetof(Smem, pred_y) + by * 64 + bx * 4);
   }
   inter_satd = wsum(inter_satd) >> 1;
   uint32_t inter_cost = inter_satd + lambda * (se_bits(mv0 - mvp0) + se_bits(mv1 - mvp1) + 1);
   if (inter_satd > 24 * lambda) {
-    int tl, ctl[2];
-    load_edges(c, sm, false, tl, ctl);
+    const Corner k0 = load_edges(c, false);
     bool ht = mby > 0, hl = mbx > 0;
-    uint32_t i16c;
-    int i16m = analyse_i16(sm, ht, hl, tl, &i16c);
-    if (i16c + lambda * 8 < inter_cost) {
-      code_i16(c, sm, i16m, ht, hl, tl, ctl);
+    const I16Fit fit16 = analyse_i16(ht, hl, k0.y);
+    if (fit16.cost + lambda * 8 < inter_cost) {
+      code_i16(c, fit16.mode, ht, hl, k0);
       return;
     }
   }
 
   // 4. P_L0_16x16 residual (enc.rs:3158-3190)
-  mc_chroma8(sd.ref_u, sd.ref_v, fp.stride_c, mbx, mby, mv0, mv1, sm);
-  uint32_t nz_lane;
-  int cbp4 = luma4x4_inter(qp, sm, &nz_lane);
+  mc_chroma8(sd.ref_u, sd.ref_v, fp.stride_c, mbx, mby, mv0, mv1);
+  int cbp4 = luma4x4_inter(qp);
   int cbpl = cbp4;
   bool use8 = false;
   if (fp.t8x8 && cbp4) {
@@ -1777,14 +1794,12 @@ __device__ __noinline__ void analyse_p_mb(const Ctx c, Smem& sm, PipeWait* pw) {
       nnz4 += ((w & 0xffffu) != 0) + ((w >> 16) != 0);
     }
     nnz4 = wsum(nnz4);
-    uint32_t nnz8;
-    int cbp8 = luma8x8_inter(qp, sm, &nnz8);
-    if (nnz8 <= nnz4) { use8 = true; cbpl = cbp8; }
+    const uint32_t r8 = luma8x8_inter(qp);
+    if ((r8 >> 4) <= nnz4) { use8 = true; cbpl = (int)(r8 & 15u); }
   }
-  uint32_t ac_any[2], ac_sc[2];
-  chroma_quant(qpc, false, sm, ac_any, ac_sc);
+  const ChromaAc ac = chroma_quant(qpc, false);
   // drop a plane's AC levels when nearly empty (enc.rs:2095)
-  bool drop_u = ac_any[0] && ac_sc[0] < 7, drop_v = ac_any[1] && ac_sc[1] < 7;
+  bool drop_u = ac.any(0) && ac.score(0) < 7, drop_v = ac.any(1) && ac.score(1) < 7;
   if (lane < 8) {
     bool d = (lane >> 2) ? drop_v : drop_u;
     if (d)
@@ -1792,10 +1807,10 @@ __device__ __noinline__ void analyse_p_mb(const Ctx c, Smem& sm, PipeWait* pw) {
       for (int i = 0; i < 16; i++) sm.ccoef[lane * 16 + i] = 0;
   }
   __syncwarp();
-  bool acu = ac_any[0] && !drop_u, acv = ac_any[1] && !drop_v;
-  int cbpc = (acu || acv) ? 2 : (chroma_dc_any(sm) ? 1 : 0);
+  bool acu = ac.any(0) && !drop_u, acv = ac.any(1) && !drop_v;
+  int cbpc = (acu || acv) ? 2 : (chroma_dc_any() ? 1 : 0);
   if (cbpl == 0 && cbpc == 0 && mv0 == ps0 && mv1 == ps1) {
-    code_skip(c, sm, mv0, mv1);
+    code_skip(c, mv0, mv1);
     return;
   }
   // code_inter (enc.rs:3196)
@@ -1809,24 +1824,23 @@ __device__ __noinline__ void analyse_p_mb(const Ctx c, Smem& sm, PipeWait* pw) {
     nzm = 0;
     for (int k = 0; k < 4; k++) if ((cbpl >> k) & 1) nzm |= (uint16_t)(0xF << (4 * k));
   } else {
-    nzm = record_luma4x4(rec, sm);
+    nzm = record_luma4x4(rec);
   }
   if (lane < 16) { rec->luma_dc[lane] = 0; rec->i4_modes[lane] = 2; }
-  record_chroma(rec, sm, cbpc);
+  record_chroma(rec, cbpc);
   if (lane == 0) {
     record_header(rec, RG_MB_P_L0_16X16, 0, 0, cbpl | (cbpc << 4), t8flag, qp, mv0, mv1, mv0 - mvp0, mv1 - mvp1, nzm);
-    write_info(c, t8flag ? kFlagT8 : 0, cbpl, mv0, mv1, 0, nzm, nullptr);
+    write_info(c, t8flag ? kFlagT8 : 0, cbpl, mv0, mv1, 0, nzm, false);
   }
   // reconstruction
   if (use8) {
-    recon_luma8x8(sm, qp, cbpl);
+    recon_luma8x8(qp, cbpl);
   } else if (cbpl) {
-    recon_luma4x4(sm, qp, cbpl);
+    recon_luma4x4(qp, cbpl);
   }
   __syncwarp();
-  chroma_recon(qpc, cbpc, sm);
-  store_recon(c, sm.pred_y, sm);
-  (void)nz_lane;
+  chroma_recon(qpc, cbpc);
+  store_recon(c, (int)offsetof(Smem, pred_y));
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1948,7 +1962,7 @@ __device__ __forceinline__ bool one_vector(const MbMv4& m) {
 }
 
 template <bool kMv4>
-__device__ __noinline__ void deblock_mb(const FrameParams& fp, const StreamDev& sd, int mbx, int mby, Smem& sm) {
+__device__ __noinline__ void deblock_mb(const FrameParams& fp, const StreamDev& sd, int mbx, int mby) {
   int lane = lane_id();
   int m = mby * fp.mb_w + mbx;
   MbInfo q = ld_info(&sd.info[m]);
@@ -1975,7 +1989,7 @@ __device__ __noinline__ void deblock_mb(const FrameParams& fp, const StreamDev& 
   }
   // tiles: luma 20x20 at (x0-4, y0-4) stride 20 in win; chroma 12x12 each in hph / hpv
   uint8_t* ty = sm.win;
-  uint8_t* tc[2] = {sm.hph, sm.hpv};
+  auto tc = [](int p) { return sm.hph + p * (int)(offsetof(Smem, hpv) - offsetof(Smem, hph)); };
   const int x0 = mbx * 16, y0 = mby * 16, cx0 = mbx * 8, cy0 = mby * 8;
   for (int w = lane; w < 100; w += 32) {  // 20 rows x 5 words
     int r = w / 5, k = w % 5;
@@ -1986,7 +2000,7 @@ __device__ __noinline__ void deblock_mb(const FrameParams& fp, const StreamDev& 
     int p = w / 36, rem = w % 36, r = rem / 3, k = rem % 3;
     if ((r < 4 && !hast) || (k == 0 && !hasl)) continue;
     const uint8_t* P = p ? sd.cur_v : sd.cur_u;
-    *(uint32_t*)&tc[p][r * 12 + 4 * k] = ldcg_u32(P + (long)(cy0 - 4 + r) * fp.stride_c + cx0 - 4 + 4 * k);
+    *(uint32_t*)&tc(p)[r * 12 + 4 * k] = ldcg_u32(P + (long)(cy0 - 4 + r) * fp.stride_c + cx0 - 4 + 4 * k);
   }
   __syncwarp();
   bool intra = q.flags & kFlagIntra;
@@ -2017,8 +2031,8 @@ __device__ __noinline__ void deblock_mb(const FrameParams& fp, const StreamDev& 
         EdgeParams ec = edge_params(qpc, bs);
         if (ec.on) {
           int j = lane - 16, p = j >> 3, k = j & 7;
-          if (dir == 0) chroma_line(&tc[p][(4 + k) * 12 + 4 + e * 2], 1, ec, ec.tc0[k >> 1]);
-          else chroma_line(&tc[p][(4 + e * 2) * 12 + 4 + k], 12, ec, ec.tc0[k >> 1]);
+          if (dir == 0) chroma_line(&tc(p)[(4 + k) * 12 + 4 + e * 2], 1, ec, ec.tc0[k >> 1]);
+          else chroma_line(&tc(p)[(4 + e * 2) * 12 + 4 + k], 12, ec, ec.tc0[k >> 1]);
         }
       }
       __syncwarp();
@@ -2036,7 +2050,7 @@ __device__ __noinline__ void deblock_mb(const FrameParams& fp, const StreamDev& 
     if (r < 4 && k == 0) continue;
     if ((r < 4 && !hast) || (k == 0 && !hasl)) continue;
     uint8_t* P = p ? sd.cur_v : sd.cur_u;
-    *(uint32_t*)(P + (long)(cy0 - 4 + r) * fp.stride_c + cx0 - 4 + 4 * k) = *(const uint32_t*)&tc[p][r * 12 + 4 * k];
+    *(uint32_t*)(P + (long)(cy0 - 4 + r) * fp.stride_c + cx0 - 4 + 4 * k) = *(const uint32_t*)&tc(p)[r * 12 + 4 * k];
   }
 }
 
@@ -2051,14 +2065,8 @@ __device__ __forceinline__ int diag_len(const FrameParams& fp, int d) {
   return hi >= lo ? hi - lo + 1 : 0;
 }
 
-struct NoSearchSmem {};
-template <int kForm>
-using FormSmem = typename std::conditional<kForm != 0, SearchSmem, NoSearchSmem>::type;
-
 template <int kForm>
 __global__ void __launch_bounds__(32) wavefront_step_kernel(const __grid_constant__ FrameParams fp, const StreamDev* __restrict__ streams, int step) {
-  __shared__ Smem sm;
-  __shared__ FormSmem<kForm> ss;
   const StreamDev& sd = streams[blockIdx.y];
   int na = diag_len(fp, step);
   int nd = fp.deblock ? diag_len(fp, step - 3) : 0;
@@ -2067,19 +2075,18 @@ __global__ void __launch_bounds__(32) wavefront_step_kernel(const __grid_constan
     int mby = diag_first(fp, step) + k, mbx = step - 2 * mby;
     Ctx c{&fp, &sd, mbx, mby, mby * fp.mb_w + mbx};
     if (sd.kind == RG_FRAME_IDR) {
-      load_source(c, sm);
-      if constexpr (kForm != 0) analyse_intra_mb_search(c, sm);
-      else analyse_intra_mb(c, sm);
+      load_source(c);
+      if constexpr (kForm != 0) analyse_intra_mb_search(c);
+      else analyse_intra_mb(c);
     } else {
-      if constexpr (kForm != 0) analyse_p_mb_search(c, sm, ss, nullptr);
-      else analyse_p_mb(c, sm, nullptr);
+      if constexpr (kForm != 0) analyse_p_mb_search(c, nullptr);
+      else analyse_p_mb(c, nullptr);
     }
   } else if (k - na < nd) {
     int d = step - 3;
     int mby = diag_first(fp, d) + (k - na), mbx = d - 2 * mby;
-    deblock_mb<kForm != 0>(fp, sd, mbx, mby, sm);
+    deblock_mb<kForm != 0>(fp, sd, mbx, mby);
   }
-  (void)ss;
 }
 
 // Border extension (enc.rs:165 extend_borders) of the padding that takes its values from
@@ -2256,8 +2263,6 @@ __device__ __noinline__ void compact_row(const rg_mb_out* rec, uint32_t* dst, in
 // which held it to 96 registers with spills).
 template <int kForm>
 __global__ void __launch_bounds__(32, 16) pipeline_kernel(const __grid_constant__ FrameGroups fg, const StreamDev* __restrict__ sds, PipeParams pp) {
-  __shared__ Smem sm;
-  __shared__ FormSmem<kForm> ss;
   const int lane = lane_id();
   // Warps on the first deblock_sms SMs take deblocking segments first, on the next intra_sms SMs
   // segments of IDR pictures (the critical path of a GOP), and the others the remaining analysis
@@ -2321,12 +2326,12 @@ __global__ void __launch_bounds__(32, 16) pipeline_kernel(const __grid_constant_
         }
         Ctx c{&fp, &sd, x, y, y * Wm + x};
         if (sd.kind == RG_FRAME_IDR) {
-          load_source(c, sm);
-          if constexpr (kForm != 0) analyse_intra_mb_search(c, sm);
-          else analyse_intra_mb(c, sm);
+          load_source(c);
+          if constexpr (kForm != 0) analyse_intra_mb_search(c);
+          else analyse_intra_mb(c);
         } else {
-          if constexpr (kForm != 0) analyse_p_mb_search(c, sm, ss, has_prev ? &pw : nullptr);
-          else analyse_p_mb(c, sm, has_prev ? &pw : nullptr);
+          if constexpr (kForm != 0) analyse_p_mb_search(c, has_prev ? &pw : nullptr);
+          else analyse_p_mb(c, has_prev ? &pw : nullptr);
           if (pw.failed) { failed = true; break; }
         }
         publish(ana_rows + y, x + 1);
@@ -2346,7 +2351,7 @@ __global__ void __launch_bounds__(32, 16) pipeline_kernel(const __grid_constant_
           failed = true;
           break;
         }
-        deblock_mb<kForm != 0>(fp, sd, x, y, sm);
+        deblock_mb<kForm != 0>(fp, sd, x, y);
         // Macroblock (x, y - 1) is final now: (x + 1, y - 1) was deblocked before this one. In
         // the last row, so is (x - 1, y), and the last macroblock is final after its own pass.
         __syncwarp();
@@ -2376,7 +2381,6 @@ __global__ void __launch_bounds__(32, 16) pipeline_kernel(const __grid_constant_
     atomicMax(pp.reach, reach_y);
     atomicMax(pp.reach + 1, reach_x);
   }
-  (void)ss;
 }
 
 // The launch's error word (and the reach its reference waits saw) into mapped host memory, queued

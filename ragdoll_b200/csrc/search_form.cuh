@@ -56,7 +56,9 @@ struct SearchSmem {
   int bmv[4][2], bmvd[4][2], own[4][2], pm[4][2], pd[4][2], qmv[4][2];
   int ccx[8], ccy[8];  // the learned form's centre candidates (ok: cok)
   bool cok[8];
+  int wbx, wby;        // integer vector of the half-sample planes held
 };
+__shared__ SearchSmem ss;
 __device__ __forceinline__ void ld_q(const MbMv4* m, int q, int* v) {
   uint32_t w = ((const uint32_t*)m)[q];
   v[0] = (int16_t)(w & 0xffffu);
@@ -90,10 +92,11 @@ __device__ __noinline__ MbNb load_nb(const Ctx c) {
 }
 // The 4x4 block at (bx, by) in 4x4 units relative to the macroblock (-1..4); own[q] / done bit q:
 // this macroblock's quadrants already decided in the current partition type.
-__device__ __forceinline__ NbMv nb4(const MbNb& n, int bx, int by, const int (*own)[2], int done) {
+__device__ __forceinline__ NbMv nb4(int bx, int by, int done) {
+  const MbNb& n = ss.nb;
   if (bx >= 0 && bx < 4 && by >= 0 && by < 4) {
     int q = (by >> 1) * 2 + (bx >> 1);
-    if ((done >> q) & 1) return {0, own[q][0], own[q][1]};
+    if ((done >> q) & 1) return {0, ss.own[q][0], ss.own[q][1]};
     return {-2, 0, 0};
   }
   if (bx == -1 && by == -1) return {n.refD, n.d[0], n.d[1]};
@@ -104,9 +107,9 @@ __device__ __forceinline__ NbMv nb4(const MbNb& n, int bx, int by, const int (*o
 }
 // Motion vector predictor of the partition whose top-left 4x4 block is (bx, by) and width pw (4x4
 // units), H.264 8.4.1.3; dir 1 16x8 top, 2 16x8 bottom, 3 8x16 left, 4 8x16 right, 0 median only.
-__device__ __noinline__ int2 mv_pred(const MbNb& n, int bx, int by, int pw, int dir, const int (*own)[2], int done) {
-  NbMv A = nb4(n, bx - 1, by, own, done), B = nb4(n, bx, by - 1, own, done), C = nb4(n, bx + pw, by - 1, own, done);
-  if (C.ref == -2) C = nb4(n, bx - 1, by - 1, own, done);
+__device__ __noinline__ int2 mv_pred(int bx, int by, int pw, int dir, int done) {
+  NbMv A = nb4(bx - 1, by, done), B = nb4(bx, by - 1, done), C = nb4(bx + pw, by - 1, done);
+  if (C.ref == -2) C = nb4(bx - 1, by - 1, done);
   if (dir == 1 && B.ref == 0) return make_int2(B.x, B.y);
   if ((dir == 2 || dir == 3) && A.ref == 0) return make_int2(A.x, A.y);
   if (dir == 4 && C.ref == 0) return make_int2(C.x, C.y);
@@ -147,8 +150,9 @@ __device__ __forceinline__ uint32_t lds4u(const uint8_t* p) {
 }
 // A window of at most 32 vectors (the learned form's): lane v takes vector v in raster order and
 // sums its four quadrant SADs over the staged band; the same costs and ties as the wide search.
-__device__ __noinline__ void int_search_small(const Ctx c, const Smem& sm, SearchSmem& ss, int xlo, int xhi, int ylo,
-                                              int yhi, int mvp0, int mvp1, uint32_t lambda, IntBest& ib) {
+__device__ __noinline__ void int_search_small(const Ctx c, int xlo, int xhi, int ylo,
+                                              int yhi, int mvp0, int mvp1, uint32_t lambda) {
+  IntBest& ib = ss.ib;
   const int lane = lane_id();
   const int x0 = c.mbx * 16, y0 = c.mby * 16, stride = c.fp->stride_y;
   const uint8_t* ref = c.sd->ref_y;
@@ -188,10 +192,11 @@ __device__ __noinline__ void int_search_small(const Ctx c, const Smem& sm, Searc
   }
 }
 
-__device__ __noinline__ void int_search(const Ctx c, const Smem& sm, SearchSmem& ss, int xlo, int xhi, int ylo, int yhi,
-                                        int mvp0, int mvp1, uint32_t lambda, IntBest& ib) {
+__device__ __noinline__ void int_search(const Ctx c, int xlo, int xhi, int ylo, int yhi,
+                                        int mvp0, int mvp1, uint32_t lambda) {
+  IntBest& ib = ss.ib;
   if ((xhi - xlo + 1) * (yhi - ylo + 1) <= 32) {
-    int_search_small(c, sm, ss, xlo, xhi, ylo, yhi, mvp0, mvp1, lambda, ib);
+    int_search_small(c, xlo, xhi, ylo, yhi, mvp0, mvp1, lambda);
     return;
   }
   const FrameParams& fp = *c.fp;
@@ -301,12 +306,12 @@ __device__ __forceinline__ uint32_t satd4_regs(const uint32_t* sa, const uint32_
   return s;
 }
 // The 4x4 prediction at window position (wx, wy), phase (fx, fy): four packed rows.
-__device__ __forceinline__ void qpel4(const Smem& sm, int wx, int wy, int fx, int fy, uint32_t* out) {
-  QSrc q = qpel_src(sm, wx, wy, fx, fy);
+__device__ __forceinline__ void qpel4(int wx, int wy, int fx, int fy, uint32_t* out) {
+  QSrc q = qpel_src(wx, wy, fx, fy);
 #pragma unroll
   for (int r = 0; r < 4; r++) {
-    uint32_t a = lds4u(q.a + r * q.sa);
-    out[r] = q.avg ? __vavgu4(a, lds4u(q.b + r * q.sb)) : a;
+    uint32_t a = lds4u(sm_at(q.a + r * q.sa));
+    out[r] = q.avg ? __vavgu4(a, lds4u(sm_at(q.b + r * q.sb))) : a;
   }
 }
 __device__ __constant__ int8_t c_hstep[8][2] = {{0, -2}, {-2, 0}, {2, 0}, {0, 2}, {-2, -2}, {2, -2}, {-2, 2}, {2, 2}};
@@ -314,22 +319,22 @@ __device__ __constant__ int8_t c_hstep[8][2] = {{0, -2}, {-2, 0}, {2, 0}, {0, 2}
 // The half-sample planes in shared memory serve every part whose integer vector they were built
 // around: a macroblock-level window (origin one sample above-left of the macroblock displaced by the
 // vector) covers every 4x4 block of the macroblock at quarter-sample offsets -3..3.
-struct WinState {
-  int bx, by;  // integer vector of the planes held, or kNoWin
-};
+// ss.wbx / wby: the integer vector of the planes held, or kNoWin.
 constexpr int kNoWin = 1 << 20;
-__device__ __forceinline__ void ensure_window(const Ctx c, Smem& sm, WinState& ws, int bx, int by) {
-  if (ws.bx == bx && ws.by == by) return;
-  stage_window(c.sd->ref_y, c.fp->stride_y, c.mbx * 16 + bx - 1, c.mby * 16 + by - 1, sm);
-  build_hpel(sm, 7);
-  ws.bx = bx;
-  ws.by = by;
+__device__ __forceinline__ void ensure_window(const Ctx c, int bx, int by) {
+  if (ss.wbx == bx && ss.wby == by) return;
+  stage_window(c.sd->ref_y, c.fp->stride_y, c.mbx * 16 + bx - 1, c.mby * 16 + by - 1);
+  build_hpel(7);
+  __syncwarp();
+  ss.wbx = bx;
+  ss.wby = by;
+  __syncwarp();
 }
 
-__device__ __noinline__ PartFit refine_part(const Ctx c, Smem& sm, WinState& ws, int px, int py, int pw, int ph, int bx,
+__device__ __noinline__ PartFit refine_part(const Ctx c, int px, int py, int pw, int ph, int bx,
                                             int by, int2 mvp, uint32_t lambda, Bounds bd) {
   const int lane = lane_id();
-  ensure_window(c, sm, ws, bx, by);
+  ensure_window(c, bx, by);
   const int bw4 = pw >> 2, nblk = bw4 * (ph >> 2);
   const int m0x = 4 * bx, m0y = 4 * by;
   int cx = m0x, cy = m0y;
@@ -351,7 +356,7 @@ __device__ __noinline__ PartFit refine_part(const Ctx c, Smem& sm, WinState& ws,
       if (ok) {
         const int ox = 4 * (blk % bw4), oy = 4 * (blk / bw4);
         uint32_t pa[4], sa[4];
-        qpel4(sm, (vx >> 2) - bx + 1 + px + ox, (vy >> 2) - by + 1 + py + oy, vx & 3, vy & 3, pa);
+        qpel4((vx >> 2) - bx + 1 + px + ox, (vy >> 2) - by + 1 + py + oy, vx & 3, vy & 3, pa);
 #pragma unroll
         for (int r = 0; r < 4; r++) sa[r] = *(const uint32_t*)&sm.src_y[(py + oy + r) * 16 + px + ox];
         s = satd4_regs(sa, pa);
@@ -383,31 +388,31 @@ __device__ __noinline__ PartFit refine_part(const Ctx c, Smem& sm, WinState& ws,
 // same at distance 1, up to two steps, each from the step's start), cost SAD + lambda * vector bits
 // against the part's predictor, the first strict minimum in that order; lanes take the part's
 // 4-sample words, one candidate at a time.
-__device__ __noinline__ uint32_t part_sad(const Smem& sm, int px, int py, int pw, int ph, int bx, int by, int vx, int vy) {
+__device__ __noinline__ uint32_t part_sad(int px, int py, int pw, int ph, int bx, int by, int vx, int vy) {
   const int lane = lane_id();
-  const QSrc q = qpel_src(sm, (vx >> 2) - bx + 1 + px, (vy >> 2) - by + 1 + py, vx & 3, vy & 3);
+  const QSrc q = qpel_src((vx >> 2) - bx + 1 + px, (vy >> 2) - by + 1 + py, vx & 3, vy & 3);
   const int wpr = pw >> 2, nw = wpr * ph;
   uint32_t s = 0;
   for (int w = lane; w < nw; w += 32) {
     const int r = w / wpr, x = (w - r * wpr) * 4;
-    uint32_t a = lds4u(q.a + r * q.sa + x);
-    if (q.avg) a = __vavgu4(a, lds4u(q.b + r * q.sb + x));
+    uint32_t a = lds4u(sm_at(q.a + r * q.sa + x));
+    if (q.avg) a = __vavgu4(a, lds4u(sm_at(q.b + r * q.sb + x)));
     s = __vsadu4(a, *(const uint32_t*)&sm.src_y[(py + r) * 16 + px + x]) + s;
   }
   return wsum(s);
 }
-__device__ __noinline__ PartFit refine_part_sad(const Ctx c, Smem& sm, WinState& ws, int px, int py, int pw, int ph,
+__device__ __noinline__ PartFit refine_part_sad(const Ctx c, int px, int py, int pw, int ph,
                                                 int bx, int by, int2 mvp, uint32_t lambda, Bounds bd) {
-  ensure_window(c, sm, ws, bx, by);
+  ensure_window(c, bx, by);
   int cx = 4 * bx, cy = 4 * by;
-  uint32_t best = part_sad(sm, px, py, pw, ph, bx, by, cx, cy) + vec_cost(cx - mvp.x, cy - mvp.y, lambda);
+  uint32_t best = part_sad(px, py, pw, ph, bx, by, cx, cy) + vec_cost(cx - mvp.x, cy - mvp.y, lambda);
   for (int st = 2; st >= 1; st--) {
     for (int it = 0; it < (st == 2 ? 1 : 2); it++) {
       const int fx = cx, fy = cy;
       for (int k = 0; k < 4; k++) {
         const int vx = fx + (k == 1 ? -st : (k == 2 ? st : 0)), vy = fy + (k == 0 ? -st : (k == 3 ? st : 0));
         if (abs(vx - 4 * bx) > 3 || abs(vy - 4 * by) > 3 || !in_bounds(bd, vx, vy)) continue;  // uniform
-        const uint32_t cost = part_sad(sm, px, py, pw, ph, bx, by, vx, vy) + vec_cost(vx - mvp.x, vy - mvp.y, lambda);
+        const uint32_t cost = part_sad(px, py, pw, ph, bx, by, vx, vy) + vec_cost(vx - mvp.x, vy - mvp.y, lambda);
         if (cost < best) { best = cost; cx = vx; cy = vy; }
       }
       if (cx == fx && cy == fy) break;
@@ -418,28 +423,28 @@ __device__ __noinline__ PartFit refine_part_sad(const Ctx c, Smem& sm, WinState&
 
 // The luma prediction of a part at quarter-sample vector mv (within 3 quarter samples of 4 (bx, by),
 // the integer vector its refinement started from) into pred_y.
-__device__ __noinline__ void predict_part(const Ctx c, Smem& sm, WinState& ws, int px, int py, int pw, int ph, int bx,
+__device__ __noinline__ void predict_part(const Ctx c, int px, int py, int pw, int ph, int bx,
                                           int by, int mvx, int mvy) {
   const int lane = lane_id();
-  ensure_window(c, sm, ws, bx, by);
-  QSrc q = qpel_src(sm, (mvx >> 2) - bx + 1 + px, (mvy >> 2) - by + 1 + py, mvx & 3, mvy & 3);
+  ensure_window(c, bx, by);
+  QSrc q = qpel_src((mvx >> 2) - bx + 1 + px, (mvy >> 2) - by + 1 + py, mvx & 3, mvy & 3);
   for (int i = lane; i < pw * ph; i += 32) {
     const int r = i / pw, x = i - r * pw;
-    int v = q.a[r * q.sa + x];
-    if (q.avg) v = (v + q.b[r * q.sb + x] + 1) >> 1;
+    int v = *sm_at(q.a + r * q.sa + x);
+    if (q.avg) v = (v + *sm_at(q.b + r * q.sb + x) + 1) >> 1;
     sm.pred_y[(py + r) * 16 + px + x] = (uint8_t)v;
   }
   __syncwarp();
 }
 // Chroma prediction of both planes with each 8x8 luma quadrant's own vector (4x4 chroma blocks;
 // the bilinear 1/8-sample filter of chroma_mc_8x8_x2, h264_enc.rs:1279, per sample).
-__device__ __noinline__ void mc_chroma_q(const Ctx c, Smem& sm, const int (*qmv)[2]) {
+__device__ __noinline__ void mc_chroma_q(const Ctx c) {
   const FrameParams& fp = *c.fp;
   const StreamDev& sd = *c.sd;
   const int lane = lane_id();
   const int plane = lane >> 4, idx = (lane & 15) * 4, r = idx >> 3, c0 = idx & 7;
   const int q = (r >> 2) * 2 + (c0 >> 2);
-  const int mvx = qmv[q][0], mvy = qmv[q][1];
+  const int mvx = ss.qmv[q][0], mvy = ss.qmv[q][1];
   const int cx = c.mbx * 8 + c0 + (mvx >> 3), cy = c.mby * 8 + r + (mvy >> 3), fx = mvx & 7, fy = mvy & 7;
   const int wa = (8 - fx) * (8 - fy), wb = fx * (8 - fy), wc = (8 - fx) * fy, wd = fx * fy;
   const uint8_t* src = (plane ? sd.ref_v : sd.ref_u) + (long)cy * fp.stride_c + cx;
@@ -453,18 +458,21 @@ __device__ __noinline__ void mc_chroma_q(const Ctx c, Smem& sm, const int (*qmv)
 }
 
 // Search-form side state of a coded macroblock: the record's partition fields and the quadrant
-// vectors later macroblocks and the deblocking filter read (lane 0 writes).
-__device__ __noinline__ void search_tail(const Ctx c, int ptype, const int (*qmv)[2], const int (*pmvd)[2]) {
+// vectors later macroblocks and the deblocking filter read (lane 0 writes). parts: the quadrants'
+// vectors ss.qmv and the partitions' differences ss.bmvd; otherwise (mvx, mvy) everywhere and no
+// differences.
+__device__ __noinline__ void search_tail(const Ctx c, int ptype, bool parts, int mvx, int mvy) {
   if (lane_id() != 0) return;
   rg_mb_out* rec = c.sd->rec + c.mb;
   MbMv4 m;
+#pragma unroll
   for (int q = 0; q < 4; q++) {
-    m.mv[q][0] = (int16_t)qmv[q][0];
-    m.mv[q][1] = (int16_t)qmv[q][1];
-    rec->part_mv[q][0] = (int16_t)qmv[q][0];
-    rec->part_mv[q][1] = (int16_t)qmv[q][1];
-    rec->part_mvd[q][0] = (int16_t)pmvd[q][0];
-    rec->part_mvd[q][1] = (int16_t)pmvd[q][1];
+    m.mv[q][0] = (int16_t)(parts ? ss.qmv[q][0] : mvx);
+    m.mv[q][1] = (int16_t)(parts ? ss.qmv[q][1] : mvy);
+    rec->part_mv[q][0] = m.mv[q][0];
+    rec->part_mv[q][1] = m.mv[q][1];
+    rec->part_mvd[q][0] = (int16_t)(parts ? ss.bmvd[q][0] : 0);
+    rec->part_mvd[q][1] = (int16_t)(parts ? ss.bmvd[q][1] : 0);
   }
   rec->part_type = (uint8_t)ptype;
   rec->reserved2[0] = rec->reserved2[1] = rec->reserved2[2] = 0;
@@ -497,13 +505,13 @@ __device__ __noinline__ bool wait_window(const Ctx c, PipeWait* pw, int xhi, int
 
 // P_Skip probe of the plain form (enc.rs:2906 try_p_skip) at skip vector (ps0, ps1): true when the
 // macroblock is coded as P_Skip (prediction left in pred_y / pred_u / pred_v).
-__device__ __noinline__ bool skip_probe(const Ctx c, Smem& sm, int ps0, int ps1, const Bounds& bd) {
+__device__ __noinline__ bool skip_probe(const Ctx c, int ps0, int ps1, const Bounds& bd) {
   const FrameParams& fp = *c.fp;
   const StreamDev& sd = *c.sd;
   const int lane = lane_id();
   if (!in_bounds(bd, ps0, ps1)) return false;
-  mc_luma16(sd.ref_y, fp.stride_y, c.mbx * 16, c.mby * 16, ps0, ps1, sm);
-  uint2 s = src8(sm), p = *(const uint2*)&sm.pred_y[(lane >> 1) * 16 + (lane & 1) * 8];
+  mc_luma16(sd.ref_y, fp.stride_y, c.mbx * 16, c.mby * 16, ps0, ps1);
+  uint2 s = src8(), p = *(const uint2*)&sm.pred_y[(lane >> 1) * 16 + (lane & 1) * 8];
   uint32_t sad = wsum(vsad8(s, p));
   if (sad >= sd.sb_probe) return false;
   bool lz = sad <= sd.sb_luma;
@@ -517,9 +525,9 @@ __device__ __noinline__ bool skip_probe(const Ctx c, Smem& sm, int ps0, int ps1,
     }
     lz = wsum(ssd) <= sd.sb_luma_ssd;
   }
-  if (!lz) lz = probe_skip_luma(sd.qp, sm);
+  if (!lz) lz = probe_skip_luma(sd.qp);
   if (!lz) return false;
-  mc_chroma8(sd.ref_u, sd.ref_v, fp.stride_c, c.mbx, c.mby, ps0, ps1, sm);
+  mc_chroma8(sd.ref_u, sd.ref_v, fp.stride_c, c.mbx, c.mby, ps0, ps1);
   int plane = lane >> 4, idx = (lane & 15) * 4;
   const uint8_t* ssrc = (plane ? sm.src_v : sm.src_u) + idx;
   const uint8_t* pp = (plane ? sm.pred_v : sm.pred_u) + idx;
@@ -530,21 +538,24 @@ __device__ __noinline__ bool skip_probe(const Ctx c, Smem& sm, int ps0, int ps1,
   uint32_t ssd_u = wsum(plane == 0 ? ssdp : 0), ssd_v = wsum(plane == 1 ? ssdp : 0);
   bool cz = (sad_u <= sd.sb_chroma || ssd_u <= sd.sb_chroma_ssd) && (sad_v <= sd.sb_chroma || ssd_v <= sd.sb_chroma_ssd);
   if (!cz) {
-    uint32_t ac_any[2], ac_sc[2];
-    chroma_quant(sd.qpc, false, sm, ac_any, ac_sc);
-    cz = !chroma_dc_any(sm) && ac_sc[0] < 7 && ac_sc[1] < 7;
+    const ChromaAc ac = chroma_quant(sd.qpc, false);
+    cz = !chroma_dc_any() && ac.score(0) < 7 && ac.score(1) < 7;
   }
   return cz;
 }
 
-// Learned form: the centre of the first +-2 window among n integer candidates (cx, cy; ok false:
+// Learned form: the centre of the first +-2 window among the integer candidates of ss.ccx / ccy (cok false:
 // absent) -- the first of least 16x16 SAD + lambda * vector bits against the 16x16 predictor.
-__device__ __noinline__ void learned_centre(const Ctx c, const Smem& sm, const int* cx, const int* cy, const bool* ok,
-                                            int n, int mvp0, int mvp1, uint32_t lambda, int& bx, int& by) {
+__device__ __noinline__ int2 learned_centre(const Ctx c, int mvp0, int mvp1, uint32_t lambda) {
+  const int* cx = ss.ccx;
+  const int* cy = ss.ccy;
+  const bool* ok = ss.cok;
+  constexpr int n = kCentreCands;
+  int bx, by;
   const int lane = lane_id();
   const int stride = c.fp->stride_y;
   const uint8_t* base = c.sd->ref_y + (long)(c.mby * 16 + (lane >> 1)) * stride + c.mbx * 16 + (lane & 1) * 8;
-  const uint2 sv = src8(sm);
+  const uint2 sv = src8();
   uint2 r[kCentreCands];
 #pragma unroll
   for (int k = 0; k < kCentreCands; k++) r[k] = k < n && ok[k] ? ldg8(base + (long)cy[k] * stride + cx[k]) : make_uint2(0u, 0u);
@@ -557,6 +568,7 @@ __device__ __noinline__ void learned_centre(const Ctx c, const Smem& sm, const i
     const uint32_t cost = fullpel_cost(sv, r[k], cx[k], cy[k], mvp0, mvp1, lambda);
     if (cost < best) { best = cost; bx = cx[k]; by = cy[k]; }
   }
+  return make_int2(bx, by);
 }
 
 // Partition geometry in coding order: {type, first part, parts}; part k: {px, py, pw, ph, bx, by,
@@ -573,7 +585,7 @@ __device__ __constant__ int8_t c_type_parts[4] = {1, 2, 2, 4};
 __device__ __constant__ uint8_t c_part_quads[9] = {15, 3, 12, 5, 10, 1, 2, 4, 8};
 
 // One macroblock of a P slice in the search forms (see the head of this file).
-__device__ __noinline__ void analyse_p_mb_search(const Ctx c, Smem& sm, SearchSmem& ss, PipeWait* pw) {
+__device__ __noinline__ void analyse_p_mb_search(const Ctx c, PipeWait* pw) {
   const FrameParams& fp = *c.fp;
   const StreamDev& sd = *c.sd;
   const int lane = lane_id();
@@ -594,18 +606,17 @@ __device__ __noinline__ void analyse_p_mb_search(const Ctx c, Smem& sm, SearchSm
   MbNb& nb = ss.nb;
   __syncwarp();
   nb = load_nb(c);
-  int none[4][2] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
-  const int2 p16 = mv_pred(nb, 0, 0, 4, 0, none, 0);
+  const int2 p16 = mv_pred(0, 0, 4, 0, 0);
   const int mvp16[2] = {p16.x, p16.y};
   int ps0 = mvp16[0], ps1 = mvp16[1];
   {
-    NbMv A = nb4(nb, -1, 0, none, 0), B = nb4(nb, 0, -1, none, 0);
+    NbMv A = nb4(-1, 0, 0), B = nb4(0, -1, 0);
     if (mbx == 0 || mby == 0 || (A.ref == 0 && A.x == 0 && A.y == 0) || (B.ref == 0 && B.x == 0 && B.y == 0)) {
       ps0 = 0;
       ps1 = 0;
     }
   }
-  load_source(c, sm);
+  load_source(c);
   const rg_mb_hint* hint = sd.hint ? sd.hint + c.mb : nullptr;
   // integer window: full search, or the learned seed's small window
   const int R = sd.search_range;
@@ -617,8 +628,8 @@ __device__ __noinline__ void analyse_p_mb_search(const Ctx c, Smem& sm, SearchSm
   int* ccy = ss.ccy;
   bool* cok = ss.cok;
   if (hint) {
-    NbMv A = nb4(nb, -1, 0, none, 0), B = nb4(nb, 0, -1, none, 0), C = nb4(nb, 4, -1, none, 0);
-    if (C.ref == -2) C = nb4(nb, -1, -1, none, 0);
+    NbMv A = nb4(-1, 0, 0), B = nb4(0, -1, 0), C = nb4(4, -1, 0);
+    if (C.ref == -2) C = nb4(-1, -1, 0);
     const int vx[kCentreCands] = {mvp16[0] + hint->mv_off[0], mvp16[0], hint->mv_coarse[0], A.x, B.x, C.x, 0};
     const int vy[kCentreCands] = {mvp16[1] + hint->mv_off[1], mvp16[1], hint->mv_coarse[1], A.y, B.y, C.y, 0};
     const bool use[kCentreCands] = {true, true, (hint->flags & 1) != 0, A.ref == 0, B.ref == 0, C.ref == 0, true};
@@ -639,25 +650,23 @@ __device__ __noinline__ void analyse_p_mb_search(const Ctx c, Smem& sm, SearchSm
   }
   // the reference region of the skip probe and the search window (learned: every candidate's)
   if (!wait_window(c, pw, max(xhi, (max(ps0, 0) + 3) >> 2), max(yhi, (max(ps1, 0) + 3) >> 2))) return;
-  const int off4[4][2] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
   // 1. skip probe
-  if (skip_probe(c, sm, ps0, ps1, bd)) {
-    code_skip(c, sm, ps0, ps1);
-    int q4[4][2] = {{ps0, ps1}, {ps0, ps1}, {ps0, ps1}, {ps0, ps1}};
-    search_tail(c, 255, q4, off4);
+  if (skip_probe(c, ps0, ps1, bd)) {
+    code_skip(c, ps0, ps1);
+    search_tail(c, 255, false, ps0, ps1);
     return;
   }
   // 2. integer search
   if (hint) {
-    int lcx, lcy;
-    learned_centre(c, sm, ccx, ccy, cok, kCentreCands, mvp16[0], mvp16[1], lambda, lcx, lcy);
+    const int2 lc = learned_centre(c, mvp16[0], mvp16[1], lambda);
+    const int lcx = lc.x, lcy = lc.y;
     xlo = max(lcx - kLearnedRange, imin0);
     xhi = min(lcx + kLearnedRange, imax0);
     ylo = max(lcy - kLearnedRange, imin1);
     yhi = min(lcy + kLearnedRange, imax1);
   }
   IntBest& ib = ss.ib;  // warp-uniform: once per warp in shared memory
-  int_search(c, sm, ss, xlo, xhi, ylo, yhi, mvp16[0], mvp16[1], lambda, ib);
+  int_search(c, xlo, xhi, ylo, yhi, mvp16[0], mvp16[1], lambda);
   if (hint) {
     bool edge = (ib.x[0] == xlo && xlo > imin0) || (ib.x[0] == xhi && xhi < imax0) ||
                 (ib.y[0] == ylo && ylo > imin1) || (ib.y[0] == yhi && yhi < imax1);
@@ -668,7 +677,7 @@ __device__ __noinline__ void analyse_p_mb_search(const Ctx c, Smem& sm, SearchSm
       ylo = max(cy - kLearnedRange, imin1);
       yhi = min(cy + kLearnedRange, imax1);
       if (!wait_window(c, pw, xhi, yhi)) return;
-      int_search(c, sm, ss, xlo, xhi, ylo, yhi, mvp16[0], mvp16[1], lambda, ib);
+      int_search(c, xlo, xhi, ylo, yhi, mvp16[0], mvp16[1], lambda);
       edge = (ib.x[0] == xlo && xlo > imin0) || (ib.x[0] == xhi && xhi < imax0) ||
              (ib.y[0] == ylo && ylo > imin1) || (ib.y[0] == yhi && yhi < imax1);
     }
@@ -676,7 +685,7 @@ __device__ __noinline__ void analyse_p_mb_search(const Ctx c, Smem& sm, SearchSm
       xlo = max(fcx - R, imin0); xhi = min(fcx + R, imax0);
       ylo = max(fcy - R, imin1); yhi = min(fcy + R, imax1);
       if (!wait_window(c, pw, xhi, yhi)) return;
-      int_search(c, sm, ss, xlo, xhi, ylo, yhi, mvp16[0], mvp16[1], lambda, ib);
+      int_search(c, xlo, xhi, ylo, yhi, mvp16[0], mvp16[1], lambda);
     }
   }
   // 3-4. refinement of every tried type, the least total cost wins
@@ -684,7 +693,7 @@ __device__ __noinline__ void analyse_p_mb_search(const Ctx c, Smem& sm, SearchSm
   uint32_t best_j = UMAX;
   int (&bmv)[4][2] = ss.bmv;  // per part (coding order) of the best type (warp-uniform, shared)
   int (&bmvd)[4][2] = ss.bmvd;
-  WinState ws{kNoWin, kNoWin};  // the skip probe's window is not a refinement window
+  ss.wbx = ss.wby = kNoWin;  // the skip probe's window is not a refinement window
   for (int t = 0; t < 4; t++) {
     if (!((part_mask >> t) & 1)) continue;
     int (&own)[4][2] = ss.own;
@@ -697,9 +706,9 @@ __device__ __noinline__ void analyse_p_mb_search(const Ctx c, Smem& sm, SearchSm
     const int first = c_type_first[t], np = c_type_parts[t];
     for (int k = 0; k < np; k++) {
       const int8_t* g = c_parts[first + k];
-      const int2 mvp = mv_pred(nb, g[4], g[5], g[6], g[7], own, done);
-      const PartFit fit = hint ? refine_part_sad(c, sm, ws, g[0], g[1], g[2], g[3], ib.x[g[8]], ib.y[g[8]], mvp, lambda, bd)
-                               : refine_part(c, sm, ws, g[0], g[1], g[2], g[3], ib.x[g[8]], ib.y[g[8]], mvp, lambda, bd);
+      const int2 mvp = mv_pred(g[4], g[5], g[6], g[7], done);
+      const PartFit fit = hint ? refine_part_sad(c, g[0], g[1], g[2], g[3], ib.x[g[8]], ib.y[g[8]], mvp, lambda, bd)
+                               : refine_part(c, g[0], g[1], g[2], g[3], ib.x[g[8]], ib.y[g[8]], mvp, lambda, bd);
       const int mv[2] = {fit.x, fit.y};
       J += fit.cost;
       pm[k][0] = mv[0]; pm[k][1] = mv[1];
@@ -728,33 +737,29 @@ __device__ __noinline__ void analyse_p_mb_search(const Ctx c, Smem& sm, SearchSm
       for (int q = 0; q < 4; q++)
         if ((qm >> q) & 1) { qmv[q][0] = bmv[k][0]; qmv[q][1] = bmv[k][1]; }
       const int8_t* g = c_parts[first + k];
-      predict_part(c, sm, ws, g[0], g[1], g[2], g[3], ib.x[g[8]], ib.y[g[8]], bmv[k][0], bmv[k][1]);
+      predict_part(c, g[0], g[1], g[2], g[3], ib.x[g[8]], ib.y[g[8]], bmv[k][0], bmv[k][1]);
     }
   }
   // 5. intra 16x16 when the inter prediction is poor (the plain form's rule, enc.rs:3121-3156)
   uint32_t inter_satd = 0;
   if (lane < 16) {
     int bx = lane & 3, by = lane >> 2;
-    inter_satd = satd4(&sm.src_y[by * 64 + bx * 4], 16, &sm.pred_y[by * 64 + bx * 4], 16);
+    inter_satd = satd4((int)offsetof(Smem, src_y) + by * 64 + bx * 4, (int)offsetof(Smem, pred_y) + by * 64 + bx * 4);
   }
   inter_satd = wsum(inter_satd) >> 1;
   if (inter_satd > 24 * lambda) {
-    int tl, ctl[2];
-    load_edges(c, sm, false, tl, ctl);
+    const Corner k0 = load_edges(c, false);
     bool ht = mby > 0, hl = mbx > 0;
-    uint32_t i16c;
-    int i16m = analyse_i16(sm, ht, hl, tl, &i16c);
-    if (i16c + lambda * 8 < best_j) {
-      code_i16(c, sm, i16m, ht, hl, tl, ctl);
-      int z[4][2] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
-      search_tail(c, best_t, z, z);
+    const I16Fit fit16 = analyse_i16(ht, hl, k0.y);
+    if (fit16.cost + lambda * 8 < best_j) {
+      code_i16(c, fit16.mode, ht, hl, k0);
+      search_tail(c, best_t, false, 0, 0);
       return;
     }
   }
   // residual (enc.rs:3158-3190)
-  mc_chroma_q(c, sm, qmv);
-  uint32_t nz_lane;
-  int cbp4 = luma4x4_inter(qp, sm, &nz_lane);
+  mc_chroma_q(c);
+  int cbp4 = luma4x4_inter(qp);
   int cbpl = cbp4;
   bool use8 = false;
   if (fp.t8x8 && cbp4) {
@@ -765,13 +770,11 @@ __device__ __noinline__ void analyse_p_mb_search(const Ctx c, Smem& sm, SearchSm
       nnz4 += ((w & 0xffffu) != 0) + ((w >> 16) != 0);
     }
     nnz4 = wsum(nnz4);
-    uint32_t nnz8;
-    int cbp8 = luma8x8_inter(qp, sm, &nnz8);
-    if (nnz8 <= nnz4) { use8 = true; cbpl = cbp8; }
+    const uint32_t r8 = luma8x8_inter(qp);
+    if ((r8 >> 4) <= nnz4) { use8 = true; cbpl = (int)(r8 & 15u); }
   }
-  uint32_t ac_any[2], ac_sc[2];
-  chroma_quant(qpc, false, sm, ac_any, ac_sc);
-  bool drop_u = ac_any[0] && ac_sc[0] < 7, drop_v = ac_any[1] && ac_sc[1] < 7;
+  const ChromaAc ac = chroma_quant(qpc, false);
+  bool drop_u = ac.any(0) && ac.score(0) < 7, drop_v = ac.any(1) && ac.score(1) < 7;
   if (lane < 8) {
     bool d = (lane >> 2) ? drop_v : drop_u;
     if (d)
@@ -779,11 +782,11 @@ __device__ __noinline__ void analyse_p_mb_search(const Ctx c, Smem& sm, SearchSm
       for (int i = 0; i < 16; i++) sm.ccoef[lane * 16 + i] = 0;
   }
   __syncwarp();
-  bool acu = ac_any[0] && !drop_u, acv = ac_any[1] && !drop_v;
-  int cbpc = (acu || acv) ? 2 : (chroma_dc_any(sm) ? 1 : 0);
+  bool acu = ac.any(0) && !drop_u, acv = ac.any(1) && !drop_v;
+  int cbpc = (acu || acv) ? 2 : (chroma_dc_any() ? 1 : 0);
   if (best_t == 0 && cbpl == 0 && cbpc == 0 && bmv[0][0] == ps0 && bmv[0][1] == ps1) {
-    code_skip(c, sm, ps0, ps1);
-    search_tail(c, best_t, qmv, off4);
+    code_skip(c, ps0, ps1);
+    search_tail(c, best_t, false, ps0, ps1);  // 16x16: every quadrant has the skip vector
     return;
   }
   rg_mb_out* rec = sd.rec + c.mb;
@@ -796,46 +799,41 @@ __device__ __noinline__ void analyse_p_mb_search(const Ctx c, Smem& sm, SearchSm
     nzm = 0;
     for (int k = 0; k < 4; k++) if ((cbpl >> k) & 1) nzm |= (uint16_t)(0xF << (4 * k));
   } else {
-    nzm = record_luma4x4(rec, sm);
+    nzm = record_luma4x4(rec);
   }
   if (lane < 16) { rec->luma_dc[lane] = 0; rec->i4_modes[lane] = 2; }
-  record_chroma(rec, sm, cbpc);
+  record_chroma(rec, cbpc);
   if (lane == 0) {
     const int types[4] = {RG_MB_P_L0_16X16, RG_MB_P_L0_16X8, RG_MB_P_L0_8X16, RG_MB_P_8X8};
     record_header(rec, types[best_t], 0, 0, cbpl | (cbpc << 4), t8flag, qp, bmv[0][0], bmv[0][1], bmvd[0][0],
                   bmvd[0][1], nzm);
-    write_info(c, t8flag ? kFlagT8 : 0, cbpl, bmv[0][0], bmv[0][1], 0, nzm, nullptr);
+    write_info(c, t8flag ? kFlagT8 : 0, cbpl, bmv[0][0], bmv[0][1], 0, nzm, false);
   }
-  search_tail(c, best_t, qmv, bmvd);
-  if (use8) recon_luma8x8(sm, qp, cbpl);
-  else if (cbpl) recon_luma4x4(sm, qp, cbpl);
+  search_tail(c, best_t, true, 0, 0);
+  if (use8) recon_luma8x8(qp, cbpl);
+  else if (cbpl) recon_luma4x4(qp, cbpl);
   __syncwarp();
-  chroma_recon(qpc, cbpc, sm);
-  store_recon(c, sm.pred_y, sm);
-  (void)nz_lane;
+  chroma_recon(qpc, cbpc);
+  store_recon(c, (int)offsetof(Smem, pred_y));
 }
 
 // One macroblock of an I slice in the search forms: the plain analysis (enc.rs:3311 code_intra),
 // intra 4x4 blocks restricted to the hinted modes in the learned form.
-__device__ __noinline__ void analyse_intra_mb_search(const Ctx c, Smem& sm) {
-  int tl, ctl[2];
-  load_edges(c, sm, true, tl, ctl);
+__device__ __noinline__ void analyse_intra_mb_search(const Ctx c) {
+  const Corner k0 = load_edges(c, true);
   bool ht = c.mby > 0, hl = c.mbx > 0;
   uint32_t lambda = c_lambda[c.sd->qp];
-  uint32_t i16c;
-  int i16m = analyse_i16(sm, ht, hl, tl, &i16c);
-  const int z[4][2] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
-  if (i16c > 40 * lambda) {
-    int cbpl;
+  const I16Fit fit16 = analyse_i16(ht, hl, k0.y);
+  if (fit16.cost > 40 * lambda) {
     const uint16_t* masks = c.sd->hint ? c.sd->hint[c.mb].i4_mask : nullptr;
-    bool ok = masks ? analyse_i4<true>(c, sm, i16c + lambda * 4, ht, hl, tl, &cbpl, masks)
-                    : analyse_i4<false>(c, sm, i16c + lambda * 4, ht, hl, tl, &cbpl, nullptr);
-    if (ok) {
-      code_i4(c, sm, cbpl, ht, hl, ctl);
-      search_tail(c, 255, z, z);
+    const int cbpl = masks ? analyse_i4<true>(c, fit16.cost + lambda * 4, ht, hl, k0.y, masks)
+                           : analyse_i4<false>(c, fit16.cost + lambda * 4, ht, hl, k0.y, nullptr);
+    if (cbpl >= 0) {
+      code_i4(c, cbpl, ht, hl, k0);
+      search_tail(c, 255, false, 0, 0);
       return;
     }
   }
-  code_i16(c, sm, i16m, ht, hl, tl, ctl);
-  search_tail(c, 255, z, z);
+  code_i16(c, fit16.mode, ht, hl, k0);
+  search_tail(c, 255, false, 0, 0);
 }
