@@ -43,6 +43,9 @@ __constant__ uint8_t c_tc0[52][3];
 
 // ---------------------------------------------------------------------------------------------
 // Shared memory of one macroblock warp.
+// Block stride (words) of the 8x8 intermediates: 8 banks apart, so the four blocks' rows and columns
+// fall into different banks.
+constexpr int kT8Block = 72;
 struct __align__(16) Smem {
   uint8_t src_y[256];
   uint8_t src_u[64];
@@ -51,36 +54,40 @@ struct __align__(16) Smem {
   uint8_t pred_u[64];
   uint8_t pred_v[64];
   uint8_t tmp_y[256];       // plane prediction / I4x4 reconstruction
-  uint8_t win[23 * 24];     // integer samples of a half-sample window (rows -2.., cols -2..)
+  alignas(16) uint8_t win[23 * 24];  // integer samples of a half-sample window (rows -2.., cols -2..)
   // The half-sample planes live until the sub-pel search ends; the 8x8 transform's intermediates
   // are needed only after it (the residual), so they share the space.
-  union {
+  union alignas(16) {
     struct {
       uint8_t hph[18 * 20];  // b samples (horizontal half)
       uint8_t hpv[18 * 20];  // h samples (vertical half)
       uint8_t hpj[18 * 20];  // j samples (centre)
       int16_t hr[23 * 18];   // unrounded horizontal 6-tap sums
     };
-    int32_t t8[256];         // 8x8 transform intermediates
+    int32_t t8[4 * kT8Block];  // 8x8 transform intermediates, block b at [kT8Block b]
   };
-  int16_t coef[256];        // luma 4x4 levels: block b (decoding order) at [16 b], raster
-  int16_t coef8[256];       // luma 8x8 levels: block b at [64 b], raster
-  int16_t ccoef[128];       // chroma levels: block (plane * 4 + b) at [16 *], raster
-  int16_t cdcraw[8];
-  int16_t cdc[8];
+  alignas(16) int16_t coef[256];  // luma 4x4 levels: block b (decoding order) at [16 b], raster
+  alignas(16) int16_t coef8[256]; // luma 8x8 levels: block b at [64 b], zig-zag order
+  alignas(16) uint8_t zz8[64];    // zig-zag index of row y, column x of an 8x8 block at [8 x + y] (init_tables)
+  alignas(16) int16_t ccoef[128]; // chroma levels: block (plane * 4 + b) at [16 *], raster
+  alignas(16) int16_t cdc[8];
   int16_t ldc[16];          // I16x16 DC levels, raster
   int16_t ldcr[16];         // I16x16 DC reconstruction, raster
   uint8_t top[24];          // luma row above the macroblock (x0 .. x0 + 23)
   uint8_t left[16];
   uint8_t ctop[2][8];
   uint8_t cleft[2][8];
-  uint8_t i4m[16];          // Intra4x4PredMode of this macroblock (decoding order)
+  alignas(16) uint8_t i4m[16];    // Intra4x4PredMode of this macroblock (decoding order)
   uint8_t i4q[16];          // edge samples of the current 4x4 block (i4_edge_index)
 };
 static_assert(offsetof(Smem, coef) % 4 == 0 && offsetof(Smem, ccoef) % 4 == 0, "level arrays cleared by words");
 static_assert(offsetof(rg_mb_out, luma) % 4 == 0 && offsetof(rg_mb_out, chroma_dc) % 4 == 0 &&
                   offsetof(rg_mb_out, chroma_ac) % 4 == 0 && sizeof(rg_mb_out) % 4 == 0,
               "record levels written by words");
+static_assert(offsetof(Smem, coef) % 8 == 0 && offsetof(Smem, ccoef) % 8 == 0 && offsetof(Smem, coef8) % 8 == 0 &&
+                  offsetof(Smem, t8) % 16 == 0 && offsetof(Smem, zz8) % 8 == 0 && offsetof(Smem, i4m) % 4 == 0 &&
+                  offsetof(Smem, src_u) % 8 == 0 && offsetof(Smem, pred_u) % 8 == 0,
+              "rows of levels, intermediates and samples move as vectors");
 static_assert(offsetof(Smem, pred_y) % 8 == 0 && offsetof(Smem, tmp_y) % 8 == 0, "16x16 predictions written 8 bytes per lane");
 
 // Every kernel of this file runs one warp per block, and its shared memory has this one name: the
@@ -105,20 +112,11 @@ __device__ __forceinline__ int16_t clamp_i16(int v) { return (int16_t)(v < -3276
 // Column and row of 4x4 block b in decoding order (enc.rs:522 blk_xy).
 __device__ __forceinline__ int blk_x(int b) { return (b & 1) + ((b >> 1) & 2); }
 __device__ __forceinline__ int blk_y(int b) { return ((b >> 1) & 1) + ((b >> 2) & 2); }
-// Position class of raster coefficient i in a 4x4 / 8x8 block (h264.rs:1204, :1343).
+// Position class of raster coefficient i in a 4x4 block (h264.rs:1204).
 __device__ __forceinline__ int pos4(int i) {
   int r = i >> 2, c = i & 3;
   if (((r | c) & 1) == 0) return 0;
   return ((r & c) & 1) ? 1 : 2;
-}
-__device__ __forceinline__ int pos8(int i) {
-  int r = (i >> 3) & 3, c = i & 3;
-  if (r == 0 && c == 0) return 0;
-  if ((r & 1) && (c & 1)) return 1;
-  if (r == 2 && c == 2) return 2;
-  if ((r == 0 && (c & 1)) || ((r & 1) && c == 0)) return 3;
-  if ((r == 0 && c == 2) || (r == 2 && c == 0)) return 4;
-  return 5;
 }
 __device__ __forceinline__ int chroma_qp(int qp) { return c_cqp[qp < 0 ? 0 : (qp > 51 ? 51 : qp)]; }
 // Bits of se(v) (enc.rs:546).
@@ -206,29 +204,6 @@ __device__ __forceinline__ void idct8_1d(const int* d, int* o) {
   o[0] = (int)(b0 + b7); o[1] = (int)(b2 + b5); o[2] = (int)(b4 + b3); o[3] = (int)(b6 + b1);
   o[4] = (int)(b6 - b1); o[5] = (int)(b4 - b3); o[6] = (int)(b2 - b5); o[7] = (int)(b0 - b7);
 }
-// SATD of a 4x4 block (metrics.rs:705, halved).
-// Byte offsets of the two blocks in Smem, rows of 16 samples.
-__device__ __noinline__ uint32_t satd4(int off_a, int off_b) {
-  const uint8_t* a = sm_at(off_a);
-  const uint8_t* b = sm_at(off_b);
-  constexpr int sa = 16, sb = 16;
-  int t[4][4];
-#pragma unroll
-  for (int y = 0; y < 4; y++) {
-    int d0 = a[y * sa] - b[y * sb], d1 = a[y * sa + 1] - b[y * sb + 1];
-    int d2 = a[y * sa + 2] - b[y * sb + 2], d3 = a[y * sa + 3] - b[y * sb + 3];
-    int s03 = d0 + d3, s12 = d1 + d2, d03 = d0 - d3, d12 = d1 - d2;
-    t[y][0] = s03 + s12; t[y][1] = d03 + d12; t[y][2] = s03 - s12; t[y][3] = d03 - d12;
-  }
-  uint32_t s = 0;
-#pragma unroll
-  for (int x = 0; x < 4; x++) {
-    int s03 = t[0][x] + t[3][x], s12 = t[1][x] + t[2][x], d03 = t[0][x] - t[3][x], d12 = t[1][x] - t[2][x];
-    s += abs(s03 + s12) + abs(d03 + d12) + abs(s03 - s12) + abs(d03 - d12);
-  }
-  return s;  // caller halves the sum of the blocks
-}
-
 // One pass of the 4x4 forward core transform along the axis whose lanes are `step` apart in a
 // 16-lane group (i = position along it): [1 1 1 1; 2 1 -1 -2; 1 -1 -1 1; 1 -2 2 -1].
 __device__ __forceinline__ int fwd4_pass(int v, int step, int i) {
@@ -414,122 +389,210 @@ __device__ __forceinline__ void quant4_params(int qp, bool intra, uint32_t& shif
   shift = 15 + qp / 6;
   bias = (1u << shift) / (intra ? 3u : 6u);
 }
+// Level of coefficient c. Every transform here is of 8-bit differences: |c| is at most 64 * 255 and
+// the scales at most 20972, so the product and the bias fit 32 bits and the level 16.
 __device__ __forceinline__ int quant_level(int c, uint32_t mf, uint32_t bias, uint32_t shift) {
   uint32_t a = (uint32_t)(c < 0 ? -c : c);
-  uint64_t l = ((uint64_t)a * mf + bias) >> shift;
-  if (l > 32767) l = 32767;
-  return c < 0 ? -(int)l : (int)l;
+  int l = (int)((a * mf + bias) >> shift);
+  return c < 0 ? -l : l;
 }
 
-// Zig-zag index of each raster position of a 4x4 block, 4 bits per position (inverse of the
-// frame scan, Table 8-12).
-constexpr unsigned long long kZigzagIndex4 = 0xfea9db83c7426510ull;
-
-// Forward 4x4 core transform (fixed.rs:104, int16 output) and quantisation of `nblocks` 4x4
-// residual blocks (src - pred): luma blocks in decoding order (chroma = false) or the eight chroma
-// blocks, U then V (chroma = true). Lane = coefficient (raster p = lane & 15); half-warp h takes
-// block 2 it + h, two blocks per step. Levels go to sm.coef / sm.ccoef [16 b + p]; the raw DC of each
-// chroma block to sm.cdcraw[b]. Lane b returns block b's: bit 0 any level (among zig-zag indices >=
-// first), bit 1 any |level| > 1 (same), and from bit 2 the decimation score of its zig-zag levels
-// from index `first` (enc.rs:559 decimate_score without its |level| > 1 rule; the caller applies it).
-__device__ __noinline__ uint32_t quant4x4_blocks(bool chroma, int nblocks, int first, int qp, uint32_t shift, uint32_t bias) {
-  int16_t* const out = chroma ? sm.ccoef : sm.coef;
-  int my_nz, my_big, my_score;
-  int lane = lane_id(), p = lane & 15, h = lane >> 4, xl = p & 3, yl = p >> 2;
-  int zi = (int)((kZigzagIndex4 >> (4 * p)) & 15);
-  uint32_t mf = c_mf4[qp % 6][pos4(p)];
-  bool counted = zi >= first;
-  my_nz = my_big = my_score = 0;
-#pragma unroll 1
-  for (int it = 0; it < nblocks / 2; it++) {
-    int b = 2 * it + h;
-    const uint8_t *s, *pr;
-    int stride;
-    if (chroma) {
-      int off = ((b & 3) >> 1) * 32 + (b & 1) * 4;
-      s = ((b >> 2) ? sm.src_v : sm.src_u) + off;
-      pr = ((b >> 2) ? sm.pred_v : sm.pred_u) + off;
-      stride = 8;
-    } else {
-      int off = blk_y(b) * 64 + blk_x(b) * 4;
-      s = sm.src_y + off;
-      pr = sm.pred_y + off;
-      stride = 16;
-    }
-    int d = (int)s[yl * stride + xl] - (int)pr[yl * stride + xl];
-    int c = (int16_t)fwd4_pass(fwd4_pass(d, 1, xl), 4, yl);
-    if (chroma && p == 0) sm.cdcraw[b] = (int16_t)c;
-    int l = quant_level(c, mf, bias, shift);
-    out[b * 16 + p] = (int16_t)l;
-    bool nz = l != 0 && counted;
-    uint32_t nzm = __ballot_sync(FULL, nz);
-    uint32_t bigm = __ballot_sync(FULL, nz && (l > 1 || l < -1));
-    uint32_t zm = __reduce_or_sync(FULL, nz ? 1u << (zi + 16 * h) : 0u);
-    uint32_t mine = (zm >> (16 * h)) & 0xffffu;
-    uint32_t contrib = 0;
-    if ((mine >> p) & 1u) {  // this lane as zig-zag index p: the run of zeros below it
-      uint32_t below = mine & ((1u << p) - 1u);
-      int prev = below ? 31 - __clz(below) : first - 1;
-      int run = p - prev - 1;
-      contrib = run == 0 ? 3u : (run <= 2 ? 2u : (run <= 5 ? 1u : 0u));
-    }
-    uint32_t sc = __reduce_add_sync(FULL, contrib << (16 * h));
-    if (lane == 2 * it || lane == 2 * it + 1) {
-      int k = lane & 1;
-      my_nz = ((nzm >> (16 * k)) & 0xffffu) != 0;
-      my_big = ((bigm >> (16 * k)) & 0xffffu) != 0;
-      my_score = (int)((sc >> (16 * k)) & 0xffffu);
-    }
+// ---- 4x4 blocks, two lanes each -----------------------------------------------------------------
+// A macroblock's 4x4 transforms are done all at once: lane 2 b + h holds half of block b, the pixel
+// rows (0, 3) when h = 0 and (1, 2) when h = 1 -- the pairs the core transform's first butterfly
+// adds -- and after the forward transform the coefficient rows (0, 2) or (1, 3), the pairs the
+// inverse starts from. Rows are transformed in registers, and a column pass needs four words of the
+// partner lane (four independent shuffles). A macroblock is one chain of instructions of one warp, so
+// what counts is the chain's length: one lane per coefficient and two blocks a step was eight steps
+// of two passes of three dependent shuffles, 7.2 k cycles for the luma quantisation even on a nearly
+// idle SM. With this split (and the record written by words) a 720p stream's launch of 30 pictures
+// went from 21.6 to 17.6 ms, 1080p 8 x 15 from 54.6 to 50.7 ms.
+struct Half4 {
+  int a[4], b[4];  // its first and second row
+};
+// The lane's two rows (r0 = the first's index) of samples at byte offset `off` in Smem.
+__device__ __forceinline__ uint2 half_rows(int off, int stride, int h) {
+  return make_uint2(*(const uint32_t*)sm_at(off + h * stride), *(const uint32_t*)sm_at(off + (3 - h) * stride));
+}
+__device__ __forceinline__ Half4 half_diff(uint2 s, uint2 p) {
+  Half4 d;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    d.a[k] = (int)((s.x >> (8 * k)) & 255u) - (int)((p.x >> (8 * k)) & 255u);
+    d.b[k] = (int)((s.y >> (8 * k)) & 255u) - (int)((p.y >> (8 * k)) & 255u);
   }
-  __syncwarp();
-  return (uint32_t)my_nz | ((uint32_t)my_big << 1) | ((uint32_t)my_score << 2);
+  return d;
+}
+// Forward core transform (fixed.rs:104).
+__device__ __forceinline__ void half_fwd(Half4& v, int h) {
+  auto row = [](int (&r)[4]) {
+    int s03 = r[0] + r[3], s12 = r[1] + r[2], d03 = r[0] - r[3], d12 = r[1] - r[2];
+    r[0] = s03 + s12; r[1] = 2 * d03 + d12; r[2] = s03 - s12; r[3] = d03 - 2 * d12;
+  };
+  row(v.a);
+  row(v.b);
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    // h = 0: sum s03 and difference d03 of rows 0 and 3; h = 1: s12 and d12 of rows 1 and 2
+    int s = v.a[k] + v.b[k], d = v.a[k] - v.b[k];
+    int o = __shfl_xor_sync(FULL, h ? s : d, 1);
+    int x = h ? o : s, y = h ? d : o;   // s03, s12 or d03, d12
+    v.a[k] = (x << h) + y;              // row 0: s03 + s12, row 1: 2 d03 + d12
+    v.b[k] = x - (y << h);              // row 2: s03 - s12, row 3: d03 - 2 d12
+  }
+}
+// Inverse core transform with its rounding (fixed.rs:192): coefficient rows in, residual rows out.
+__device__ __forceinline__ void half_inv(Half4& v, int h) {
+  auto row = [](int (&r)[4]) {
+    int e0 = r[0] + r[2], e1 = r[0] - r[2], e2 = (r[1] >> 1) - r[3], e3 = r[1] + (r[3] >> 1);
+    r[0] = e0 + e3; r[1] = e1 + e2; r[2] = e1 - e2; r[3] = e0 - e3;
+  };
+  row(v.a);
+  row(v.b);
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    // h = 0 (rows 0, 2): e0, e1; h = 1 (rows 1, 3): e2, e3
+    int p = h ? (v.a[k] >> 1) - v.b[k] : v.a[k] + v.b[k];
+    int q = h ? v.a[k] + (v.b[k] >> 1) : v.a[k] - v.b[k];
+    int o = __shfl_xor_sync(FULL, q, 1);
+    int x = h ? o : p, y = h ? p : o;  // h = 0: e0, e3 -> rows 0, 3; h = 1: e1, e2 -> rows 1, 2
+    v.a[k] = (x + y + 32) >> 6;
+    v.b[k] = (x - y + 32) >> 6;
+  }
+}
+// This half's share of the block's SATD (metrics.rs:705): a column's four Hadamard outputs are
+// |x + y| and |x - y| of each lane's (x, y), and |x + y| + |x - y| = 2 max(|x|, |y|), so the sums
+// below are the halved ones.
+__device__ __forceinline__ uint32_t half_satd(Half4 v, int h) {
+  auto row = [](int (&r)[4]) {
+    int s03 = r[0] + r[3], s12 = r[1] + r[2], d03 = r[0] - r[3], d12 = r[1] - r[2];
+    r[0] = s03 + s12; r[1] = d03 + d12; r[2] = s03 - s12; r[3] = d03 - d12;
+  };
+  row(v.a);
+  row(v.b);
+  uint32_t sum = 0;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    int s = v.a[k] + v.b[k], d = v.a[k] - v.b[k];
+    int o = __shfl_xor_sync(FULL, h ? s : d, 1);
+    sum += (uint32_t)max(abs(h ? d : s), abs(o));
+  }
+  return sum;
+}
+// The per-lane scales of the half's even and odd columns (position classes 0, 2 / 2, 1).
+__device__ __forceinline__ void half_scales(uint32_t c0, uint32_t c1, uint32_t c2, int h, uint32_t& even, uint32_t& odd) {
+  even = h ? c2 : c0;
+  odd = h ? c1 : c2;
+}
+// The half's zig-zag indices: rows 0 and 2, or rows 1 and 3, of the frame scan (Table 8-12).
+__device__ __forceinline__ uint32_t half_zigzag_bit(int row, int k, int h) {
+  constexpr uint32_t z[2][2][4] = {{{0, 1, 5, 6}, {3, 8, 11, 13}}, {{2, 4, 7, 12}, {9, 10, 14, 15}}};
+  return h ? 1u << z[1][row][k] : 1u << z[0][row][k];
+}
+// Quantises the half. Returns, alike in both lanes, the block's nonzero levels by zig-zag index
+// (bits 0..15, indices >= first) and in bit 16 whether one of them is above 1.
+__device__ __forceinline__ uint32_t half_quant(Half4& v, int h, int first, uint32_t mf_even, uint32_t mf_odd, uint32_t bias,
+                                               uint32_t shift) {
+  uint32_t mask = 0, big = 0;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const uint32_t mf = (k & 1) ? mf_odd : mf_even;
+    const uint32_t la = ((uint32_t)abs(v.a[k]) * mf + bias) >> shift, lb = ((uint32_t)abs(v.b[k]) * mf + bias) >> shift;
+    const bool dc = k == 0 && first && !h;
+    if (la && !dc) mask |= half_zigzag_bit(0, k, h);
+    if (lb) mask |= half_zigzag_bit(1, k, h);
+    big |= (dc ? 0u : la) | lb;
+    v.a[k] = v.a[k] < 0 ? -(int)la : (int)la;
+    v.b[k] = v.b[k] < 0 ? -(int)lb : (int)lb;
+  }
+  mask |= big > 1u ? 0x10000u : 0u;
+  return mask | __shfl_xor_sync(FULL, mask, 1);
+}
+// Decimation score (enc.rs:559, without its |level| > 1 rule) of a block's nonzero zig-zag
+// positions: 3 / 2 / 1 / 0 for a zero run of 0 / 1-2 / 3-5 / longer below each -- the positions with
+// another one (or the start, index first - 1) at most 1, 3 and 6 below, counted.
+__device__ __forceinline__ uint32_t score4(uint32_t m, int first) {
+  m &= 0xffffu;
+  const uint32_t w1 = (first ? m | 1u : m) << 1, w3 = w1 | (w1 << 1) | (w1 << 2), w6 = w3 | (w3 << 3);
+  const uint32_t u = first ? 0u : 0x3fu;  // the start, one below index 0
+  return __popc(m & (w1 | (u & 1u))) + __popc(m & (w3 | (u & 7u))) + __popc(m & (w6 | u));
+}
+__device__ __forceinline__ uint2 pack_half(const int (&r)[4]) {
+  return make_uint2(__byte_perm((uint32_t)r[0], (uint32_t)r[1], 0x5410), __byte_perm((uint32_t)r[2], (uint32_t)r[3], 0x5410));
+}
+__device__ __forceinline__ void unpack_half(uint2 w, int (&r)[4]) {
+  r[0] = (int16_t)(w.x & 0xffffu); r[1] = (int)w.x >> 16;
+  r[2] = (int16_t)(w.y & 0xffffu); r[3] = (int)w.y >> 16;
+}
+// Four clipped samples p + r, packed.
+__device__ __forceinline__ uint32_t add_clip4(uint32_t p, const int (&r)[4]) {
+  uint32_t w = 0;
+#pragma unroll
+  for (int k = 0; k < 4; k++) w |= (uint32_t)clip255((int)((p >> (8 * k)) & 255u) + r[k]) << (8 * k);
+  return w;
+}
+// Byte offset of 4x4 luma block b (decoding order) in a 16x16 plane, and of chroma block b (plane b
+// / 4) in the two 8x8 planes u, v (v right behind u).
+__device__ __forceinline__ int blk_off16(int b) { return blk_y(b) * 64 + blk_x(b) * 4; }
+__device__ __forceinline__ int blk_off8(int b) { return (b >> 2) * 64 + ((b & 3) >> 1) * 32 + (b & 1) * 4; }
+static_assert(offsetof(Smem, src_v) == offsetof(Smem, src_u) + 64 && offsetof(Smem, pred_v) == offsetof(Smem, pred_u) + 64,
+              "the chroma planes lie back to back");
+// The even bits of w (one per lane pair) as 16 bits.
+__device__ __forceinline__ uint32_t even_bits(uint32_t w) {
+  w &= 0x55555555u;
+  w = (w | (w >> 1)) & 0x33333333u;
+  w = (w | (w >> 2)) & 0x0f0f0f0fu;
+  w = (w | (w >> 4)) & 0x00ff00ffu;
+  return (w | (w >> 8)) & 0xffffu;
+}
+
+// SATD (metrics.rs:705, halved) of the macroblock's source against the 16x16 plane at byte offset `at`.
+__device__ __noinline__ uint32_t satd16(int at) {
+  const int lane = lane_id(), h = lane & 1, off = blk_off16(lane >> 1);
+  return wsum(half_satd(half_diff(half_rows((int)offsetof(Smem, src_y) + off, 16, h), half_rows(at + off, 16, h)), h));
+}
+// Forward transform and inter quantisation of the macroblock's luma residual, one block per lane pair.
+__device__ __forceinline__ uint32_t luma4x4_levels(int qp, Half4& v) {
+  const int lane = lane_id(), b = lane >> 1, h = lane & 1, off = blk_off16(b);
+  uint32_t shift, bias, even, odd;
+  quant4_params(qp, false, shift, bias);
+  const int rem = qp % 6;
+  half_scales(c_mf4[rem][0], c_mf4[rem][1], c_mf4[rem][2], h, even, odd);
+  v = half_diff(half_rows((int)offsetof(Smem, src_y) + off, 16, h), half_rows((int)offsetof(Smem, pred_y) + off, 16, h));
+  half_fwd(v, h);
+  return half_quant(v, h, 0, even, odd, bias, shift);
 }
 
 // Luma 4x4 residual of pred_y, quantised (inter) and decimated into sm.coef
-// (enc.rs:1810 quant_luma_4x4_inter). Returns cbp.
-__device__ __noinline__ int luma4x4_inter(int qp) {
-  int lane = lane_id();
-  uint32_t shift, bias;
-  quant4_params(qp, false, shift, bias);
-  const uint32_t mine = quant4x4_blocks(false, 16, 0, qp, shift, bias);
-  int my_nz = mine & 1, my_big = (mine >> 1) & 1, my_score = mine >> 2;
-  // per-8x8 aggregates (lanes 4g..4g+3)
-  int g_nz = my_nz | __shfl_xor_sync(FULL, my_nz, 1);
-  g_nz |= __shfl_xor_sync(FULL, g_nz, 2);
-  int g_big = my_big | __shfl_xor_sync(FULL, my_big, 1);
-  g_big |= __shfl_xor_sync(FULL, g_big, 2);
-  uint32_t g_sc = my_score + __shfl_xor_sync(FULL, my_score, 1);
-  g_sc += __shfl_xor_sync(FULL, g_sc, 2);
-  int cbp = 0;
-  uint32_t total = 0;
-#pragma unroll
-  for (int g = 0; g < 4; g++) {
-    int nz = __shfl_sync(FULL, g_nz, 4 * g), big = __shfl_sync(FULL, g_big, 4 * g);
-    uint32_t sc = __shfl_sync(FULL, g_sc, 4 * g);
-    if (!nz) continue;
-    if (big) { cbp |= 1 << g; total += 9; continue; }
-    if (sc >= 4) cbp |= 1 << g;
-    total += sc;
-  }
-  if (total < 6 && cbp) cbp = 0;
-  // clear the levels of dropped 8x8 groups: word lane + 32 k of sm.coef lies in group k
-#pragma unroll
-  for (int k = 0; k < 4; k++)
-    if (!((cbp >> k) & 1)) ((uint32_t*)sm.coef)[lane + 32 * k] = 0u;
+// (enc.rs:1810 quant_luma_4x4_inter).
+struct Luma4 {
+  uint32_t cbp, nnz, nz16;  // coded block pattern, nonzero levels kept, blocks holding levels (bit b)
+};
+__device__ __noinline__ Luma4 luma4x4_inter(int qp) {
+  const int lane = lane_id(), b = lane >> 1, h = lane & 1;
+  Half4 v;
+  const uint32_t m = luma4x4_levels(qp, v);
+  // the 8x8 group's any, |level| > 1 and score sums over its four blocks (lanes 8 g .. 8 g + 7)
+  uint32_t g = score4(m, 0) | ((m >> 16) << 12) | ((m & 0xffffu) ? 1u << 16 : 0u);
+  g += __shfl_xor_sync(FULL, g, 2);
+  g += __shfl_xor_sync(FULL, g, 4);
+  const bool any = (g >> 16) != 0, big = ((g >> 12) & 15u) != 0;
+  const uint32_t sc = g & 0xfffu;
+  const uint32_t keep = __ballot_sync(FULL, any && (big || sc >= 4));
+  const uint32_t total = wsum((lane & 7) == 0 && any ? (big ? 9u : sc) : 0u);
+  uint32_t cbp = (keep & 1u) | ((keep >> 7) & 2u) | ((keep >> 14) & 4u) | ((keep >> 21) & 8u);
+  if (total < 6) cbp = 0;
+  const bool coded = (cbp >> (lane >> 3)) & 1u;  // levels of dropped groups are cleared
+  uint2 ra = pack_half(v.a), rb = pack_half(v.b);
+  if (!coded) ra = rb = make_uint2(0u, 0u);
+  *(uint2*)&sm.coef[b * 16 + h * 4] = ra;
+  *(uint2*)&sm.coef[b * 16 + h * 4 + 8] = rb;
+  Luma4 r;
+  r.cbp = cbp;
+  r.nz16 = even_bits(__ballot_sync(FULL, coded && (m & 0xffffu)));
+  r.nnz = wsum(h == 0 && coded ? __popc(m & 0xffffu) : 0u);
   __syncwarp();
-  return cbp;
-}
-
-// The 1-D forward 8x8 transform in place on sm.t8[at], [at + stride], ..., [at + 7 * stride] (row and column
-// passes share it).
-__device__ __noinline__ void fdct8_inplace(int at, int stride) {
-  int* p = &sm.t8[at];
-  int a[8], o[8];
-#pragma unroll
-  for (int k = 0; k < 8; k++) a[k] = p[k * stride];
-  fdct8_1d(a, o);
-#pragma unroll
-  for (int k = 0; k < 8; k++) p[k * stride] = o[k];
+  return r;
 }
 
 // Zig-zag index of (row y, column x) of an 8x8 block (frame scan, Table 8-13): diagonal s = x + y,
@@ -539,145 +602,165 @@ __device__ __forceinline__ int zigzag8(int y, int x) {
   if (s < 8) return s * (s + 1) / 2 + ((s & 1) ? y : x);
   return 64 - (16 - s) * (15 - s) / 2 + ((s & 1) ? 7 - x : 7 - y);
 }
+// The tables a warp keeps in its shared memory, once per kernel.
+__device__ __forceinline__ void init_tables() {
+  for (int i = lane_id(); i < 64; i += 32) sm.zz8[i] = (uint8_t)zigzag8(i & 7, i >> 3);
+  __syncwarp();
+}
+// The scales of row (or column) q of an 8x8 block by the other coordinate's low two bits: position
+// classes (h264.rs:1343) {0, 3, 4, 3}, {3, 1, 5, 1}, {4, 5, 2, 5}, {3, 1, 5, 1}.
+struct Scale8 {
+  int m0, m1, m2;  // index 0, odd, 2
+  __device__ __forceinline__ int at(int k) const { return (k & 1) ? m1 : ((k & 2) ? m2 : m0); }
+};
+template <typename T>
+__device__ __forceinline__ Scale8 scale8(const T* c, int q) {
+  const int k0 = c[0], k1 = c[1], k2 = c[2], k3 = c[3], k4 = c[4], k5 = c[5];
+  const bool odd = q & 1, two = (q & 3) == 2;
+  return {odd ? k3 : (two ? k4 : k0), odd ? k1 : (two ? k5 : k3), odd ? k5 : (two ? k2 : k4)};
+}
+// Eight words of a block's row (contiguous) to and from shared memory.
+__device__ __forceinline__ void t8_store_row(int at, const int (&r)[8]) {
+  *(int4*)&sm.t8[at] = make_int4(r[0], r[1], r[2], r[3]);
+  *(int4*)&sm.t8[at + 4] = make_int4(r[4], r[5], r[6], r[7]);
+}
 
 // Luma 8x8 residual of pred_y, quantised (inter) and decimated into sm.coef8
-// (enc.rs:2041 quant_luma_8x8_inter). Lanes 8b..8b+7 own block b: a row each in the first pass,
-// column q each in the second. The decimation score of a block comes from the bitmask of its
-// nonzero zig-zag positions (run of zeros below each, weights 3 / 2 / 1 / 0 for runs of
-// 0-3 / 4-11 / 12-23 / longer, enc.rs:559 with the 8x8 table). Returns cbp | nonzero levels << 4.
+// (enc.rs:2041 quant_luma_8x8_inter). Lanes 8b..8b+7 own block b: row q in registers for the first
+// pass, column q (through shared memory) for the second. The decimation score of a block comes from
+// the bitmask of its nonzero zig-zag positions (weights 3 / 2 / 1 / 0 for zero runs of 0-3 / 4-11 /
+// 12-23 / longer below each, enc.rs:559 with the 8x8 table), counted as in score4. Returns cbp |
+// nonzero levels << 4.
 __device__ __noinline__ uint32_t luma8x8_inter(int qp) {
-  int lane = lane_id();
-  int b = lane >> 3, q = lane & 7;
-  int bx = (b & 1) * 8, by = (b >> 1) * 8;
-  uint32_t shift = 16 + qp / 6, bias = (1u << shift) / 6u;
-  // residual of row q, then the row pass and (after all rows) the column pass in place
-#pragma unroll 1
-  for (int x = 0; x < 8; x++) {
-    int off = (by + q) * 16 + bx + x;
-    sm.t8[b * 64 + q * 8 + x] = (int)sm.src_y[off] - (int)sm.pred_y[off];
-  }
-  fdct8_inplace(b * 64 + q * 8, 1);
-  __syncwarp();
-  uint32_t mf6[6];
+  const int lane = lane_id(), b = lane >> 3, q = lane & 7;
+  const int off = ((b >> 1) * 8 + q) * 16 + (b & 1) * 8;
+  const uint32_t shift = 16 + qp / 6, bias = (1u << shift) / 6u;
+  int d[8], o[8];
+  {
+    const uint2 s = *(const uint2*)&sm.src_y[off], p = *(const uint2*)&sm.pred_y[off];
 #pragma unroll
-  for (int k = 0; k < 6; k++) mf6[k] = c_mf8[qp % 6][k];
-  int any = 0, big = 0;
-  unsigned long long zmask = 0;
-  fdct8_inplace(b * 64 + q, 8);  // column q; then quantisation row by row
-#pragma unroll 1
-  for (int y = 0; y < 8; y++) {
-    int i = y * 8 + q, cls = pos8(i);
-    uint32_t mf = cls == 0 ? mf6[0] : cls == 1 ? mf6[1] : cls == 2 ? mf6[2] : cls == 3 ? mf6[3] : cls == 4 ? mf6[4] : mf6[5];
-    int l = quant_level((int16_t)sm.t8[b * 64 + i], mf, bias, shift);
-    sm.coef8[b * 64 + i] = (int16_t)l;
-    any |= l != 0;
-    big |= l > 1 || l < -1;
-    if (l) zmask |= 1ull << zigzag8(y, q);
-  }
-#pragma unroll
-  for (int o = 1; o < 8; o <<= 1) {
-    any |= __shfl_xor_sync(FULL, any, o);
-    big |= __shfl_xor_sync(FULL, big, o);
-    zmask |= __shfl_xor_sync(FULL, zmask, o);
-  }
-  // lane q scores zig-zag positions 8q .. 8q + 7
-  uint32_t part = 0;
-#pragma unroll 1
-  for (int k = 0; k < 8; k++) {
-    int z = 8 * q + k;
-    if ((zmask >> z) & 1ull) {
-      unsigned long long below = zmask & ((1ull << z) - 1ull);
-      int run = z - (below ? 63 - __clzll((long long)below) : -1) - 1;
-      part += run < 4 ? 3u : (run < 12 ? 2u : (run < 24 ? 1u : 0u));
+    for (int k = 0; k < 4; k++) {
+      d[k] = (int)((s.x >> (8 * k)) & 255u) - (int)((p.x >> (8 * k)) & 255u);
+      d[k + 4] = (int)((s.y >> (8 * k)) & 255u) - (int)((p.y >> (8 * k)) & 255u);
     }
   }
+  fdct8_1d(d, o);
+  t8_store_row(b * kT8Block + q * 8, o);
+  __syncwarp();
 #pragma unroll
-  for (int o = 1; o < 8; o <<= 1) part += __shfl_xor_sync(FULL, part, o);
-  uint32_t score = !any ? 0u : (big ? 9u : part);
-  int cbp = 0;
-  uint32_t total = 0;
+  for (int y = 0; y < 8; y++) d[y] = sm.t8[b * kT8Block + y * 8 + q];
+  fdct8_1d(d, o);
+  const Scale8 mf = scale8(c_mf8[qp % 6], q);
+  const uint2 zz = *(const uint2*)&sm.zz8[q * 8];
+  uint32_t lo = 0, hi = 0, big = 0;
 #pragma unroll
-  for (int k = 0; k < 4; k++) {
-    uint32_t s = __shfl_sync(FULL, score, 8 * k);
-    total += s;
-    if (s >= 4) cbp |= 1 << k;
+  for (int y = 0; y < 8; y++) {
+    const uint32_t l = ((uint32_t)abs(o[y]) * (uint32_t)mf.at(y) + bias) >> shift;
+    const uint32_t z = ((y < 4 ? zz.x : zz.y) >> (8 * (y & 3))) & 255u, bit = l ? 1u << (z & 31u) : 0u;
+    if (z & 32u) hi |= bit; else lo |= bit;
+    big |= l;
+    o[y] = o[y] < 0 ? -(int)l : (int)l;
   }
-  if (total < 6 && cbp) cbp = 0;
-  uint32_t cnt = 0;
-  if (!((cbp >> b) & 1)) {
 #pragma unroll
-    for (int y = 0; y < 8; y++) sm.coef8[b * 64 + y * 8 + q] = 0;
-  } else {
-    cnt = __popcll(zmask) * (q == 0);
+  for (int k = 1; k < 8; k <<= 1) {
+    lo |= __shfl_xor_sync(FULL, lo, k);
+    hi |= __shfl_xor_sync(FULL, hi, k);
+  }
+  const bool anybig = ((__ballot_sync(FULL, big > 1u) >> (8 * b)) & 0xffu) != 0;
+  const unsigned long long m = ((unsigned long long)hi << 32) | lo;
+  const unsigned long long s1 = m << 1, s2 = s1 | (s1 << 1), s4 = s2 | (s2 << 2), s8 = s4 | (s4 << 4),
+                           s12 = s8 | (s4 << 8), s24 = s12 | (s12 << 12);
+  uint32_t score = __popcll(m & (s4 | 0xfull)) + __popcll(m & (s12 | 0xfffull)) + __popcll(m & (s24 | 0xffffffull));
+  if (anybig) score = 9u;
+  const uint32_t keep = __ballot_sync(FULL, score >= 4);
+  const uint32_t total = wsum(q == 0 ? score : 0u);
+  uint32_t cbp = (keep & 1u) | ((keep >> 7) & 2u) | ((keep >> 14) & 4u) | ((keep >> 21) & 8u);
+  if (total < 6) cbp = 0;
+  const bool coded = (cbp >> b) & 1u;
+#pragma unroll
+  for (int y = 0; y < 8; y++) {
+    const uint32_t z = ((y < 4 ? zz.x : zz.y) >> (8 * (y & 3))) & 255u;
+    sm.coef8[b * 64 + z] = (int16_t)(coded ? o[y] : 0);
   }
   __syncwarp();
-  return (uint32_t)cbp | (wsum(cnt) << 4);
+  return cbp | (wsum(q == 0 && coded ? (uint32_t)__popcll(m) : 0u) << 4);
 }
 
-// Chroma residual of pred_u/pred_v (enc.rs:1899 quant_chroma): lanes 0..7 own block
-// (plane = lane / 4, b = lane % 4). Levels into sm.ccoef (raster), DC levels into sm.cdc.
-// Returns, in every lane and per plane: AC present and AC decimation score.
+// Chroma residual of pred_u/pred_v (enc.rs:1899 quant_chroma): lane pair b < 8 owns block b
+// (plane = b / 4); the other lanes repeat them. Levels into sm.ccoef (raster), DC levels into sm.cdc.
+// Returns, in every lane and per plane: AC present, AC decimation score, and any DC level.
 struct ChromaAc {
-  uint32_t w;  // byte p: the score of plane p (at most 4 x 45); bits 16, 17: AC present
+  uint32_t w;  // byte p: the score of plane p (at most 4 x 45); bits 16, 17: AC present; bit 18: DC present
   __device__ __forceinline__ bool any(int p) const { return (w >> (16 + p)) & 1u; }
   __device__ __forceinline__ uint32_t score(int p) const { return (w >> (8 * p)) & 255u; }
+  __device__ __forceinline__ bool dc() const { return (w >> 18) & 1u; }
 };
 __device__ __noinline__ ChromaAc chroma_quant(int qpc, bool intra) {
-  int lane = lane_id();
-  uint32_t shift, bias;
+  const int lane = lane_id(), h = lane & 1, b = (lane >> 1) & 7, off = blk_off8(b);
+  uint32_t shift, bias, even, odd;
   quant4_params(qpc, intra, shift, bias);
-  const uint32_t mine = quant4x4_blocks(true, 8, 1, qpc, shift, bias);
-  int ac = mine & 1, big = (mine >> 1) & 1, sc = mine >> 2;
-  uint32_t my_ac = lane < 8 ? (uint32_t)ac : 0u;
-  uint32_t my_score = lane < 8 ? (big ? 9u : (uint32_t)sc) : 0u;  // decimate_score's |level| > 1 rule
-  __syncwarp();
-  // 2x2 DC transform + quantisation (enc.rs:1938 quant_chroma_dc; f = 2^qbits / 3 always)
-  if (lane == 0 || lane == 4) {
-    int d0 = sm.cdcraw[lane], d1 = sm.cdcraw[lane + 1], d2 = sm.cdcraw[lane + 2], d3 = sm.cdcraw[lane + 3];
-    int had[4] = {d0 + d1 + d2 + d3, d0 - d1 + d2 - d3, d0 + d1 - d2 - d3, d0 - d1 - d2 + d3};
-    int qbits = 16 + qpc / 6, mf = c_mf4[qpc % 6][0], f = (1 << qbits) / 3;
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      int a = had[i] < 0 ? -had[i] : had[i];
-      int l = (a * mf + f) >> qbits;
-      sm.cdc[lane + i] = (int16_t)(had[i] < 0 ? -l : l);
-    }
+  const int rem = qpc % 6;
+  const uint32_t mf0 = c_mf4[rem][0];
+  half_scales(mf0, c_mf4[rem][1], c_mf4[rem][2], h, even, odd);
+  Half4 v = half_diff(half_rows((int)offsetof(Smem, src_u) + off, 8, h), half_rows((int)offsetof(Smem, pred_u) + off, 8, h));
+  half_fwd(v, h);
+  // 2x2 DC transform + quantisation (enc.rs:1938 quant_chroma_dc; f = 2^qbits / 3 always); block b & 3
+  // of the plane ends with output b & 3
+  int dc = v.a[0];
+  {
+    int o = __shfl_xor_sync(FULL, dc, 2);
+    dc = (b & 1) ? o - dc : dc + o;
+    o = __shfl_xor_sync(FULL, dc, 4);
+    dc = (b & 2) ? o - dc : dc + o;
+    const int qbits = 16 + qpc / 6, f = (1 << qbits) / 3;
+    const int l = (abs(dc) * (int)mf0 + f) >> qbits;
+    dc = dc < 0 ? -l : l;
   }
-  uint32_t pa = my_ac | __shfl_xor_sync(FULL, my_ac, 1);
-  pa |= __shfl_xor_sync(FULL, pa, 2);
-  uint32_t ps = my_score + __shfl_xor_sync(FULL, my_score, 1);
-  ps += __shfl_xor_sync(FULL, ps, 2);
-  const uint32_t both = ps | (pa << 16);
-  const uint32_t u = __shfl_sync(FULL, both, 0), v = __shfl_sync(FULL, both, 4);
+  const uint32_t m = half_quant(v, h, 1, even, odd, bias, shift);
+  if (lane < 16) {
+    *(uint2*)&sm.ccoef[b * 16 + h * 4] = pack_half(v.a);
+    *(uint2*)&sm.ccoef[b * 16 + h * 4 + 8] = pack_half(v.b);
+    if (!h) sm.cdc[b] = (int16_t)dc;
+  }
+  const bool dcany = __ballot_sync(FULL, !h && dc != 0) != 0;
+  // a plane's score (9 for a block with a level above 1) and AC count over its four blocks
+  uint32_t g = ((m >> 16) ? 9u : score4(m, 1)) | ((m & 0xffffu) ? 1u << 16 : 0u);
+  g += __shfl_xor_sync(FULL, g, 2);
+  g += __shfl_xor_sync(FULL, g, 4);
+  const uint32_t u = __shfl_sync(FULL, g, 0), w = __shfl_sync(FULL, g, 8);
   __syncwarp();
-  return ChromaAc{(u & 0x100ffu) | ((v & 0xffu) << 8) | ((v & 0x10000u) << 1)};
-}
-__device__ __forceinline__ bool chroma_dc_any() {
-  bool a = false;
-#pragma unroll
-  for (int i = 0; i < 8; i++) a |= sm.cdc[i] != 0;
-  return a;
+  return ChromaAc{(u & 0xffu) | ((w & 0xffu) << 8) | ((u >> 16) ? 1u << 16 : 0u) | ((w >> 16) ? 1u << 17 : 0u) |
+                  (dcany ? 1u << 18 : 0u)};
 }
 
 // Adds the dequantised chroma residual to pred_u / pred_v (enc.rs:1992 recon_chroma): the DC of
 // each block from the 2x2 inverse (h264.rs:1674 dequantize_idct_chroma_dc2x2), its AC dequantised
-// when cbpc == 2, then the inverse core transform. Lane = coefficient, two blocks per step.
+// when cbpc == 2, then the inverse core transform. Two lanes per block as in chroma_quant.
 __device__ __noinline__ void chroma_recon(int qpc, int cbpc) {
   if (cbpc == 0) return;
-  int lane = lane_id(), p = lane & 15, h = lane >> 4, xl = p & 3, yl = p >> 2;
-  int qmul = (c_dq4[qpc % 6][0] * 16) << (qpc / 6 + 2);
-  int dqs = (int)c_dq4[qpc % 6][pos4(p)] << (qpc / 6);
-#pragma unroll 1
-  for (int it = 0; it < 4; it++) {
-    int b = 2 * it + h, pl = b >> 2, bb = b & 3;
-    int a = sm.cdc[pl * 4], bv = sm.cdc[pl * 4 + 1], c = sm.cdc[pl * 4 + 2], d = sm.cdc[pl * 4 + 3];
-    int e = a - bv, apb = a + bv, cmd = c - d, cpd = c + d;
-    int dcv = bb == 0 ? apb + cpd : (bb == 1 ? e + cmd : (bb == 2 ? apb - cpd : e - cmd));
-    int v = p == 0 ? (int)(int16_t)((dcv * qmul) >> 7)
-                   : (cbpc >= 2 ? (int)clamp_i16((int)sm.ccoef[b * 16 + p] * dqs) : 0);
-    int r = (int16_t)((inv4_pass(inv4_pass(v, 1, xl), 4, yl) + 32) >> 6);
-    uint8_t* pr = (pl ? sm.pred_v : sm.pred_u) + (bb >> 1) * 32 + (bb & 1) * 4 + yl * 8 + xl;
-    *pr = (uint8_t)clip255(*pr + r);
+  const int lane = lane_id(), h = lane & 1, b = (lane >> 1) & 7, bb = b & 3, off = blk_off8(b) + (int)offsetof(Smem, pred_u);
+  const int rem = qpc % 6, qdiv = qpc / 6, qmul = (c_dq4[rem][0] * 16) << (qdiv + 2);
+  uint32_t even, odd;
+  half_scales(c_dq4[rem][0], c_dq4[rem][1], c_dq4[rem][2], h, even, odd);
+  int lv[4];
+  unpack_half(*(const uint2*)&sm.cdc[b & 4], lv);
+  const int e = lv[0] - lv[1], apb = lv[0] + lv[1], cmd = lv[2] - lv[3], cpd = lv[2] + lv[3];
+  const int dcv = bb == 0 ? apb + cpd : (bb == 1 ? e + cmd : (bb == 2 ? apb - cpd : e - cmd));
+  Half4 v;
+  unpack_half(*(const uint2*)&sm.ccoef[b * 16 + h * 4], v.a);
+  unpack_half(*(const uint2*)&sm.ccoef[b * 16 + h * 4 + 8], v.b);
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const int dq = (int)((k & 1) ? odd : even) << qdiv;
+    v.a[k] = cbpc >= 2 ? (int)clamp_i16(v.a[k] * dq) : 0;
+    v.b[k] = cbpc >= 2 ? (int)clamp_i16(v.b[k] * dq) : 0;
+  }
+  if (!h) v.a[0] = (int16_t)((dcv * qmul) >> 7);
+  half_inv(v, h);
+  const uint2 p = half_rows(off, 8, h);
+  if (lane < 16) {
+    *(uint32_t*)sm_at(off + h * 8) = add_clip4(p.x, v.a);
+    *(uint32_t*)sm_at(off + (3 - h) * 8) = add_clip4(p.y, v.b);
   }
   __syncwarp();
 }
@@ -685,69 +768,56 @@ __device__ __noinline__ void chroma_recon(int qpc, int cbpc) {
 // Raster position of each 4x4 zig-zag index, 4 bits per index (frame scan, Table 8-12).
 constexpr unsigned long long kScan4Packed = 0xfeb7adc963258410ull;
 
-// The 1-D inverse 8x8 transform in place on sm.t8[at], [at + stride], ..., [at + 7 * stride] (rows and columns
-// of the 8x8 reconstruction share it).
-__device__ __noinline__ void idct8_inplace(int at, int stride) {
-  int* p = &sm.t8[at];
-  int d[8], o[8];
-#pragma unroll
-  for (int k = 0; k < 8; k++) d[k] = p[k * stride];
-  idct8_1d(d, o);
-#pragma unroll
-  for (int k = 0; k < 8; k++) p[k * stride] = o[k];
-}
-
 // Adds the dequantised 8x8 residual of the coded blocks of sm.coef8 to pred_y (enc.rs:2013
 // recon_8x8: dequantize_block8x8, h264.rs:1403, then h264_idct8_add, h264_idct.rs:207).
-// Lanes 8b..8b+7 own block b: row q, then column q.
+// Lanes 8b..8b+7 own block b: row q, then column q. Blocks that are not coded add zero.
 __device__ __noinline__ void recon_luma8x8(int qp, int cbp) {
-  int lane = lane_id(), b = lane >> 3, q = lane & 7;
-  bool coded = (cbp >> b) & 1;
-  int qdiv = qp / 6, rem = qp % 6;
-  int dq6[6];
+  const int lane = lane_id(), b = lane >> 3, q = lane & 7;
+  const bool coded = (cbp >> b) & 1;
+  const int qdiv = qp / 6;
+  const Scale8 dq = scale8(c_dq8[qp % 6], q);
+  int d[8], o[8];
 #pragma unroll
-  for (int k = 0; k < 6; k++) dq6[k] = c_dq8[rem][k];
-  if (coded) {
-#pragma unroll 1
-    for (int x = 0; x < 8; x++) {
-      int i = q * 8 + x, cls = pos8(i);
-      int v = cls == 0 ? dq6[0] : cls == 1 ? dq6[1] : cls == 2 ? dq6[2] : cls == 3 ? dq6[3] : cls == 4 ? dq6[4] : dq6[5];
-      int l = sm.coef8[b * 64 + i];
-      int dv = qdiv >= 2 ? l * (v << (qdiv - 2)) : ((l * v + (1 << (1 - qdiv))) >> (2 - qdiv));
-      sm.t8[b * 64 + i] = clamp_i16(dv);
-    }
-    idct8_inplace(b * 64 + q * 8, 1);
+  for (int x = 0; x < 8; x++) {
+    const int l = coded ? sm.coef8[b * 64 + sm.zz8[x * 8 + q]] : 0, v = dq.at(x);
+    const int dv = qdiv >= 2 ? l * (v << (qdiv - 2)) : ((l * v + (1 << (1 - qdiv))) >> (2 - qdiv));
+    d[x] = clamp_i16(dv);
   }
+  idct8_1d(d, o);
+  t8_store_row(b * kT8Block + q * 8, o);
   __syncwarp();
-  if (coded) {
-    idct8_inplace(b * 64 + q, 8);
-    int bx = (b & 1) * 8, by = (b >> 1) * 8;
-#pragma unroll 1
-    for (int y = 0; y < 8; y++) {
-      int off = (by + y) * 16 + bx + q;
-      int v = (int)((unsigned)sm.t8[b * 64 + y * 8 + q] + 32u) >> 6;
-      sm.pred_y[off] = (uint8_t)clip255((int)((unsigned)sm.pred_y[off] + (unsigned)v));
-    }
+#pragma unroll
+  for (int y = 0; y < 8; y++) d[y] = sm.t8[b * kT8Block + y * 8 + q];
+  idct8_1d(d, o);
+  uint8_t* px = &sm.pred_y[(b >> 1) * 128 + (b & 1) * 8 + q];
+#pragma unroll
+  for (int y = 0; y < 8; y++) {
+    const int v = (int)((unsigned)o[y] + 32u) >> 6;
+    px[y * 16] = (uint8_t)clip255((int)((unsigned)px[y * 16] + (unsigned)v));
   }
   __syncwarp();
 }
 
-// Adds the dequantised luma 4x4 residual of the coded 8x8 groups of sm.coef to pred_y
-// (enc.rs:1978 recon_luma_4x4). Lane = coefficient, two blocks per step.
-__device__ __noinline__ void recon_luma4x4(int qp, int cbp) {
-  int lane = lane_id(), p = lane & 15, h = lane >> 4, xl = p & 3, yl = p >> 2;
-  int dqs = (int)c_dq4[qp % 6][pos4(p)] << (qp / 6);
-#pragma unroll 1
-  for (int it = 0; it < 8; it++) {
-    int b = 2 * it + h;
-    bool coded = (cbp >> (b >> 2)) & 1;
-    int v = coded ? (int)clamp_i16((int)sm.coef[b * 16 + p] * dqs) : 0;
-    int r = (int16_t)((inv4_pass(inv4_pass(v, 1, xl), 4, yl) + 32) >> 6);
-    if (coded) {
-      int o = (blk_y(b) * 4 + yl) * 16 + blk_x(b) * 4 + xl;
-      sm.pred_y[o] = (uint8_t)clip255(sm.pred_y[o] + r);
-    }
+// Adds the dequantised luma 4x4 residual of sm.coef to pred_y (enc.rs:1978 recon_luma_4x4; blocks
+// without levels add zero), two lanes per block.
+__device__ __noinline__ void recon_luma4x4(int qp) {
+  const int lane = lane_id(), b = lane >> 1, h = lane & 1, off = blk_off16(b) + (int)offsetof(Smem, pred_y);
+  const int rem = qp % 6, qdiv = qp / 6;
+  uint32_t even, odd;
+  half_scales(c_dq4[rem][0], c_dq4[rem][1], c_dq4[rem][2], h, even, odd);
+  Half4 v;
+  unpack_half(*(const uint2*)&sm.coef[b * 16 + h * 4], v.a);
+  unpack_half(*(const uint2*)&sm.coef[b * 16 + h * 4 + 8], v.b);
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const int dq = (int)((k & 1) ? odd : even) << qdiv;
+    v.a[k] = clamp_i16(v.a[k] * dq);
+    v.b[k] = clamp_i16(v.b[k] * dq);
   }
+  half_inv(v, h);
+  const uint2 p = half_rows(off, 16, h);
+  *(uint32_t*)sm_at(off + h * 16) = add_clip4(p.x, v.a);
+  *(uint32_t*)sm_at(off + (3 - h) * 16) = add_clip4(p.y, v.b);
   __syncwarp();
 }
 
@@ -855,12 +925,7 @@ __device__ __noinline__ I16Fit analyse_i16(bool ht, bool hl, int tl) {
   if (hl && sh < best) { best = sh; mode = 1; }
   if (ht && hl) {
     pred16_into(3, (int)offsetof(Smem, tmp_y), ht, hl, tl);
-    uint32_t s = 0;
-    if (lane < 16) {
-      int bx = lane & 3, by = lane >> 2;
-      s = satd4((int)offsetof(Smem, src_y) + by * 64 + bx * 4, (int)offsetof(Smem, tmp_y) + by * 64 + bx * 4);
-    }
-    s = wsum(s) >> 1;
+    const uint32_t s = satd16((int)offsetof(Smem, tmp_y));
     if (s < best) { best = s; mode = 3; }
   }
   return I16Fit{mode, best};
@@ -1047,80 +1112,65 @@ __device__ __noinline__ void store_recon(const Ctx c, int ly) {
   }
 }
 
-// Writes the chroma part of the record (chroma levels in zig-zag) and clears the rest.
-// The chroma levels of the record, a word (two zig-zag levels) per lane and store: word w of the
-// AC levels holds slots 2 (w & 7), 2 (w & 7) + 1 of block w / 8 (plane * 4 + block); slot 0 (the
-// DC position) stays 0. Lanes 0..3 write the DC levels.
+// The record is written by 32-bit words, a word per lane and store (it is 8-byte aligned at best, so
+// no wider): words 0..8 the head, 9..136 the luma levels, 137..144 the Intra16x16 DC levels, 145..148
+// and 149..212 the chroma levels.
+constexpr int kWordLuma = offsetof(rg_mb_out, luma) / 4, kWordLumaDc = offsetof(rg_mb_out, luma_dc) / 4,
+              kWordChromaDc = offsetof(rg_mb_out, chroma_dc) / 4, kWordChromaAc = offsetof(rg_mb_out, chroma_ac) / 4,
+              kWordParts = offsetof(rg_mb_out, part_mv) / 4;
+static_assert(kWordLuma == 9 && offsetof(rg_mb_out, mv) == 8 && offsetof(rg_mb_out, mvd) == 12 &&
+                  offsetof(rg_mb_out, i4_modes) == 16 && offsetof(rg_mb_out, nz_mask) == 32,
+              "the head's words");
+__device__ __forceinline__ uint32_t pack16(int lo, int hi) { return __byte_perm((uint32_t)lo, (uint32_t)hi, 0x5410); }
+// The chroma levels of the record (zig-zag): word w of the AC levels holds slots 2 (w & 7), 2 (w & 7)
+// + 1 of block w / 8 (plane * 4 + block); slot 0 (the DC position) stays 0.
 __device__ __noinline__ void record_chroma(rg_mb_out* rec, int cbpc) {
-  int lane = lane_id();
-#pragma unroll 1
-  for (int k = 0; k < 2; k++) {
-    int w = lane + 32 * k, blk = w >> 3, i = (w & 7) * 2;
-    int r0 = (int)((kScan4Packed >> (4 * i)) & 15), r1 = (int)((kScan4Packed >> (4 * i + 4)) & 15);
-    int16_t v0 = (i && cbpc >= 2) ? sm.ccoef[blk * 16 + r0] : 0, v1 = cbpc >= 2 ? sm.ccoef[blk * 16 + r1] : 0;
-    ((uint32_t*)rec->chroma_ac)[w] = (uint32_t)(uint16_t)v0 | ((uint32_t)(uint16_t)v1 << 16);
-  }
-  if (lane < 4) {
-    int16_t d0 = cbpc >= 1 ? sm.cdc[2 * lane] : 0, d1 = cbpc >= 1 ? sm.cdc[2 * lane + 1] : 0;
-    ((uint32_t*)rec->chroma_dc)[lane] = (uint32_t)(uint16_t)d0 | ((uint32_t)(uint16_t)d1 << 16);
-  }
-}
-// The 4x4 luma levels of the record in zig-zag order, a word per lane and store: word w holds
-// levels 2 (w & 7), 2 (w & 7) + 1 of block w / 8; lanes 8j..8j+7 of step k cover block 4k + j.
-// Returns the blocks holding levels (bit b: block b).
-__device__ __noinline__ uint16_t record_luma4x4(rg_mb_out* rec) {
-  int lane = lane_id();
-  uint32_t nz = 0;
-#pragma unroll 1
-  for (int k = 0; k < 4; k++) {
-    int w = lane + 32 * k, b = w >> 3, i = (w & 7) * 2;
-    int r0 = (int)((kScan4Packed >> (4 * i)) & 15), r1 = (int)((kScan4Packed >> (4 * i + 4)) & 15);
-    int16_t v0 = sm.coef[b * 16 + r0], v1 = sm.coef[b * 16 + r1];
-    ((uint32_t*)rec->luma)[w] = (uint32_t)(uint16_t)v0 | ((uint32_t)(uint16_t)v1 << 16);
-    uint32_t bal = __ballot_sync(FULL, (v0 | v1) != 0);
+  const int lane = lane_id(), i = (lane & 7) * 2;
+  const int r0 = (int)((kScan4Packed >> (4 * i)) & 15), r1 = (int)((kScan4Packed >> (4 * i + 4)) & 15);
+  uint32_t* w = (uint32_t*)rec;
 #pragma unroll
-    for (int j = 0; j < 4; j++)
-      if ((bal >> (8 * j)) & 0xffu) nz |= 1u << (4 * k + j);
+  for (int k = 0; k < 2; k++) {
+    const int blk = (lane >> 3) + 4 * k;
+    const uint32_t v = pack16(i ? sm.ccoef[blk * 16 + r0] : 0, sm.ccoef[blk * 16 + r1]);
+    w[kWordChromaAc + lane + 32 * k] = cbpc >= 2 ? v : 0u;
   }
-  return (uint16_t)nz;
+  if (lane < 4) w[kWordChromaDc + lane] = cbpc >= 1 ? ((const uint32_t*)sm.cdc)[lane] : 0u;
 }
-__device__ __noinline__ void record_header(rg_mb_out* rec, int type, int i16_mode, int cmode, int cbp, int t8, int qp, int mvx, int mvy,
-                              int mvdx, int mvdy, uint16_t nz) {
-  rec->mb_type = (uint8_t)type;
-  rec->i16_mode = (uint8_t)i16_mode;
-  rec->chroma_mode = (uint8_t)cmode;
-  rec->cbp = (uint8_t)cbp;
-  rec->transform_8x8 = (uint8_t)t8;
-  rec->qp = (uint8_t)qp;
-  rec->qp_delta = 0;
-  rec->reserved0 = 0;
-  rec->mv[0] = (int16_t)mvx;
-  rec->mv[1] = (int16_t)mvy;
-  rec->mvd[0] = (int16_t)mvdx;
-  rec->mvd[1] = (int16_t)mvdy;
-  rec->nz_mask = nz;
-  rec->reserved1 = 0;
-}
-__device__ __noinline__ void write_info(const Ctx c, int flags, int cbpl, int mvx, int mvy, int ref, uint16_t nz, bool i4) {
-  MbInfo inf;
-  inf.mv[0] = (int16_t)mvx;
-  inf.mv[1] = (int16_t)mvy;
-  inf.ref = (int8_t)ref;
-  inf.flags = (uint8_t)flags;
-  inf.cbp_luma = (uint8_t)cbpl;
-  inf.qp = (uint8_t)c.sd->qp;
-  inf.nz16 = nz;
-  inf.i4_bottom = 0;
-  inf.i4_right = 0;
+// The 4x4 luma levels of the record in zig-zag order: word w holds levels 2 (w & 7), 2 (w & 7) + 1 of
+// block w / 8.
+__device__ __noinline__ void record_luma4x4(rg_mb_out* rec) {
+  const int lane = lane_id(), i = (lane & 7) * 2;
+  const int r0 = (int)((kScan4Packed >> (4 * i)) & 15), r1 = (int)((kScan4Packed >> (4 * i + 4)) & 15);
+#pragma unroll
   for (int k = 0; k < 4; k++) {
-    // bottom row blocks (x = k, y = 3) and right column blocks (x = 3, y = k), decoding order
-    int bb = ((3 >> 1) << 3) | ((k >> 1) << 2) | ((3 & 1) << 1) | (k & 1);
-    int br = ((k >> 1) << 3) | ((3 >> 1) << 2) | ((k & 1) << 1) | (3 & 1);
-    inf.i4_bottom |= (uint16_t)((i4 ? sm.i4m[bb] : 2) << (4 * k));
-    inf.i4_right |= (uint16_t)((i4 ? sm.i4m[br] : 2) << (4 * k));
+    const int16_t* c = &sm.coef[((lane >> 3) + 4 * k) * 16];
+    ((uint32_t*)rec)[kWordLuma + lane + 32 * k] = pack16(c[r0], c[r1]);
   }
-  inf.pad_ = 0;
-  c.sd->info[c.mb] = inf;
+}
+// The head's words. i4: the modes of sm.i4m, otherwise all DC (2).
+__device__ __noinline__ void record_header(rg_mb_out* rec, int type, int i16_mode, int cmode, int cbp, int t8, int qp, int mvx, int mvy,
+                              int mvdx, int mvdy, uint32_t nz, bool i4) {
+  const int lane = lane_id();
+  uint32_t v = i4 ? ((const uint32_t*)sm.i4m)[lane & 3] : 0x02020202u;  // words 4..7
+  v = lane == 0 ? (uint32_t)(type | (i16_mode << 8) | (cmode << 16) | (cbp << 24)) : v;
+  v = lane == 1 ? (uint32_t)(t8 | (qp << 8)) : v;
+  v = lane == 2 ? pack16(mvx, mvy) : v;
+  v = lane == 3 ? pack16(mvdx, mvdy) : v;
+  v = lane == 8 ? nz : v;
+  if (lane < 9) ((uint32_t*)rec)[lane] = v;
+}
+// What later macroblocks and the deblocking filter read of this one (lane 0 stores it).
+__device__ __forceinline__ void write_info(const Ctx c, int flags, int cbpl, int mvx, int mvy, int ref, uint32_t nz, bool i4) {
+  if (lane_id() != 0) return;
+  uint32_t bottom = 0x2222u, right = 0x2222u;
+  if (i4) {  // bottom row blocks 10, 11, 14, 15 and right column blocks 5, 7, 13, 15 (decoding order)
+    bottom = sm.i4m[10] | (sm.i4m[11] << 4) | (sm.i4m[14] << 8) | (sm.i4m[15] << 12);
+    right = sm.i4m[5] | (sm.i4m[7] << 4) | (sm.i4m[13] << 8) | (sm.i4m[15] << 12);
+  }
+  static_assert(offsetof(MbInfo, ref) == 4 && offsetof(MbInfo, qp) == 7 && offsetof(MbInfo, i4_bottom) == 10 &&
+                    offsetof(MbInfo, i4_right) == 12, "MbInfo packed by words");
+  *(uint4*)(c.sd->info + c.mb) = make_uint4(pack16(mvx, mvy), (uint32_t)(ref & 255) | (flags << 8) | (cbpl << 16) | (c.sd->qp << 24),
+                                            nz | (bottom << 16), right);
 }
 
 // I16x16 coding and reconstruction (enc.rs:3587 code_i16) with prediction mode `mode`.
@@ -1204,20 +1254,15 @@ __device__ __noinline__ void code_i16(const Ctx c, int mode, bool ht, bool hl, C
     }
   }
   const ChromaAc ac = chroma_quant(qpc, true);
-  int cbpc = (ac.any(0) || ac.any(1)) ? 2 : (chroma_dc_any() ? 1 : 0);
+  int cbpc = (ac.any(0) || ac.any(1)) ? 2 : (ac.dc() ? 1 : 0);
   __syncwarp();
   // record
   rg_mb_out* rec = c.sd->rec + c.mb;
-  uint16_t nzm = 0;
-  if (lane < 16) {
-#pragma unroll
-    for (int i = 0; i < 16; i++) rec->luma[lane * 16 + i] = sm.coef[lane * 16 + c_scan4[i]];
-    rec->luma_dc[lane] = sm.ldc[c_scan4[lane]];
-    rec->i4_modes[lane] = 2;
-  }
-  nzm = (uint16_t)__ballot_sync(FULL, lane < 16 && cbpl && my_ac);
+  record_luma4x4(rec);
+  if (lane < 16) rec->luma_dc[lane] = sm.ldc[(kScan4Packed >> (4 * lane)) & 15];
+  const uint32_t nzm = __ballot_sync(FULL, lane < 16 && cbpl && my_ac);
   record_chroma(rec, cbpc);
-  if (lane == 0) record_header(rec, RG_MB_I16X16, mode, cmode, cbpl | (cbpc << 4), 0, qp, 0, 0, 0, 0, nzm);
+  record_header(rec, RG_MB_I16X16, mode, cmode, cbpl | (cbpc << 4), 0, qp, 0, 0, 0, 0, nzm, false);
   // reconstruction
   if (lane < 16) {
     int bx = blk_x(lane), by = blk_y(lane);
@@ -1240,7 +1285,7 @@ __device__ __noinline__ void code_i16(const Ctx c, int mode, bool ht, bool hl, C
   __syncwarp();
   chroma_recon(qpc, cbpc);
   store_recon(c, (int)offsetof(Smem, pred_y));
-  if (lane == 0) write_info(c, kFlagIntra, cbpl, 0, 0, -1, nzm, false);
+  write_info(c, kFlagIntra, cbpl, 0, 0, -1, nzm, false);
 }
 
 // I4x4 analysis (enc.rs:3336 analyse_i4): sixteen blocks in decoding order, each choosing among
@@ -1248,7 +1293,8 @@ __device__ __noinline__ void code_i16(const Ctx c, int mode, bool ht, bool hl, C
 // reconstructing before the next block. Per block the warp gathers the edge samples (lane k ->
 // Q[k]), builds all nine predictions (lane -> pixel, the two half-warps taking even / odd modes),
 // costs the modes (lane -> mode), and transforms the chosen residual with shuffles (lane ->
-// coefficient). Returns the luma coded block pattern, or -1 as soon as the running cost reaches `budget`.
+// coefficient). Returns the luma coded block pattern with the blocks
+// holding levels in bits 4.. (bit 4 + b: block b), or -1 as soon as the running cost reaches `budget`.
 // kMask: only the modes of masks[b] (bit m: Intra4x4PredMode m) that are available at block b are
 // tried -- DC alone when none is (the learned form); the plain form tries every available mode.
 template <bool kMask>
@@ -1366,7 +1412,7 @@ __device__ __noinline__ int analyse_i4(const Ctx c, uint32_t budget, bool ht_mb,
     int lvl = acc < 0 ? -l : l;
     if (lane < 16) sm.coef[b * 16 + p] = (int16_t)lvl;
     bool nz = __ballot_sync(FULL, lane < 16 && lvl != 0) != 0;
-    if (nz) cbpl |= 1 << (b >> 2);
+    if (nz) cbpl |= (1 << (b >> 2)) | (16 << b);
     // inverse transform (rows then columns) and reconstruction
     int rec = pred;
     if (nz) {
@@ -1380,23 +1426,23 @@ __device__ __noinline__ int analyse_i4(const Ctx c, uint32_t budget, bool ht_mb,
   return cbpl;
 }
 
-__device__ __noinline__ void code_i4(const Ctx c, int cbpl, bool ht, bool hl, Corner k0) {
+// `luma`: what analyse_i4 returned.
+__device__ __noinline__ void code_i4(const Ctx c, int luma, bool ht, bool hl, Corner k0) {
   int lane = lane_id();
   int qpc = c.sd->qpc;
+  const int cbpl = luma & 15;
+  const uint32_t nzm = (uint32_t)luma >> 4;
   int cmode = analyse_chroma(ht, hl, k0);
   const ChromaAc ac = chroma_quant(qpc, true);
-  int cbpc = (ac.any(0) || ac.any(1)) ? 2 : (chroma_dc_any() ? 1 : 0);
+  int cbpc = (ac.any(0) || ac.any(1)) ? 2 : (ac.dc() ? 1 : 0);
   rg_mb_out* rec = c.sd->rec + c.mb;
-  uint16_t nzm = record_luma4x4(rec);
-  if (lane < 16) {
-    rec->luma_dc[lane] = 0;
-    rec->i4_modes[lane] = sm.i4m[lane];
-  }
+  record_luma4x4(rec);
+  if (lane < 8) ((uint32_t*)rec)[kWordLumaDc + lane] = 0u;
   record_chroma(rec, cbpc);
-  if (lane == 0) record_header(rec, RG_MB_I4X4, 0, cmode, cbpl | (cbpc << 4), 0, c.sd->qp, 0, 0, 0, 0, nzm);
+  record_header(rec, RG_MB_I4X4, 0, cmode, cbpl | (cbpc << 4), 0, c.sd->qp, 0, 0, 0, 0, nzm, true);
   chroma_recon(qpc, cbpc);
   store_recon(c, (int)offsetof(Smem, tmp_y));
-  if (lane == 0) write_info(c, kFlagIntra, cbpl, 0, 0, -1, nzm, true);
+  write_info(c, kFlagIntra, cbpl, 0, 0, -1, nzm, true);
 }
 
 // One macroblock of an I slice (enc.rs:3311 code_intra).
@@ -1417,37 +1463,69 @@ __device__ __noinline__ void analyse_intra_mb(const Ctx c) {
 
 // Codes P_Skip with vector mv; prediction already in pred_y / pred_u / pred_v.
 __device__ __noinline__ void code_skip(const Ctx c, int mvx, int mvy) {
-  int lane = lane_id();
+  const int lane = lane_id();
   rg_mb_out* rec = c.sd->rec + c.mb;
-  if (lane < 16) {
 #pragma unroll
-    for (int i = 0; i < 16; i++) rec->luma[lane * 16 + i] = 0;
-    rec->luma_dc[lane] = 0;
-    rec->i4_modes[lane] = 2;
-  }
-  if (lane < 8) {
-#pragma unroll
-    for (int i = 0; i < 16; i++) rec->chroma_ac[lane >> 2][lane & 3][i] = 0;
-    rec->chroma_dc[lane >> 2][lane & 3] = 0;
-  }
-  if (lane == 0) {
-    record_header(rec, RG_MB_P_SKIP, 0, 0, 0, 0, c.sd->qp, mvx, mvy, 0, 0, 0);
-    write_info(c, kFlagSkip, 0, mvx, mvy, 0, 0, false);
-  }
+  for (int k = 0; k < 7; k++)
+    if (kWordLuma + lane + 32 * k < kWordParts) ((uint32_t*)rec)[kWordLuma + lane + 32 * k] = 0u;
+  record_header(rec, RG_MB_P_SKIP, 0, 0, 0, 0, c.sd->qp, mvx, mvy, 0, 0, 0, false);
+  write_info(c, kFlagSkip, 0, mvx, mvy, 0, 0, false);
   store_recon(c, (int)offsetof(Smem, pred_y));
 }
 
 // Probe of the skip residual (enc.rs:2163 probe_skip_luma): no level above 1 and a total
 // decimation score below 6.
 __device__ __noinline__ bool probe_skip_luma(int qp) {
-  int lane = lane_id();
-  uint32_t shift, bias;
-  quant4_params(qp, false, shift, bias);
-  // levels go to sm.coef as scratch: a skipped macroblock records none
-  const uint32_t mine = quant4x4_blocks(false, 16, 0, qp, shift, bias);
-  uint32_t b = wor(lane < 16 ? mine & 2u : 0u);
-  uint32_t score = wsum(lane < 16 ? mine >> 2 : 0u);
-  return !b && score < 6;
+  Half4 v;
+  const uint32_t m = luma4x4_levels(qp, v);
+  const uint32_t score = (lane_id() & 1) ? 0u : score4(m, 0);
+  return wsum(score | ((m >> 16) << 16)) < 6;
+}
+
+// The residual of an inter macroblock whose prediction lies in pred_y / pred_u / pred_v
+// (enc.rs:3158-3190), its record (code_inter, enc.rs:3196) and its reconstruction. can_skip: nothing
+// coded makes it P_Skip with vector (mvx, mvy). Returns whether it did.
+__device__ __noinline__ bool code_inter(const Ctx c, int type, bool can_skip, int mvx, int mvy, int mvdx, int mvdy) {
+  const int lane = lane_id(), qp = c.sd->qp, qpc = c.sd->qpc;
+  const Luma4 l4 = luma4x4_inter(qp);
+  uint32_t cbpl = l4.cbp;
+  bool use8 = false;
+  if (c.fp->t8x8 && l4.cbp) {
+    const uint32_t r8 = luma8x8_inter(qp);
+    if ((r8 >> 4) <= l4.nnz) { use8 = true; cbpl = r8 & 15u; }
+  }
+  const ChromaAc ac = chroma_quant(qpc, false);
+  // drop a plane's AC levels when nearly empty (enc.rs:2095)
+  const bool drop_u = ac.any(0) && ac.score(0) < 7, drop_v = ac.any(1) && ac.score(1) < 7;
+  if ((lane & 16) ? drop_v : drop_u) *(uint2*)&sm.ccoef[lane * 4] = make_uint2(0u, 0u);
+  __syncwarp();
+  const bool acu = ac.any(0) && !drop_u, acv = ac.any(1) && !drop_v;
+  const int cbpc = (acu || acv) ? 2 : (ac.dc() ? 1 : 0);
+  if (cbpl == 0 && cbpc == 0 && can_skip) {
+    code_skip(c, mvx, mvy);
+    return true;
+  }
+  rg_mb_out* rec = c.sd->rec + c.mb;
+  const bool t8flag = use8 && cbpl != 0;
+  uint32_t nzm = l4.nz16;
+  if (use8) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) ((uint32_t*)rec)[kWordLuma + lane + 32 * k] = ((const uint32_t*)sm.coef8)[lane + 32 * k];
+    nzm = (cbpl & 1u ? 0xfu : 0u) | (cbpl & 2u ? 0xf0u : 0u) | (cbpl & 4u ? 0xf00u : 0u) | (cbpl & 8u ? 0xf000u : 0u);
+  } else {
+    record_luma4x4(rec);
+  }
+  if (lane < 8) ((uint32_t*)rec)[kWordLumaDc + lane] = 0u;
+  record_chroma(rec, cbpc);
+  record_header(rec, type, 0, 0, (int)cbpl | (cbpc << 4), t8flag, qp, mvx, mvy, mvdx, mvdy, nzm, false);
+  write_info(c, t8flag ? kFlagT8 : 0, (int)cbpl, mvx, mvy, 0, nzm, false);
+  if (cbpl) {
+    if (use8) recon_luma8x8(qp, (int)cbpl);
+    else recon_luma4x4(qp);
+  }
+  chroma_recon(qpc, cbpc);
+  store_recon(c, (int)offsetof(Smem, pred_y));
+  return false;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1645,7 +1723,7 @@ __device__ __noinline__ void analyse_p_mb(const Ctx c, PipeWait* pw) {
         bool cz = zu && zv;
         if (!cz) {
           const ChromaAc ac = chroma_quant(qpc, false);
-          cz = !chroma_dc_any() && ac.score(0) < 7 && ac.score(1) < 7;
+          cz = !ac.dc() && ac.score(0) < 7 && ac.score(1) < 7;
         }
         if (cz) {
           code_skip(c, ps0, ps1);
@@ -1764,12 +1842,7 @@ __device__ __noinline__ void analyse_p_mb(const Ctx c, PipeWait* pw) {
   }
 
   // 3. intra 16x16 when the inter prediction is poor (enc.rs:3121-3156)
-  uint32_t inter_satd = 0;
-  if (lane < 16) {
-    int bx = lane & 3, by = lane >> 2;
-    inter_satd = satd4((int)offsetof(Smem, src_y) + by * 64 + bx * 4, (int)offsetof(Smem, pred_y) + by * 64 + bx * 4);
-  }
-  inter_satd = wsum(inter_satd) >> 1;
+  const uint32_t inter_satd = satd16((int)offsetof(Smem, pred_y));
   uint32_t inter_cost = inter_satd + lambda * (se_bits(mv0 - mvp0) + se_bits(mv1 - mvp1) + 1);
   if (inter_satd > 24 * lambda) {
     const Corner k0 = load_edges(c, false);
@@ -1781,66 +1854,9 @@ __device__ __noinline__ void analyse_p_mb(const Ctx c, PipeWait* pw) {
     }
   }
 
-  // 4. P_L0_16x16 residual (enc.rs:3158-3190)
+  // 4. P_L0_16x16 residual, record and reconstruction
   mc_chroma8(sd.ref_u, sd.ref_v, fp.stride_c, mbx, mby, mv0, mv1);
-  int cbp4 = luma4x4_inter(qp);
-  int cbpl = cbp4;
-  bool use8 = false;
-  if (fp.t8x8 && cbp4) {
-    uint32_t nnz4 = 0;  // nonzero levels of the 4x4 coding: four words (eight levels) per lane
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      uint32_t w = ((const uint32_t*)sm.coef)[lane + 32 * k];
-      nnz4 += ((w & 0xffffu) != 0) + ((w >> 16) != 0);
-    }
-    nnz4 = wsum(nnz4);
-    const uint32_t r8 = luma8x8_inter(qp);
-    if ((r8 >> 4) <= nnz4) { use8 = true; cbpl = (int)(r8 & 15u); }
-  }
-  const ChromaAc ac = chroma_quant(qpc, false);
-  // drop a plane's AC levels when nearly empty (enc.rs:2095)
-  bool drop_u = ac.any(0) && ac.score(0) < 7, drop_v = ac.any(1) && ac.score(1) < 7;
-  if (lane < 8) {
-    bool d = (lane >> 2) ? drop_v : drop_u;
-    if (d)
-#pragma unroll
-      for (int i = 0; i < 16; i++) sm.ccoef[lane * 16 + i] = 0;
-  }
-  __syncwarp();
-  bool acu = ac.any(0) && !drop_u, acv = ac.any(1) && !drop_v;
-  int cbpc = (acu || acv) ? 2 : (chroma_dc_any() ? 1 : 0);
-  if (cbpl == 0 && cbpc == 0 && mv0 == ps0 && mv1 == ps1) {
-    code_skip(c, mv0, mv1);
-    return;
-  }
-  // code_inter (enc.rs:3196)
-  rg_mb_out* rec = c.sd->rec + c.mb;
-  bool t8flag = use8 && cbpl != 0;
-  uint16_t nzm;
-  if (use8) {
-    int b = lane >> 3, q = lane & 7;  // column q of block b, each level to its zig-zag slot
-#pragma unroll 1
-    for (int y = 0; y < 8; y++) rec->luma[b * 64 + zigzag8(y, q)] = sm.coef8[b * 64 + y * 8 + q];
-    nzm = 0;
-    for (int k = 0; k < 4; k++) if ((cbpl >> k) & 1) nzm |= (uint16_t)(0xF << (4 * k));
-  } else {
-    nzm = record_luma4x4(rec);
-  }
-  if (lane < 16) { rec->luma_dc[lane] = 0; rec->i4_modes[lane] = 2; }
-  record_chroma(rec, cbpc);
-  if (lane == 0) {
-    record_header(rec, RG_MB_P_L0_16X16, 0, 0, cbpl | (cbpc << 4), t8flag, qp, mv0, mv1, mv0 - mvp0, mv1 - mvp1, nzm);
-    write_info(c, t8flag ? kFlagT8 : 0, cbpl, mv0, mv1, 0, nzm, false);
-  }
-  // reconstruction
-  if (use8) {
-    recon_luma8x8(qp, cbpl);
-  } else if (cbpl) {
-    recon_luma4x4(qp, cbpl);
-  }
-  __syncwarp();
-  chroma_recon(qpc, cbpc);
-  store_recon(c, (int)offsetof(Smem, pred_y));
+  code_inter(c, RG_MB_P_L0_16X16, mv0 == ps0 && mv1 == ps1, mv0, mv1, mv0 - mvp0, mv1 - mvp1);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -2067,6 +2083,7 @@ __device__ __forceinline__ int diag_len(const FrameParams& fp, int d) {
 
 template <int kForm>
 __global__ void __launch_bounds__(32) wavefront_step_kernel(const __grid_constant__ FrameParams fp, const StreamDev* __restrict__ streams, int step) {
+  init_tables();
   const StreamDev& sd = streams[blockIdx.y];
   int na = diag_len(fp, step);
   int nd = fp.deblock ? diag_len(fp, step - 3) : 0;
@@ -2275,6 +2292,7 @@ __global__ void __launch_bounds__(32, 16) pipeline_kernel(const __grid_constant_
     int k = blockIdx.x % 9;
     role = k == 0 ? 1 : (k == 1 ? 2 : 0);
   }
+  init_tables();
   bool empty[3] = {pp.qbeg[0] >= pp.qend[0], pp.qbeg[1] >= pp.qend[1], pp.qbeg[2] >= pp.qend[2]};
   int reach_y = 0, reach_x = 0;  // this warp's, published once as it exits
   while (true) {

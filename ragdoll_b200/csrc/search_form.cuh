@@ -539,7 +539,7 @@ __device__ __noinline__ bool skip_probe(const Ctx c, int ps0, int ps1, const Bou
   bool cz = (sad_u <= sd.sb_chroma || ssd_u <= sd.sb_chroma_ssd) && (sad_v <= sd.sb_chroma || ssd_v <= sd.sb_chroma_ssd);
   if (!cz) {
     const ChromaAc ac = chroma_quant(sd.qpc, false);
-    cz = !chroma_dc_any() && ac.score(0) < 7 && ac.score(1) < 7;
+    cz = !ac.dc() && ac.score(0) < 7 && ac.score(1) < 7;
   }
   return cz;
 }
@@ -591,7 +591,7 @@ __device__ __noinline__ void analyse_p_mb_search(const Ctx c, PipeWait* pw) {
   const int lane = lane_id();
   const int mbx = c.mbx, mby = c.mby;
   const int x0 = mbx * 16, y0 = mby * 16;
-  const int qp = sd.qp, qpc = sd.qpc;
+  const int qp = sd.qp;
   const uint32_t lambda = c_lambda[qp];
   const int cw = fp.mb_w * 16, chh = fp.mb_h * 16;
   Bounds bd;
@@ -741,12 +741,7 @@ __device__ __noinline__ void analyse_p_mb_search(const Ctx c, PipeWait* pw) {
     }
   }
   // 5. intra 16x16 when the inter prediction is poor (the plain form's rule, enc.rs:3121-3156)
-  uint32_t inter_satd = 0;
-  if (lane < 16) {
-    int bx = lane & 3, by = lane >> 2;
-    inter_satd = satd4((int)offsetof(Smem, src_y) + by * 64 + bx * 4, (int)offsetof(Smem, pred_y) + by * 64 + bx * 4);
-  }
-  inter_satd = wsum(inter_satd) >> 1;
+  const uint32_t inter_satd = satd16((int)offsetof(Smem, pred_y));
   if (inter_satd > 24 * lambda) {
     const Corner k0 = load_edges(c, false);
     bool ht = mby > 0, hl = mbx > 0;
@@ -757,64 +752,12 @@ __device__ __noinline__ void analyse_p_mb_search(const Ctx c, PipeWait* pw) {
       return;
     }
   }
-  // residual (enc.rs:3158-3190)
+  // residual, late skip (a 16x16 macroblock at the skip vector), record and reconstruction
   mc_chroma_q(c);
-  int cbp4 = luma4x4_inter(qp);
-  int cbpl = cbp4;
-  bool use8 = false;
-  if (fp.t8x8 && cbp4) {
-    uint32_t nnz4 = 0;
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      uint32_t w = ((const uint32_t*)sm.coef)[lane + 32 * k];
-      nnz4 += ((w & 0xffffu) != 0) + ((w >> 16) != 0);
-    }
-    nnz4 = wsum(nnz4);
-    const uint32_t r8 = luma8x8_inter(qp);
-    if ((r8 >> 4) <= nnz4) { use8 = true; cbpl = (int)(r8 & 15u); }
-  }
-  const ChromaAc ac = chroma_quant(qpc, false);
-  bool drop_u = ac.any(0) && ac.score(0) < 7, drop_v = ac.any(1) && ac.score(1) < 7;
-  if (lane < 8) {
-    bool d = (lane >> 2) ? drop_v : drop_u;
-    if (d)
-#pragma unroll
-      for (int i = 0; i < 16; i++) sm.ccoef[lane * 16 + i] = 0;
-  }
-  __syncwarp();
-  bool acu = ac.any(0) && !drop_u, acv = ac.any(1) && !drop_v;
-  int cbpc = (acu || acv) ? 2 : (chroma_dc_any() ? 1 : 0);
-  if (best_t == 0 && cbpl == 0 && cbpc == 0 && bmv[0][0] == ps0 && bmv[0][1] == ps1) {
-    code_skip(c, ps0, ps1);
-    search_tail(c, best_t, false, ps0, ps1);  // 16x16: every quadrant has the skip vector
-    return;
-  }
-  rg_mb_out* rec = sd.rec + c.mb;
-  bool t8flag = use8 && cbpl != 0;
-  uint16_t nzm;
-  if (use8) {
-    int b = lane >> 3, q = lane & 7;
-#pragma unroll 1
-    for (int y = 0; y < 8; y++) rec->luma[b * 64 + zigzag8(y, q)] = sm.coef8[b * 64 + y * 8 + q];
-    nzm = 0;
-    for (int k = 0; k < 4; k++) if ((cbpl >> k) & 1) nzm |= (uint16_t)(0xF << (4 * k));
-  } else {
-    nzm = record_luma4x4(rec);
-  }
-  if (lane < 16) { rec->luma_dc[lane] = 0; rec->i4_modes[lane] = 2; }
-  record_chroma(rec, cbpc);
-  if (lane == 0) {
-    const int types[4] = {RG_MB_P_L0_16X16, RG_MB_P_L0_16X8, RG_MB_P_L0_8X16, RG_MB_P_8X8};
-    record_header(rec, types[best_t], 0, 0, cbpl | (cbpc << 4), t8flag, qp, bmv[0][0], bmv[0][1], bmvd[0][0],
-                  bmvd[0][1], nzm);
-    write_info(c, t8flag ? kFlagT8 : 0, cbpl, bmv[0][0], bmv[0][1], 0, nzm, false);
-  }
-  search_tail(c, best_t, true, 0, 0);
-  if (use8) recon_luma8x8(qp, cbpl);
-  else if (cbpl) recon_luma4x4(qp, cbpl);
-  __syncwarp();
-  chroma_recon(qpc, cbpc);
-  store_recon(c, (int)offsetof(Smem, pred_y));
+  const int type = best_t == 0 ? RG_MB_P_L0_16X16 : (best_t == 1 ? RG_MB_P_L0_16X8 : (best_t == 2 ? RG_MB_P_L0_8X16 : RG_MB_P_8X8));
+  const bool skipped = code_inter(c, type, best_t == 0 && bmv[0][0] == ps0 && bmv[0][1] == ps1, bmv[0][0], bmv[0][1],
+                                  bmvd[0][0], bmvd[0][1]);
+  search_tail(c, best_t, !skipped, ps0, ps1);
 }
 
 // One macroblock of an I slice in the search forms: the plain analysis (enc.rs:3311 code_intra),
