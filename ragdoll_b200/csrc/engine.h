@@ -63,8 +63,8 @@ struct StreamDev {
   // SkipBounds (enc.rs:2104) of the stream's QP
   uint32_t sb_luma, sb_luma_ssd, sb_chroma, sb_chroma_ssd, sb_probe;
   // pipelined launches: the descriptor's size group (its FrameParams), the offset of its rows in the
-  // launch's row counters, and the descriptor of the previous picture of its stream (-1: none)
-  int32_t group, rows_base, prev_ps;
+  // launch's row counters, and that of the previous picture of its stream (-1: none in this launch)
+  int32_t group, rows_base, prev_rows;
   // search forms only (null / 0 in the plain form)
   MbMv4* mv4;              // this picture's quadrant vectors
   const rg_mb_hint* hint;  // learned form: this picture's hints (null: full search)
@@ -76,6 +76,7 @@ struct StreamDev {
   // ready array at the descriptor's index, if any)
   int32_t* ready;
 };
+static_assert(sizeof(StreamDev) % 8 == 0, "descriptors are copied by 8-byte words");
 
 // Frame-constant parameters of one wavefront (all streams share the size; qp / qpc / sb_* are the
 // context's default QP -- the kernels read each stream's own from its StreamDev). A pipelined launch

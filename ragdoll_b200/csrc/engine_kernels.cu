@@ -77,6 +77,10 @@ struct __align__(16) Smem {
   uint8_t left[16];
   uint8_t ctop[2][8];
   uint8_t cleft[2][8];
+  alignas(16) StreamDev sd;       // the picture worked on (load_desc) and its stream's size (load_params)
+  alignas(16) FrameParams fp;
+  int db_row, seen_db;            // last acquired progress db_prev[db_row] of the reference picture
+  int reach_y, reach_x;           // 1 + the largest reach waited for beyond zero motion, in macroblocks
   alignas(16) uint8_t i4m[16];    // Intra4x4PredMode of this macroblock (decoding order)
   uint8_t i4q[16];          // edge samples of the current 4x4 block (i4_edge_index)
 };
@@ -1038,26 +1042,45 @@ __host__ __device__ __forceinline__ int i4_tap(int m, int x, int y) {
 // min(i + 2, 15) << 8 | kind << 12, at [16 m + 4 y + x] (filled from i4_tap by upload_tables).
 __device__ uint16_t g_i4tap[9 * 16];
 // ---------------------------------------------------------------------------------------------
+// A macroblock; its picture's descriptor and parameters are in shared memory (sm.sd, sm.fp): the
+// acquire of every wait drops the SM's L1, so read through global memory each use of them was an
+// L2 access.
 struct Ctx {
-  const FrameParams* fp;
-  const StreamDev* sd;
   int mbx, mby, mb;
 };
+__device__ __forceinline__ void load_desc(const StreamDev* p) {
+  constexpr int n = (int)(sizeof(StreamDev) / 8);
+  static_assert(n <= 32, "a word a lane");
+  const int lane = lane_id();
+  uint2 a = make_uint2(0u, 0u);
+  if (lane < n) a = ((const uint2*)p)[lane];
+  __syncwarp();
+  if (lane < n) ((uint2*)&sm.sd)[lane] = a;
+  __syncwarp();
+}
+__device__ __forceinline__ void load_params(const FrameParams& fp) {
+  constexpr int n = (int)(sizeof(FrameParams) / 4);
+  static_assert(n <= 32, "a word a lane");
+  const int lane = lane_id();
+  __syncwarp();
+  if (lane < n) ((int*)&sm.fp)[lane] = ((const int*)&fp)[lane];
+  __syncwarp();
+}
 
 // Loads the source macroblock, replicating the last row / column past the picture edges
 // (enc.rs:400 MbSrc::load, h264.rs:3660 extract_mb_planes).
 __device__ __noinline__ void load_source(const Ctx c) {
-  const FrameParams& fp = *c.fp;
+  const FrameParams& fp = sm.fp;
   int lane = lane_id();
   int W = fp.width, H = fp.height, cw = (W + 1) >> 1, ch = (H + 1) >> 1;
   int y = min(c.mby * 16 + (lane >> 1), H - 1);
-  const uint8_t* row = c.sd->src_y + (long)y * fp.src_stride_y;
+  const uint8_t* row = sm.sd.src_y + (long)y * fp.src_stride_y;
   int x0 = c.mbx * 16 + (lane & 1) * 8;
 #pragma unroll
   for (int k = 0; k < 8; k++) sm.src_y[(lane >> 1) * 16 + (lane & 1) * 8 + k] = __ldg(row + min(x0 + k, W - 1));
   int plane = lane >> 4, idx = (lane & 15) * 4, r = idx >> 3, c0 = idx & 7;
   int cy = min(c.mby * 8 + r, ch - 1);
-  const uint8_t* crow = (plane ? c.sd->src_v : c.sd->src_u) + (long)cy * fp.src_stride_uv;
+  const uint8_t* crow = (plane ? sm.sd.src_v : sm.sd.src_u) + (long)cy * fp.src_stride_uv;
   uint8_t* dst = (plane ? sm.src_v : sm.src_u) + r * 8 + c0;
 #pragma unroll
   for (int k = 0; k < 4; k++) dst[k] = __ldg(crow + min(c.mbx * 8 + c0 + k, cw - 1));
@@ -1066,9 +1089,9 @@ __device__ __noinline__ void load_source(const Ctx c) {
 // Intra edges from the unfiltered reconstruction of this picture (enc.rs:1459-1521) into shared
 // memory; returns the samples at the corner.
 __device__ __noinline__ Corner load_edges(const Ctx c, bool want_topright) {
-  const FrameParams& fp = *c.fp;
+  const FrameParams& fp = sm.fp;
   int lane = lane_id();
-  const uint8_t* Y = c.sd->cur_y;
+  const uint8_t* Y = sm.sd.cur_y;
   int x0 = c.mbx * 16, y0 = c.mby * 16;
   bool ht = c.mby > 0, hl = c.mbx > 0;
   if (ht && lane < 24) {
@@ -1079,35 +1102,35 @@ __device__ __noinline__ Corner load_edges(const Ctx c, bool want_topright) {
   int cx0 = c.mbx * 8, cy0 = c.mby * 8;
   if (lane < 16) {
     int p = lane >> 3, k = lane & 7;
-    const uint8_t* P = p ? c.sd->cur_v : c.sd->cur_u;
+    const uint8_t* P = p ? sm.sd.cur_v : sm.sd.cur_u;
     if (ht) sm.ctop[p][k] = ldcg_u8(P + (long)(cy0 - 1) * fp.stride_c + cx0 + k);
     if (hl) sm.cleft[p][k] = ldcg_u8(P + (long)(cy0 + k) * fp.stride_c + cx0 - 1);
   }
   Corner k;
   k.y = (ht && hl) ? ldcg_u8(Y + (long)(y0 - 1) * fp.stride_y + x0 - 1) : 128;
-  k.u = (ht && hl) ? ldcg_u8(c.sd->cur_u + (long)(cy0 - 1) * fp.stride_c + cx0 - 1) : 128;
-  k.v = (ht && hl) ? ldcg_u8(c.sd->cur_v + (long)(cy0 - 1) * fp.stride_c + cx0 - 1) : 128;
+  k.u = (ht && hl) ? ldcg_u8(sm.sd.cur_u + (long)(cy0 - 1) * fp.stride_c + cx0 - 1) : 128;
+  k.v = (ht && hl) ? ldcg_u8(sm.sd.cur_v + (long)(cy0 - 1) * fp.stride_c + cx0 - 1) : 128;
   __syncwarp();
   return k;
 }
 
 // Stores the reconstruction of pred_y/u/v (or tmp_y for luma: its byte offset in Smem) into the current picture.
 __device__ __noinline__ void store_recon(const Ctx c, int ly) {
-  const FrameParams& fp = *c.fp;
+  const FrameParams& fp = sm.fp;
   int lane = lane_id();
   int y = lane >> 1, x = (lane & 1) * 8;
   uint2 v = *(const uint2*)sm_at(ly + y * 16 + x);
-  *(uint2*)(c.sd->cur_y + (long)(c.mby * 16 + y) * fp.stride_y + c.mbx * 16 + x) = v;
-  if (c.sd->unf_y) {
+  *(uint2*)(sm.sd.cur_y + (long)(c.mby * 16 + y) * fp.stride_y + c.mbx * 16 + x) = v;
+  if (sm.sd.unf_y) {
     int cw = fp.mb_w * 16;
-    *(uint2*)(c.sd->unf_y + (long)(c.mby * 16 + y) * cw + c.mbx * 16 + x) = v;
+    *(uint2*)(sm.sd.unf_y + (long)(c.mby * 16 + y) * cw + c.mbx * 16 + x) = v;
   }
   if (lane < 16) {
     int p = lane >> 3, r = lane & 7;
     uint2 cv = *(const uint2*)&(p ? sm.pred_v : sm.pred_u)[r * 8];
-    uint8_t* P = p ? c.sd->cur_v : c.sd->cur_u;
+    uint8_t* P = p ? sm.sd.cur_v : sm.sd.cur_u;
     *(uint2*)(P + (long)(c.mby * 8 + r) * fp.stride_c + c.mbx * 8) = cv;
-    uint8_t* U = p ? c.sd->unf_v : c.sd->unf_u;
+    uint8_t* U = p ? sm.sd.unf_v : sm.sd.unf_u;
     if (U) *(uint2*)(U + (long)(c.mby * 8 + r) * (fp.mb_w * 8) + c.mbx * 8) = cv;
   }
 }
@@ -1169,14 +1192,14 @@ __device__ __forceinline__ void write_info(const Ctx c, int flags, int cbpl, int
   }
   static_assert(offsetof(MbInfo, ref) == 4 && offsetof(MbInfo, qp) == 7 && offsetof(MbInfo, i4_bottom) == 10 &&
                     offsetof(MbInfo, i4_right) == 12, "MbInfo packed by words");
-  *(uint4*)(c.sd->info + c.mb) = make_uint4(pack16(mvx, mvy), (uint32_t)(ref & 255) | (flags << 8) | (cbpl << 16) | (c.sd->qp << 24),
+  *(uint4*)(sm.sd.info + c.mb) = make_uint4(pack16(mvx, mvy), (uint32_t)(ref & 255) | (flags << 8) | (cbpl << 16) | (sm.sd.qp << 24),
                                             nz | (bottom << 16), right);
 }
 
 // I16x16 coding and reconstruction (enc.rs:3587 code_i16) with prediction mode `mode`.
 __device__ __noinline__ void code_i16(const Ctx c, int mode, bool ht, bool hl, Corner k0) {
   int lane = lane_id();
-  int qp = c.sd->qp, qpc = c.sd->qpc;
+  int qp = sm.sd.qp, qpc = sm.sd.qpc;
   pred16_into(mode, (int)offsetof(Smem, pred_y), ht, hl, k0.y);
   int cmode = analyse_chroma(ht, hl, k0);
   uint32_t shift, bias;
@@ -1257,7 +1280,7 @@ __device__ __noinline__ void code_i16(const Ctx c, int mode, bool ht, bool hl, C
   int cbpc = (ac.any(0) || ac.any(1)) ? 2 : (ac.dc() ? 1 : 0);
   __syncwarp();
   // record
-  rg_mb_out* rec = c.sd->rec + c.mb;
+  rg_mb_out* rec = sm.sd.rec + c.mb;
   record_luma4x4(rec);
   if (lane < 16) rec->luma_dc[lane] = sm.ldc[(kScan4Packed >> (4 * lane)) & 15];
   const uint32_t nzm = __ballot_sync(FULL, lane < 16 && cbpl && my_ac);
@@ -1300,10 +1323,10 @@ __device__ __noinline__ void code_i16(const Ctx c, int mode, bool ht, bool hl, C
 template <bool kMask>
 __device__ __noinline__ int analyse_i4(const Ctx c, uint32_t budget, bool ht_mb, bool hl_mb, int tl_mb,
                                         const uint16_t* masks) {
-  const FrameParams& fp = *c.fp;
+  const FrameParams& fp = sm.fp;
   int lane = lane_id();
   int p = lane & 15, xl = p & 3, yl = p >> 2;
-  int qp = c.sd->qp;
+  int qp = sm.sd.qp;
   uint32_t lambda = c_lambda[qp];
   uint32_t shift, bias;
   quant4_params(qp, true, shift, bias);
@@ -1311,7 +1334,7 @@ __device__ __noinline__ int analyse_i4(const Ctx c, uint32_t budget, bool ht_mb,
   int dqs = (int)c_dq4[qp % 6][pos4(p)] << (qp / 6);
   uint32_t total = lambda * 24;
   int cbpl = 0;
-  const MbInfo* info = c.sd->info;
+  const MbInfo* info = sm.sd.info;
   uint32_t lmodes = hl_mb ? ld_info(&info[c.mb - 1]).i4_right : 0x2222u;
   uint32_t tmodes = ht_mb ? ld_info(&info[c.mb - fp.mb_w]).i4_bottom : 0x2222u;
   // this lane's taps for its predictions (modes lane / 16 + 2 k, sample p): the same for every block
@@ -1429,17 +1452,17 @@ __device__ __noinline__ int analyse_i4(const Ctx c, uint32_t budget, bool ht_mb,
 // `luma`: what analyse_i4 returned.
 __device__ __noinline__ void code_i4(const Ctx c, int luma, bool ht, bool hl, Corner k0) {
   int lane = lane_id();
-  int qpc = c.sd->qpc;
+  int qpc = sm.sd.qpc;
   const int cbpl = luma & 15;
   const uint32_t nzm = (uint32_t)luma >> 4;
   int cmode = analyse_chroma(ht, hl, k0);
   const ChromaAc ac = chroma_quant(qpc, true);
   int cbpc = (ac.any(0) || ac.any(1)) ? 2 : (ac.dc() ? 1 : 0);
-  rg_mb_out* rec = c.sd->rec + c.mb;
+  rg_mb_out* rec = sm.sd.rec + c.mb;
   record_luma4x4(rec);
   if (lane < 8) ((uint32_t*)rec)[kWordLumaDc + lane] = 0u;
   record_chroma(rec, cbpc);
-  record_header(rec, RG_MB_I4X4, 0, cmode, cbpl | (cbpc << 4), 0, c.sd->qp, 0, 0, 0, 0, nzm, true);
+  record_header(rec, RG_MB_I4X4, 0, cmode, cbpl | (cbpc << 4), 0, sm.sd.qp, 0, 0, 0, 0, nzm, true);
   chroma_recon(qpc, cbpc);
   store_recon(c, (int)offsetof(Smem, tmp_y));
   write_info(c, kFlagIntra, cbpl, 0, 0, -1, nzm, true);
@@ -1449,7 +1472,7 @@ __device__ __noinline__ void code_i4(const Ctx c, int luma, bool ht, bool hl, Co
 __device__ __noinline__ void analyse_intra_mb(const Ctx c) {
   const Corner k0 = load_edges(c, true);
   bool ht = c.mby > 0, hl = c.mbx > 0;
-  uint32_t lambda = c_lambda[c.sd->qp];
+  uint32_t lambda = c_lambda[sm.sd.qp];
   const I16Fit fit16 = analyse_i16(ht, hl, k0.y);
   if (fit16.cost > 40 * lambda) {
     const int cbpl = analyse_i4<false>(c, fit16.cost + lambda * 4, ht, hl, k0.y, nullptr);
@@ -1464,11 +1487,11 @@ __device__ __noinline__ void analyse_intra_mb(const Ctx c) {
 // Codes P_Skip with vector mv; prediction already in pred_y / pred_u / pred_v.
 __device__ __noinline__ void code_skip(const Ctx c, int mvx, int mvy) {
   const int lane = lane_id();
-  rg_mb_out* rec = c.sd->rec + c.mb;
+  rg_mb_out* rec = sm.sd.rec + c.mb;
 #pragma unroll
   for (int k = 0; k < 7; k++)
     if (kWordLuma + lane + 32 * k < kWordParts) ((uint32_t*)rec)[kWordLuma + lane + 32 * k] = 0u;
-  record_header(rec, RG_MB_P_SKIP, 0, 0, 0, 0, c.sd->qp, mvx, mvy, 0, 0, 0, false);
+  record_header(rec, RG_MB_P_SKIP, 0, 0, 0, 0, sm.sd.qp, mvx, mvy, 0, 0, 0, false);
   write_info(c, kFlagSkip, 0, mvx, mvy, 0, 0, false);
   store_recon(c, (int)offsetof(Smem, pred_y));
 }
@@ -1486,11 +1509,11 @@ __device__ __noinline__ bool probe_skip_luma(int qp) {
 // (enc.rs:3158-3190), its record (code_inter, enc.rs:3196) and its reconstruction. can_skip: nothing
 // coded makes it P_Skip with vector (mvx, mvy). Returns whether it did.
 __device__ __noinline__ bool code_inter(const Ctx c, int type, bool can_skip, int mvx, int mvy, int mvdx, int mvdy) {
-  const int lane = lane_id(), qp = c.sd->qp, qpc = c.sd->qpc;
+  const int lane = lane_id(), qp = sm.sd.qp, qpc = sm.sd.qpc;
   const Luma4 l4 = luma4x4_inter(qp);
   uint32_t cbpl = l4.cbp;
   bool use8 = false;
-  if (c.fp->t8x8 && l4.cbp) {
+  if (sm.fp.t8x8 && l4.cbp) {
     const uint32_t r8 = luma8x8_inter(qp);
     if ((r8 >> 4) <= l4.nnz) { use8 = true; cbpl = r8 & 15u; }
   }
@@ -1505,7 +1528,7 @@ __device__ __noinline__ bool code_inter(const Ctx c, int type, bool can_skip, in
     code_skip(c, mvx, mvy);
     return true;
   }
-  rg_mb_out* rec = c.sd->rec + c.mb;
+  rg_mb_out* rec = sm.sd.rec + c.mb;
   const bool t8flag = use8 && cbpl != 0;
   uint32_t nzm = l4.nz16;
   if (use8) {
@@ -1558,42 +1581,41 @@ __device__ __forceinline__ unsigned long long global_ns() {
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
-// Waits until *p >= need. The first check and the final one are acquire loads by every lane;
-// in between lane 0 polls with relaxed loads (which leave the SM's L1 alone) and sleeps 32 ns
-// doubling to 512 ns. Returns the acquired value, or -1 on timeout (recorded in *error) or
-// when another warp failed.
-__device__ __noinline__ int wait_geq(const int* p, int need, int* error, unsigned long long timeout_ns) {
-  int v = ld_acquire(p);
-  if (__all_sync(FULL, v >= need)) return v;
-  unsigned long long t0 = global_ns();
+// Waits until every lane's counter has reached its need (p null: the lane waits for nothing). The
+// counters a macroblock depends on are taken by different lanes at once: one round trip, and one
+// drop of the SM's L1 by the acquires, instead of one per counter. `seen` is the lane's last acquired
+// value: no load when it covers `need` already (the acquire that returned it orders every later load
+// of this warp). The first check and the final one are acquire loads; in between the lanes poll with
+// relaxed loads (which leave the L1 alone) and sleep 32 ns doubling to 512 ns. False on timeout
+// (recorded in *error) or when another warp failed.
+__device__ __noinline__ bool wait_all(const int* p, int need, int& seen, int* error, unsigned long long timeout_ns) {
+  bool ok = !p || seen >= need;
+  if (__all_sync(FULL, ok)) return true;
+  unsigned long long t0 = 0;
   unsigned int sleep = 32;
   while (true) {
-    int r = 0;
-    if (lane_id() == 0) r = ld_relaxed(p) >= need ? 1 : (ld_relaxed(error) ? 2 : 0);
-    r = __shfl_sync(FULL, r, 0);
-    if (r == 1) {
-      v = ld_acquire(p);
-      if (__all_sync(FULL, v >= need)) return v;
+    if (!ok) seen = ld_acquire(p);
+    ok = !p || seen >= need;
+    if (__all_sync(FULL, ok)) {
+      __syncwarp();  // every lane's later loads follow the acquires
+      return true;
     }
-    if (r == 2) return -1;
-    unsigned long long dt = __shfl_sync(FULL, global_ns() - t0, 0);
-    if (dt > timeout_ns) {
-      if (lane_id() == 0) atomicCAS(error, 0, 1);
-      return -1;
+    if (!t0) t0 = global_ns();
+    while (true) {  // until no lane is behind
+      const bool behind = !ok && ld_relaxed(p) < need;
+      const bool fail = lane_id() == 0 && ld_relaxed(error);
+      const bool late = lane_id() == 0 && global_ns() - t0 > timeout_ns;
+      const uint32_t b = __ballot_sync(FULL, behind);
+      if (!b) break;
+      if (__any_sync(FULL, fail)) return false;
+      if (__any_sync(FULL, late)) {
+        if (lane_id() == 0) atomicCAS(error, 0, 1);
+        return false;
+      }
+      __nanosleep(sleep);
+      sleep = min(sleep * 2, 512u);
     }
-    __nanosleep(sleep);
-    sleep = min(sleep * 2, 512u);
   }
-}
-// wait_geq with the last acquired value of the counter kept in `seen`: no load when it already
-// covers `need` (the acquire that returned it orders every later load of this warp).
-__device__ __forceinline__ bool wait_seen(const int* p, int need, int& seen, int* error,
-                                          unsigned long long timeout_ns) {
-  if (seen >= need) return true;
-  int v = wait_geq(p, need, error, timeout_ns);
-  if (v < 0) return false;
-  seen = v;
-  return true;
 }
 // Publishes v after this warp's global writes: the warp barrier orders every lane's writes before lane
 // 0's release store, which is cumulative over them.
@@ -1601,28 +1623,45 @@ __device__ __forceinline__ void publish(int* p, int v) {
   __syncwarp();
   if (lane_id() == 0) st_release(p, v);
 }
-// What a P macroblock of the pipelined mode waits for in its reference picture.
+// What a P macroblock of the pipelined mode waits for in its reference picture (kernel constants and
+// addresses; the state is in shared memory).
 struct PipeWait {
-  const int* ana_prev;   // analysis progress per macroblock row of the reference picture
-  const int* db_prev;    // deblocking progress per row of the reference picture (padding included)
+  const int* db_prev;    // deblocking progress per row of the reference picture (padding included); null: no wait
   int* error;
   unsigned long long timeout_ns;
-  int seen_ana;          // last acquired ana_prev[row of this segment]
-  int db_row, seen_db;   // last acquired db_prev[db_row]
-  int reach_y, reach_x;  // 1 + the largest reach waited for beyond zero motion, in macroblocks
-  bool failed;
 };
+// Waits until the reference picture is final over the macroblocks left of and above (xx, rr),
+// clamped to the picture: rows above the last are final where the row below is deblocked; the last
+// row where its right neighbour is.
+__device__ __noinline__ bool wait_reference(const Ctx c, const PipeWait pw, int xb, int rb) {
+  const FrameParams& fp = sm.fp;
+  const int rr = min(max(rb, 0), fp.mb_h - 1), xx = min(max(xb, 0), fp.mb_w - 1);
+  const int row = rr < fp.mb_h - 1 ? rr + 1 : rr, need = rr < fp.mb_h - 1 ? xx + 1 : min(xx + 2, fp.mb_w);
+  int seen = row == sm.db_row ? sm.seen_db : 0;
+  // zero motion reaches (mbx + 2, mby + 2); the host sizes the picture lag from the maximum
+  const int ry = max(sm.reach_y, max(rr - c.mby - 2, 0) + 1), rx = max(sm.reach_x, max(xx - c.mbx - 2, 0) + 1);
+  const bool ok = wait_all(lane_id() == 0 ? pw.db_prev + row : nullptr, need, seen, pw.error, pw.timeout_ns);
+  __syncwarp();
+  if (lane_id() == 0) {
+    sm.reach_y = ry;
+    sm.reach_x = rx;
+    sm.db_row = row;
+    sm.seen_db = seen;
+  }
+  __syncwarp();
+  return ok;
+}
 
-// One macroblock of a P slice (enc.rs:3011 code_p_mb). In the pipelined mode (pw != null) it
-// first waits for the reference frame to be final over every sample its search can read; when
-// a wait gives up it returns with pw->failed set and writes nothing.
-__device__ __noinline__ void analyse_p_mb(const Ctx c, PipeWait* pw) {
-  const FrameParams& fp = *c.fp;
-  const StreamDev& sd = *c.sd;
+// One macroblock of a P slice (enc.rs:3011 code_p_mb). In the pipelined mode (pw.db_prev) it first
+// waits for the reference frame to be final over every sample its search can read; when a wait
+// gives up it returns false and writes nothing.
+__device__ __noinline__ bool analyse_p_mb(const Ctx c, const PipeWait pw) {
+  const FrameParams& fp = sm.fp;
+  const StreamDev& sd = sm.sd;
   int lane = lane_id();
   int mbx = c.mbx, mby = c.mby, mb_w = fp.mb_w;
   int x0 = mbx * 16, y0 = mby * 16;
-  int qp = c.sd->qp;
+  int qp = sm.sd.qp;
   uint32_t lambda = c_lambda[qp];
   int cw = fp.mb_w * 16, chh = fp.mb_h * 16;
   // MvBounds (enc.rs:1105)
@@ -1652,14 +1691,10 @@ __device__ __noinline__ void analyse_p_mb(const Ctx c, PipeWait* pw) {
   int ps0 = mvp0, ps1 = mvp1;
   if (mbx == 0 || mby == 0 || (lref == 0 && a0 == 0 && a1 == 0) || (tref == 0 && b0 == 0 && b1 == 0)) { ps0 = 0; ps1 = 0; }
   load_source(c);
-  int qpc = c.sd->qpc;
+  int qpc = sm.sd.qpc;
   // co-located vector of the previous picture: a search candidate (enc.rs:3094)
-  if (pw && !wait_seen(pw->ana_prev + mby, mbx + 1, pw->seen_ana, pw->error, pw->timeout_ns)) {
-    pw->failed = true;
-    return;
-  }
   MbInfo prevmb = ld_info(&sd.prev_info[c.mb]);
-  if (pw) {
+  if (pw.db_prev) {
     // The right- and bottom-most reference sample this macroblock can read: the full-pel
     // candidates, a diamond of at most 16 steps around the best, the half-sample window
     // (-3..+20) and 8-byte loads. Everything above and to the left of it (padding included) is
@@ -1667,26 +1702,12 @@ __device__ __noinline__ void analyse_p_mb(const Ctx c, PipeWait* pw) {
     int cx[5] = {mvp0, 0, a0, b0, prevmb.mv[0]}, cy[5] = {mvp1, 0, a1, b1, prevmb.mv[1]};
     int hi0 = -(1 << 20), hi1 = -(1 << 20);
     int imn0 = (bmin0 + 3) >> 2, imn1 = (bmin1 + 3) >> 2, imx0 = bmax0 >> 2, imx1 = bmax1 >> 2;
+#pragma unroll
     for (int k = 0; k < 5; k++) {
       hi0 = max(hi0, min(max((cx[k] + 2) >> 2, imn0), imx0));
       hi1 = max(hi1, min(max((cy[k] + 2) >> 2, imn1), imx1));
     }
-    int xb = (x0 + hi0 + 44) >> 4, rb = (y0 + hi1 + 40) >> 4;
-    int rr = min(max(rb, 0), fp.mb_h - 1), xx = min(max(xb, 0), fp.mb_w - 1);
-    // rows above the last are final where the row below is deblocked; the last row where its
-    // right neighbour is
-    int row = rr < fp.mb_h - 1 ? rr + 1 : rr, need = rr < fp.mb_h - 1 ? xx + 1 : min(xx + 2, fp.mb_w);
-    // zero motion reaches (mbx + 2, mby + 2); the host sizes the picture lag from the maximum
-    pw->reach_y = max(pw->reach_y, max(rr - mby - 2, 0) + 1);
-    pw->reach_x = max(pw->reach_x, max(xx - mbx - 2, 0) + 1);
-    if (row != pw->db_row) {
-      pw->db_row = row;
-      pw->seen_db = 0;
-    }
-    if (!wait_seen(pw->db_prev + row, need, pw->seen_db, pw->error, pw->timeout_ns)) {
-      pw->failed = true;
-      return;
-    }
+    if (!wait_reference(c, pw, (x0 + hi0 + 44) >> 4, (y0 + hi1 + 40) >> 4)) return false;
   }
 
   // 1. skip probe (enc.rs:2906 try_p_skip)
@@ -1694,8 +1715,8 @@ __device__ __noinline__ void analyse_p_mb(const Ctx c, PipeWait* pw) {
     mc_luma16(sd.ref_y, fp.stride_y, x0, y0, ps0, ps1);
     uint2 s = src8(), p = *(const uint2*)&sm.pred_y[(lane >> 1) * 16 + (lane & 1) * 8];
     uint32_t sad = wsum(vsad8(s, p));
-    if (sad < c.sd->sb_probe) {
-      bool lz = sad <= c.sd->sb_luma;
+    if (sad < sm.sd.sb_probe) {
+      bool lz = sad <= sm.sd.sb_luma;
       if (!lz) {
         uint32_t ssd = 0;
 #pragma unroll
@@ -1704,7 +1725,7 @@ __device__ __noinline__ void analyse_p_mb(const Ctx c, PipeWait* pw) {
           int d1 = (int)((s.y >> (8 * k)) & 255) - (int)((p.y >> (8 * k)) & 255);
           ssd += d0 * d0 + d1 * d1;
         }
-        lz = wsum(ssd) <= c.sd->sb_luma_ssd;
+        lz = wsum(ssd) <= sm.sd.sb_luma_ssd;
       }
       if (!lz) lz = probe_skip_luma(qp);
       if (lz) {
@@ -1718,8 +1739,8 @@ __device__ __noinline__ void analyse_p_mb(const Ctx c, PipeWait* pw) {
         for (int k = 0; k < 4; k++) { int d = (int)ss[k] - (int)pp[k]; sadp += abs(d); ssdp += d * d; }
         uint32_t sad_u = wsum(plane == 0 ? sadp : 0), sad_v = wsum(plane == 1 ? sadp : 0);
         uint32_t ssd_u = wsum(plane == 0 ? ssdp : 0), ssd_v = wsum(plane == 1 ? ssdp : 0);
-        bool zu = sad_u <= c.sd->sb_chroma || ssd_u <= c.sd->sb_chroma_ssd;
-        bool zv = sad_v <= c.sd->sb_chroma || ssd_v <= c.sd->sb_chroma_ssd;
+        bool zu = sad_u <= sm.sd.sb_chroma || ssd_u <= sm.sd.sb_chroma_ssd;
+        bool zv = sad_v <= sm.sd.sb_chroma || ssd_v <= sm.sd.sb_chroma_ssd;
         bool cz = zu && zv;
         if (!cz) {
           const ChromaAc ac = chroma_quant(qpc, false);
@@ -1727,7 +1748,7 @@ __device__ __noinline__ void analyse_p_mb(const Ctx c, PipeWait* pw) {
         }
         if (cz) {
           code_skip(c, ps0, ps1);
-          return;
+          return true;
         }
       }
     }
@@ -1800,7 +1821,7 @@ __device__ __noinline__ void analyse_p_mb(const Ctx c, PipeWait* pw) {
   {
     int fm0 = best0 * 4, fm1 = best1 * 4;
     uint32_t full_mvc = mvd_cost(fm0 - mvp0, lambda) + mvd_cost(fm1 - mvp1, lambda);
-    if (best_cost - full_mvc <= c.sd->sb_luma) {
+    if (best_cost - full_mvc <= sm.sd.sb_luma) {
       mv0 = fm0; mv1 = fm1;
       uint2 v = ldg8(base + (long)best1 * stride + best0);
       *(uint2*)&sm.pred_y[(lane >> 1) * 16 + (lane & 1) * 8] = v;
@@ -1850,13 +1871,14 @@ __device__ __noinline__ void analyse_p_mb(const Ctx c, PipeWait* pw) {
     const I16Fit fit16 = analyse_i16(ht, hl, k0.y);
     if (fit16.cost + lambda * 8 < inter_cost) {
       code_i16(c, fit16.mode, ht, hl, k0);
-      return;
+      return true;
     }
   }
 
   // 4. P_L0_16x16 residual, record and reconstruction
   mc_chroma8(sd.ref_u, sd.ref_v, fp.stride_c, mbx, mby, mv0, mv1);
   code_inter(c, RG_MB_P_L0_16X16, mv0 == ps0 && mv1 == ps1, mv0, mv1, mv0 - mvp0, mv1 - mvp1);
+  return true;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1978,7 +2000,9 @@ __device__ __forceinline__ bool one_vector(const MbMv4& m) {
 }
 
 template <bool kMv4>
-__device__ __noinline__ void deblock_mb(const FrameParams& fp, const StreamDev& sd, int mbx, int mby) {
+__device__ __noinline__ void deblock_mb(int mbx, int mby) {
+  const FrameParams& fp = sm.fp;
+  const StreamDev& sd = sm.sd;
   int lane = lane_id();
   int m = mby * fp.mb_w + mbx;
   MbInfo q = ld_info(&sd.info[m]);
@@ -2084,25 +2108,28 @@ __device__ __forceinline__ int diag_len(const FrameParams& fp, int d) {
 template <int kForm>
 __global__ void __launch_bounds__(32) wavefront_step_kernel(const __grid_constant__ FrameParams fp, const StreamDev* __restrict__ streams, int step) {
   init_tables();
-  const StreamDev& sd = streams[blockIdx.y];
+  load_params(fp);
+  load_desc(streams + blockIdx.y);
+  const StreamDev& sd = sm.sd;
   int na = diag_len(fp, step);
   int nd = fp.deblock ? diag_len(fp, step - 3) : 0;
   int k = blockIdx.x;
   if (k < na) {
     int mby = diag_first(fp, step) + k, mbx = step - 2 * mby;
-    Ctx c{&fp, &sd, mbx, mby, mby * fp.mb_w + mbx};
+    Ctx c{mbx, mby, mby * fp.mb_w + mbx};
+    const PipeWait none{nullptr, nullptr, 0};
     if (sd.kind == RG_FRAME_IDR) {
       load_source(c);
       if constexpr (kForm != 0) analyse_intra_mb_search(c);
       else analyse_intra_mb(c);
     } else {
-      if constexpr (kForm != 0) analyse_p_mb_search(c, nullptr);
-      else analyse_p_mb(c, nullptr);
+      if constexpr (kForm != 0) analyse_p_mb_search(c, none);
+      else analyse_p_mb(c, none);
     }
   } else if (k - na < nd) {
     int d = step - 3;
     int mby = diag_first(fp, d) + (k - na), mbx = d - 2 * mby;
-    deblock_mb<kForm != 0>(fp, sd, mbx, mby);
+    deblock_mb<kForm != 0>(mbx, mby);
   }
 }
 
@@ -2112,7 +2139,9 @@ __global__ void __launch_bounds__(32) wavefront_step_kernel(const __grid_constan
 // first / last row -- corners included, which come from the corner macroblocks. Applied to every
 // macroblock of the picture this writes every padding sample exactly once, so a picture's
 // padding is complete wherever the macroblocks it copies are final. One warp, 4-byte stores.
-__device__ __noinline__ void extend_mb(const FrameParams& fp, const StreamDev& sd, int a, int b) {
+__device__ __noinline__ void extend_mb(int a, int b) {
+  const FrameParams& fp = sm.fp;
+  const StreamDev& sd = sm.sd;
   int lane = lane_id();
   bool left = a == 0, right = a == fp.mb_w - 1, top = b == 0, bottom = b == fp.mb_h - 1;
   if (!(left || right || top || bottom)) return;
@@ -2195,10 +2224,12 @@ __device__ __noinline__ void picture_row_done(int* rows_done, int* ready, int se
 }
 
 static_assert(sizeof(rg_mb_out) == 4 * kRecordWords, "a record is kRecordWords words");
-// Staging of compact records in the warp's shared memory (its Smem, which no task reads before
-// writing it): kStageWords words, flushed to host memory in 16-byte stores.
+// Staging of compact records in the warp's shared memory (the front of its Smem, which no task reads
+// before writing it): kStageWords words, flushed to host memory in 16-byte stores.
 constexpr int kStageWords = 512;
-static_assert(sizeof(Smem) >= 4 * kStageWords, "the staging buffer fits the warp's shared memory");
+static_assert(offsetof(Smem, coef) >= 4 * kStageWords && offsetof(Smem, zz8) > offsetof(Smem, coef) &&
+                  offsetof(Smem, sd) > offsetof(Smem, coef),
+              "the staging buffer ends before what a warp keeps between macroblocks");
 static_assert(kStageWords >= 2 * (kCompactMaskWords + kRecordWords), "a flush leaves room for a whole record");
 
 // Writes the first n (a multiple of 4) staged words to dst + at (16-byte aligned) while they fit
@@ -2294,7 +2325,8 @@ __global__ void __launch_bounds__(32, 16) pipeline_kernel(const __grid_constant_
   }
   init_tables();
   bool empty[3] = {pp.qbeg[0] >= pp.qend[0], pp.qbeg[1] >= pp.qend[1], pp.qbeg[2] >= pp.qend[2]};
-  int reach_y = 0, reach_x = 0;  // this warp's, published once as it exits
+  if (lane == 0) sm.reach_y = sm.reach_x = 0;  // this warp's, published once as it exits
+  int group = -1;                              // whose parameters sm.fp holds
   while (true) {
     int t = -1;
     if (lane == 0) {
@@ -2310,73 +2342,68 @@ __global__ void __launch_bounds__(32, 16) pipeline_kernel(const __grid_constant_
     if (__shfl_sync(FULL, lane == 0 ? ld_relaxed(pp.error) : 0, 0)) break;
     int2 task = __ldg(pp.tasks + t);
     int ps = task.x;
-    const StreamDev& sd = sds[ps];
-    const FrameParams& fp = fg.g[sd.group];  // the descriptor's picture size
-    const int H = fp.mb_h, Wm = fp.mb_w;
-    int y = task.y >> 16, x0 = (task.y >> 1) & 0x7fff, x1 = min(x0 + pp.seg, Wm);
-    bool ana = (task.y & 1) == 0;
+    load_desc(sds + ps);
+    const StreamDev& sd = sm.sd;
+    if (sd.group != group) {  // the descriptor's picture size
+      group = sd.group;
+      load_params(fg.g[group]);
+    }
+    const int H = sm.fp.mb_h, Wm = sm.fp.mb_w;
+    const int y = task.y >> 16, x0 = (task.y >> 1) & 0x7fff, x1 = min(x0 + pp.seg, Wm);
+    const bool ana = (task.y & 1) == 0;
     int* ana_rows = pp.ana + sd.rows_base;
     int* db_rows = pp.db + sd.rows_base;
     bool failed = false;
+    int seen = 0;  // of this lane's counter (wait_all)
     if (ana) {
-      PipeWait pw;
-      bool has_prev = sd.prev_ps >= 0 && sd.kind == RG_FRAME_P;
-      if (has_prev) {
-        const int pb = sds[sd.prev_ps].rows_base;
-        pw.ana_prev = pp.ana + pb;
-        pw.db_prev = pp.db + pb;
-      }
-      pw.error = pp.error;
-      pw.timeout_ns = pp.timeout_ns;
-      pw.seen_ana = 0;
-      pw.db_row = -1;
-      pw.seen_db = 0;
-      pw.reach_y = reach_y;
-      pw.reach_x = reach_x;
-      pw.failed = false;
-      int seen_own = 0, seen_up = 0;
-      // the previous segment of this row, then per macroblock the row above two ahead
-      if (x0 > 0 && !wait_seen(ana_rows + y, x0, seen_own, pp.error, pp.timeout_ns)) failed = true;
-      for (int x = x0; x < x1 && !failed; x++) {
-        if (y > 0 && !wait_seen(ana_rows + y - 1, min(x + 2, Wm), seen_up, pp.error, pp.timeout_ns)) {
+      const bool has_prev = sd.prev_rows >= 0 && sd.kind == RG_FRAME_P;
+      const PipeWait pw{has_prev ? pp.db + sd.prev_rows : nullptr, pp.error, pp.timeout_ns};
+      if (lane == 0) sm.db_row = -1;
+      // lane 0: the previous segment of this row; lane 1: the row above two macroblocks ahead; lane 2
+      // (plain form): the co-located macroblock of the previous picture, whose vector is a candidate
+      const int* flag = lane == 0 && x0 > 0 ? ana_rows + y : nullptr;
+      if (lane == 1 && y > 0) flag = ana_rows + y - 1;
+      if (kForm == 0 && lane == 2 && has_prev) flag = pp.ana + sd.prev_rows + y;
+      for (int x = x0; x < x1; x++) {
+        if (!wait_all(flag, lane == 0 ? x0 : (lane == 1 ? min(x + 2, Wm) : x + 1), seen, pp.error, pp.timeout_ns)) {
           failed = true;
           break;
         }
-        Ctx c{&fp, &sd, x, y, y * Wm + x};
+        Ctx c{x, y, y * Wm + x};
         if (sd.kind == RG_FRAME_IDR) {
           load_source(c);
           if constexpr (kForm != 0) analyse_intra_mb_search(c);
           else analyse_intra_mb(c);
         } else {
-          if constexpr (kForm != 0) analyse_p_mb_search(c, has_prev ? &pw : nullptr);
-          else analyse_p_mb(c, has_prev ? &pw : nullptr);
-          if (pw.failed) { failed = true; break; }
+          if constexpr (kForm != 0) failed = !analyse_p_mb_search(c, pw);
+          else failed = !analyse_p_mb(c, pw);
+          if (failed) break;
         }
         publish(ana_rows + y, x + 1);
       }
       // (with compact records, the row is counted once its deblocking warp has compacted it)
       int* const rdy = sd.ready ? sd.ready : (pp.ready ? pp.ready + ps : nullptr);
       if (!failed && x1 == Wm && rdy && !pp.cwords) picture_row_done(pp.rows_done + ps, rdy, pp.seq, H);
-      reach_y = pw.reach_y;
-      reach_x = pw.reach_x;
     } else {
-      int seen_own = 0, seen_a0 = 0, seen_a1 = 0, seen_up = 0;
-      if (x0 > 0 && !wait_seen(db_rows + y, x0, seen_own, pp.error, pp.timeout_ns)) failed = true;
-      for (int x = x0; x < x1 && !failed; x++) {
-        if (!wait_seen(ana_rows + y, min(x + 2, Wm), seen_a0, pp.error, pp.timeout_ns) ||
-            (y + 1 < H && !wait_seen(ana_rows + y + 1, min(x + 1, Wm), seen_a1, pp.error, pp.timeout_ns)) ||
-            (y > 0 && !wait_seen(db_rows + y - 1, min(x + 2, Wm), seen_up, pp.error, pp.timeout_ns))) {
+      // lane 0: the analysis of this row one macroblock further; lane 1: of the row below; lane 2: the
+      // deblocking of the row above one further; lane 3: the previous segment of this row
+      const int* flag = lane == 0 ? ana_rows + y : nullptr;
+      if (lane == 1 && y + 1 < H) flag = ana_rows + y + 1;
+      if (lane == 2 && y > 0) flag = db_rows + y - 1;
+      if (lane == 3 && x0 > 0) flag = db_rows + y;
+      for (int x = x0; x < x1; x++) {
+        if (!wait_all(flag, lane == 3 ? x0 : min(x + (lane == 1 ? 1 : 2), Wm), seen, pp.error, pp.timeout_ns)) {
           failed = true;
           break;
         }
-        deblock_mb<kForm != 0>(fp, sd, x, y);
+        deblock_mb<kForm != 0>(x, y);
         // Macroblock (x, y - 1) is final now: (x + 1, y - 1) was deblocked before this one. In
         // the last row, so is (x - 1, y), and the last macroblock is final after its own pass.
         __syncwarp();
-        if (y >= 1) extend_mb(fp, sd, x, y - 1);
+        if (y >= 1) extend_mb(x, y - 1);
         if (y == H - 1) {
-          if (x >= 1) extend_mb(fp, sd, x - 1, y);
-          if (x == Wm - 1) extend_mb(fp, sd, x, y);
+          if (x >= 1) extend_mb(x - 1, y);
+          if (x == Wm - 1) extend_mb(x, y);
         }
         publish(db_rows + y, x + 1);
       }
@@ -2395,9 +2422,9 @@ __global__ void __launch_bounds__(32, 16) pipeline_kernel(const __grid_constant_
     }
     if (failed) break;
   }
-  if (lane == 0 && reach_y) {
-    atomicMax(pp.reach, reach_y);
-    atomicMax(pp.reach + 1, reach_x);
+  if (lane == 0 && sm.reach_y) {
+    atomicMax(pp.reach, sm.reach_y);
+    atomicMax(pp.reach + 1, sm.reach_x);
   }
 }
 

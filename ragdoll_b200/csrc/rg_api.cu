@@ -540,7 +540,7 @@ static int enqueue_wavefront(rg_ctx* c, const uint8_t* const* dev_planes, size_t
     apply_qp(d, c->qps[s]);
     d.group = 0;
     d.rows_base = 0;
-    d.prev_ps = -1;
+    d.prev_rows = -1;
     d.mv4 = c->mv4s ? c->mv4s + ((size_t)s * c->nslots + par) * c->n_mb : nullptr;
     d.hint = hints ? hints[i] : nullptr;
     d.search_range = c->search_range;
@@ -569,11 +569,11 @@ static int enqueue_wavefront(rg_ctx* c, const uint8_t* const* dev_planes, size_t
 // previous wave then runs during that wave's own launch and slows it.) ready / seq: per-picture
 // flags in mapped host memory (rg_analyse_gops_stream), or null.
 // Descriptor of picture f of stream s of a pipelined call (records at rec_base, [f][s]); in a launch
-// of several contexts, this context's descriptors start at desc_base, its row counters at
-// rows_base, and its picture size is group `group`.
+// of several contexts, this context's row counters start at rows_base, and its picture size is
+// group `group`.
 static void gop_desc(const rg_ctx* c, StreamDev& d, int f, int s, const uint8_t* const* dev_planes,
-                     const int32_t* kinds, rg_mb_out* rec_base, const rg_mb_hint* hint, int group, int desc_base,
-                     int rows_base, int* ready = nullptr) {
+                     const int32_t* kinds, rg_mb_out* rec_base, const rg_mb_hint* hint, int group, int rows_base,
+                     int* ready = nullptr) {
   const int S = c->S, g = c->frames[s] + f;
   const int cur = g % c->nslots, prv = (g + c->nslots - 1) % c->nslots;
   d.src_y = dev_planes[(f * S + s) * 3];
@@ -593,7 +593,7 @@ static void gop_desc(const rg_ctx* c, StreamDev& d, int f, int s, const uint8_t*
   apply_qp(d, c->qps[s]);
   d.group = group;
   d.rows_base = rows_base + (f * S + s) * c->fp.mb_h;
-  d.prev_ps = f > 0 ? desc_base + (f - 1) * S + s : -1;
+  d.prev_rows = f > 0 ? d.rows_base - S * c->fp.mb_h : -1;
   d.mv4 = c->mv4s ? c->mv4s + ((size_t)s * c->nslots + cur) * c->n_mb : nullptr;
   d.hint = hint;
   d.search_range = c->search_range;
@@ -656,7 +656,7 @@ static int enqueue_gops(rg_ctx* c, const uint8_t* const* dev_planes, size_t stri
   StreamDev* h = c->h_streams[slot];
   for (int f = 0; f < frames; f++)
     for (int s = 0; s < S; s++)
-      gop_desc(c, h[f * S + s], f, s, dev_planes, kinds, rec_base, hv.empty() ? nullptr : hv[f * S + s], 0, 0, 0);
+      gop_desc(c, h[f * S + s], f, s, dev_planes, kinds, rec_base, hv.empty() ? nullptr : hv[f * S + s], 0, 0);
   FrameParams fp = c->fp;
   fp.src_stride_y = (int)stride_y;
   fp.src_stride_uv = (int)stride_uv;
@@ -810,7 +810,7 @@ static int group_launch(rg_ctx* const* ctxs, int32_t n, const uint8_t* const* co
     for (int f = 0; f < frames; f++)
       for (int s = 0; s < c->S; s++)
         gop_desc(c, L->g_hstreams[desc_base[i] + f * c->S + s], f, s, dev_planes[i], kinds[i],
-                 rec_bases && rec_bases[i] ? rec_bases[i] : c->recs, nullptr, i, desc_base[i], rows_base[i],
+                 rec_bases && rec_bases[i] ? rec_bases[i] : c->recs, nullptr, i, rows_base[i],
                  readies ? readies[i] : nullptr);
   }
   // launch shape: the segment length and SM roles of the context with the most macroblocks (its

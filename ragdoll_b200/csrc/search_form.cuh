@@ -65,8 +65,8 @@ __device__ __forceinline__ void ld_q(const MbMv4* m, int q, int* v) {
   v[1] = (int16_t)(w >> 16);
 }
 __device__ __noinline__ MbNb load_nb(const Ctx c) {
-  const StreamDev& sd = *c.sd;
-  const int mb_w = c.fp->mb_w, mb = c.mb;
+  const StreamDev& sd = sm.sd;
+  const int mb_w = sm.fp.mb_w, mb = c.mb;
   MbNb n;
   n.refA = n.refB = n.refC = n.refD = -2;
   n.a[0][0] = n.a[0][1] = n.a[1][0] = n.a[1][1] = 0;
@@ -154,8 +154,8 @@ __device__ __noinline__ void int_search_small(const Ctx c, int xlo, int xhi, int
                                               int yhi, int mvp0, int mvp1, uint32_t lambda) {
   IntBest& ib = ss.ib;
   const int lane = lane_id();
-  const int x0 = c.mbx * 16, y0 = c.mby * 16, stride = c.fp->stride_y;
-  const uint8_t* ref = c.sd->ref_y;
+  const int x0 = c.mbx * 16, y0 = c.mby * 16, stride = sm.fp.stride_y;
+  const uint8_t* ref = sm.sd.ref_y;
   const int xs = (x0 + xlo) & ~3;
   const int bw = ((x0 + xhi + 20 - xs) + 3) & ~3;
   const int nwx = xhi - xlo + 1, nwy = yhi - ylo + 1, wpr = bw >> 2;
@@ -199,10 +199,10 @@ __device__ __noinline__ void int_search(const Ctx c, int xlo, int xhi, int ylo, 
     int_search_small(c, xlo, xhi, ylo, yhi, mvp0, mvp1, lambda);
     return;
   }
-  const FrameParams& fp = *c.fp;
+  const FrameParams& fp = sm.fp;
   const int lane = lane_id();
   const int x0 = c.mbx * 16, y0 = c.mby * 16, stride = fp.stride_y;
-  const uint8_t* ref = c.sd->ref_y;
+  const uint8_t* ref = sm.sd.ref_y;
   const int xs = (x0 + xlo) & ~3;                        // picture column of band column 0
   const int bw = ((x0 + xhi + 20 - xs) + 3) & ~3;        // band row bytes
   const int nwx = xhi - xlo + 1;
@@ -323,7 +323,7 @@ __device__ __constant__ int8_t c_hstep[8][2] = {{0, -2}, {-2, 0}, {2, 0}, {0, 2}
 constexpr int kNoWin = 1 << 20;
 __device__ __forceinline__ void ensure_window(const Ctx c, int bx, int by) {
   if (ss.wbx == bx && ss.wby == by) return;
-  stage_window(c.sd->ref_y, c.fp->stride_y, c.mbx * 16 + bx - 1, c.mby * 16 + by - 1);
+  stage_window(sm.sd.ref_y, sm.fp.stride_y, c.mbx * 16 + bx - 1, c.mby * 16 + by - 1);
   build_hpel(7);
   __syncwarp();
   ss.wbx = bx;
@@ -439,8 +439,8 @@ __device__ __noinline__ void predict_part(const Ctx c, int px, int py, int pw, i
 // Chroma prediction of both planes with each 8x8 luma quadrant's own vector (4x4 chroma blocks;
 // the bilinear 1/8-sample filter of chroma_mc_8x8_x2, h264_enc.rs:1279, per sample).
 __device__ __noinline__ void mc_chroma_q(const Ctx c) {
-  const FrameParams& fp = *c.fp;
-  const StreamDev& sd = *c.sd;
+  const FrameParams& fp = sm.fp;
+  const StreamDev& sd = sm.sd;
   const int lane = lane_id();
   const int plane = lane >> 4, idx = (lane & 15) * 4, r = idx >> 3, c0 = idx & 7;
   const int q = (r >> 2) * 2 + (c0 >> 2);
@@ -463,7 +463,7 @@ __device__ __noinline__ void mc_chroma_q(const Ctx c) {
 // differences.
 __device__ __noinline__ void search_tail(const Ctx c, int ptype, bool parts, int mvx, int mvy) {
   if (lane_id() != 0) return;
-  rg_mb_out* rec = c.sd->rec + c.mb;
+  rg_mb_out* rec = sm.sd.rec + c.mb;
   MbMv4 m;
 #pragma unroll
   for (int q = 0; q < 4; q++) {
@@ -476,38 +476,22 @@ __device__ __noinline__ void search_tail(const Ctx c, int ptype, bool parts, int
   }
   rec->part_type = (uint8_t)ptype;
   rec->reserved2[0] = rec->reserved2[1] = rec->reserved2[2] = 0;
-  c.sd->mv4[c.mb] = m;
+  sm.sd.mv4[c.mb] = m;
 }
 
 // Reach of a search window for the pipelined mode's wait on the reference picture: every
 // sample the integer search (band staging), the refinement windows and the final prediction can
 // read lies above row (y0 + yhi + 28) and left of column (x0 + xhi + 36); everything above and
 // to the left of the macroblock holding that sample is final once it is.
-__device__ __noinline__ bool wait_window(const Ctx c, PipeWait* pw, int xhi, int yhi) {
-  const FrameParams& fp = *c.fp;
-  if (!pw) return true;
-  const int x0 = c.mbx * 16, y0 = c.mby * 16;
-  const int xb = (x0 + xhi + 36) >> 4, rb = (y0 + yhi + 28) >> 4;
-  const int rr = min(max(rb, 0), fp.mb_h - 1), xx = min(max(xb, 0), fp.mb_w - 1);
-  const int row = rr < fp.mb_h - 1 ? rr + 1 : rr, need = rr < fp.mb_h - 1 ? xx + 1 : min(xx + 2, fp.mb_w);
-  pw->reach_y = max(pw->reach_y, max(rr - c.mby - 2, 0) + 1);
-  pw->reach_x = max(pw->reach_x, max(xx - c.mbx - 2, 0) + 1);
-  if (row != pw->db_row) {
-    pw->db_row = row;
-    pw->seen_db = 0;
-  }
-  if (!wait_seen(pw->db_prev + row, need, pw->seen_db, pw->error, pw->timeout_ns)) {
-    pw->failed = true;
-    return false;
-  }
-  return true;
+__device__ __forceinline__ bool wait_window(const Ctx c, const PipeWait& pw, int xhi, int yhi) {
+  return !pw.db_prev || wait_reference(c, pw, (c.mbx * 16 + xhi + 36) >> 4, (c.mby * 16 + yhi + 28) >> 4);
 }
 
 // P_Skip probe of the plain form (enc.rs:2906 try_p_skip) at skip vector (ps0, ps1): true when the
 // macroblock is coded as P_Skip (prediction left in pred_y / pred_u / pred_v).
 __device__ __noinline__ bool skip_probe(const Ctx c, int ps0, int ps1, const Bounds& bd) {
-  const FrameParams& fp = *c.fp;
-  const StreamDev& sd = *c.sd;
+  const FrameParams& fp = sm.fp;
+  const StreamDev& sd = sm.sd;
   const int lane = lane_id();
   if (!in_bounds(bd, ps0, ps1)) return false;
   mc_luma16(sd.ref_y, fp.stride_y, c.mbx * 16, c.mby * 16, ps0, ps1);
@@ -553,8 +537,8 @@ __device__ __noinline__ int2 learned_centre(const Ctx c, int mvp0, int mvp1, uin
   constexpr int n = kCentreCands;
   int bx, by;
   const int lane = lane_id();
-  const int stride = c.fp->stride_y;
-  const uint8_t* base = c.sd->ref_y + (long)(c.mby * 16 + (lane >> 1)) * stride + c.mbx * 16 + (lane & 1) * 8;
+  const int stride = sm.fp.stride_y;
+  const uint8_t* base = sm.sd.ref_y + (long)(c.mby * 16 + (lane >> 1)) * stride + c.mbx * 16 + (lane & 1) * 8;
   const uint2 sv = src8();
   uint2 r[kCentreCands];
 #pragma unroll
@@ -584,10 +568,11 @@ __device__ __constant__ int8_t c_type_parts[4] = {1, 2, 2, 4};
 // quadrants covered by part k (bit mask)
 __device__ __constant__ uint8_t c_part_quads[9] = {15, 3, 12, 5, 10, 1, 2, 4, 8};
 
-// One macroblock of a P slice in the search forms (see the head of this file).
-__device__ __noinline__ void analyse_p_mb_search(const Ctx c, PipeWait* pw) {
-  const FrameParams& fp = *c.fp;
-  const StreamDev& sd = *c.sd;
+// One macroblock of a P slice in the search forms (see the head of this file); false when a wait for
+// the reference picture gave up.
+__device__ __noinline__ bool analyse_p_mb_search(const Ctx c, const PipeWait pw) {
+  const FrameParams& fp = sm.fp;
+  const StreamDev& sd = sm.sd;
   const int lane = lane_id();
   const int mbx = c.mbx, mby = c.mby;
   const int x0 = mbx * 16, y0 = mby * 16;
@@ -649,12 +634,12 @@ __device__ __noinline__ void analyse_p_mb_search(const Ctx c, PipeWait* pw) {
     if (!part_mask) part_mask = 1;
   }
   // the reference region of the skip probe and the search window (learned: every candidate's)
-  if (!wait_window(c, pw, max(xhi, (max(ps0, 0) + 3) >> 2), max(yhi, (max(ps1, 0) + 3) >> 2))) return;
+  if (!wait_window(c, pw, max(xhi, (max(ps0, 0) + 3) >> 2), max(yhi, (max(ps1, 0) + 3) >> 2))) return false;
   // 1. skip probe
   if (skip_probe(c, ps0, ps1, bd)) {
     code_skip(c, ps0, ps1);
     search_tail(c, 255, false, ps0, ps1);
-    return;
+    return true;
   }
   // 2. integer search
   if (hint) {
@@ -676,7 +661,7 @@ __device__ __noinline__ void analyse_p_mb_search(const Ctx c, PipeWait* pw) {
       xhi = min(cx + kLearnedRange, imax0);
       ylo = max(cy - kLearnedRange, imin1);
       yhi = min(cy + kLearnedRange, imax1);
-      if (!wait_window(c, pw, xhi, yhi)) return;
+      if (!wait_window(c, pw, xhi, yhi)) return false;
       int_search(c, xlo, xhi, ylo, yhi, mvp16[0], mvp16[1], lambda);
       edge = (ib.x[0] == xlo && xlo > imin0) || (ib.x[0] == xhi && xhi < imax0) ||
              (ib.y[0] == ylo && ylo > imin1) || (ib.y[0] == yhi && yhi < imax1);
@@ -684,7 +669,7 @@ __device__ __noinline__ void analyse_p_mb_search(const Ctx c, PipeWait* pw) {
     if (edge) {  // the walk did not reach the minimum: full search
       xlo = max(fcx - R, imin0); xhi = min(fcx + R, imax0);
       ylo = max(fcy - R, imin1); yhi = min(fcy + R, imax1);
-      if (!wait_window(c, pw, xhi, yhi)) return;
+      if (!wait_window(c, pw, xhi, yhi)) return false;
       int_search(c, xlo, xhi, ylo, yhi, mvp16[0], mvp16[1], lambda);
     }
   }
@@ -749,7 +734,7 @@ __device__ __noinline__ void analyse_p_mb_search(const Ctx c, PipeWait* pw) {
     if (fit16.cost + lambda * 8 < best_j) {
       code_i16(c, fit16.mode, ht, hl, k0);
       search_tail(c, best_t, false, 0, 0);
-      return;
+      return true;
     }
   }
   // residual, late skip (a 16x16 macroblock at the skip vector), record and reconstruction
@@ -758,6 +743,7 @@ __device__ __noinline__ void analyse_p_mb_search(const Ctx c, PipeWait* pw) {
   const bool skipped = code_inter(c, type, best_t == 0 && bmv[0][0] == ps0 && bmv[0][1] == ps1, bmv[0][0], bmv[0][1],
                                   bmvd[0][0], bmvd[0][1]);
   search_tail(c, best_t, !skipped, ps0, ps1);
+  return true;
 }
 
 // One macroblock of an I slice in the search forms: the plain analysis (enc.rs:3311 code_intra),
@@ -765,10 +751,10 @@ __device__ __noinline__ void analyse_p_mb_search(const Ctx c, PipeWait* pw) {
 __device__ __noinline__ void analyse_intra_mb_search(const Ctx c) {
   const Corner k0 = load_edges(c, true);
   bool ht = c.mby > 0, hl = c.mbx > 0;
-  uint32_t lambda = c_lambda[c.sd->qp];
+  uint32_t lambda = c_lambda[sm.sd.qp];
   const I16Fit fit16 = analyse_i16(ht, hl, k0.y);
   if (fit16.cost > 40 * lambda) {
-    const uint16_t* masks = c.sd->hint ? c.sd->hint[c.mb].i4_mask : nullptr;
+    const uint16_t* masks = sm.sd.hint ? sm.sd.hint[c.mb].i4_mask : nullptr;
     const int cbpl = masks ? analyse_i4<true>(c, fit16.cost + lambda * 4, ht, hl, k0.y, masks)
                            : analyse_i4<false>(c, fit16.cost + lambda * 4, ht, hl, k0.y, nullptr);
     if (cbpl >= 0) {
