@@ -27,15 +27,22 @@ namespace {
 constexpr unsigned FULL = 0xffffffffu;
 constexpr uint32_t UMAX = 0xffffffffu;
 
-__constant__ uint16_t c_lambda[52];
-__constant__ uint8_t c_dec4[16];
-__constant__ uint8_t c_dec8[64];
-__constant__ uint8_t c_scan4[16];
-__constant__ uint8_t c_scan8[64];
-__constant__ uint16_t c_mf4[6][3];
-__constant__ uint8_t c_dq4[6][3];
-__constant__ uint16_t c_mf8[6][6];
-__constant__ uint8_t c_dq8[6][6];
+// Everything the analysis needs of one QP, in the form its lanes use it (upload_tables); a warp keeps
+// its picture's luma and chroma entries in shared memory (load_desc).
+struct QTab {
+  uint32_t mf[2][2];   // quantiser scales of a 4x4 half (quant_half): [coefficient rows h, h + 2][column parity]
+  int32_t dq[2][2];    // dequantiser scales alike, shifted by qp / 6
+  uint32_t bias[2];    // inter, intra
+  uint32_t shift;
+  int32_t dc_mf, dc_dq;  // DC transforms: quantiser scale, dequantiser scale
+  uint32_t lambda;
+  uint32_t mf8[3][3];  // 8x8: [column 0, odd, 2 of four][row 0, odd, 2 of four]
+  int32_t dq8[3][3];
+  uint32_t bias8;
+  int32_t rnd8, sh8;   // dequantised level = (level * dq8 + rnd8) >> sh8
+};
+__device__ QTab g_qtab[52];
+constexpr int kQTabWords = (int)(sizeof(QTab) / 4), kQTabWords4 = (int)(offsetof(QTab, mf8) / 4);  // all, and chroma's
 __constant__ uint8_t c_cqp[52];
 __constant__ uint8_t c_alpha[52];
 __constant__ uint8_t c_beta[52];
@@ -46,6 +53,8 @@ __constant__ uint8_t c_tc0[52][3];
 // Block stride (words) of the 8x8 intermediates: 8 banks apart, so the four blocks' rows and columns
 // fall into different banks.
 constexpr int kT8Block = 72;
+// A plane of the interpolation window: 23 rows of 24 samples.
+constexpr int kWinPlane = 23 * 24 + 8;
 struct __align__(16) Smem {
   uint8_t src_y[256];
   uint8_t src_u[64];
@@ -54,15 +63,17 @@ struct __align__(16) Smem {
   uint8_t pred_u[64];
   uint8_t pred_v[64];
   uint8_t tmp_y[256];       // plane prediction / I4x4 reconstruction
-  alignas(16) uint8_t win[23 * 24];  // integer samples of a half-sample window (rows -2.., cols -2..)
-  // The half-sample planes live until the sub-pel search ends; the 8x8 transform's intermediates
-  // are needed only after it (the residual), so they share the space.
+  // Samples around an integer position of the reference (ensure_window): plane 0 the integer samples
+  // (23 rows of 24 from two rows / columns above-left of one sample above-left of the position), and
+  // on the same grid b (between a sample and its right neighbour), h (and the one below) and j (the
+  // four); rows and columns 2..19 of those hold values.
+  alignas(16) uint8_t win[kWinPlane];
+  // The half-sample planes live until the prediction is made; the 8x8 transform's intermediates are
+  // needed only after it (the residual), so they share the space.
   union alignas(16) {
     struct {
-      uint8_t hph[18 * 20];  // b samples (horizontal half)
-      uint8_t hpv[18 * 20];  // h samples (vertical half)
-      uint8_t hpj[18 * 20];  // j samples (centre)
-      int16_t hr[23 * 18];   // unrounded horizontal 6-tap sums
+      uint8_t hp[3][kWinPlane];     // b, h, j
+      alignas(8) int16_t hr[23 * 20];  // unrounded horizontal 6-tap sums, columns 0..19
     };
     int32_t t8[4 * kT8Block];  // 8x8 transform intermediates, block b at [kT8Block b]
   };
@@ -73,12 +84,16 @@ struct __align__(16) Smem {
   alignas(16) int16_t cdc[8];
   int16_t ldc[16];          // I16x16 DC levels, raster
   int16_t ldcr[16];         // I16x16 DC reconstruction, raster
-  uint8_t top[24];          // luma row above the macroblock (x0 .. x0 + 23)
-  uint8_t left[16];
-  uint8_t ctop[2][8];
+  alignas(4) uint8_t top[24];  // luma row above the macroblock (x0 .. x0 + 23)
+  alignas(4) uint8_t left[16];
+  alignas(4) uint8_t ctop[2][8];
   uint8_t cleft[2][8];
   alignas(16) StreamDev sd;       // the picture worked on (load_desc) and its stream's size (load_params)
   alignas(16) FrameParams fp;
+  alignas(16) QTab qt[2];         // the picture's luma and chroma QP
+  int qt_qp;                      // the luma QP they are of
+  uint32_t qpt[16];               // quarter-sample phases: the two planes averaged (init_tables)
+  int win_x, win_y, win_have;     // ensure_window: the position held (kNoWin: none), its planes built (bits 0..2)
   int db_row, seen_db;            // last acquired progress db_prev[db_row] of the reference picture
   int reach_y, reach_x;           // 1 + the largest reach waited for beyond zero motion, in macroblocks
   alignas(16) uint8_t i4m[16];    // Intra4x4PredMode of this macroblock (decoding order)
@@ -102,6 +117,7 @@ __shared__ Smem sm;
 __device__ __forceinline__ uint8_t* sm_at(int off) { return (uint8_t*)&sm + off; }
 
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
+__device__ __forceinline__ uint32_t pack16(int lo, int hi) { return __byte_perm((uint32_t)lo, (uint32_t)hi, 0x5410); }
 __device__ __forceinline__ MbInfo ld_info(const MbInfo* p) {
   int4 v = *(const int4*)p;
   MbInfo m;
@@ -109,19 +125,12 @@ __device__ __forceinline__ MbInfo ld_info(const MbInfo* p) {
   return m;
 }
 __device__ __forceinline__ uint32_t wsum(uint32_t v) { return __reduce_add_sync(FULL, v); }
-__device__ __forceinline__ uint32_t wor(uint32_t v) { return __reduce_or_sync(FULL, v); }
 __device__ __forceinline__ int clip255(int v) { return v < 0 ? 0 : (v > 255 ? 255 : v); }
 __device__ __forceinline__ int16_t clamp_i16(int v) { return (int16_t)(v < -32768 ? -32768 : (v > 32767 ? 32767 : v)); }
 
 // Column and row of 4x4 block b in decoding order (enc.rs:522 blk_xy).
 __device__ __forceinline__ int blk_x(int b) { return (b & 1) + ((b >> 1) & 2); }
 __device__ __forceinline__ int blk_y(int b) { return ((b >> 1) & 1) + ((b >> 2) & 2); }
-// Position class of raster coefficient i in a 4x4 block (h264.rs:1204).
-__device__ __forceinline__ int pos4(int i) {
-  int r = i >> 2, c = i & 3;
-  if (((r | c) & 1) == 0) return 0;
-  return ((r & c) & 1) ? 1 : 2;
-}
 __device__ __forceinline__ int chroma_qp(int qp) { return c_cqp[qp < 0 ? 0 : (qp > 51 ? 51 : qp)]; }
 // Bits of se(v) (enc.rs:546).
 __device__ __forceinline__ uint32_t se_bits(int d) {
@@ -151,38 +160,7 @@ __device__ __forceinline__ uint2 ldg8(const uint8_t* p) {
 __device__ __forceinline__ uint32_t vsad8(uint2 a, uint2 b) { return __vsadu4(a.x, b.x) + __vsadu4(a.y, b.y); }
 
 // ---------------------------------------------------------------------------------------------
-// Per-lane transforms (crates/ragdoll-simd/src/fixed.rs:104,192,322; h264_idct.rs:225)
-__device__ __forceinline__ void fdct4(const int* d, int* o) {
-  int t[16];
-#pragma unroll
-  for (int r = 0; r < 4; r++) {
-    int s03 = d[r * 4] + d[r * 4 + 3], s12 = d[r * 4 + 1] + d[r * 4 + 2];
-    int d03 = d[r * 4] - d[r * 4 + 3], d12 = d[r * 4 + 1] - d[r * 4 + 2];
-    t[r * 4] = s03 + s12; t[r * 4 + 1] = 2 * d03 + d12; t[r * 4 + 2] = s03 - s12; t[r * 4 + 3] = d03 - 2 * d12;
-  }
-#pragma unroll
-  for (int c = 0; c < 4; c++) {
-    int s03 = t[c] + t[c + 12], s12 = t[c + 4] + t[c + 8], d03 = t[c] - t[c + 12], d12 = t[c + 4] - t[c + 8];
-    o[c] = (int16_t)(s03 + s12); o[c + 4] = (int16_t)(2 * d03 + d12);
-    o[c + 8] = (int16_t)(s03 - s12); o[c + 12] = (int16_t)(d03 - 2 * d12);
-  }
-}
-__device__ __forceinline__ void idct4(const int* c, int* o) {
-  int t[16];
-#pragma unroll
-  for (int r = 0; r < 4; r++) {
-    int e0 = c[r * 4] + c[r * 4 + 2], e1 = c[r * 4] - c[r * 4 + 2];
-    int e2 = (c[r * 4 + 1] >> 1) - c[r * 4 + 3], e3 = c[r * 4 + 1] + (c[r * 4 + 3] >> 1);
-    t[r * 4] = e0 + e3; t[r * 4 + 1] = e1 + e2; t[r * 4 + 2] = e1 - e2; t[r * 4 + 3] = e0 - e3;
-  }
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    int e0 = t[k] + t[k + 8], e1 = t[k] - t[k + 8];
-    int e2 = (t[k + 4] >> 1) - t[k + 12], e3 = t[k + 4] + (t[k + 12] >> 1);
-    o[k] = (int16_t)((e0 + e3 + 32) >> 6); o[k + 4] = (int16_t)((e1 + e2 + 32) >> 6);
-    o[k + 8] = (int16_t)((e1 - e2 + 32) >> 6); o[k + 12] = (int16_t)((e0 - e3 + 32) >> 6);
-  }
-}
+// Per-lane 8-point transforms (crates/ragdoll-simd/src/fixed.rs:392; h264_idct.rs:225)
 // One row / column of the 8x8 forward transform (fixed.rs:392).
 __device__ __forceinline__ void fdct8_1d(const int* a, int* o) {
   int a0 = a[0] + a[7], a1 = a[1] + a[6], a2 = a[2] + a[5], a3 = a[3] + a[4];
@@ -230,56 +208,132 @@ __device__ __forceinline__ int inv4_pass(int v, int step, int i) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// Half-sample window (h264_enc.rs:747 hpel_window, :803 hpel_window_centre): integer origin
-// (ox, oy); plane coordinate (r, c) is the sample at (ox + c, oy + r).
-__device__ __noinline__ void stage_window(const uint8_t* ref, int stride, int ox, int oy) {
-  int lane = lane_id();
+// Half-sample window (h264_enc.rs:747 hpel_window, :803 hpel_window_centre) around the integer
+// position (px, py) of a 16x16 block: quarter-sample vectors up to 3 away from it. Window row y,
+// column x is the sample at (px - 3 + x, py - 3 + y); the block itself starts at (3, 3).
+constexpr int kNoWin = 1 << 20;
+__device__ __forceinline__ void stage_window(int px, int py) {
+  const int lane = lane_id(), stride = sm.fp.stride_y;
+  const uint8_t* ref = sm.sd.ref_y + (long)(py - 3) * stride + px - 3;
+  const uint32_t sh = (uint32_t)((uintptr_t)ref & 3) * 8u;  // rows are 64-byte multiples apart
+  ref = (const uint8_t*)((uintptr_t)ref & ~(uintptr_t)3);
   // 23 rows x 6 words: five words per lane, all loads issued before the first use
-  uint32_t lo[5], hi[5], sh[5];
+  uint32_t lo[5], hi[5];
 #pragma unroll
   for (int r = 0; r < 5; r++) {
-    int q = min(lane + 32 * r, 23 * 6 - 1);
-    int k = q / 6, w = q - 6 * (q / 6);
-    uintptr_t a = (uintptr_t)(ref + (long)(oy - 2 + k) * stride + (ox - 2) + 4 * w);
-    const uint32_t* b = (const uint32_t*)(a & ~(uintptr_t)3);
-    sh[r] = (uint32_t)(a & 3) * 8u;
+    const int q = min(lane + 32 * r, 23 * 6 - 1), k = q / 6, w = q - 6 * k;
+    const uint32_t* b = (const uint32_t*)(ref + k * stride + 4 * w);
     lo[r] = b[0];
     hi[r] = b[1];
   }
 #pragma unroll
   for (int r = 0; r < 5; r++) {
-    int q = lane + 32 * r;
-    if (q < 23 * 6) {
-      int k = q / 6, w = q - 6 * (q / 6);
-      *(uint32_t*)&sm.win[k * 24 + 4 * w] = __funnelshift_r(lo[r], hi[r], sh[r]);
-    }
+    const int q = lane + 32 * r;
+    if (q < 23 * 6) *(uint32_t*)&sm.win[4 * q] = __funnelshift_r(lo[r], hi[r], sh);
   }
-  __syncwarp();
 }
-// need: bit 0 b plane (h), bit 1 h plane (v), bit 2 j plane (c)
-__device__ __noinline__ void build_hpel(int need) {
-  int lane = lane_id();
-  if (need & 5) {
-    for (int i = lane; i < 23 * 18; i += 32) {
-      int k = i / 18, c = i - k * 18;
-      const uint8_t* w = &sm.win[k * 24 + c];
-      sm.hr[i] = (int16_t)(w[0] - 5 * w[1] + 20 * w[2] + 20 * w[3] - 5 * w[4] + w[5]);
+__device__ __forceinline__ int dp4a_us(uint32_t a, int b, int c) {
+  int d;
+  asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  return d;
+}
+__device__ __forceinline__ int dp2a_ss(uint32_t a, int b, int c) {
+  int d;
+  asm("dp2a.lo.s32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  return d;
+}
+constexpr int taps4(int t0, int t1, int t2, int t3) {
+  return (t0 & 255) | ((t1 & 255) << 8) | ((t2 & 255) << 16) | (int)((unsigned)(t3 & 255) << 24);
+}
+__device__ __forceinline__ uint32_t pack_clip(int a, int b, int c, int d) {
+  return (uint32_t)clip255(a) | ((uint32_t)clip255(b) << 8) | ((uint32_t)clip255(c) << 16) | ((uint32_t)clip255(d) << 24);
+}
+// The 6-tap filter (1, -5, 20, 20, -5, 1) along rows: four outputs of an item from three words by
+// byte dot products; the unrounded sums for j, and plane b of rows 2..19.
+__device__ __forceinline__ void build_b() {
+#pragma unroll 1
+  for (int i = lane_id(); i < 23 * 5; i += 32) {
+    const int y = i / 5, k = i - 5 * y;
+    const uint32_t* w = (const uint32_t*)&sm.win[y * 24 + 4 * k];
+    const uint32_t w0 = w[-1], w1 = w[0], w2 = w[1];  // (word -1 of item 0: columns 0, 1, never read)
+    const int h0 = dp4a_us(w0, taps4(0, 0, 1, -5), dp4a_us(w1, taps4(20, 20, -5, 1), 0));
+    const int h1 = dp4a_us(w0, taps4(0, 0, 0, 1), dp4a_us(w1, taps4(-5, 20, 20, -5), dp4a_us(w2, taps4(1, 0, 0, 0), 0)));
+    const int h2 = dp4a_us(w1, taps4(1, -5, 20, 20), dp4a_us(w2, taps4(-5, 1, 0, 0), 0));
+    const int h3 = dp4a_us(w1, taps4(0, 1, -5, 20), dp4a_us(w2, taps4(20, -5, 1, 0), 0));
+    *(uint2*)&sm.hr[y * 20 + 4 * k] = make_uint2(pack16(h0, h1), pack16(h2, h3));
+    if (y >= 2 && y < 20)
+      *(uint32_t*)&sm.hp[0][y * 24 + 4 * k] = pack_clip((h0 + 16) >> 5, (h1 + 16) >> 5, (h2 + 16) >> 5, (h3 + 16) >> 5);
+  }
+}
+// Down the columns: lane = (word column, three rows); two samples per word in 16-bit halves, biased by
+// 80 << 5 so that no half goes negative.
+__device__ __forceinline__ void build_h() {
+  const int lane = lane_id(), seg = lane / 5, k = lane - 5 * seg;
+  if (seg > 5) return;
+  const uint8_t* w = &sm.win[3 * seg * 24 + 4 * k];
+  uint32_t e[8], o[8];
+#pragma unroll
+  for (int r = 0; r < 8; r++) {
+    const uint32_t v = *(const uint32_t*)(w + r * 24);
+    e[r] = v & 0x00ff00ffu;
+    o[r] = (v >> 8) & 0x00ff00ffu;
+  }
+  auto tap = [](const uint32_t* a) {
+    const uint32_t v = (a[0] + a[5]) + 20u * (a[2] + a[3]) + 0x0a100a10u - 5u * (a[1] + a[4]);
+    return __vminu2(__vmaxu2((v >> 5) & 0x07ff07ffu, 0x00500050u), 0x014f014fu) - 0x00500050u;
+  };
+#pragma unroll
+  for (int r = 0; r < 3; r++) *(uint32_t*)&sm.hp[1][(3 * seg + 2 + r) * 24 + 4 * k] = tap(e + r) | (tap(o + r) << 8);
+}
+// j: the filter down the unrounded row sums, the same split, by 16-bit dot products of vertical pairs.
+__device__ __forceinline__ void build_j() {
+  const int lane = lane_id(), seg = lane / 5, k = lane - 5 * seg;
+  if (seg > 5) return;
+  uint32_t r[3] = {0u, 0u, 0u};
+#pragma unroll 1
+  for (int half = 0; half < 2; half++) {  // two columns
+    uint32_t v[8];
+#pragma unroll
+    for (int y = 0; y < 8; y++) v[y] = *(const uint32_t*)&sm.hr[(3 * seg + y) * 20 + 4 * k + 2 * half];
+    int j[3][2];
+#pragma unroll
+    for (int x = 0; x < 2; x++) {
+      uint32_t w[7];
+#pragma unroll
+      for (int y = 0; y < 7; y++) w[y] = __byte_perm(v[y], v[y + 1], x ? 0x7632 : 0x5410);
+#pragma unroll
+      for (int y = 0; y < 3; y++)
+        j[y][x] = dp2a_ss(w[y], taps4(1, -5, 0, 0), dp2a_ss(w[y + 2], taps4(20, 20, 0, 0), dp2a_ss(w[y + 4], taps4(-5, 1, 0, 0), 512))) >> 10;
     }
+#pragma unroll
+    for (int y = 0; y < 3; y++)
+      r[y] = (r[y] >> 16) | ((uint32_t)clip255(j[y][0]) << 16) | ((uint32_t)clip255(j[y][1]) << 24);
+  }
+#pragma unroll
+  for (int y = 0; y < 3; y++) *(uint32_t*)&sm.hp[2][(3 * seg + 2 + y) * 24 + 4 * k] = r[y];
+}
+// Makes the window around (px, py) hold its integer samples and the planes of `need` (bit 0 b, bit 1
+// h, bit 2 j); what is there already is kept.
+__device__ __noinline__ void ensure_window(int px, int py, int need) {
+  int have = sm.win_have;
+  if (sm.win_x != px || sm.win_y != py) {
+    __syncwarp();
+    stage_window(px, py);
+    have = 0;
   }
   __syncwarp();
-  for (int i = lane; i < 18 * 18; i += 32) {
-    int r = i / 18, c = i - r * 18;
-    if (need & 1) sm.hph[r * 20 + c] = (uint8_t)clip255((sm.hr[(r + 2) * 18 + c] + 16) >> 5);
-    if (need & 2) {
-      const uint8_t* w = &sm.win[r * 24 + c + 2];
-      int v = w[0] - 5 * w[24] + 20 * w[48] + 20 * w[72] - 5 * w[96] + w[120];
-      sm.hpv[r * 20 + c] = (uint8_t)clip255((v + 16) >> 5);
-    }
-    if (need & 4) {
-      const int16_t* t = &sm.hr[r * 18 + c];
-      int j = t[0] - 5 * t[18] + 20 * t[36] + 20 * t[54] - 5 * t[72] + t[90];
-      sm.hpj[r * 20 + c] = (uint8_t)clip255((j + 512) >> 10);
-    }
+  const int miss = need & ~have;
+  if ((miss & 5) && !(have & 1)) { build_b(); have |= 1; }
+  if (miss & 2) { build_h(); have |= 2; }
+  if (miss & 4) {
+    __syncwarp();
+    build_j();
+    have |= 4;
+  }
+  if (lane_id() == 0) {
+    sm.win_x = px;
+    sm.win_y = py;
+    sm.win_have = have;
   }
   __syncwarp();
 }
@@ -293,38 +347,16 @@ __device__ __forceinline__ int planes_needed(int fx, int fy) {
   if (fy == 2) return 6;
   return 3;
 }
-// Quarter-sample prediction of the 16x16 block whose integer position is (wx, wy) in window
-// coordinates: one window plane, or the rounded average of two (window_src, enc.rs:1395; equal
-// to h264_luma_mc_scalar, h264_mc.rs:148, by enc.rs:4030). Returns the two source rows' bases.
-// (byte offsets in Smem).
-struct QSrc {
-  int a, b, sa, sb, avg;
-};
-__device__ __noinline__ QSrc qpel_src(int wx, int wy, int fx, int fy) {
-  const int G = (int)offsetof(Smem, win) + (wy + 2) * 24 + wx + 2;
-  const int B = (int)offsetof(Smem, hph) + wy * 20 + wx;
-  const int V = (int)offsetof(Smem, hpv) + wy * 20 + wx;
-  const int J = (int)offsetof(Smem, hpj) + wy * 20 + wx;
-  switch (fx | (fy << 2)) {
-    case 0: return {G, G, 24, 24, 0};
-    case 1: return {G, B, 24, 20, 1};
-    case 2: return {B, B, 20, 20, 0};
-    case 3: return {B, G + 1, 20, 24, 1};
-    case 4: return {G, V, 24, 20, 1};
-    case 5: return {B, V, 20, 20, 1};
-    case 6: return {B, J, 20, 20, 1};
-    case 7: return {B, V + 1, 20, 20, 1};
-    case 8: return {V, V, 20, 20, 0};
-    case 9: return {V, J, 20, 20, 1};
-    case 10: return {J, J, 20, 20, 0};
-    case 11: return {J, V + 1, 20, 20, 1};
-    case 12: return {V, G + 24, 20, 24, 1};
-    case 13: return {V, B + 20, 20, 20, 1};
-    case 14: return {J, B + 20, 20, 20, 1};
-    default: return {V + 1, B + 20, 20, 20, 1};
-  }
+// Quarter-sample prediction (window_src, enc.rs:1395; equal to h264_luma_mc_scalar, h264_mc.rs:148, by
+// enc.rs:4030): phase fx | fy << 2 is the rounded average of two planes at fixed offsets, the same one
+// twice where it is a plane itself. The offsets, in bytes from sm.win, packed in sm.qpt.
+constexpr uint32_t qpel_entry(int phase) {
+  constexpr uint32_t P = kWinPlane, B = (uint32_t)(offsetof(Smem, hp) - offsetof(Smem, win)), V = B + P, J = V + P;
+  constexpr uint32_t a[16] = {0, 0, B, B, 0, B, B, B, V, V, J, J, V, V, J, V + 1};
+  constexpr uint32_t b[16] = {0, B, B, 1, V, V, J, V + 1, V, J, J, V + 1, 24, B + 24, B + 24, B + 24};
+  return a[phase] | (b[phase] << 16);
 }
-// 8 bytes of shared memory at any alignment (rows of the window planes are 4-byte aligned).
+// 8 bytes of shared memory at any alignment.
 __device__ __forceinline__ uint2 lds8(const uint8_t* p) {
   uintptr_t a = (uintptr_t)p;
   const uint32_t* b = (const uint32_t*)(a & ~(uintptr_t)3);
@@ -332,42 +364,58 @@ __device__ __forceinline__ uint2 lds8(const uint8_t* p) {
   uint32_t w0 = b[0], w1 = b[1], w2 = b[2];
   return make_uint2(__funnelshift_r(w0, w1, sh), __funnelshift_r(w1, w2, sh));
 }
-// This lane's 8 prediction samples (row lane/2, columns 8 (lane&1) ..) packed in two words.
-__device__ __forceinline__ uint2 qpel8(const QSrc& q) {
-  int lane = lane_id(), i = lane >> 1, j0 = (lane & 1) * 8;
-  uint2 a = lds8(sm_at(q.a + i * q.sa + j0));
-  if (!q.avg) return a;
-  uint2 b = lds8(sm_at(q.b + i * q.sb + j0));
+// Offset in a plane of the sample a quarter-sample vector (dx, dy) from the window's position points
+// at, for the block's sample (0, 0).
+__device__ __forceinline__ int qpel_pos(int dx, int dy) { return ((dy >> 2) + 3) * 24 + (dx >> 2) + 3; }
+// This lane's 8 prediction samples (row lane / 2, columns 8 (lane & 1) ..) for the vector (dx, dy) from
+// the window's position.
+__device__ __noinline__ uint2 qpel8(int dx, int dy) {
+  const int lane = lane_id(), at = qpel_pos(dx, dy) + (lane >> 1) * 24 + (lane & 1) * 8;
+  const uint32_t e = sm.qpt[(dx & 3) | ((dy & 3) << 2)];
+  const uint2 a = lds8(&sm.win[0] + at + (e & 0xffffu)), b = lds8(&sm.win[0] + at + (e >> 16));
   return make_uint2(__vavgu4(a.x, b.x), __vavgu4(a.y, b.y));
 }
 // Cost of a full-pel position (mx, my): the warp's SAD of the 16x16 block (this lane's 8 source
 // samples sv against its 8 reference samples r) plus lambda * bits of the vector difference to
-// the predictor (enc.rs:1207 cost). Shared by the candidates and the diamond steps.
+// the predictor (enc.rs:1207 cost).
 __device__ __noinline__ uint32_t fullpel_cost(uint2 sv, uint2 r, int mx, int my, int mvp0, int mvp1, uint32_t lambda) {
   return wsum(vsad8(sv, r)) + mvd_cost(mx * 4 - mvp0, lambda) + mvd_cost(my * 4 - mvp1, lambda);
 }
-// This lane's SAD against the quarter-sample prediction at window position (wx, wy), phase
-// (fx, fy): shared by the candidates of the sub-pel search.
-__device__ __noinline__ uint32_t qpel_sad(uint2 sv, int wx, int wy, int fx, int fy) {
-  return vsad8(sv, qpel8(qpel_src(wx, wy, fx, fy)));
+// The cheapest of the four neighbours of (x, y) at distance st (quarter samples) inside the bounds:
+// up, left, right, down, the first on ties. s01, s23: this lane's share of their SADs, two to a word
+// (a 16x16 SAD fits 16 bits). Lane k costs neighbour k. Returns cost << 2 | k, all ones when none is
+// inside. exact_bits: vector bits by vec_cost's rule, without mvd_cost's 16-bit wrap.
+struct Box {
+  int lo0, hi0, lo1, hi1;
+};
+__device__ __noinline__ uint32_t best4(uint32_t s01, uint32_t s23, int x, int y, int st, Box b, int mvp0, int mvp1, uint32_t lambda,
+                                       bool exact_bits) {
+  s01 = wsum(s01);
+  s23 = wsum(s23);
+  const int k = lane_id() & 3;
+  x += k == 1 ? -st : (k == 2 ? st : 0);
+  y += k == 0 ? -st : (k == 3 ? st : 0);
+  const uint32_t sad = ((k & 2 ? s23 : s01) >> (16 * (k & 1))) & 0xffffu;
+  const uint32_t cost = sad + (exact_bits ? lambda * (se_bits(x - mvp0) + se_bits(y - mvp1))
+                                          : mvd_cost(x - mvp0, lambda) + mvd_cost(y - mvp1, lambda));
+  const bool ok = x >= b.lo0 && x <= b.hi0 && y >= b.lo1 && y <= b.hi1;
+  return __reduce_min_sync(FULL, ok ? (cost << 2) | (uint32_t)k : UMAX);
 }
 __device__ __forceinline__ uint2 src8() {
   int lane = lane_id();
   return *(const uint2*)&sm.src_y[(lane >> 1) * 16 + (lane & 1) * 8];
 }
-// Prediction of the 16x16 block displaced by mv into pred_y (enc.rs:1058 mc_luma).
-__device__ __noinline__ void mc_luma16(const uint8_t* ref, int stride, int x0, int y0, int mvx, int mvy) {
-  int ix = x0 + (mvx >> 2), iy = y0 + (mvy >> 2), fx = mvx & 3, fy = mvy & 3;
-  int lane = lane_id();
+// Prediction of the 16x16 block at (x0, y0) displaced by mv into pred_y (enc.rs:1058 mc_luma). A
+// fractional vector leaves its window behind for the sub-pel search, which often starts there.
+__device__ __noinline__ void mc_luma16(int x0, int y0, int mvx, int mvy) {
+  const int ix = x0 + (mvx >> 2), iy = y0 + (mvy >> 2), fx = mvx & 3, fy = mvy & 3, lane = lane_id();
+  uint2 v;
   if ((fx | fy) == 0) {
-    uint2 v = ldg8(ref + (long)(iy + (lane >> 1)) * stride + ix + (lane & 1) * 8);
-    *(uint2*)&sm.pred_y[(lane >> 1) * 16 + (lane & 1) * 8] = v;
-    __syncwarp();
-    return;
+    v = ldg8(sm.sd.ref_y + (long)(iy + (lane >> 1)) * sm.fp.stride_y + ix + (lane & 1) * 8);
+  } else {
+    ensure_window(ix, iy, planes_needed(fx, fy));
+    v = qpel8(fx, fy);
   }
-  stage_window(ref, stride, ix, iy);
-  build_hpel(planes_needed(fx, fy));
-  uint2 v = qpel8(qpel_src(0, 0, fx, fy));
   *(uint2*)&sm.pred_y[(lane >> 1) * 16 + (lane & 1) * 8] = v;
   __syncwarp();
 }
@@ -389,17 +437,8 @@ __device__ __noinline__ void mc_chroma8(const uint8_t* ru, const uint8_t* rv, in
 
 // ---------------------------------------------------------------------------------------------
 // Quantisation helpers (enc.rs:1703-1779, h264_enc.rs:408)
-__device__ __forceinline__ void quant4_params(int qp, bool intra, uint32_t& shift, uint32_t& bias) {
-  shift = 15 + qp / 6;
-  bias = (1u << shift) / (intra ? 3u : 6u);
-}
-// Level of coefficient c. Every transform here is of 8-bit differences: |c| is at most 64 * 255 and
-// the scales at most 20972, so the product and the bias fit 32 bits and the level 16.
-__device__ __forceinline__ int quant_level(int c, uint32_t mf, uint32_t bias, uint32_t shift) {
-  uint32_t a = (uint32_t)(c < 0 ? -c : c);
-  int l = (int)((a * mf + bias) >> shift);
-  return c < 0 ? -l : l;
-}
+// (Every transform here is of 8-bit differences: |coefficient| is at most 64 * 255 and the scales at
+// most 20972, so a product and the bias fit 32 bits, and a level 16.)
 
 // ---- 4x4 blocks, two lanes each -----------------------------------------------------------------
 // A macroblock's 4x4 transforms are done all at once: lane 2 b + h holds half of block b, the pixel
@@ -411,39 +450,36 @@ __device__ __forceinline__ int quant_level(int c, uint32_t mf, uint32_t bias, ui
 // of two passes of three dependent shuffles, 7.2 k cycles for the luma quantisation even on a nearly
 // idle SM. With this split (and the record written by words) a 720p stream's launch of 30 pictures
 // went from 21.6 to 17.6 ms, 1080p 8 x 15 from 54.6 to 50.7 ms.
+// A helper is one copy of code for luma and chroma, inter and intra: the warps of an SM run different
+// phases of their macroblocks, and what they fetch is the kernel's scarcest resource (the code of a P
+// macroblock is several times the instruction cache).
 struct Half4 {
   int a[4], b[4];  // its first and second row
 };
-// The lane's two rows (r0 = the first's index) of samples at byte offset `off` in Smem.
+// Rows of samples at byte offset `off` in Smem: the lane's two.
 __device__ __forceinline__ uint2 half_rows(int off, int stride, int h) {
   return make_uint2(*(const uint32_t*)sm_at(off + h * stride), *(const uint32_t*)sm_at(off + (3 - h) * stride));
 }
-__device__ __forceinline__ Half4 half_diff(uint2 s, uint2 p) {
-  Half4 d;
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    d.a[k] = (int)((s.x >> (8 * k)) & 255u) - (int)((p.x >> (8 * k)) & 255u);
-    d.b[k] = (int)((s.y >> (8 * k)) & 255u) - (int)((p.y >> (8 * k)) & 255u);
-  }
-  return d;
-}
-// Forward core transform (fixed.rs:104).
-__device__ __forceinline__ void half_fwd(Half4& v, int h) {
-  auto row = [](int (&r)[4]) {
-    int s03 = r[0] + r[3], s12 = r[1] + r[2], d03 = r[0] - r[3], d12 = r[1] - r[2];
-    r[0] = s03 + s12; r[1] = 2 * d03 + d12; r[2] = s03 - s12; r[3] = d03 - 2 * d12;
+// The column pass of the forward transform and of the Hadamard transform: differences of the lane's
+// rows of s and p, columns 0, 2 and 1, 3 packed as hi * 65536 + lo (sums, differences and small
+// multiples of such pairs are the pairs of the results), then the butterfly with the partner lane.
+// m = 1 + h for the core transform, 1 for Hadamard.
+__device__ __forceinline__ void half_columns(uint2 s, uint2 p, int h, int m, int (&a)[4], int (&b)[4]) {
+  const int ae = (int)(s.x & 0x00ff00ffu) - (int)(p.x & 0x00ff00ffu), be = (int)(s.y & 0x00ff00ffu) - (int)(p.y & 0x00ff00ffu);
+  const int ao = (int)__byte_perm(s.x, 0u, 0x4341) - (int)__byte_perm(p.x, 0u, 0x4341),
+            bo = (int)__byte_perm(s.y, 0u, 0x4341) - (int)__byte_perm(p.y, 0u, 0x4341);
+  // h = 0: sum s03 and difference d03 of rows 0 and 3; h = 1: s12 and d12 of rows 1 and 2
+  auto exchange = [&](int r0, int r1, int& x, int& y) {
+    const int sum = r0 + r1, dif = r0 - r1, o = __shfl_xor_sync(FULL, h ? sum : dif, 1);
+    const int u = h ? o : sum, v = h ? dif : o;  // s03, s12 or d03, d12
+    x = u * m + v;  // row 0: s03 + s12, row 1: 2 d03 + d12
+    y = u - v * m;  // row 2: s03 - s12, row 3: d03 - 2 d12
   };
-  row(v.a);
-  row(v.b);
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    // h = 0: sum s03 and difference d03 of rows 0 and 3; h = 1: s12 and d12 of rows 1 and 2
-    int s = v.a[k] + v.b[k], d = v.a[k] - v.b[k];
-    int o = __shfl_xor_sync(FULL, h ? s : d, 1);
-    int x = h ? o : s, y = h ? d : o;   // s03, s12 or d03, d12
-    v.a[k] = (x << h) + y;              // row 0: s03 + s12, row 1: 2 d03 + d12
-    v.b[k] = x - (y << h);              // row 2: s03 - s12, row 3: d03 - 2 d12
-  }
+  int xe, ye, xo, yo;
+  exchange(ae, be, xe, ye);
+  exchange(ao, bo, xo, yo);
+  a[0] = (int16_t)xe; a[2] = (xe + 0x8000) >> 16; a[1] = (int16_t)xo; a[3] = (xo + 0x8000) >> 16;
+  b[0] = (int16_t)ye; b[2] = (ye + 0x8000) >> 16; b[1] = (int16_t)yo; b[3] = (yo + 0x8000) >> 16;
 }
 // Inverse core transform with its rounding (fixed.rs:192): coefficient rows in, residual rows out.
 __device__ __forceinline__ void half_inv(Half4& v, int h) {
@@ -464,65 +500,8 @@ __device__ __forceinline__ void half_inv(Half4& v, int h) {
     v.b[k] = (x - y + 32) >> 6;
   }
 }
-// This half's share of the block's SATD (metrics.rs:705): a column's four Hadamard outputs are
-// |x + y| and |x - y| of each lane's (x, y), and |x + y| + |x - y| = 2 max(|x|, |y|), so the sums
-// below are the halved ones.
-__device__ __forceinline__ uint32_t half_satd(Half4 v, int h) {
-  auto row = [](int (&r)[4]) {
-    int s03 = r[0] + r[3], s12 = r[1] + r[2], d03 = r[0] - r[3], d12 = r[1] - r[2];
-    r[0] = s03 + s12; r[1] = d03 + d12; r[2] = s03 - s12; r[3] = d03 - d12;
-  };
-  row(v.a);
-  row(v.b);
-  uint32_t sum = 0;
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    int s = v.a[k] + v.b[k], d = v.a[k] - v.b[k];
-    int o = __shfl_xor_sync(FULL, h ? s : d, 1);
-    sum += (uint32_t)max(abs(h ? d : s), abs(o));
-  }
-  return sum;
-}
-// The per-lane scales of the half's even and odd columns (position classes 0, 2 / 2, 1).
-__device__ __forceinline__ void half_scales(uint32_t c0, uint32_t c1, uint32_t c2, int h, uint32_t& even, uint32_t& odd) {
-  even = h ? c2 : c0;
-  odd = h ? c1 : c2;
-}
-// The half's zig-zag indices: rows 0 and 2, or rows 1 and 3, of the frame scan (Table 8-12).
-__device__ __forceinline__ uint32_t half_zigzag_bit(int row, int k, int h) {
-  constexpr uint32_t z[2][2][4] = {{{0, 1, 5, 6}, {3, 8, 11, 13}}, {{2, 4, 7, 12}, {9, 10, 14, 15}}};
-  return h ? 1u << z[1][row][k] : 1u << z[0][row][k];
-}
-// Quantises the half. Returns, alike in both lanes, the block's nonzero levels by zig-zag index
-// (bits 0..15, indices >= first) and in bit 16 whether one of them is above 1.
-__device__ __forceinline__ uint32_t half_quant(Half4& v, int h, int first, uint32_t mf_even, uint32_t mf_odd, uint32_t bias,
-                                               uint32_t shift) {
-  uint32_t mask = 0, big = 0;
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    const uint32_t mf = (k & 1) ? mf_odd : mf_even;
-    const uint32_t la = ((uint32_t)abs(v.a[k]) * mf + bias) >> shift, lb = ((uint32_t)abs(v.b[k]) * mf + bias) >> shift;
-    const bool dc = k == 0 && first && !h;
-    if (la && !dc) mask |= half_zigzag_bit(0, k, h);
-    if (lb) mask |= half_zigzag_bit(1, k, h);
-    big |= (dc ? 0u : la) | lb;
-    v.a[k] = v.a[k] < 0 ? -(int)la : (int)la;
-    v.b[k] = v.b[k] < 0 ? -(int)lb : (int)lb;
-  }
-  mask |= big > 1u ? 0x10000u : 0u;
-  return mask | __shfl_xor_sync(FULL, mask, 1);
-}
-// Decimation score (enc.rs:559, without its |level| > 1 rule) of a block's nonzero zig-zag
-// positions: 3 / 2 / 1 / 0 for a zero run of 0 / 1-2 / 3-5 / longer below each -- the positions with
-// another one (or the start, index first - 1) at most 1, 3 and 6 below, counted.
-__device__ __forceinline__ uint32_t score4(uint32_t m, int first) {
-  m &= 0xffffu;
-  const uint32_t w1 = (first ? m | 1u : m) << 1, w3 = w1 | (w1 << 1) | (w1 << 2), w6 = w3 | (w3 << 3);
-  const uint32_t u = first ? 0u : 0x3fu;  // the start, one below index 0
-  return __popc(m & (w1 | (u & 1u))) + __popc(m & (w3 | (u & 7u))) + __popc(m & (w6 | u));
-}
 __device__ __forceinline__ uint2 pack_half(const int (&r)[4]) {
-  return make_uint2(__byte_perm((uint32_t)r[0], (uint32_t)r[1], 0x5410), __byte_perm((uint32_t)r[2], (uint32_t)r[3], 0x5410));
+  return make_uint2(pack16(r[0], r[1]), pack16(r[2], r[3]));
 }
 __device__ __forceinline__ void unpack_half(uint2 w, int (&r)[4]) {
   r[0] = (int16_t)(w.x & 0xffffu); r[1] = (int)w.x >> 16;
@@ -550,21 +529,73 @@ __device__ __forceinline__ uint32_t even_bits(uint32_t w) {
   return (w | (w >> 8)) & 0xffffu;
 }
 
-// SATD (metrics.rs:705, halved) of the macroblock's source against the 16x16 plane at byte offset `at`.
+// SATD (metrics.rs:705, halved) of the macroblock's source against the 16x16 plane at byte offset
+// `at`: half the sum of the magnitudes of every block's Hadamard coefficients.
 __device__ __noinline__ uint32_t satd16(int at) {
   const int lane = lane_id(), h = lane & 1, off = blk_off16(lane >> 1);
-  return wsum(half_satd(half_diff(half_rows((int)offsetof(Smem, src_y) + off, 16, h), half_rows(at + off, 16, h)), h));
+  int a[4], b[4];
+  half_columns(half_rows((int)offsetof(Smem, src_y) + off, 16, h), half_rows(at + off, 16, h), h, 1, a, b);
+  // |x + y| + |x - y| = 2 max(|x|, |y|): the last butterfly and the halving in one
+  auto row = [](const int (&r)[4]) {
+    const int s03 = r[0] + r[3], s12 = r[1] + r[2], d03 = r[0] - r[3], d12 = r[1] - r[2];
+    return (uint32_t)(max(abs(s03), abs(s12)) + max(abs(d03), abs(d12)));
+  };
+  return wsum(row(a) + row(b));
 }
-// Forward transform and inter quantisation of the macroblock's luma residual, one block per lane pair.
-__device__ __forceinline__ uint32_t luma4x4_levels(int qp, Half4& v) {
-  const int lane = lane_id(), b = lane >> 1, h = lane & 1, off = blk_off16(b);
-  uint32_t shift, bias, even, odd;
-  quant4_params(qp, false, shift, bias);
-  const int rem = qp % 6;
-  half_scales(c_mf4[rem][0], c_mf4[rem][1], c_mf4[rem][2], h, even, odd);
-  v = half_diff(half_rows((int)offsetof(Smem, src_y) + off, 16, h), half_rows((int)offsetof(Smem, pred_y) + off, 16, h));
-  half_fwd(v, h);
-  return half_quant(v, h, 0, even, odd, bias, shift);
+// Forward transform (fixed.rs:104) and quantisation (enc.rs:1703-1779) of the lane's half of the block
+// at byte offsets src and pred of Smem. mask, alike in both lanes: the block's nonzero levels by
+// zig-zag index (bits 0..15, the DC of a chroma block left out) and in bit 16 whether one of them is above 1. ra, rb:
+// the levels of its two coefficient rows; dc: the block's DC coefficient before quantisation (h = 0).
+struct HalfLevels {
+  uint2 ra, rb;
+  uint32_t mask;
+  int dc;
+};
+__device__ __noinline__ HalfLevels quant_half(int src, int pred, int stride, int chroma, bool intra) {
+  const int first = chroma;  // a chroma block's DC is coded apart
+  const int h = lane_id() & 1;
+  const QTab& qt = sm.qt[chroma];
+  const uint32_t shift = qt.shift, bias = qt.bias[intra], mf[2] = {qt.mf[h][0], qt.mf[h][1]};
+  Half4 v;
+  half_columns(half_rows(src, stride, h), half_rows(pred, stride, h), h, 1 + h, v.a, v.b);
+  auto row = [](int (&r)[4]) {
+    const int s03 = r[0] + r[3], s12 = r[1] + r[2], d03 = r[0] - r[3], d12 = r[1] - r[2];
+    r[0] = s03 + s12; r[1] = 2 * d03 + d12; r[2] = s03 - s12; r[3] = d03 - 2 * d12;
+  };
+  row(v.a);
+  row(v.b);
+  HalfLevels q;
+  q.dc = v.a[0];
+  // zig-zag indices (Table 8-12) of rows 0 and 2, or 1 and 3, four bits each
+  uint32_t zz = h ? 0xfea9c742u : 0xdb836510u, mask = 0, big = 0;
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    int& c = k < 4 ? v.a[k & 3] : v.b[k & 3];
+    const uint32_t l = ((uint32_t)abs(c) * mf[k & 1] + bias) >> shift;
+    if (l) mask |= 1u << ((zz >> (4 * k)) & 15u);
+    big |= k == 0 && first && !h ? 0u : l;
+    c = c < 0 ? -(int)l : (int)l;
+  }
+  mask &= first ? 0xfffeu : 0xffffu;
+  mask |= big > 1u ? 0x10000u : 0u;
+  q.mask = mask | __shfl_xor_sync(FULL, mask, 1);
+  q.ra = pack_half(v.a);
+  q.rb = pack_half(v.b);
+  return q;
+}
+// Decimation score (enc.rs:559, without its |level| > 1 rule) of a block's nonzero zig-zag
+// positions: 3 / 2 / 1 / 0 for a zero run of 0 / 1-2 / 3-5 / longer below each -- the positions with
+// another one (or the start, index first - 1) at most 1, 3 and 6 below, counted.
+__device__ __forceinline__ uint32_t score4(uint32_t m, int first) {
+  m &= 0xffffu;
+  const uint32_t w1 = (first ? m | 1u : m) << 1, w3 = w1 | (w1 << 1) | (w1 << 2), w6 = w3 | (w3 << 3);
+  const uint32_t u = first ? 0u : 0x3fu;  // the start, one below index 0
+  return __popc(m & (w1 | (u & 1u))) + __popc(m & (w3 | (u & 7u))) + __popc(m & (w6 | u));
+}
+// quant_half of the macroblock's luma: lane pair b owns block b.
+__device__ __forceinline__ HalfLevels quant_luma(bool intra) {
+  const int off = blk_off16(lane_id() >> 1);
+  return quant_half((int)offsetof(Smem, src_y) + off, (int)offsetof(Smem, pred_y) + off, 16, 0, intra);
 }
 
 // Luma 4x4 residual of pred_y, quantised (inter) and decimated into sm.coef
@@ -572,10 +603,10 @@ __device__ __forceinline__ uint32_t luma4x4_levels(int qp, Half4& v) {
 struct Luma4 {
   uint32_t cbp, nnz, nz16;  // coded block pattern, nonzero levels kept, blocks holding levels (bit b)
 };
-__device__ __noinline__ Luma4 luma4x4_inter(int qp) {
+__device__ __noinline__ Luma4 luma4x4_inter() {
   const int lane = lane_id(), b = lane >> 1, h = lane & 1;
-  Half4 v;
-  const uint32_t m = luma4x4_levels(qp, v);
+  HalfLevels q = quant_luma(false);
+  const uint32_t m = q.mask;
   // the 8x8 group's any, |level| > 1 and score sums over its four blocks (lanes 8 g .. 8 g + 7)
   uint32_t g = score4(m, 0) | ((m >> 16) << 12) | ((m & 0xffffu) ? 1u << 16 : 0u);
   g += __shfl_xor_sync(FULL, g, 2);
@@ -587,10 +618,9 @@ __device__ __noinline__ Luma4 luma4x4_inter(int qp) {
   uint32_t cbp = (keep & 1u) | ((keep >> 7) & 2u) | ((keep >> 14) & 4u) | ((keep >> 21) & 8u);
   if (total < 6) cbp = 0;
   const bool coded = (cbp >> (lane >> 3)) & 1u;  // levels of dropped groups are cleared
-  uint2 ra = pack_half(v.a), rb = pack_half(v.b);
-  if (!coded) ra = rb = make_uint2(0u, 0u);
-  *(uint2*)&sm.coef[b * 16 + h * 4] = ra;
-  *(uint2*)&sm.coef[b * 16 + h * 4 + 8] = rb;
+  if (!coded) q.ra = q.rb = make_uint2(0u, 0u);
+  *(uint2*)&sm.coef[b * 16 + h * 4] = q.ra;
+  *(uint2*)&sm.coef[b * 16 + h * 4 + 8] = q.rb;
   Luma4 r;
   r.cbp = cbp;
   r.nz16 = even_bits(__ballot_sync(FULL, coded && (m & 0xffffu)));
@@ -609,20 +639,15 @@ __device__ __forceinline__ int zigzag8(int y, int x) {
 // The tables a warp keeps in its shared memory, once per kernel.
 __device__ __forceinline__ void init_tables() {
   for (int i = lane_id(); i < 64; i += 32) sm.zz8[i] = (uint8_t)zigzag8(i & 7, i >> 3);
+#pragma unroll
+  for (int k = 0; k < 16; k++)
+    if (lane_id() == k) sm.qpt[k] = qpel_entry(k);
+  if (lane_id() == 0) sm.qt_qp = -1;
   __syncwarp();
 }
-// The scales of row (or column) q of an 8x8 block by the other coordinate's low two bits: position
-// classes (h264.rs:1343) {0, 3, 4, 3}, {3, 1, 5, 1}, {4, 5, 2, 5}, {3, 1, 5, 1}.
-struct Scale8 {
-  int m0, m1, m2;  // index 0, odd, 2
-  __device__ __forceinline__ int at(int k) const { return (k & 1) ? m1 : ((k & 2) ? m2 : m0); }
-};
-template <typename T>
-__device__ __forceinline__ Scale8 scale8(const T* c, int q) {
-  const int k0 = c[0], k1 = c[1], k2 = c[2], k3 = c[3], k4 = c[4], k5 = c[5];
-  const bool odd = q & 1, two = (q & 3) == 2;
-  return {odd ? k3 : (two ? k4 : k0), odd ? k1 : (two ? k5 : k3), odd ? k5 : (two ? k2 : k4)};
-}
+// Row of the 8x8 scale tables (QTab::mf8, dq8) for coordinate k: position classes (h264.rs:1343)
+// {0, 3, 4, 3}, {3, 1, 5, 1}, {4, 5, 2, 5}, {3, 1, 5, 1} by the low two bits of row and column.
+__device__ __forceinline__ int class8(int k) { return (k & 1) ? 1 : (k & 2); }
 // Eight words of a block's row (contiguous) to and from shared memory.
 __device__ __forceinline__ void t8_store_row(int at, const int (&r)[8]) {
   *(int4*)&sm.t8[at] = make_int4(r[0], r[1], r[2], r[3]);
@@ -635,10 +660,11 @@ __device__ __forceinline__ void t8_store_row(int at, const int (&r)[8]) {
 // the bitmask of its nonzero zig-zag positions (weights 3 / 2 / 1 / 0 for zero runs of 0-3 / 4-11 /
 // 12-23 / longer below each, enc.rs:559 with the 8x8 table), counted as in score4. Returns cbp |
 // nonzero levels << 4.
-__device__ __noinline__ uint32_t luma8x8_inter(int qp) {
+__device__ __noinline__ uint32_t luma8x8_inter() {
   const int lane = lane_id(), b = lane >> 3, q = lane & 7;
   const int off = ((b >> 1) * 8 + q) * 16 + (b & 1) * 8;
-  const uint32_t shift = 16 + qp / 6, bias = (1u << shift) / 6u;
+  const QTab& qt = sm.qt[0];
+  const uint32_t shift = qt.shift + 1, bias = qt.bias8;
   int d[8], o[8];
   {
     const uint2 s = *(const uint2*)&sm.src_y[off], p = *(const uint2*)&sm.pred_y[off];
@@ -654,12 +680,12 @@ __device__ __noinline__ uint32_t luma8x8_inter(int qp) {
 #pragma unroll
   for (int y = 0; y < 8; y++) d[y] = sm.t8[b * kT8Block + y * 8 + q];
   fdct8_1d(d, o);
-  const Scale8 mf = scale8(c_mf8[qp % 6], q);
+  const uint32_t* mf = qt.mf8[class8(q)];
   const uint2 zz = *(const uint2*)&sm.zz8[q * 8];
   uint32_t lo = 0, hi = 0, big = 0;
 #pragma unroll
   for (int y = 0; y < 8; y++) {
-    const uint32_t l = ((uint32_t)abs(o[y]) * (uint32_t)mf.at(y) + bias) >> shift;
+    const uint32_t l = ((uint32_t)abs(o[y]) * mf[class8(y)] + bias) >> shift;
     const uint32_t z = ((y < 4 ? zz.x : zz.y) >> (8 * (y & 3))) & 255u, bit = l ? 1u << (z & 31u) : 0u;
     if (z & 32u) hi |= bit; else lo |= bit;
     big |= l;
@@ -690,6 +716,12 @@ __device__ __noinline__ uint32_t luma8x8_inter(int qp) {
   return cbp | (wsum(q == 0 && coded ? (uint32_t)__popcll(m) : 0u) << 4);
 }
 
+// |Level| of a DC transform's coefficient (enc.rs:1938, :1960: one bit more, f = 2^qbits / 3).
+__device__ __forceinline__ int quant_dc(int a, const QTab& q) {
+  const uint32_t qbits = q.shift + 1;
+  return (int)(((uint32_t)a * (uint32_t)q.dc_mf + (1u << qbits) / 3u) >> qbits);
+}
+
 // Chroma residual of pred_u/pred_v (enc.rs:1899 quant_chroma): lane pair b < 8 owns block b
 // (plane = b / 4); the other lanes repeat them. Levels into sm.ccoef (raster), DC levels into sm.cdc.
 // Returns, in every lane and per plane: AC present, AC decimation score, and any DC level.
@@ -699,31 +731,24 @@ struct ChromaAc {
   __device__ __forceinline__ uint32_t score(int p) const { return (w >> (8 * p)) & 255u; }
   __device__ __forceinline__ bool dc() const { return (w >> 18) & 1u; }
 };
-__device__ __noinline__ ChromaAc chroma_quant(int qpc, bool intra) {
+__device__ __noinline__ ChromaAc chroma_quant(bool intra) {
   const int lane = lane_id(), h = lane & 1, b = (lane >> 1) & 7, off = blk_off8(b);
-  uint32_t shift, bias, even, odd;
-  quant4_params(qpc, intra, shift, bias);
-  const int rem = qpc % 6;
-  const uint32_t mf0 = c_mf4[rem][0];
-  half_scales(mf0, c_mf4[rem][1], c_mf4[rem][2], h, even, odd);
-  Half4 v = half_diff(half_rows((int)offsetof(Smem, src_u) + off, 8, h), half_rows((int)offsetof(Smem, pred_u) + off, 8, h));
-  half_fwd(v, h);
+  const HalfLevels q = quant_half((int)offsetof(Smem, src_u) + off, (int)offsetof(Smem, pred_u) + off, 8, 1, intra);
+  const uint32_t m = q.mask;
   // 2x2 DC transform + quantisation (enc.rs:1938 quant_chroma_dc; f = 2^qbits / 3 always); block b & 3
   // of the plane ends with output b & 3
-  int dc = v.a[0];
+  int dc = q.dc;
   {
     int o = __shfl_xor_sync(FULL, dc, 2);
     dc = (b & 1) ? o - dc : dc + o;
     o = __shfl_xor_sync(FULL, dc, 4);
     dc = (b & 2) ? o - dc : dc + o;
-    const int qbits = 16 + qpc / 6, f = (1 << qbits) / 3;
-    const int l = (abs(dc) * (int)mf0 + f) >> qbits;
+    const int l = quant_dc(abs(dc), sm.qt[1]);
     dc = dc < 0 ? -l : l;
   }
-  const uint32_t m = half_quant(v, h, 1, even, odd, bias, shift);
   if (lane < 16) {
-    *(uint2*)&sm.ccoef[b * 16 + h * 4] = pack_half(v.a);
-    *(uint2*)&sm.ccoef[b * 16 + h * 4 + 8] = pack_half(v.b);
+    *(uint2*)&sm.ccoef[b * 16 + h * 4] = q.ra;
+    *(uint2*)&sm.ccoef[b * 16 + h * 4 + 8] = q.rb;
     if (!h) sm.cdc[b] = (int16_t)dc;
   }
   const bool dcany = __ballot_sync(FULL, !h && dc != 0) != 0;
@@ -737,36 +762,44 @@ __device__ __noinline__ ChromaAc chroma_quant(int qpc, bool intra) {
                   (dcany ? 1u << 18 : 0u)};
 }
 
+// Adds the dequantised residual (levels of coefficient rows h, h + 2 in ra, rb; has_dc: the DC
+// coefficient given, dequantised, instead) of the lane's half of a block to the samples at byte offset
+// `off` of Smem; lanes not `on` leave them.
+__device__ __noinline__ void recon_half(uint2 ra, uint2 rb, int chroma, bool has_dc, int dc, int off, int stride, bool on) {
+  const int h = lane_id() & 1, dq[2] = {sm.qt[chroma].dq[h][0], sm.qt[chroma].dq[h][1]};
+  Half4 v;
+  unpack_half(ra, v.a);
+  unpack_half(rb, v.b);
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    v.a[k] = clamp_i16(v.a[k] * dq[k & 1]);
+    v.b[k] = clamp_i16(v.b[k] * dq[k & 1]);
+  }
+  if (has_dc && !h) v.a[0] = dc;
+  half_inv(v, h);
+  const uint2 p = half_rows(off, stride, h);
+  if (on) {
+    *(uint32_t*)sm_at(off + h * stride) = add_clip4(p.x, v.a);
+    *(uint32_t*)sm_at(off + (3 - h) * stride) = add_clip4(p.y, v.b);
+  }
+  __syncwarp();
+}
+// The lane's rows of block b of sm.coef / sm.ccoef.
+__device__ __forceinline__ uint2 level_row(const int16_t* c, int b, int row) { return *(const uint2*)&c[b * 16 + row * 4]; }
+
 // Adds the dequantised chroma residual to pred_u / pred_v (enc.rs:1992 recon_chroma): the DC of
 // each block from the 2x2 inverse (h264.rs:1674 dequantize_idct_chroma_dc2x2), its AC dequantised
 // when cbpc == 2, then the inverse core transform. Two lanes per block as in chroma_quant.
-__device__ __noinline__ void chroma_recon(int qpc, int cbpc) {
+__device__ __noinline__ void chroma_recon(int cbpc) {
   if (cbpc == 0) return;
-  const int lane = lane_id(), h = lane & 1, b = (lane >> 1) & 7, bb = b & 3, off = blk_off8(b) + (int)offsetof(Smem, pred_u);
-  const int rem = qpc % 6, qdiv = qpc / 6, qmul = (c_dq4[rem][0] * 16) << (qdiv + 2);
-  uint32_t even, odd;
-  half_scales(c_dq4[rem][0], c_dq4[rem][1], c_dq4[rem][2], h, even, odd);
+  const int lane = lane_id(), h = lane & 1, b = (lane >> 1) & 7, bb = b & 3;
   int lv[4];
   unpack_half(*(const uint2*)&sm.cdc[b & 4], lv);
   const int e = lv[0] - lv[1], apb = lv[0] + lv[1], cmd = lv[2] - lv[3], cpd = lv[2] + lv[3];
   const int dcv = bb == 0 ? apb + cpd : (bb == 1 ? e + cmd : (bb == 2 ? apb - cpd : e - cmd));
-  Half4 v;
-  unpack_half(*(const uint2*)&sm.ccoef[b * 16 + h * 4], v.a);
-  unpack_half(*(const uint2*)&sm.ccoef[b * 16 + h * 4 + 8], v.b);
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    const int dq = (int)((k & 1) ? odd : even) << qdiv;
-    v.a[k] = cbpc >= 2 ? (int)clamp_i16(v.a[k] * dq) : 0;
-    v.b[k] = cbpc >= 2 ? (int)clamp_i16(v.b[k] * dq) : 0;
-  }
-  if (!h) v.a[0] = (int16_t)((dcv * qmul) >> 7);
-  half_inv(v, h);
-  const uint2 p = half_rows(off, 8, h);
-  if (lane < 16) {
-    *(uint32_t*)sm_at(off + h * 8) = add_clip4(p.x, v.a);
-    *(uint32_t*)sm_at(off + (3 - h) * 8) = add_clip4(p.y, v.b);
-  }
-  __syncwarp();
+  uint2 ra = level_row(sm.ccoef, b, h), rb = level_row(sm.ccoef, b, h + 2);
+  if (cbpc < 2) ra = rb = make_uint2(0u, 0u);
+  recon_half(ra, rb, 1, true, (int16_t)((dcv * sm.qt[1].dc_dq) >> 7), blk_off8(b) + (int)offsetof(Smem, pred_u), 8, lane < 16);
 }
 
 // Raster position of each 4x4 zig-zag index, 4 bits per index (frame scan, Table 8-12).
@@ -775,17 +808,16 @@ constexpr unsigned long long kScan4Packed = 0xfeb7adc963258410ull;
 // Adds the dequantised 8x8 residual of the coded blocks of sm.coef8 to pred_y (enc.rs:2013
 // recon_8x8: dequantize_block8x8, h264.rs:1403, then h264_idct8_add, h264_idct.rs:207).
 // Lanes 8b..8b+7 own block b: row q, then column q. Blocks that are not coded add zero.
-__device__ __noinline__ void recon_luma8x8(int qp, int cbp) {
+__device__ __noinline__ void recon_luma8x8(int cbp) {
   const int lane = lane_id(), b = lane >> 3, q = lane & 7;
   const bool coded = (cbp >> b) & 1;
-  const int qdiv = qp / 6;
-  const Scale8 dq = scale8(c_dq8[qp % 6], q);
+  const int* dq = sm.qt[0].dq8[class8(q)];
+  const int rnd = sm.qt[0].rnd8, sh = sm.qt[0].sh8;
   int d[8], o[8];
 #pragma unroll
   for (int x = 0; x < 8; x++) {
-    const int l = coded ? sm.coef8[b * 64 + sm.zz8[x * 8 + q]] : 0, v = dq.at(x);
-    const int dv = qdiv >= 2 ? l * (v << (qdiv - 2)) : ((l * v + (1 << (1 - qdiv))) >> (2 - qdiv));
-    d[x] = clamp_i16(dv);
+    const int l = coded ? sm.coef8[b * 64 + sm.zz8[x * 8 + q]] : 0;
+    d[x] = clamp_i16((l * dq[class8(x)] + rnd) >> sh);
   }
   idct8_1d(d, o);
   t8_store_row(b * kT8Block + q * 8, o);
@@ -804,25 +836,9 @@ __device__ __noinline__ void recon_luma8x8(int qp, int cbp) {
 
 // Adds the dequantised luma 4x4 residual of sm.coef to pred_y (enc.rs:1978 recon_luma_4x4; blocks
 // without levels add zero), two lanes per block.
-__device__ __noinline__ void recon_luma4x4(int qp) {
-  const int lane = lane_id(), b = lane >> 1, h = lane & 1, off = blk_off16(b) + (int)offsetof(Smem, pred_y);
-  const int rem = qp % 6, qdiv = qp / 6;
-  uint32_t even, odd;
-  half_scales(c_dq4[rem][0], c_dq4[rem][1], c_dq4[rem][2], h, even, odd);
-  Half4 v;
-  unpack_half(*(const uint2*)&sm.coef[b * 16 + h * 4], v.a);
-  unpack_half(*(const uint2*)&sm.coef[b * 16 + h * 4 + 8], v.b);
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    const int dq = (int)((k & 1) ? odd : even) << qdiv;
-    v.a[k] = clamp_i16(v.a[k] * dq);
-    v.b[k] = clamp_i16(v.b[k] * dq);
-  }
-  half_inv(v, h);
-  const uint2 p = half_rows(off, 16, h);
-  *(uint32_t*)sm_at(off + h * 16) = add_clip4(p.x, v.a);
-  *(uint32_t*)sm_at(off + (3 - h) * 16) = add_clip4(p.y, v.b);
-  __syncwarp();
+__device__ __forceinline__ void recon_luma4x4() {
+  const int lane = lane_id(), b = lane >> 1, h = lane & 1;
+  recon_half(level_row(sm.coef, b, h), level_row(sm.coef, b, h + 2), 0, false, 0, blk_off16(b) + (int)offsetof(Smem, pred_y), 16, true);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -855,6 +871,10 @@ __device__ __forceinline__ int dc16(bool ht, bool hl) {
   if (hl) return (int)((sl + 8) >> 4);
   return 128;
 }
+// Four samples of a plane prediction, (v + k step) >> 5 clipped.
+__device__ __forceinline__ uint32_t plane4(int v, int step) {
+  return pack_clip(v >> 5, (v + step) >> 5, (v + 2 * step) >> 5, (v + 3 * step) >> 5);
+}
 __device__ __noinline__ void pred16_into(int mode, int dst, bool ht, bool hl, int tl) {
   int lane = lane_id();
   int y = lane >> 1, x0 = (lane & 1) * 8;
@@ -862,11 +882,8 @@ __device__ __noinline__ void pred16_into(int mode, int dst, bool ht, bool hl, in
   if (mode == 3) {
     int pa, pb, pc;
     plane16_params(ht, hl, tl, pa, pb, pc);
-    uint32_t w[2] = {0u, 0u};
-#pragma unroll
-    for (int k = 0; k < 8; k++)
-      w[k >> 2] |= (uint32_t)clip255((pa + pb * (x0 + k - 7) + pc * (y - 7) + 16) >> 5) << (8 * (k & 3));
-    *(uint2*)o = make_uint2(w[0], w[1]);
+    const int v = pa + pb * (x0 - 7) + pc * (y - 7) + 16;
+    *(uint2*)o = make_uint2(plane4(v, pb), plane4(v + 4 * pb, pb));
   } else {
     uint2 v;
     if (mode == 0) {
@@ -879,50 +896,43 @@ __device__ __noinline__ void pred16_into(int mode, int dst, bool ht, bool hl, in
   }
   __syncwarp();
 }
-// Intra 16x16 analysis (enc.rs:1637 analyse_i16_edges): SATD per mode; the best mode and its cost.
+// Intra 16x16 analysis (enc.rs:1637 analyse_i16_edges): SATD per mode; the best mode and its cost. The
+// vertical, horizontal and DC predictions have one nonzero row, column or coefficient of each
+// block's Hadamard transform, so their SATDs are the source's with those terms replaced.
 struct I16Fit {
   int mode;
   uint32_t cost;
 };
 __device__ __noinline__ I16Fit analyse_i16(bool ht, bool hl, int tl) {
-  int lane = lane_id();
-  int dc = dc16(ht, hl);
-  uint32_t sv = 0, sh = 0, sd = 0;
-  if (lane < 16) {
-    int bx = lane & 3, by = lane >> 2;
-    // hadamard4x4_16x4_scalar of the source block, out[4 v + h]
-    int rows[4][4];
+  const int lane = lane_id(), h = lane & 1, b = lane >> 1, off = blk_off16(b);
+  const int dc = 16 * dc16(ht, hl);
+  int a[4], c[4];  // coefficient rows: h = 0: all rows' sum, s03 - s12; h = 1: d03 + d12, d03 - d12
+  half_columns(half_rows((int)offsetof(Smem, src_y) + off, 16, h), make_uint2(0u, 0u), h, 1, a, c);
+  auto row = [](int (&r)[4]) {
+    const int s03 = r[0] + r[3], s12 = r[1] + r[2], d03 = r[0] - r[3], d12 = r[1] - r[2];
+    r[0] = s03 + s12; r[1] = d03 + d12; r[2] = s03 - s12; r[3] = d03 - d12;
+  };
+  row(a);
+  row(c);
+  int top[4], left[4];
+  const uint32_t tw = ht ? *(const uint32_t*)&sm.top[blk_x(b) * 4] : 0u, lw = hl ? *(const uint32_t*)&sm.left[blk_y(b) * 4] : 0u;
 #pragma unroll
-    for (int y = 0; y < 4; y++) {
-      const uint8_t* s = &sm.src_y[(by * 4 + y) * 16 + bx * 4];
-      int s01 = s[0] + s[1], d01 = s[0] - s[1], s23 = s[2] + s[3], d23 = s[2] - s[3];
-      rows[y][0] = s01 + s23; rows[y][1] = s01 - s23; rows[y][2] = d01 + d23; rows[y][3] = d01 - d23;
-    }
-    int tv[4], th[4];
-    {
-      const uint8_t* t = &sm.top[bx * 4];
-      int e0 = ht ? t[0] : 0, e1 = ht ? t[1] : 0, e2 = ht ? t[2] : 0, e3 = ht ? t[3] : 0;
-      int s01 = e0 + e1, d01 = e0 - e1, s23 = e2 + e3, d23 = e2 - e3;
-      tv[0] = 4 * (s01 + s23); tv[1] = 4 * (s01 - s23); tv[2] = 4 * (d01 + d23); tv[3] = 4 * (d01 - d23);
-      const uint8_t* l = &sm.left[by * 4];
-      e0 = hl ? l[0] : 0; e1 = hl ? l[1] : 0; e2 = hl ? l[2] : 0; e3 = hl ? l[3] : 0;
-      s01 = e0 + e1; d01 = e0 - e1; s23 = e2 + e3; d23 = e2 - e3;
-      th[0] = 4 * (s01 + s23); th[1] = 4 * (s01 - s23); th[2] = 4 * (d01 + d23); th[3] = 4 * (d01 - d23);
-    }
-#pragma unroll
-    for (int h = 0; h < 4; h++) {
-      int c0 = rows[0][h], c1 = rows[1][h], c2 = rows[2][h], c3 = rows[3][h];
-      int s01 = c0 + c1, d01 = c0 - c1, s23 = c2 + c3, d23 = c2 - c3;
-      int col[4] = {s01 + s23, s01 - s23, d01 + d23, d01 - d23};
-#pragma unroll
-      for (int v = 0; v < 4; v++) {
-        int c = col[v], k = 4 * v + h;
-        int pv = v == 0 ? tv[h] : 0, ph = h == 0 ? th[v] : 0, pd = k == 0 ? 16 * dc : 0;
-        sv += abs(c - pv); sh += abs(c - ph); sd += abs(c - pd);
-      }
-    }
+  for (int k = 0; k < 4; k++) {
+    top[k] = (int)((tw >> (8 * k)) & 255u) * 4;
+    left[k] = (int)((lw >> (8 * k)) & 255u) * 4;
   }
-  sv = wsum(sv) >> 1; sh = wsum(sh) >> 1; sd = wsum(sd) >> 1;
+  row(top);
+  row(left);
+  uint32_t all = 0, row0 = 0, row0v = 0;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    all += (uint32_t)(abs(a[k]) + abs(c[k]));
+    row0 += (uint32_t)abs(a[k]);
+    row0v += (uint32_t)abs(a[k] - top[k]);
+  }
+  const uint32_t col0 = (uint32_t)(abs(a[0]) + abs(c[0])), col0h = (uint32_t)(abs(a[0] - left[h]) + abs(c[0] - left[h + 2]));
+  const uint32_t sv = wsum(h ? all : all - row0 + row0v) >> 1, sh = wsum(all - col0 + col0h) >> 1,
+                 sd = wsum(h ? all : all - (uint32_t)abs(a[0]) + (uint32_t)abs(a[0] - dc)) >> 1;
   uint32_t best = sd;
   int mode = 2;
   if (ht && sv < best) { best = sv; mode = 0; }
@@ -933,16 +943,6 @@ __device__ __noinline__ I16Fit analyse_i16(bool ht, bool hl, int tl) {
     if (s < best) { best = s; mode = 3; }
   }
   return I16Fit{mode, best};
-}
-// Chroma intra prediction sample of mode for plane p at (x, y).
-__device__ __forceinline__ int predc_sample(int mode, int p, bool ht, bool hl, int tl, int x, int y,
-                                            const int* dcv, int pa, int pb, int pc) {
-  switch (mode) {
-    case 0: return dcv[(y >> 2) * 2 + (x >> 2)];
-    case 1: return hl ? sm.cleft[p][y] : 128;
-    case 2: return ht ? sm.ctop[p][x] : 128;
-    default: return clip255((pa + pb * (x - 3) + pc * (y - 3) + 16) >> 5);
-  }
 }
 // DC and plane parameters of plane p's chroma prediction; called by the whole warp with p =
 // lane / 16. In each half-warp lanes 0..7 hold top[0..7], lanes 8..15 left[0..7] (DC sums of four
@@ -983,26 +983,26 @@ struct Corner {
 };
 // Intra chroma mode by SAD (enc.rs:1526 analyse_chroma_intra); best prediction into pred_u/v.
 __device__ __noinline__ int analyse_chroma(bool ht, bool hl, Corner k0) {
-  int lane = lane_id();
-  int plane = lane >> 4, idx = (lane & 15) * 4, y = idx >> 3, x0 = idx & 7;
-  const int plane_tl = plane ? k0.v : k0.u;
+  const int lane = lane_id(), plane = lane >> 4, idx = (lane & 15) * 4, y = idx >> 3, x0 = idx & 7;
   int dcv[4], pa, pb, pc;
-  chroma_pred_params(plane, ht, hl, plane_tl, dcv, pa, pb, pc);
-  const uint8_t* s = (plane ? sm.src_v : sm.src_u) + y * 8 + x0;
-  uint32_t best = UMAX;
+  chroma_pred_params(plane, ht, hl, plane ? k0.v : k0.u, dcv, pa, pb, pc);
+  // this lane's four samples of every mode: DC, horizontal, vertical, plane
+  const int dc = (y & 4) ? (x0 ? dcv[3] : dcv[2]) : (x0 ? dcv[1] : dcv[0]);
+  const uint32_t w0 = (uint32_t)dc * 0x01010101u, w1 = hl ? sm.cleft[plane][y] * 0x01010101u : 0x80808080u,
+                 w2 = ht ? *(const uint32_t*)&sm.ctop[plane][x0] : 0x80808080u,
+                 w3 = plane4(pa + pb * (x0 - 3) + pc * (y - 3) + 16, pb);
+  const uint32_t src = *(const uint32_t*)&sm.src_u[lane * 4];
+  // the SADs of two modes per reduction (each below 2^16)
+  const uint32_t s01 = wsum(__vsadu4(src, w0) | (__vsadu4(src, w1) << 16)), s23 = wsum(__vsadu4(src, w2) | (__vsadu4(src, w3) << 16));
+  uint32_t best = s01 & 0xffffu, w = w0;
   int bm = 0;
-  for (int mode = 0; mode < 4; mode++) {
-    bool ok = mode == 1 ? hl : (mode == 2 ? ht : (mode == 3 ? (ht && hl) : true));
-    if (!ok) continue;
-    uint32_t sad = 0;
-#pragma unroll
-    for (int k = 0; k < 4; k++) sad += abs((int)s[k] - predc_sample(mode, plane, ht, hl, plane_tl, x0 + k, y, dcv, pa, pb, pc));
-    uint32_t cost = wsum(sad) + (mode == 0 ? 0u : 8u);
-    if (cost < best) { best = cost; bm = mode; }
-  }
-  uint8_t* out = (plane ? sm.pred_v : sm.pred_u) + y * 8 + x0;
-#pragma unroll
-  for (int k = 0; k < 4; k++) out[k] = (uint8_t)predc_sample(bm, plane, ht, hl, plane_tl, x0 + k, y, dcv, pa, pb, pc);
+  auto take = [&](int m, bool ok, uint32_t sad, uint32_t v) {
+    if (ok && sad + 8u < best) { best = sad + 8u; bm = m; w = v; }
+  };
+  take(1, hl, s01 >> 16, w1);
+  take(2, ht, s23 & 0xffffu, w2);
+  take(3, ht && hl, s23 >> 16, w3);
+  *(uint32_t*)&sm.pred_u[lane * 4] = w;
   __syncwarp();
   return bm;
 }
@@ -1057,7 +1057,19 @@ __device__ __forceinline__ void load_desc(const StreamDev* p) {
   __syncwarp();
   if (lane < n) ((uint2*)&sm.sd)[lane] = a;
   __syncwarp();
+  if (sm.sd.qp != sm.qt_qp) {  // another QP than the last picture's (init_tables: none)
+    const uint32_t* l = (const uint32_t*)&g_qtab[sm.sd.qp];
+    const uint32_t* ch = (const uint32_t*)&g_qtab[sm.sd.qpc];
+    const uint32_t w0 = l[lane], w1 = lane + 32 < kQTabWords ? l[lane + 32] : 0u, w2 = lane < kQTabWords4 ? ch[lane] : 0u;
+    __syncwarp();
+    ((uint32_t*)&sm.qt[0])[lane] = w0;
+    if (lane + 32 < kQTabWords) ((uint32_t*)&sm.qt[0])[lane + 32] = w1;
+    if (lane < kQTabWords4) ((uint32_t*)&sm.qt[1])[lane] = w2;
+    if (lane == 0) sm.qt_qp = sm.sd.qp;
+    __syncwarp();
+  }
 }
+static_assert(kQTabWords > 32 && kQTabWords <= 64 && kQTabWords4 <= 32, "a luma entry is two words a lane, a chroma one less");
 __device__ __forceinline__ void load_params(const FrameParams& fp) {
   constexpr int n = (int)(sizeof(FrameParams) / 4);
   static_assert(n <= 32, "a word a lane");
@@ -1071,19 +1083,25 @@ __device__ __forceinline__ void load_params(const FrameParams& fp) {
 // (enc.rs:400 MbSrc::load, h264.rs:3660 extract_mb_planes).
 __device__ __noinline__ void load_source(const Ctx c) {
   const FrameParams& fp = sm.fp;
-  int lane = lane_id();
-  int W = fp.width, H = fp.height, cw = (W + 1) >> 1, ch = (H + 1) >> 1;
-  int y = min(c.mby * 16 + (lane >> 1), H - 1);
-  const uint8_t* row = sm.sd.src_y + (long)y * fp.src_stride_y;
-  int x0 = c.mbx * 16 + (lane & 1) * 8;
-#pragma unroll
-  for (int k = 0; k < 8; k++) sm.src_y[(lane >> 1) * 16 + (lane & 1) * 8 + k] = __ldg(row + min(x0 + k, W - 1));
-  int plane = lane >> 4, idx = (lane & 15) * 4, r = idx >> 3, c0 = idx & 7;
-  int cy = min(c.mby * 8 + r, ch - 1);
-  const uint8_t* crow = (plane ? sm.sd.src_v : sm.sd.src_u) + (long)cy * fp.src_stride_uv;
-  uint8_t* dst = (plane ? sm.src_v : sm.src_u) + r * 8 + c0;
-#pragma unroll
-  for (int k = 0; k < 4; k++) dst[k] = __ldg(crow + min(c.mbx * 8 + c0 + k, cw - 1));
+  const int lane = lane_id(), W = fp.width, H = fp.height, cw = (W + 1) >> 1, ch = (H + 1) >> 1;
+  const int y = min(c.mby * 16 + (lane >> 1), H - 1), x0 = c.mbx * 16 + (lane & 1) * 8;
+  const uint8_t* row = sm.sd.src_y + (long)y * fp.src_stride_y + x0;
+  const int idx = (lane & 15) * 4, cy = min(c.mby * 8 + (idx >> 3), ch - 1), cx0 = c.mbx * 8 + (idx & 7);
+  const uint8_t* crow = ((lane & 16) ? sm.sd.src_v : sm.sd.src_u) + (long)cy * fp.src_stride_uv + cx0;
+  // inside the picture's width and aligned: a vector per lane (an 8-byte and a 4-byte load instead of
+  // twelve of a byte)
+  const bool fast = c.mbx * 16 + 16 <= W && (((uintptr_t)row & 7) | ((uintptr_t)crow & 3)) == 0;
+  if (__all_sync(FULL, fast)) {
+    const uint2 v = __ldg((const uint2*)row);
+    const uint32_t w = __ldg((const uint32_t*)crow);
+    *(uint2*)&sm.src_y[lane * 8] = v;
+    *(uint32_t*)&sm.src_u[lane * 4] = w;
+  } else {
+#pragma unroll 4
+    for (int k = 0; k < 8; k++) sm.src_y[lane * 8 + k] = __ldg(row + min(k, W - 1 - x0));
+#pragma unroll 4
+    for (int k = 0; k < 4; k++) sm.src_u[lane * 4 + k] = __ldg(crow + min(k, cw - 1 - cx0));
+  }
   __syncwarp();
 }
 // Intra edges from the unfiltered reconstruction of this picture (enc.rs:1459-1521) into shared
@@ -1144,7 +1162,6 @@ constexpr int kWordLuma = offsetof(rg_mb_out, luma) / 4, kWordLumaDc = offsetof(
 static_assert(kWordLuma == 9 && offsetof(rg_mb_out, mv) == 8 && offsetof(rg_mb_out, mvd) == 12 &&
                   offsetof(rg_mb_out, i4_modes) == 16 && offsetof(rg_mb_out, nz_mask) == 32,
               "the head's words");
-__device__ __forceinline__ uint32_t pack16(int lo, int hi) { return __byte_perm((uint32_t)lo, (uint32_t)hi, 0x5410); }
 // The chroma levels of the record (zig-zag): word w of the AC levels holds slots 2 (w & 7), 2 (w & 7)
 // + 1 of block w / 8 (plane * 4 + block); slot 0 (the DC position) stays 0.
 __device__ __noinline__ void record_chroma(rg_mb_out* rec, int cbpc) {
@@ -1196,117 +1213,59 @@ __device__ __forceinline__ void write_info(const Ctx c, int flags, int cbpl, int
                                             nz | (bottom << 16), right);
 }
 
+// The 4x4 Hadamard transform of sixteen values, lane i < 16 holding entry i (row-major; the upper
+// half-warp repeats it): outputs in the rows / columns order ++++, ++--, +--+, +-+- of both the
+// forward (enc.rs:1960) and the inverse (h264.rs:1645) luma DC transform.
+__device__ __noinline__ int hadamard16(int v) {
+  const int lane = lane_id();
+#pragma unroll
+  for (int k = 1; k < 16; k <<= 1) {
+    const int o = __shfl_xor_sync(FULL, v, k);
+    v = (lane & k) ? o - v : v + o;
+  }
+  // natural order (bit 0: +-+-, bit 1: ++--) to the order above: 0, 2, 3, 1
+  const int x = lane & 3, y = (lane >> 2) & 3;
+  return __shfl_sync(FULL, v, (((0x1320 >> (4 * y)) & 3) << 2) | ((0x1320 >> (4 * x)) & 3));
+}
 // I16x16 coding and reconstruction (enc.rs:3587 code_i16) with prediction mode `mode`.
 __device__ __noinline__ void code_i16(const Ctx c, int mode, bool ht, bool hl, Corner k0) {
-  int lane = lane_id();
-  int qp = sm.sd.qp, qpc = sm.sd.qpc;
+  const int lane = lane_id(), b = lane >> 1, h = lane & 1;
+  const int qp = sm.sd.qp;
   pred16_into(mode, (int)offsetof(Smem, pred_y), ht, hl, k0.y);
-  int cmode = analyse_chroma(ht, hl, k0);
-  uint32_t shift, bias;
-  quant4_params(qp, true, shift, bias);
-  uint32_t my_ac = 0, my_nz = 0;
-  int lv[16];
-  if (lane < 16) {
-    int bx = blk_x(lane), by = blk_y(lane);
-    int d[16], cc[16];
-#pragma unroll
-    for (int y = 0; y < 4; y++)
-#pragma unroll
-      for (int x = 0; x < 4; x++) {
-        int o = (by * 4 + y) * 16 + bx * 4 + x;
-        d[y * 4 + x] = (int)sm.src_y[o] - (int)sm.pred_y[o];
-      }
-    fdct4(d, cc);
-    sm.ldc[by * 4 + bx] = (int16_t)cc[0];
-#pragma unroll
-    for (int i = 0; i < 16; i++) {
-      lv[i] = quant_level(cc[i], c_mf4[qp % 6][pos4(i)], bias, shift);
-      if (lv[i]) my_nz = 1;
-    }
+  const int cmode = analyse_chroma(ht, hl, k0);
+  HalfLevels q = quant_luma(true);
+  const int raster = blk_y(b) * 4 + blk_x(b);
+  if (!h) {
+    sm.ldc[raster] = (int16_t)q.dc;
+    q.ra.x &= 0xffff0000u;  // the DC is coded apart
   }
-  // a group with any level drops its DC slots; AC presence counts only slots 1..15
-  uint32_t gnz = my_nz | __shfl_xor_sync(FULL, my_nz, 1);
-  gnz |= __shfl_xor_sync(FULL, gnz, 2);
-  if (lane < 16) {
-    if (gnz) lv[0] = 0;
-    else {
-#pragma unroll
-      for (int i = 0; i < 16; i++) lv[i] = 0;
-    }
-#pragma unroll
-    for (int i = 1; i < 16; i++) if (lv[i]) my_ac = 1;
-#pragma unroll
-    for (int i = 0; i < 16; i++) sm.coef[lane * 16 + i] = (int16_t)lv[i];
-  }
+  // without an AC level the macroblock codes none (cbp 0)
+  const bool ac = (q.mask & 0xfffeu) != 0;
+  const uint32_t nz = even_bits(__ballot_sync(FULL, ac));
+  const int cbpl = nz ? 15 : 0;
+  const uint32_t nzm = cbpl ? nz : 0u;
+  *(uint2*)&sm.coef[b * 16 + h * 4] = q.ra;
+  *(uint2*)&sm.coef[b * 16 + h * 4 + 8] = q.rb;
   __syncwarp();
-  int cbpl = wor(my_ac) ? 15 : 0;
-  // luma DC: Hadamard (>> 1) + quantisation (enc.rs:1960), then inverse (h264.rs:1645)
-  if (lane == 0) {
-    int t[16], had[16];
-    for (int r = 0; r < 4; r++) {
-      int b0 = sm.ldc[r * 4], b1 = sm.ldc[r * 4 + 1], b2 = sm.ldc[r * 4 + 2], b3 = sm.ldc[r * 4 + 3];
-      int s03 = b0 + b3, s12 = b1 + b2, d03 = b0 - b3, d12 = b1 - b2;
-      t[r * 4] = s03 + s12; t[r * 4 + 1] = d03 + d12; t[r * 4 + 2] = s03 - s12; t[r * 4 + 3] = d03 - d12;
-    }
-    for (int k = 0; k < 4; k++) {
-      int s03 = t[k] + t[k + 12], s12 = t[k + 4] + t[k + 8], d03 = t[k] - t[k + 12], d12 = t[k + 4] - t[k + 8];
-      had[k] = (int16_t)((s03 + s12) >> 1); had[k + 4] = (int16_t)((d03 + d12) >> 1);
-      had[k + 8] = (int16_t)((s03 - s12) >> 1); had[k + 12] = (int16_t)((d03 - d12) >> 1);
-    }
-    int qbits = 16 + qp / 6, mf = c_mf4[qp % 6][0], f = (1 << qbits) / 3;
-    int lvl[16];
-    for (int i = 0; i < 16; i++) {
-      int a = had[i] < 0 ? -had[i] : had[i];
-      int l = (a * mf + f) >> qbits;
-      lvl[i] = had[i] < 0 ? -l : l;
-      sm.ldc[i] = (int16_t)lvl[i];
-    }
-    int qmul = (c_dq4[qp % 6][0] * 16) << (qp / 6 + 2);
-    int tt[16];
-    for (int i = 0; i < 4; i++) {
-      int z0 = lvl[4 * i] + lvl[4 * i + 1], z1 = lvl[4 * i] - lvl[4 * i + 1];
-      int z2 = lvl[4 * i + 2] - lvl[4 * i + 3], z3 = lvl[4 * i + 2] + lvl[4 * i + 3];
-      tt[4 * i] = z0 + z3; tt[4 * i + 1] = z0 - z3; tt[4 * i + 2] = z1 - z2; tt[4 * i + 3] = z1 + z2;
-    }
-    for (int i = 0; i < 4; i++) {
-      int z0 = tt[i] + tt[8 + i], z1 = tt[i] - tt[8 + i], z2 = tt[4 + i] - tt[12 + i], z3 = tt[4 + i] + tt[12 + i];
-      sm.ldcr[i] = (int16_t)(((z0 + z3) * qmul + 128) >> 8);
-      sm.ldcr[4 + i] = (int16_t)(((z1 + z2) * qmul + 128) >> 8);
-      sm.ldcr[8 + i] = (int16_t)(((z1 - z2) * qmul + 128) >> 8);
-      sm.ldcr[12 + i] = (int16_t)(((z0 - z3) * qmul + 128) >> 8);
-    }
-  }
-  const ChromaAc ac = chroma_quant(qpc, true);
-  int cbpc = (ac.any(0) || ac.any(1)) ? 2 : (ac.dc() ? 1 : 0);
+  // luma DC: Hadamard (>> 1) + quantisation (enc.rs:1960), then the inverse (h264.rs:1645)
+  const int had = hadamard16(sm.ldc[lane & 15]) >> 1;
+  const int l = quant_dc(abs(had), sm.qt[0]), level = had < 0 ? -l : l;
+  const int dcr = (hadamard16(level) * sm.qt[0].dc_dq + 128) >> 8;
   __syncwarp();
-  // record
+  if (lane < 16) {
+    sm.ldc[lane] = (int16_t)level;
+    sm.ldcr[lane] = (int16_t)dcr;
+  }
+  const ChromaAc ca = chroma_quant(true);
+  const int cbpc = (ca.any(0) || ca.any(1)) ? 2 : (ca.dc() ? 1 : 0);
+  __syncwarp();
   rg_mb_out* rec = sm.sd.rec + c.mb;
   record_luma4x4(rec);
   if (lane < 16) rec->luma_dc[lane] = sm.ldc[(kScan4Packed >> (4 * lane)) & 15];
-  const uint32_t nzm = __ballot_sync(FULL, lane < 16 && cbpl && my_ac);
   record_chroma(rec, cbpc);
   record_header(rec, RG_MB_I16X16, mode, cmode, cbpl | (cbpc << 4), 0, qp, 0, 0, 0, 0, nzm, false);
-  // reconstruction
-  if (lane < 16) {
-    int bx = blk_x(lane), by = blk_y(lane);
-    int blk[16], res[16];
-#pragma unroll
-    for (int i = 0; i < 16; i++) {
-      int v = sm.coef[lane * 16 + i];
-      blk[i] = cbpl ? clamp_i16(v * ((int)c_dq4[qp % 6][pos4(i)] << (qp / 6))) : v;
-    }
-    blk[0] = sm.ldcr[by * 4 + bx];
-    idct4(blk, res);
-#pragma unroll
-    for (int y = 0; y < 4; y++)
-#pragma unroll
-      for (int x = 0; x < 4; x++) {
-        int o = (by * 4 + y) * 16 + bx * 4 + x;
-        sm.pred_y[o] = (uint8_t)clip255(sm.pred_y[o] + res[y * 4 + x]);
-      }
-  }
-  __syncwarp();
-  chroma_recon(qpc, cbpc);
+  recon_half(q.ra, q.rb, 0, true, sm.ldcr[raster], blk_off16(b) + (int)offsetof(Smem, pred_y), 16, true);
+  chroma_recon(cbpc);
   store_recon(c, (int)offsetof(Smem, pred_y));
   write_info(c, kFlagIntra, cbpl, 0, 0, -1, nzm, false);
 }
@@ -1326,12 +1285,9 @@ __device__ __noinline__ int analyse_i4(const Ctx c, uint32_t budget, bool ht_mb,
   const FrameParams& fp = sm.fp;
   int lane = lane_id();
   int p = lane & 15, xl = p & 3, yl = p >> 2;
-  int qp = sm.sd.qp;
-  uint32_t lambda = c_lambda[qp];
-  uint32_t shift, bias;
-  quant4_params(qp, true, shift, bias);
-  uint32_t mf = c_mf4[qp % 6][pos4(p)];
-  int dqs = (int)c_dq4[qp % 6][pos4(p)] << (qp / 6);
+  const QTab& qt = sm.qt[0];
+  const uint32_t lambda = qt.lambda, shift = qt.shift, bias = qt.bias[1], mf = qt.mf[yl & 1][xl & 1];
+  const int dqs = qt.dq[yl & 1][xl & 1];
   uint32_t total = lambda * 24;
   int cbpl = 0;
   const MbInfo* info = sm.sd.info;
@@ -1452,18 +1408,17 @@ __device__ __noinline__ int analyse_i4(const Ctx c, uint32_t budget, bool ht_mb,
 // `luma`: what analyse_i4 returned.
 __device__ __noinline__ void code_i4(const Ctx c, int luma, bool ht, bool hl, Corner k0) {
   int lane = lane_id();
-  int qpc = sm.sd.qpc;
   const int cbpl = luma & 15;
   const uint32_t nzm = (uint32_t)luma >> 4;
   int cmode = analyse_chroma(ht, hl, k0);
-  const ChromaAc ac = chroma_quant(qpc, true);
+  const ChromaAc ac = chroma_quant(true);
   int cbpc = (ac.any(0) || ac.any(1)) ? 2 : (ac.dc() ? 1 : 0);
   rg_mb_out* rec = sm.sd.rec + c.mb;
   record_luma4x4(rec);
   if (lane < 8) ((uint32_t*)rec)[kWordLumaDc + lane] = 0u;
   record_chroma(rec, cbpc);
   record_header(rec, RG_MB_I4X4, 0, cmode, cbpl | (cbpc << 4), 0, sm.sd.qp, 0, 0, 0, 0, nzm, true);
-  chroma_recon(qpc, cbpc);
+  chroma_recon(cbpc);
   store_recon(c, (int)offsetof(Smem, tmp_y));
   write_info(c, kFlagIntra, cbpl, 0, 0, -1, nzm, true);
 }
@@ -1472,7 +1427,7 @@ __device__ __noinline__ void code_i4(const Ctx c, int luma, bool ht, bool hl, Co
 __device__ __noinline__ void analyse_intra_mb(const Ctx c) {
   const Corner k0 = load_edges(c, true);
   bool ht = c.mby > 0, hl = c.mbx > 0;
-  uint32_t lambda = c_lambda[sm.sd.qp];
+  uint32_t lambda = sm.qt[0].lambda;
   const I16Fit fit16 = analyse_i16(ht, hl, k0.y);
   if (fit16.cost > 40 * lambda) {
     const int cbpl = analyse_i4<false>(c, fit16.cost + lambda * 4, ht, hl, k0.y, nullptr);
@@ -1498,9 +1453,8 @@ __device__ __noinline__ void code_skip(const Ctx c, int mvx, int mvy) {
 
 // Probe of the skip residual (enc.rs:2163 probe_skip_luma): no level above 1 and a total
 // decimation score below 6.
-__device__ __noinline__ bool probe_skip_luma(int qp) {
-  Half4 v;
-  const uint32_t m = luma4x4_levels(qp, v);
+__device__ __noinline__ bool probe_skip_luma() {
+  const uint32_t m = quant_luma(false).mask;
   const uint32_t score = (lane_id() & 1) ? 0u : score4(m, 0);
   return wsum(score | ((m >> 16) << 16)) < 6;
 }
@@ -1509,15 +1463,15 @@ __device__ __noinline__ bool probe_skip_luma(int qp) {
 // (enc.rs:3158-3190), its record (code_inter, enc.rs:3196) and its reconstruction. can_skip: nothing
 // coded makes it P_Skip with vector (mvx, mvy). Returns whether it did.
 __device__ __noinline__ bool code_inter(const Ctx c, int type, bool can_skip, int mvx, int mvy, int mvdx, int mvdy) {
-  const int lane = lane_id(), qp = sm.sd.qp, qpc = sm.sd.qpc;
-  const Luma4 l4 = luma4x4_inter(qp);
+  const int lane = lane_id(), qp = sm.sd.qp;
+  const Luma4 l4 = luma4x4_inter();
   uint32_t cbpl = l4.cbp;
   bool use8 = false;
   if (sm.fp.t8x8 && l4.cbp) {
-    const uint32_t r8 = luma8x8_inter(qp);
+    const uint32_t r8 = luma8x8_inter();
     if ((r8 >> 4) <= l4.nnz) { use8 = true; cbpl = r8 & 15u; }
   }
-  const ChromaAc ac = chroma_quant(qpc, false);
+  const ChromaAc ac = chroma_quant(false);
   // drop a plane's AC levels when nearly empty (enc.rs:2095)
   const bool drop_u = ac.any(0) && ac.score(0) < 7, drop_v = ac.any(1) && ac.score(1) < 7;
   if ((lane & 16) ? drop_v : drop_u) *(uint2*)&sm.ccoef[lane * 4] = make_uint2(0u, 0u);
@@ -1543,10 +1497,10 @@ __device__ __noinline__ bool code_inter(const Ctx c, int type, bool can_skip, in
   record_header(rec, type, 0, 0, (int)cbpl | (cbpc << 4), t8flag, qp, mvx, mvy, mvdx, mvdy, nzm, false);
   write_info(c, t8flag ? kFlagT8 : 0, (int)cbpl, mvx, mvy, 0, nzm, false);
   if (cbpl) {
-    if (use8) recon_luma8x8(qp, (int)cbpl);
-    else recon_luma4x4(qp);
+    if (use8) recon_luma8x8((int)cbpl);
+    else recon_luma4x4();
   }
-  chroma_recon(qpc, cbpc);
+  chroma_recon(cbpc);
   store_recon(c, (int)offsetof(Smem, pred_y));
   return false;
 }
@@ -1652,224 +1606,187 @@ __device__ __noinline__ bool wait_reference(const Ctx c, const PipeWait pw, int 
   return ok;
 }
 
+struct Bounds {
+  int min0, min1, max0, max1;  // quarter samples (MvBounds, enc.rs:1105)
+};
+__device__ __forceinline__ bool in_bounds(const Bounds& b, int x, int y) {
+  return x >= b.min0 && x <= b.max0 && y >= b.min1 && y <= b.max1;
+}
+__device__ __forceinline__ Bounds mv_bounds(int x0, int y0) {
+  const int cw = sm.fp.mb_w * 16, ch = sm.fp.mb_h * 16;
+  return {-4 * (x0 + 28), max(-4 * (y0 + 28), -2048), 4 * (cw - 16 - x0 + 28), min(4 * (ch - 16 - y0 + 28), 2044)};
+}
+__device__ __forceinline__ int lo16(int w) { return (int16_t)(w & 0xffff); }
+
+// P_Skip probe (enc.rs:2906 try_p_skip) at skip vector (ps0, ps1): true when the macroblock is coded as
+// P_Skip (prediction left in pred_y / pred_u / pred_v).
+__device__ __noinline__ bool skip_probe(const Ctx c, int ps0, int ps1) {
+  const StreamDev& sd = sm.sd;
+  const int lane = lane_id();
+  mc_luma16(c.mbx * 16, c.mby * 16, ps0, ps1);
+  {
+    const uint2 s = src8(), p = *(const uint2*)&sm.pred_y[lane * 8];
+    const uint32_t dx = __vabsdiffu4(s.x, p.x), dy = __vabsdiffu4(s.y, p.y);
+    const uint32_t sad = wsum(__dp4a(dx, 0x01010101u, __dp4a(dy, 0x01010101u, 0u)));
+    if (sad >= sd.sb_probe) return false;
+    if (sad > sd.sb_luma && wsum(__dp4a(dx, dx, __dp4a(dy, dy, 0u))) > sd.sb_luma_ssd && !probe_skip_luma()) return false;
+  }
+  mc_chroma8(sd.ref_u, sd.ref_v, sm.fp.stride_c, c.mbx, c.mby, ps0, ps1);
+  // per plane SAD / SSD bounds (lanes 0..15 U, 16..31 V, 4 samples each)
+  const uint32_t d = __vabsdiffu4(*(const uint32_t*)&sm.src_u[lane * 4], *(const uint32_t*)&sm.pred_u[lane * 4]);
+  const uint32_t sad = __dp4a(d, 0x01010101u, 0u), ssd = __dp4a(d, d, 0u);
+  const bool v = lane & 16;
+  const uint32_t sads = wsum(v ? sad << 16 : sad), ssd_u = wsum(v ? 0u : ssd), ssd_v = wsum(v ? ssd : 0u);
+  if (((sads & 0xffffu) <= sd.sb_chroma || ssd_u <= sd.sb_chroma_ssd) && ((sads >> 16) <= sd.sb_chroma || ssd_v <= sd.sb_chroma_ssd))
+    return true;
+  const ChromaAc ac = chroma_quant(false);
+  return !ac.dc() && ac.score(0) < 7 && ac.score(1) < 7;
+}
+
+// This lane's SADs of the source (sv) against the predictions of the vectors (dx0, dy0) and (dx1, dy1)
+// from the window's position, two to a word.
+__device__ __forceinline__ uint32_t qpel_sad2(uint2 sv, int dx0, int dy0, int dx1, int dy1) {
+  const uint32_t a = vsad8(sv, qpel8(dx0, dy0));
+  return a | (vsad8(sv, qpel8(dx1, dy1)) << 16);
+}
+
 // One macroblock of a P slice (enc.rs:3011 code_p_mb). In the pipelined mode (pw.db_prev) it first
 // waits for the reference frame to be final over every sample its search can read; when a wait
 // gives up it returns false and writes nothing.
 __device__ __noinline__ bool analyse_p_mb(const Ctx c, const PipeWait pw) {
   const FrameParams& fp = sm.fp;
   const StreamDev& sd = sm.sd;
-  int lane = lane_id();
-  int mbx = c.mbx, mby = c.mby, mb_w = fp.mb_w;
-  int x0 = mbx * 16, y0 = mby * 16;
-  int qp = sm.sd.qp;
-  uint32_t lambda = c_lambda[qp];
-  int cw = fp.mb_w * 16, chh = fp.mb_h * 16;
-  // MvBounds (enc.rs:1105)
-  int bmin0 = -4 * (x0 + 28), bmin1 = max(-4 * (y0 + 28), -2048);
-  int bmax0 = 4 * (cw - 16 - x0 + 28), bmax1 = min(4 * (chh - 16 - y0 + 28), 2044);
-  // neighbours (this picture)
-  const MbInfo* info = sd.info;
-  int lref = -2, tref = -2, dref = -2;
-  int a0 = 0, a1 = 0, b0 = 0, b1 = 0, c0 = 0, c1 = 0;
-  if (mbx > 0) { MbInfo n = ld_info(&info[c.mb - 1]); lref = n.ref; a0 = n.mv[0]; a1 = n.mv[1]; }
-  if (mby > 0) { MbInfo n = ld_info(&info[c.mb - mb_w]); tref = n.ref; b0 = n.mv[0]; b1 = n.mv[1]; }
-  if (mby > 0 && mbx + 1 < mb_w) { MbInfo n = ld_info(&info[c.mb - mb_w + 1]); dref = n.ref; c0 = n.mv[0]; c1 = n.mv[1]; }
-  else if (mby > 0 && mbx > 0) { MbInfo n = ld_info(&info[c.mb - mb_w - 1]); dref = n.ref; c0 = n.mv[0]; c1 = n.mv[1]; }
-  // pred_motion_partition (h264.rs:3577), 16x16, ref 0
-  int mvp0, mvp1;
+  const int lane = lane_id(), mbx = c.mbx, mby = c.mby, x0 = mbx * 16, y0 = mby * 16;
+  const uint32_t lambda = sm.qt[0].lambda;
+  const Bounds bd = mv_bounds(x0, y0);
+  // neighbours (this picture) and the co-located macroblock of the previous one, a lane each: left,
+  // top, top-right (top-left where that is absent), co-located; ref -2 when absent
+  const MbInfo* nb = nullptr;
+  if (lane == 0 && mbx > 0) nb = &sd.info[c.mb - 1];
+  if (lane == 1 && mby > 0) nb = &sd.info[c.mb - fp.mb_w];
+  if (lane == 2 && mby > 0 && fp.mb_w > 1) nb = &sd.info[c.mb - fp.mb_w + (mbx + 1 < fp.mb_w ? 1 : -1)];
+  if (lane == 3) nb = &sd.prev_info[c.mb];
+  const uint2 nw = nb ? *(const uint2*)nb : make_uint2(0u, 0xfeu);
+  load_source(c);
+  const int va = __shfl_sync(FULL, (int)nw.x, 0), vb = __shfl_sync(FULL, (int)nw.x, 1), vc = __shfl_sync(FULL, (int)nw.x, 2),
+            vp = __shfl_sync(FULL, (int)nw.x, 3);
+  const int ref = (int8_t)(nw.y & 255u);
+  const uint32_t inter = __ballot_sync(FULL, ref == 0) & 7u, absent = __ballot_sync(FULL, ref == -2) & 7u;
+  // pred_motion_partition (h264.rs:3577), 16x16, ref 0: the only inter neighbour, the left one when
+  // it is the only one there is, else the median
+  int mvp;
   {
     auto med = [](int x, int y, int z) { return min(max(x, y), max(min(x, y), z)); };
-    int m = (lref == 0) + (tref == 0) + (dref == 0);
-    if (m > 1) { mvp0 = med(a0, b0, c0); mvp1 = med(a1, b1, c1); }
-    else if (m == 1) {
-      if (lref == 0) { mvp0 = a0; mvp1 = a1; }
-      else if (tref == 0) { mvp0 = b0; mvp1 = b1; }
-      else { mvp0 = c0; mvp1 = c1; }
-    } else if (tref == -2 && dref == -2 && lref != -2) { mvp0 = a0; mvp1 = a1; }
-    else { mvp0 = med(a0, b0, c0); mvp1 = med(a1, b1, c1); }
+    mvp = (int)pack16(med(lo16(va), lo16(vb), lo16(vc)), med(va >> 16, vb >> 16, vc >> 16));
+    if (inter == 1u || (inter == 0u && absent == 6u)) mvp = va;
+    if (inter == 2u) mvp = vb;
+    if (inter == 4u) mvp = vc;
   }
-  int ps0 = mvp0, ps1 = mvp1;
-  if (mbx == 0 || mby == 0 || (lref == 0 && a0 == 0 && a1 == 0) || (tref == 0 && b0 == 0 && b1 == 0)) { ps0 = 0; ps1 = 0; }
-  load_source(c);
-  int qpc = sm.sd.qpc;
-  // co-located vector of the previous picture: a search candidate (enc.rs:3094)
-  MbInfo prevmb = ld_info(&sd.prev_info[c.mb]);
+  const int ps = mbx == 0 || mby == 0 || ((inter & 1u) && va == 0) || ((inter & 2u) && vb == 0) ? 0 : mvp;
+  const int mvp0 = lo16(mvp), mvp1 = mvp >> 16, ps0 = lo16(ps), ps1 = ps >> 16;
+  // Full-pel candidates (enc.rs:3084-3105): predictor, zero, left (if any), top (if any) and the
+  // co-located vector of the previous picture, rounded and clamped; lane k holds candidate k.
+  const int imin0 = (bd.min0 + 3) >> 2, imin1 = (bd.min1 + 3) >> 2, imax0 = bd.max0 >> 2, imax1 = bd.max1 >> 2;
+  int cx, cy;
+  {
+    const int v = lane == 1 ? 0 : (lane == 2 ? va : (lane == 3 ? vb : (lane == 4 ? vp : mvp)));
+    cx = min(max((lo16(v) + 2) >> 2, imin0), imax0);
+    cy = min(max(((v >> 16) + 2) >> 2, imin1), imax1);
+  }
   if (pw.db_prev) {
     // The right- and bottom-most reference sample this macroblock can read: the full-pel
     // candidates, a diamond of at most 16 steps around the best, the half-sample window
     // (-3..+20) and 8-byte loads. Everything above and to the left of it (padding included) is
     // final once the macroblock holding it is.
-    int cx[5] = {mvp0, 0, a0, b0, prevmb.mv[0]}, cy[5] = {mvp1, 0, a1, b1, prevmb.mv[1]};
-    int hi0 = -(1 << 20), hi1 = -(1 << 20);
-    int imn0 = (bmin0 + 3) >> 2, imn1 = (bmin1 + 3) >> 2, imx0 = bmax0 >> 2, imx1 = bmax1 >> 2;
-#pragma unroll
-    for (int k = 0; k < 5; k++) {
-      hi0 = max(hi0, min(max((cx[k] + 2) >> 2, imn0), imx0));
-      hi1 = max(hi1, min(max((cy[k] + 2) >> 2, imn1), imx1));
-    }
+    const int hi0 = __reduce_max_sync(FULL, cx), hi1 = __reduce_max_sync(FULL, cy);
     if (!wait_reference(c, pw, (x0 + hi0 + 44) >> 4, (y0 + hi1 + 40) >> 4)) return false;
   }
+  if (lane == 0) sm.win_x = kNoWin;  // the last macroblock's window
+  __syncwarp();
 
-  // 1. skip probe (enc.rs:2906 try_p_skip)
-  if (ps0 >= bmin0 && ps0 <= bmax0 && ps1 >= bmin1 && ps1 <= bmax1) {
-    mc_luma16(sd.ref_y, fp.stride_y, x0, y0, ps0, ps1);
-    uint2 s = src8(), p = *(const uint2*)&sm.pred_y[(lane >> 1) * 16 + (lane & 1) * 8];
-    uint32_t sad = wsum(vsad8(s, p));
-    if (sad < sm.sd.sb_probe) {
-      bool lz = sad <= sm.sd.sb_luma;
-      if (!lz) {
-        uint32_t ssd = 0;
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-          int d0 = (int)((s.x >> (8 * k)) & 255) - (int)((p.x >> (8 * k)) & 255);
-          int d1 = (int)((s.y >> (8 * k)) & 255) - (int)((p.y >> (8 * k)) & 255);
-          ssd += d0 * d0 + d1 * d1;
-        }
-        lz = wsum(ssd) <= sm.sd.sb_luma_ssd;
-      }
-      if (!lz) lz = probe_skip_luma(qp);
-      if (lz) {
-        mc_chroma8(sd.ref_u, sd.ref_v, fp.stride_c, mbx, mby, ps0, ps1);
-        // per plane SAD / SSD bounds (lanes 0..15 U, 16..31 V, 4 samples each)
-        int plane = lane >> 4, idx = (lane & 15) * 4;
-        const uint8_t* ss = (plane ? sm.src_v : sm.src_u) + idx;
-        const uint8_t* pp = (plane ? sm.pred_v : sm.pred_u) + idx;
-        uint32_t sadp = 0, ssdp = 0;
-#pragma unroll
-        for (int k = 0; k < 4; k++) { int d = (int)ss[k] - (int)pp[k]; sadp += abs(d); ssdp += d * d; }
-        uint32_t sad_u = wsum(plane == 0 ? sadp : 0), sad_v = wsum(plane == 1 ? sadp : 0);
-        uint32_t ssd_u = wsum(plane == 0 ? ssdp : 0), ssd_v = wsum(plane == 1 ? ssdp : 0);
-        bool zu = sad_u <= sm.sd.sb_chroma || ssd_u <= sm.sd.sb_chroma_ssd;
-        bool zv = sad_v <= sm.sd.sb_chroma || ssd_v <= sm.sd.sb_chroma_ssd;
-        bool cz = zu && zv;
-        if (!cz) {
-          const ChromaAc ac = chroma_quant(qpc, false);
-          cz = !ac.dc() && ac.score(0) < 7 && ac.score(1) < 7;
-        }
-        if (cz) {
-          code_skip(c, ps0, ps1);
-          return true;
-        }
-      }
-    }
+  // 1. skip probe
+  if (in_bounds(bd, ps0, ps1) && skip_probe(c, ps0, ps1)) {
+    code_skip(c, ps0, ps1);
+    return true;
   }
 
-  // 2. motion search (enc.rs:3084-3117)
-  const uint8_t* ref = sd.ref_y;
-  int stride = fp.stride_y;
-  // candidates in order: predictor, zero, left (if any), top (if any), co-located of the previous
-  // picture -- five fixed slots, the left / top ones skipped when absent
-  int imin0 = (bmin0 + 3) >> 2, imin1 = (bmin1 + 3) >> 2, imax0 = bmax0 >> 2, imax1 = bmax1 >> 2;
-  uint2 sv = src8();
-  const uint8_t* base = ref + (long)(y0 + (lane >> 1)) * stride + x0 + (lane & 1) * 8;
-  int best0 = 0, best1 = 0;
-  uint32_t best_cost = UMAX;
-  // clamped full-pel candidates, their samples loaded together, then costed in order (a
-  // repeated position is skipped)
-  int cmx[5], cmy[5];
-  bool cval[5];
-  uint2 cref[5];
+  // 2. motion search (enc.rs:3084-3117): the first of the cheapest candidates
+  const int stride = fp.stride_y;
+  const uint2 sv = src8();
+  const uint8_t* base = sd.ref_y + (long)(y0 + (lane >> 1)) * stride + x0 + (lane & 1) * 8;
+  int best0, best1;
+  uint32_t best_cost;
+  {
+    const int at = cy * stride + cx;
+    uint2 r[5];
 #pragma unroll
-  for (int k = 0; k < 5; k++) {
-    int vx = k == 0 ? mvp0 : k == 1 ? 0 : k == 2 ? a0 : k == 3 ? b0 : prevmb.mv[0];
-    int vy = k == 0 ? mvp1 : k == 1 ? 0 : k == 2 ? a1 : k == 3 ? b1 : prevmb.mv[1];
-    cval[k] = k == 2 ? mbx > 0 : (k == 3 ? mby > 0 : true);
-    cmx[k] = min(max((vx + 2) >> 2, imin0), imax0);
-    cmy[k] = min(max((vy + 2) >> 2, imin1), imax1);
-    cref[k] = ldg8(base + (long)cmy[k] * stride + cmx[k]);
-  }
-#pragma unroll
-  for (int k = 0; k < 5; k++) {
-    bool use = cval[k];  // absent, or at the position of an earlier candidate: skipped
-#pragma unroll
-    for (int j = 0; j < k; j++) use &= !(cval[j] && cmx[j] == cmx[k] && cmy[j] == cmy[k]);
-    if (!use) continue;  // uniform across the warp
-    uint32_t cost = fullpel_cost(sv, cref[k], cmx[k], cmy[k], mvp0, mvp1, lambda);
-    if (cost < best_cost) { best_cost = cost; best0 = cmx[k]; best1 = cmy[k]; }
+    for (int k = 0; k < 5; k++) r[k] = ldg8(base + __shfl_sync(FULL, at, k));
+    const uint32_t s01 = wsum(vsad8(sv, r[0]) | (vsad8(sv, r[1]) << 16)), s23 = wsum(vsad8(sv, r[2]) | (vsad8(sv, r[3]) << 16)),
+                   s4 = wsum(vsad8(sv, r[4]));
+    const uint32_t w = lane < 2 ? s01 : (lane < 4 ? s23 : s4);
+    const uint32_t cost = ((w >> (16 * (lane & 1))) & 0xffffu) + mvd_cost(cx * 4 - mvp0, lambda) + mvd_cost(cy * 4 - mvp1, lambda);
+    const bool use = lane < 5 && (lane != 2 || mbx > 0) && (lane != 3 || mby > 0);
+    const uint32_t key = __reduce_min_sync(FULL, use ? (cost << 3) | (uint32_t)lane : UMAX);
+    best_cost = key >> 3;
+    best0 = __shfl_sync(FULL, cx, (int)(key & 7u));
+    best1 = __shfl_sync(FULL, cy, (int)(key & 7u));
   }
   // diamond (enc.rs:1207-1272): up, left, right, down around the best, first strict minimum
-  // wins; each step's four loads are issued together
+  // wins; each step's four loads are issued together (a neighbour past the bounds is still inside
+  // the padded picture, and not counted)
+  const Box ibox{4 * imin0, 4 * imax0, 4 * imin1, 4 * imax1};
 #pragma unroll 1
   for (int it = 0; it < 16; it++) {
-    const uint8_t* cp = base + (long)best1 * stride + best0;
-    uint2 r[4];
-    bool in[4];
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      int dx = k == 1 ? -1 : (k == 2 ? 1 : 0), dy = k == 0 ? -1 : (k == 3 ? 1 : 0);
-      int px = best0 + dx, py = best1 + dy;
-      in[k] = px >= imin0 && px <= imax0 && py >= imin1 && py <= imax1;
-      r[k] = in[k] ? ldg8(cp + dy * stride + dx) : make_uint2(0u, 0u);
-    }
-    int nb0 = best0, nb1 = best1;
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      int dx = k == 1 ? -1 : (k == 2 ? 1 : 0), dy = k == 0 ? -1 : (k == 3 ? 1 : 0);
-      if (!in[k]) continue;  // uniform across the warp
-      uint32_t cost = fullpel_cost(sv, r[k], best0 + dx, best1 + dy, mvp0, mvp1, lambda);
-      if (cost < best_cost) {
-        best_cost = cost;
-        nb0 = best0 + dx;
-        nb1 = best1 + dy;
-      }
-    }
-    if (nb0 == best0 && nb1 == best1) break;
-    best0 = nb0;
-    best1 = nb1;
+    const uint8_t* cp = base + best1 * stride + best0;
+    const uint2 u = ldg8(cp - stride), l = ldg8(cp - 1), r = ldg8(cp + 1), d = ldg8(cp + stride);
+    const uint32_t key = best4(vsad8(sv, u) | (vsad8(sv, l) << 16), vsad8(sv, r) | (vsad8(sv, d) << 16), 4 * best0, 4 * best1, 4, ibox,
+                               mvp0, mvp1, lambda, false);
+    if ((key >> 2) >= best_cost) break;
+    best_cost = key >> 2;
+    const int k = (int)(key & 3u);
+    best0 += k == 1 ? -1 : (k == 2 ? 1 : 0);
+    best1 += k == 0 ? -1 : (k == 3 ? 1 : 0);
   }
-  int mv0, mv1;
+  int mv0 = best0 * 4, mv1 = best1 * 4;
   {
-    int fm0 = best0 * 4, fm1 = best1 * 4;
-    uint32_t full_mvc = mvd_cost(fm0 - mvp0, lambda) + mvd_cost(fm1 - mvp1, lambda);
-    if (best_cost - full_mvc <= sm.sd.sb_luma) {
-      mv0 = fm0; mv1 = fm1;
-      uint2 v = ldg8(base + (long)best1 * stride + best0);
-      *(uint2*)&sm.pred_y[(lane >> 1) * 16 + (lane & 1) * 8] = v;
-      __syncwarp();
-    } else {
-      // sub-pel refinement over a half-sample window around the full-pel best (enc.rs:1283)
-      int bxp = x0 + best0, byp = y0 + best1;
-      stage_window(ref, stride, bxp - 1, byp - 1);
-      build_hpel(7);
-      int q0 = fm0, q1 = fm1;
-      uint32_t bc = best_cost;
+    uint2 v = ldg8(base + best1 * stride + best0);
+    if (wsum(vsad8(sv, v)) > sd.sb_luma) {
+      // sub-pel refinement over a half-sample window around the full-pel best (enc.rs:1283): a
+      // half-sample diamond step, then up to two quarter-sample ones. The steps from the full-pel
+      // position itself never read plane j.
+      ensure_window(x0 + best0, y0 + best1, 3);
+      const Box box{max(bd.min0, mv0 - 3), min(bd.max0, mv0 + 3), max(bd.min1, mv1 - 3), min(bd.max1, mv1 + 3)};
+      int q0 = 0, q1 = 0;  // from the full-pel best
 #pragma unroll 1
-      for (int si = 0; si < 2; si++) {
-        int st = si == 0 ? 2 : 1, iters = si == 0 ? 1 : 2;
-#pragma unroll 1
-        for (int it = 0; it < iters; it++) {
-          int f0 = q0, f1 = q1;
-          int dd[4][2] = {{0, -st}, {-st, 0}, {st, 0}, {0, st}};
-          uint32_t cc[4];
-#pragma unroll
-          for (int k = 0; k < 4; k++) {
-            int cx = f0 + dd[k][0], cy = f1 + dd[k][1];
-            bool ok = abs(cx - fm0) <= 3 && abs(cy - fm1) <= 3 && cx >= bmin0 && cx <= bmax0 && cy >= bmin1 && cy <= bmax1;
-            uint32_t s = ok ? qpel_sad(sv, (cx >> 2) - best0 + 1, (cy >> 2) - best1 + 1, cx & 3, cy & 3) : 0u;
-            s = wsum(s);
-            cc[k] = ok ? s + mvd_cost(cx - mvp0, lambda) + mvd_cost(cy - mvp1, lambda) : UMAX;
-          }
-#pragma unroll
-          for (int k = 0; k < 4; k++)
-            if (cc[k] < bc) { bc = cc[k]; q0 = f0 + dd[k][0]; q1 = f1 + dd[k][1]; }
-          if (q0 == f0 && q1 == f1) break;
+      for (int it = 0; it < 3; it++) {
+        const int st = it == 0 ? 2 : 1;
+        if (it == 1 && (q0 | q1)) ensure_window(x0 + best0, y0 + best1, 7);
+        const uint32_t s01 = qpel_sad2(sv, q0, q1 - st, q0 - st, q1), s23 = qpel_sad2(sv, q0 + st, q1, q0, q1 + st);
+        const uint32_t key = best4(s01, s23, mv0 + q0, mv1 + q1, st, box, mvp0, mvp1, lambda, false);
+        if ((key >> 2) < best_cost) {
+          best_cost = key >> 2;
+          const int k = (int)(key & 3u);
+          q0 += k == 1 ? -st : (k == 2 ? st : 0);
+          q1 += k == 0 ? -st : (k == 3 ? st : 0);
+        } else if (it) {
+          break;
         }
       }
-      mv0 = q0; mv1 = q1;
-      uint2 v = qpel8(qpel_src((q0 >> 2) - best0 + 1, (q1 >> 2) - best1 + 1, q0 & 3, q1 & 3));
-      *(uint2*)&sm.pred_y[(lane >> 1) * 16 + (lane & 1) * 8] = v;
-      __syncwarp();
+      v = qpel8(q0, q1);
+      mv0 += q0;
+      mv1 += q1;
     }
+    *(uint2*)&sm.pred_y[lane * 8] = v;
+    __syncwarp();
   }
 
   // 3. intra 16x16 when the inter prediction is poor (enc.rs:3121-3156)
   const uint32_t inter_satd = satd16((int)offsetof(Smem, pred_y));
-  uint32_t inter_cost = inter_satd + lambda * (se_bits(mv0 - mvp0) + se_bits(mv1 - mvp1) + 1);
   if (inter_satd > 24 * lambda) {
     const Corner k0 = load_edges(c, false);
-    bool ht = mby > 0, hl = mbx > 0;
+    const bool ht = mby > 0, hl = mbx > 0;
     const I16Fit fit16 = analyse_i16(ht, hl, k0.y);
-    if (fit16.cost + lambda * 8 < inter_cost) {
+    if (fit16.cost + lambda * 8 < inter_satd + lambda * (se_bits(mv0 - mvp0) + se_bits(mv1 - mvp1) + 1)) {
       code_i16(c, fit16.mode, ht, hl, k0);
       return true;
     }
@@ -2027,9 +1944,9 @@ __device__ __noinline__ void deblock_mb(int mbx, int mby) {
         (!hast || (quiet(tp) && tp.mv[0] == q.mv[0] && tp.mv[1] == q.mv[1])))
       return;
   }
-  // tiles: luma 20x20 at (x0-4, y0-4) stride 20 in win; chroma 12x12 each in hph / hpv
+  // tiles: luma 20x20 at (x0-4, y0-4) stride 20 in win; chroma 12x12 each in two half-sample planes
   uint8_t* ty = sm.win;
-  auto tc = [](int p) { return sm.hph + p * (int)(offsetof(Smem, hpv) - offsetof(Smem, hph)); };
+  auto tc = [](int p) { return sm.hp[p]; };
   const int x0 = mbx * 16, y0 = mby * 16, cx0 = mbx * 8, cy0 = mby * 8;
   for (int w = lane; w < 100; w += 32) {  // 20 rows x 5 words
     int r = w / 5, k = w % 5;
@@ -2470,17 +2387,31 @@ __global__ void extend_borders_kernel(FrameParams fp, const StreamDev* __restric
 
 void upload_tables() {
   using namespace tables;
-  cudaMemcpyToSymbol(c_lambda, kLambda, sizeof(kLambda));
-  cudaMemcpyToSymbol(c_dec4, kDecimate4, sizeof(kDecimate4));
-  uint8_t d8[64] = {0};
-  for (int i = 0; i < 24; i++) d8[i] = kDecimate8[i];
-  cudaMemcpyToSymbol(c_dec8, d8, sizeof(d8));
-  cudaMemcpyToSymbol(c_scan4, kScan4, sizeof(kScan4));
-  cudaMemcpyToSymbol(c_scan8, kScan8, sizeof(kScan8));
-  cudaMemcpyToSymbol(c_mf4, kMf4, sizeof(kMf4));
-  cudaMemcpyToSymbol(c_dq4, kDq4, sizeof(kDq4));
-  cudaMemcpyToSymbol(c_mf8, kMf8, sizeof(kMf8));
-  cudaMemcpyToSymbol(c_dq8, kDq8, sizeof(kDq8));
+  QTab qt[52];
+  for (int qp = 0; qp < 52; qp++) {
+    QTab& t = qt[qp];
+    const int rem = qp % 6, d = qp / 6;
+    const uint16_t* m = kMf4[rem];
+    const uint8_t* k = kDq4[rem];
+    t.mf[0][0] = m[0]; t.mf[0][1] = t.mf[1][0] = m[2]; t.mf[1][1] = m[1];
+    t.dq[0][0] = k[0] << d; t.dq[0][1] = t.dq[1][0] = k[2] << d; t.dq[1][1] = k[1] << d;
+    t.shift = 15 + d;
+    t.bias[0] = (1u << t.shift) / 6u;
+    t.bias[1] = (1u << t.shift) / 3u;
+    t.dc_mf = m[0];
+    t.dc_dq = (k[0] * 16) << (d + 2);
+    t.lambda = kLambda[qp];
+    const int cls[3][3] = {{0, 3, 4}, {3, 1, 5}, {4, 5, 2}};
+    for (int x = 0; x < 3; x++)
+      for (int y = 0; y < 3; y++) {
+        t.mf8[x][y] = kMf8[rem][cls[x][y]];
+        t.dq8[x][y] = kDq8[rem][cls[x][y]] << (d >= 2 ? d - 2 : 0);
+      }
+    t.bias8 = (1u << (16 + d)) / 6u;
+    t.rnd8 = d >= 2 ? 0 : 1 << (1 - d);
+    t.sh8 = d >= 2 ? 0 : 2 - d;
+  }
+  cudaMemcpyToSymbol(g_qtab, qt, sizeof(qt));
   cudaMemcpyToSymbol(c_cqp, kChromaQp, sizeof(kChromaQp));
   cudaMemcpyToSymbol(c_alpha, kAlpha, sizeof(kAlpha));
   cudaMemcpyToSymbol(c_beta, kBeta, sizeof(kBeta));

@@ -56,7 +56,6 @@ struct SearchSmem {
   int bmv[4][2], bmvd[4][2], own[4][2], pm[4][2], pd[4][2], qmv[4][2];
   int ccx[8], ccy[8];  // the learned form's centre candidates (ok: cok)
   bool cok[8];
-  int wbx, wby;        // integer vector of the half-sample planes held
 };
 __shared__ SearchSmem ss;
 __device__ __forceinline__ void ld_q(const MbMv4* m, int q, int* v) {
@@ -128,12 +127,6 @@ struct PartFit {
   int x, y;
 };
 
-struct Bounds {
-  int min0, min1, max0, max1;  // quarter samples (MvBounds, enc.rs:1105)
-};
-__device__ __forceinline__ bool in_bounds(const Bounds& b, int x, int y) {
-  return x >= b.min0 && x <= b.max0 && y >= b.min1 && y <= b.max1;
-}
 __device__ __forceinline__ uint32_t vec_cost(int dx, int dy, uint32_t lambda) {
   return lambda * (se_bits(dx) + se_bits(dy));
 }
@@ -305,36 +298,27 @@ __device__ __forceinline__ uint32_t satd4_regs(const uint32_t* sa, const uint32_
   }
   return s;
 }
-// The 4x4 prediction at window position (wx, wy), phase (fx, fy): four packed rows.
-__device__ __forceinline__ void qpel4(int wx, int wy, int fx, int fy, uint32_t* out) {
-  QSrc q = qpel_src(wx, wy, fx, fy);
+// The 4x4 prediction at the block's sample (ox, oy) for the vector (dx, dy) from the window's position:
+// four packed rows.
+__device__ __forceinline__ void qpel4(int ox, int oy, int dx, int dy, uint32_t* out) {
+  const uint8_t* p = &sm.win[0] + qpel_pos(dx, dy) + oy * 24 + ox;
+  const uint32_t e = sm.qpt[(dx & 3) | ((dy & 3) << 2)];
 #pragma unroll
-  for (int r = 0; r < 4; r++) {
-    uint32_t a = lds4u(sm_at(q.a + r * q.sa));
-    out[r] = q.avg ? __vavgu4(a, lds4u(sm_at(q.b + r * q.sb))) : a;
-  }
+  for (int r = 0; r < 4; r++) out[r] = __vavgu4(lds4u(p + r * 24 + (e & 0xffffu)), lds4u(p + r * 24 + (e >> 16)));
 }
 __device__ __constant__ int8_t c_hstep[8][2] = {{0, -2}, {-2, 0}, {2, 0}, {0, 2}, {-2, -2}, {2, -2}, {-2, 2}, {2, 2}};
 
 // The half-sample planes in shared memory serve every part whose integer vector they were built
-// around: a macroblock-level window (origin one sample above-left of the macroblock displaced by the
-// vector) covers every 4x4 block of the macroblock at quarter-sample offsets -3..3.
-// ss.wbx / wby: the integer vector of the planes held, or kNoWin.
-constexpr int kNoWin = 1 << 20;
-__device__ __forceinline__ void ensure_window(const Ctx c, int bx, int by) {
-  if (ss.wbx == bx && ss.wby == by) return;
-  stage_window(sm.sd.ref_y, sm.fp.stride_y, c.mbx * 16 + bx - 1, c.mby * 16 + by - 1);
-  build_hpel(7);
-  __syncwarp();
-  ss.wbx = bx;
-  ss.wby = by;
-  __syncwarp();
+// around: the macroblock's window (ensure_window) covers every 4x4 block of the macroblock at
+// quarter-sample offsets -3..3.
+__device__ __forceinline__ void ensure_mb_window(const Ctx c, int bx, int by) {
+  ensure_window(c.mbx * 16 + bx, c.mby * 16 + by, 7);
 }
 
 __device__ __noinline__ PartFit refine_part(const Ctx c, int px, int py, int pw, int ph, int bx,
                                             int by, int2 mvp, uint32_t lambda, Bounds bd) {
   const int lane = lane_id();
-  ensure_window(c, bx, by);
+  ensure_mb_window(c, bx, by);
   const int bw4 = pw >> 2, nblk = bw4 * (ph >> 2);
   const int m0x = 4 * bx, m0y = 4 * by;
   int cx = m0x, cy = m0y;
@@ -356,7 +340,7 @@ __device__ __noinline__ PartFit refine_part(const Ctx c, int px, int py, int pw,
       if (ok) {
         const int ox = 4 * (blk % bw4), oy = 4 * (blk / bw4);
         uint32_t pa[4], sa[4];
-        qpel4((vx >> 2) - bx + 1 + px + ox, (vy >> 2) - by + 1 + py + oy, vx & 3, vy & 3, pa);
+        qpel4(px + ox, py + oy, vx - m0x, vy - m0y, pa);
 #pragma unroll
         for (int r = 0; r < 4; r++) sa[r] = *(const uint32_t*)&sm.src_y[(py + oy + r) * 16 + px + ox];
         s = satd4_regs(sa, pa);
@@ -387,38 +371,49 @@ __device__ __noinline__ PartFit refine_part(const Ctx c, int px, int py, int pw,
 // diamond (up, left, right, down at distance 2, one step), then the quarter-sample diamond (the
 // same at distance 1, up to two steps, each from the step's start), cost SAD + lambda * vector bits
 // against the part's predictor, the first strict minimum in that order; lanes take the part's
-// 4-sample words, one candidate at a time.
-__device__ __noinline__ uint32_t part_sad(int px, int py, int pw, int ph, int bx, int by, int vx, int vy) {
+// 4-sample words.
+// This lane's share of the part's SAD at the vector (dx, dy) from the window's position: the part's
+// 4-sample words lane, lane + 32 (shift: log2 of the words per row).
+__device__ __noinline__ uint32_t part_sad(int at, int src, int shift, int nw, int dx, int dy) {
   const int lane = lane_id();
-  const QSrc q = qpel_src((vx >> 2) - bx + 1 + px, (vy >> 2) - by + 1 + py, vx & 3, vy & 3);
-  const int wpr = pw >> 2, nw = wpr * ph;
+  const uint32_t e = sm.qpt[(dx & 3) | ((dy & 3) << 2)];
+  const uint8_t* p = &sm.win[0] + qpel_pos(dx, dy) + at;
   uint32_t s = 0;
   for (int w = lane; w < nw; w += 32) {
-    const int r = w / wpr, x = (w - r * wpr) * 4;
-    uint32_t a = lds4u(sm_at(q.a + r * q.sa + x));
-    if (q.avg) a = __vavgu4(a, lds4u(sm_at(q.b + r * q.sb + x)));
-    s = __vsadu4(a, *(const uint32_t*)&sm.src_y[(py + r) * 16 + px + x]) + s;
+    const int r = w >> shift, x = (w - (r << shift)) * 4;
+    const uint8_t* q = p + r * 24 + x;
+    s = __vsadu4(__vavgu4(lds4u(q + (e & 0xffffu)), lds4u(q + (e >> 16))), *(const uint32_t*)&sm.src_y[src + r * 16 + x]) + s;
   }
-  return wsum(s);
+  return s;
 }
 __device__ __noinline__ PartFit refine_part_sad(const Ctx c, int px, int py, int pw, int ph,
                                                 int bx, int by, int2 mvp, uint32_t lambda, Bounds bd) {
-  ensure_window(c, bx, by);
-  int cx = 4 * bx, cy = 4 * by;
-  uint32_t best = part_sad(px, py, pw, ph, bx, by, cx, cy) + vec_cost(cx - mvp.x, cy - mvp.y, lambda);
-  for (int st = 2; st >= 1; st--) {
-    for (int it = 0; it < (st == 2 ? 1 : 2); it++) {
-      const int fx = cx, fy = cy;
-      for (int k = 0; k < 4; k++) {
-        const int vx = fx + (k == 1 ? -st : (k == 2 ? st : 0)), vy = fy + (k == 0 ? -st : (k == 3 ? st : 0));
-        if (abs(vx - 4 * bx) > 3 || abs(vy - 4 * by) > 3 || !in_bounds(bd, vx, vy)) continue;  // uniform
-        const uint32_t cost = part_sad(px, py, pw, ph, bx, by, vx, vy) + vec_cost(vx - mvp.x, vy - mvp.y, lambda);
-        if (cost < best) { best = cost; cx = vx; cy = vy; }
-      }
-      if (cx == fx && cy == fy) break;
+  ensure_mb_window(c, bx, by);
+  const int at = py * 24 + px, src = py * 16 + px, shift = pw == 16 ? 2 : 1, nw = (pw * ph) >> 2;
+  const int m0x = 4 * bx, m0y = 4 * by;
+  uint32_t best = wsum(part_sad(at, src, shift, nw, 0, 0)) + vec_cost(m0x - mvp.x, m0y - mvp.y, lambda);
+  const Box box{max(bd.min0, m0x - 3), min(bd.max0, m0x + 3), max(bd.min1, m0y - 3), min(bd.max1, m0y + 3)};
+  int q0 = 0, q1 = 0;
+#pragma unroll 1
+  for (int it = 0; it < 3; it++) {
+    const int st = it == 0 ? 2 : 1;
+    uint32_t sums = 0, s01 = 0;  // neighbours k = 3, 2 (right, down), then 1, 0
+#pragma unroll 1
+    for (int k = 3; k >= 0; k--) {
+      if (k == 1) { s01 = sums; sums = 0; }
+      sums = (sums << 16) | part_sad(at, src, shift, nw, q0 + (k == 1 ? -st : (k == 2 ? st : 0)), q1 + (k == 0 ? -st : (k == 3 ? st : 0)));
+    }
+    const uint32_t key = best4(sums, s01, m0x + q0, m0y + q1, st, box, mvp.x, mvp.y, lambda, true);
+    if ((key >> 2) < best) {
+      best = key >> 2;
+      const int k = (int)(key & 3u);
+      q0 += k == 1 ? -st : (k == 2 ? st : 0);
+      q1 += k == 0 ? -st : (k == 3 ? st : 0);
+    } else if (it) {
+      break;
     }
   }
-  return PartFit{best, cx, cy};
+  return PartFit{best, m0x + q0, m0y + q1};
 }
 
 // The luma prediction of a part at quarter-sample vector mv (within 3 quarter samples of 4 (bx, by),
@@ -426,13 +421,14 @@ __device__ __noinline__ PartFit refine_part_sad(const Ctx c, int px, int py, int
 __device__ __noinline__ void predict_part(const Ctx c, int px, int py, int pw, int ph, int bx,
                                           int by, int mvx, int mvy) {
   const int lane = lane_id();
-  ensure_window(c, bx, by);
-  QSrc q = qpel_src((mvx >> 2) - bx + 1 + px, (mvy >> 2) - by + 1 + py, mvx & 3, mvy & 3);
-  for (int i = lane; i < pw * ph; i += 32) {
-    const int r = i / pw, x = i - r * pw;
-    int v = *sm_at(q.a + r * q.sa + x);
-    if (q.avg) v = (v + *sm_at(q.b + r * q.sb + x) + 1) >> 1;
-    sm.pred_y[(py + r) * 16 + px + x] = (uint8_t)v;
+  ensure_mb_window(c, bx, by);
+  const int dx = mvx - 4 * bx, dy = mvy - 4 * by, shift = pw == 16 ? 2 : 1, nw = (pw * ph) >> 2;
+  const uint32_t e = sm.qpt[(dx & 3) | ((dy & 3) << 2)];
+  const uint8_t* p = &sm.win[0] + qpel_pos(dx, dy) + py * 24 + px;
+  for (int w = lane; w < nw; w += 32) {
+    const int r = w >> shift, x = (w - (r << shift)) * 4;
+    const uint8_t* q = p + r * 24 + x;
+    *(uint32_t*)&sm.pred_y[(py + r) * 16 + px + x] = __vavgu4(lds4u(q + (e & 0xffffu)), lds4u(q + (e >> 16)));
   }
   __syncwarp();
 }
@@ -487,47 +483,6 @@ __device__ __forceinline__ bool wait_window(const Ctx c, const PipeWait& pw, int
   return !pw.db_prev || wait_reference(c, pw, (c.mbx * 16 + xhi + 36) >> 4, (c.mby * 16 + yhi + 28) >> 4);
 }
 
-// P_Skip probe of the plain form (enc.rs:2906 try_p_skip) at skip vector (ps0, ps1): true when the
-// macroblock is coded as P_Skip (prediction left in pred_y / pred_u / pred_v).
-__device__ __noinline__ bool skip_probe(const Ctx c, int ps0, int ps1, const Bounds& bd) {
-  const FrameParams& fp = sm.fp;
-  const StreamDev& sd = sm.sd;
-  const int lane = lane_id();
-  if (!in_bounds(bd, ps0, ps1)) return false;
-  mc_luma16(sd.ref_y, fp.stride_y, c.mbx * 16, c.mby * 16, ps0, ps1);
-  uint2 s = src8(), p = *(const uint2*)&sm.pred_y[(lane >> 1) * 16 + (lane & 1) * 8];
-  uint32_t sad = wsum(vsad8(s, p));
-  if (sad >= sd.sb_probe) return false;
-  bool lz = sad <= sd.sb_luma;
-  if (!lz) {
-    uint32_t ssd = 0;
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      int d0 = (int)((s.x >> (8 * k)) & 255) - (int)((p.x >> (8 * k)) & 255);
-      int d1 = (int)((s.y >> (8 * k)) & 255) - (int)((p.y >> (8 * k)) & 255);
-      ssd += d0 * d0 + d1 * d1;
-    }
-    lz = wsum(ssd) <= sd.sb_luma_ssd;
-  }
-  if (!lz) lz = probe_skip_luma(sd.qp);
-  if (!lz) return false;
-  mc_chroma8(sd.ref_u, sd.ref_v, fp.stride_c, c.mbx, c.mby, ps0, ps1);
-  int plane = lane >> 4, idx = (lane & 15) * 4;
-  const uint8_t* ssrc = (plane ? sm.src_v : sm.src_u) + idx;
-  const uint8_t* pp = (plane ? sm.pred_v : sm.pred_u) + idx;
-  uint32_t sadp = 0, ssdp = 0;
-#pragma unroll
-  for (int k = 0; k < 4; k++) { int d = (int)ssrc[k] - (int)pp[k]; sadp += abs(d); ssdp += d * d; }
-  uint32_t sad_u = wsum(plane == 0 ? sadp : 0), sad_v = wsum(plane == 1 ? sadp : 0);
-  uint32_t ssd_u = wsum(plane == 0 ? ssdp : 0), ssd_v = wsum(plane == 1 ? ssdp : 0);
-  bool cz = (sad_u <= sd.sb_chroma || ssd_u <= sd.sb_chroma_ssd) && (sad_v <= sd.sb_chroma || ssd_v <= sd.sb_chroma_ssd);
-  if (!cz) {
-    const ChromaAc ac = chroma_quant(sd.qpc, false);
-    cz = !ac.dc() && ac.score(0) < 7 && ac.score(1) < 7;
-  }
-  return cz;
-}
-
 // Learned form: the centre of the first +-2 window among the integer candidates of ss.ccx / ccy (cok false:
 // absent) -- the first of least 16x16 SAD + lambda * vector bits against the 16x16 predictor.
 __device__ __noinline__ int2 learned_centre(const Ctx c, int mvp0, int mvp1, uint32_t lambda) {
@@ -571,19 +526,12 @@ __device__ __constant__ uint8_t c_part_quads[9] = {15, 3, 12, 5, 10, 1, 2, 4, 8}
 // One macroblock of a P slice in the search forms (see the head of this file); false when a wait for
 // the reference picture gave up.
 __device__ __noinline__ bool analyse_p_mb_search(const Ctx c, const PipeWait pw) {
-  const FrameParams& fp = sm.fp;
   const StreamDev& sd = sm.sd;
   const int lane = lane_id();
   const int mbx = c.mbx, mby = c.mby;
   const int x0 = mbx * 16, y0 = mby * 16;
-  const int qp = sd.qp;
-  const uint32_t lambda = c_lambda[qp];
-  const int cw = fp.mb_w * 16, chh = fp.mb_h * 16;
-  Bounds bd;
-  bd.min0 = -4 * (x0 + 28);
-  bd.min1 = max(-4 * (y0 + 28), -2048);
-  bd.max0 = 4 * (cw - 16 - x0 + 28);
-  bd.max1 = min(4 * (chh - 16 - y0 + 28), 2044);
+  const uint32_t lambda = sm.qt[0].lambda;
+  const Bounds bd = mv_bounds(x0, y0);
   const int imin0 = (bd.min0 + 3) >> 2, imin1 = (bd.min1 + 3) >> 2, imax0 = bd.max0 >> 2, imax1 = bd.max1 >> 2;
   // Warp-uniform state (every lane computes the same values) is held once per warp in shared memory
   // (SearchSmem) instead of once per lane on the stack; every lane writes the same value, and a
@@ -635,8 +583,10 @@ __device__ __noinline__ bool analyse_p_mb_search(const Ctx c, const PipeWait pw)
   }
   // the reference region of the skip probe and the search window (learned: every candidate's)
   if (!wait_window(c, pw, max(xhi, (max(ps0, 0) + 3) >> 2), max(yhi, (max(ps1, 0) + 3) >> 2))) return false;
+  if (lane == 0) sm.win_x = kNoWin;  // the last macroblock's window
+  __syncwarp();
   // 1. skip probe
-  if (skip_probe(c, ps0, ps1, bd)) {
+  if (in_bounds(bd, ps0, ps1) && skip_probe(c, ps0, ps1)) {
     code_skip(c, ps0, ps1);
     search_tail(c, 255, false, ps0, ps1);
     return true;
@@ -678,7 +628,6 @@ __device__ __noinline__ bool analyse_p_mb_search(const Ctx c, const PipeWait pw)
   uint32_t best_j = UMAX;
   int (&bmv)[4][2] = ss.bmv;  // per part (coding order) of the best type (warp-uniform, shared)
   int (&bmvd)[4][2] = ss.bmvd;
-  ss.wbx = ss.wby = kNoWin;  // the skip probe's window is not a refinement window
   for (int t = 0; t < 4; t++) {
     if (!((part_mask >> t) & 1)) continue;
     int (&own)[4][2] = ss.own;
@@ -751,7 +700,7 @@ __device__ __noinline__ bool analyse_p_mb_search(const Ctx c, const PipeWait pw)
 __device__ __noinline__ void analyse_intra_mb_search(const Ctx c) {
   const Corner k0 = load_edges(c, true);
   bool ht = c.mby > 0, hl = c.mbx > 0;
-  uint32_t lambda = c_lambda[sm.sd.qp];
+  uint32_t lambda = sm.qt[0].lambda;
   const I16Fit fit16 = analyse_i16(ht, hl, k0.y);
   if (fit16.cost > 40 * lambda) {
     const uint16_t* masks = sm.sd.hint ? sm.sd.hint[c.mb].i4_mask : nullptr;
