@@ -44,9 +44,8 @@ struct QTab {
 __device__ QTab g_qtab[52];
 constexpr int kQTabWords = (int)(sizeof(QTab) / 4), kQTabWords4 = (int)(offsetof(QTab, mf8) / 4);  // all, and chroma's
 __constant__ uint8_t c_cqp[52];
-__constant__ uint8_t c_alpha[52];
-__constant__ uint8_t c_beta[52];
-__constant__ uint8_t c_tc0[52][3];
+// Deblocking thresholds by QP: {alpha | beta << 8, tC0 of strengths 1..3 a byte each}.
+__constant__ uint2 c_deblock[52];
 
 // ---------------------------------------------------------------------------------------------
 // Shared memory of one macroblock warp.
@@ -93,11 +92,12 @@ struct __align__(16) Smem {
   alignas(16) QTab qt[2];         // the picture's luma and chroma QP
   int qt_qp;                      // the luma QP they are of
   uint32_t qpt[16];               // quarter-sample phases: the two planes averaged (init_tables)
+  alignas(16) uint32_t dbmv[12];  // deblocking, search forms: quadrant vectors of the macroblock, its left and top neighbours
   int win_x, win_y, win_have;     // ensure_window: the position held (kNoWin: none), its planes built (bits 0..2)
   int db_row, seen_db;            // last acquired progress db_prev[db_row] of the reference picture
   int reach_y, reach_x;           // 1 + the largest reach waited for beyond zero motion, in macroblocks
   alignas(16) uint8_t i4m[16];    // Intra4x4PredMode of this macroblock (decoding order)
-  uint8_t i4q[16];          // edge samples of the current 4x4 block (i4_edge_index)
+  uint8_t i4e[48];          // the current 4x4 block's edge samples Q, their avg2 and their avg3 (i4_tap)
 };
 static_assert(offsetof(Smem, coef) % 4 == 0 && offsetof(Smem, ccoef) % 4 == 0, "level arrays cleared by words");
 static_assert(offsetof(rg_mb_out, luma) % 4 == 0 && offsetof(rg_mb_out, chroma_dc) % 4 == 0 &&
@@ -107,6 +107,7 @@ static_assert(offsetof(Smem, coef) % 8 == 0 && offsetof(Smem, ccoef) % 8 == 0 &&
                   offsetof(Smem, t8) % 16 == 0 && offsetof(Smem, zz8) % 8 == 0 && offsetof(Smem, i4m) % 4 == 0 &&
                   offsetof(Smem, src_u) % 8 == 0 && offsetof(Smem, pred_u) % 8 == 0,
               "rows of levels, intermediates and samples move as vectors");
+static_assert(20 * 24 <= kWinPlane && 24 * 12 <= kWinPlane, "the deblocking tiles fit the window's planes");
 static_assert(offsetof(Smem, pred_y) % 8 == 0 && offsetof(Smem, tmp_y) % 8 == 0, "16x16 predictions written 8 bytes per lane");
 
 // Every kernel of this file runs one warp per block, and its shared memory has this one name: the
@@ -186,27 +187,6 @@ __device__ __forceinline__ void idct8_1d(const int* d, int* o) {
   o[0] = (int)(b0 + b7); o[1] = (int)(b2 + b5); o[2] = (int)(b4 + b3); o[3] = (int)(b6 + b1);
   o[4] = (int)(b6 - b1); o[5] = (int)(b4 - b3); o[6] = (int)(b2 - b5); o[7] = (int)(b0 - b7);
 }
-// One pass of the 4x4 forward core transform along the axis whose lanes are `step` apart in a
-// 16-lane group (i = position along it): [1 1 1 1; 2 1 -1 -2; 1 -1 -1 1; 1 -2 2 -1].
-__device__ __forceinline__ int fwd4_pass(int v, int step, int i) {
-  int b = __shfl_xor_sync(FULL, v, 3 * step);
-  int s = v + b, dd = v - b;
-  int ps = __shfl_xor_sync(FULL, s, step), pd = __shfl_xor_sync(FULL, dd, step);
-  return i == 0 ? s + ps : (i == 1 ? 2 * pd + dd : (i == 2 ? ps - s : 2 * pd - dd));
-}
-// One pass of the inverse core transform (fixed.rs:192): e0 = c0 + c2, e1 = c0 - c2,
-// e2 = (c1 >> 1) - c3, e3 = c1 + (c3 >> 1); out = e0 + e3, e1 + e2, e1 - e2, e0 - e3.
-__device__ __forceinline__ int inv4_pass(int v, int step, int i) {
-  int b = __shfl_xor_sync(FULL, v, 2 * step);
-  int ea, eb;
-  if (i == 0) { ea = v + b; eb = v - b; }
-  else if (i == 2) { ea = b + v; eb = b - v; }
-  else if (i == 1) { ea = (v >> 1) - b; eb = v + (b >> 1); }
-  else { ea = (b >> 1) - v; eb = b + (v >> 1); }
-  int pa = __shfl_xor_sync(FULL, ea, step), pb = __shfl_xor_sync(FULL, eb, step);
-  return i == 0 ? ea + pb : (i == 1 ? pb + ea : (i == 2 ? eb - pa : pa - eb));
-}
-
 // ---------------------------------------------------------------------------------------------
 // Half-sample window (h264_enc.rs:747 hpel_window, :803 hpel_window_centre) around the integer
 // position (px, py) of a 16x16 block: quarter-sample vectors up to 3 away from it. Window row y,
@@ -1007,7 +987,6 @@ __device__ __noinline__ int analyse_chroma(bool ht, bool hl, Corner k0) {
   return bm;
 }
 
-// Intra 4x4 prediction of mode m (h264_dsp.rs:799 predict_intra_4x4_u8_scalar) into out[16].
 // Intra 4x4 prediction (h264.rs:3223 predict_4x4, the nine modes of H.264 8.3.1.2) in closed
 // form. The block's edge samples are gathered into Q[16]:
 //   Q[0] = Q[1] = l3, Q[2] = l2, Q[3] = l1, Q[4] = l0, Q[5] = top-left, Q[6..13] = t0..t7,
@@ -1038,9 +1017,9 @@ __host__ __device__ __forceinline__ int i4_tap(int m, int x, int y) {
     }
   }
 }
-// The taps of every (mode, sample) for the nine-prediction loop: i | min(i + 1, 15) << 4 |
-// min(i + 2, 15) << 8 | kind << 12, at [16 m + 4 y + x] (filled from i4_tap by upload_tables).
-__device__ uint16_t g_i4tap[9 * 16];
+// The taps of half h of mode m (its rows as in Half4) at [2 m + h], a byte 16 kind + i per sample:
+// offsets into sm.i4e, the edge samples, their avg2 and their avg3 (filled by upload_tables).
+__device__ uint2 g_i4tap[18];
 // ---------------------------------------------------------------------------------------------
 // A macroblock; its picture's descriptor and parameters are in shared memory (sm.sd, sm.fp): the
 // acquire of every wait drops the SM's L1, so read through global memory each use of them was an
@@ -1272,137 +1251,134 @@ __device__ __noinline__ void code_i16(const Ctx c, int mode, bool ht, bool hl, C
 
 // I4x4 analysis (enc.rs:3336 analyse_i4): sixteen blocks in decoding order, each choosing among
 // the available modes by SATD + lambda * (1 if the predicted mode else 4), then quantising and
-// reconstructing before the next block. Per block the warp gathers the edge samples (lane k ->
-// Q[k]), builds all nine predictions (lane -> pixel, the two half-warps taking even / odd modes),
-// costs the modes (lane -> mode), and transforms the chosen residual with shuffles (lane ->
-// coefficient). Returns the luma coded block pattern with the blocks
-// holding levels in bits 4.. (bit 4 + b: block b), or -1 as soon as the running cost reaches `budget`.
-// kMask: only the modes of masks[b] (bit m: Intra4x4PredMode m) that are available at block b are
-// tried -- DC alone when none is (the learned form); the plain form tries every available mode.
-template <bool kMask>
-__device__ __noinline__ int analyse_i4(const Ctx c, uint32_t budget, bool ht_mb, bool hl_mb, int tl_mb,
-                                        const uint16_t* masks) {
-  const FrameParams& fp = sm.fp;
-  int lane = lane_id();
-  int p = lane & 15, xl = p & 3, yl = p >> 2;
+// reconstructing before the next block: a serial chain, and the head of every GOP. Lane 2 m + h takes
+// half of the block under mode m (Half4): all nine modes are predicted, costed, transformed,
+// quantised and reconstructed side by side, the residual's chain beside the cost's, and the winner's
+// two lanes store theirs (one mode per step and the residual after the choice: 3.4 k cycles a block
+// on an idle SM). The macroblock and its edges form one tile (sm.win: sample (x, y) at 24 (y + 1) + 4 + x,
+// unavailable samples 128). `masks`: lane b's mask of the modes tried in block b (the learned form's
+// hints; bit m: Intra4x4PredMode m) -- those of them available, DC alone when none is. Returns the
+// luma coded block pattern with the blocks holding levels in bits 4.. (bit 4 + b: block b), or -1 as
+// soon as the running cost reaches `budget`.
+__device__ __noinline__ int analyse_i4(const Ctx c, uint32_t budget, bool ht_mb, bool hl_mb, int tl_mb, uint32_t masks) {
+  const int lane = lane_id(), h = lane & 1, m = lane >> 1, p = lane & 15;
   const QTab& qt = sm.qt[0];
-  const uint32_t lambda = qt.lambda, shift = qt.shift, bias = qt.bias[1], mf = qt.mf[yl & 1][xl & 1];
-  const int dqs = qt.dq[yl & 1][xl & 1];
-  uint32_t total = lambda * 24;
-  int cbpl = 0;
+  const uint32_t lambda = qt.lambda, shift = qt.shift, bias = qt.bias[1], mf[2] = {qt.mf[h][0], qt.mf[h][1]};
+  const int dq[2] = {qt.dq[h][0], qt.dq[h][1]};
   const MbInfo* info = sm.sd.info;
-  uint32_t lmodes = hl_mb ? ld_info(&info[c.mb - 1]).i4_right : 0x2222u;
-  uint32_t tmodes = ht_mb ? ld_info(&info[c.mb - fp.mb_w]).i4_bottom : 0x2222u;
-  // this lane's taps for its predictions (modes lane / 16 + 2 k, sample p): the same for every block
-  uint32_t taps[5];
-#pragma unroll
-  for (int k = 0; k < 5; k++) {
-    int m = (lane >> 4) + 2 * k;
-    taps[k] = m < 9 ? __ldg(&g_i4tap[m * 16 + p]) : 0u;
-  }
+  const uint32_t lmodes = hl_mb ? info[c.mb - 1].i4_right : 0x2222u, tmodes = ht_mb ? info[c.mb - sm.fp.mb_w].i4_bottom : 0x2222u;
+  const uint2 taps = __ldg(&g_i4tap[min(lane, 17)]);
+  // the tile's edges: the row above from its corner to the top-right neighbour's first four samples,
+  // the column to the left
+  if (lane < 20) sm.win[4 + lane] = ht_mb ? sm.top[lane] : 128;
+  if (lane < 16) sm.win[24 * (lane + 1) + 3] = hl_mb ? sm.left[lane] : 128;
+  if (lane == 20) sm.win[3] = (uint8_t)tl_mb;
+  // this lane's edge sample relative to the block (lanes 0..14: Q[p]), and where t4.. are unavailable
+  const int eoff = p <= 4 ? 24 * (p <= 1 ? 3 : 4 - p) - 1 : (p == 5 ? -25 : min(p - 6, 7) - 24), eoff3 = p >= 10 ? -21 : eoff;
+  uint32_t total = lambda * 24;
+  int luma = 0;
+  __syncwarp();
+#pragma unroll 1
   for (int b = 0; b < 16; b++) {
-    int bx = blk_x(b), by = blk_y(b), px = bx * 4, py = by * 4;
-    bool ht = by > 0 || ht_mb, hl = bx > 0 || hl_mb;
-    bool tr = !(b == 3 || b == 7 || b == 11 || b == 13 || b == 15) && (b != 5 || c.mbx + 1 < fp.mb_w);
-    // edge samples (unavailable ones 128; top-right replicated from t3 when unavailable)
-    int q = 128;
-    if (p <= 4) {
-      int j = p <= 1 ? 3 : 4 - p;
-      if (hl) q = bx > 0 ? sm.tmp_y[(py + j) * 16 + px - 1] : sm.left[py + j];
-    } else if (p == 5) {
-      if (ht && hl)
-        q = (by > 0 && bx > 0) ? sm.tmp_y[(py - 1) * 16 + px - 1]
-                               : (by > 0 ? sm.left[py - 1] : (bx > 0 ? sm.top[px - 1] : tl_mb));
-    } else if (p <= 14) {
-      int i = min(p - 6, 7);
-      if (i >= 4 && !tr) i = 3;
-      if (ht) q = by > 0 ? sm.tmp_y[(py - 1) * 16 + px + i] : sm.top[px + i];
+    const int bx = blk_x(b), by = blk_y(b), px = bx * 4, py = by * 4;
+    const bool ht = by > 0 || ht_mb, hl = bx > 0 || hl_mb;
+    const bool tr = !((0xa888 >> b) & 1) && (b != 5 || c.mbx + 1 < sm.fp.mb_w);  // blocks 3, 7, 11, 13, 15 have none
+    uint8_t* tile = &sm.win[24 * (py + 1) + 4 + px];
+    const int q = tile[tr ? eoff : eoff3];
+    const uint32_t sums = wsum(lane >= 6 && lane <= 9 ? (uint32_t)q : (lane >= 1 && lane <= 4 ? (uint32_t)q << 16 : 0u));
+    const int st = (int)(sums & 0xffffu), sl = (int)(sums >> 16);
+    const int dc = ht && hl ? (st + sl + 4) >> 3 : (ht ? (st + 2) >> 2 : (hl ? (sl + 2) >> 2 : 128));
+    const int q1 = __shfl_down_sync(FULL, q, 1), q2 = __shfl_down_sync(FULL, q, 2);
+    if (lane < 16) {
+      sm.i4e[p] = (uint8_t)(p == 15 ? dc : q);
+      sm.i4e[16 + p] = (uint8_t)((q + q1 + 1) >> 1);
+      sm.i4e[32 + p] = (uint8_t)((q + 2 * q1 + q2 + 2) >> 2);
     }
-    uint32_t sums = wsum(lane < 16 ? ((p >= 6 && p <= 9) ? (uint32_t)q : 0u) + ((p >= 1 && p <= 4) ? (uint32_t)q << 16 : 0u) : 0u);
-    int st = (int)(sums & 0xffff), sl = (int)(sums >> 16);
-    int dc = ht && hl ? (st + sl + 4) >> 3 : (ht ? (st + 2) >> 2 : (hl ? (sl + 2) >> 2 : 128));
-    if (lane < 16) sm.i4q[p] = (uint8_t)(p == 15 ? dc : q);
     // predicted mode (h264.rs:3283)
-    int gx = c.mbx * 4 + bx, gy = c.mby * 4 + by;
-    int pm;
-    if (gx == 0 || gy == 0) pm = 2;
-    else {
-      int ml = bx > 0 ? sm.i4m[(((by >> 1) << 3) | (((bx - 1) >> 1) << 2) | ((by & 1) << 1) | ((bx - 1) & 1))]
-                      : (int)((lmodes >> (4 * by)) & 15);
-      int mt = by > 0 ? sm.i4m[((((by - 1) >> 1) << 3) | ((bx >> 1) << 2) | (((by - 1) & 1) << 1) | (bx & 1))]
-                      : (int)((tmodes >> (4 * bx)) & 15);
+    int pm = 2;
+    if ((c.mbx | bx) && (c.mby | by)) {
+      const int ml = bx > 0 ? sm.i4m[((by >> 1) << 3) | (((bx - 1) >> 1) << 2) | ((by & 1) << 1) | ((bx - 1) & 1)]
+                            : (int)((lmodes >> (4 * by)) & 15);
+      const int mt = by > 0 ? sm.i4m[(((by - 1) >> 1) << 3) | ((bx >> 1) << 2) | (((by - 1) & 1) << 1) | (bx & 1)]
+                            : (int)((tmodes >> (4 * bx)) & 15);
       pm = min(ml, mt);
     }
+    const uint32_t avail = 0x4u | (ht ? 0x89u : 0u) | (hl ? 0x102u : 0u) | (ht && hl ? 0x70u : 0u);
+    uint32_t allow = __shfl_sync(FULL, masks, b) & avail;
+    if (!allow) allow = 0x4u;
     __syncwarp();
-    // nine predictions and their SATDs: half-warp h takes modes h, h + 2, ... (k = 0..4), lane p
-    // sample p; the 4x4 Hadamard of the difference (metrics.rs:705) by four shuffle butterflies,
-    // both halves' sums of magnitudes in one reduction (each below 2^16). Every lane ends with
-    // the same key, the least cost first and the lower mode on a tie.
-    int srcp = sm.src_y[(py + yl) * 16 + px + xl];
-    int pv[5];
-    uint32_t key = UMAX;
-    uint32_t allow = 0x1ffu;
-    if constexpr (kMask) {
-      uint32_t avail = 0x4u | (ht ? 0x89u : 0u) | (hl ? 0x102u : 0u) | (ht && hl ? 0x70u : 0u);
-      allow = masks[b] & avail;
-      if (!allow) allow = 0x4u;
+    // this lane's two predicted rows and their residual's columns; the butterflies of the Hadamard and
+    // of the core transform share the exchange (half_columns)
+    uint2 pr, sr = half_rows((int)offsetof(Smem, src_y) + py * 16 + px, 16, h);
+    {
+      uint32_t w[2] = {0u, 0u};
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        const uint32_t tp = ((k < 4 ? taps.x : taps.y) >> (8 * (k & 3))) & 255u;
+        w[k >> 2] |= (uint32_t)sm.i4e[tp] << (8 * (k & 3));
+      }
+      pr = make_uint2(w[0], w[1]);
     }
+    Half4 v;
+    uint32_t cost;
+    {
+      int u[2], w[2];
 #pragma unroll
-    for (int k = 0; k < 5; k++) {
-      if constexpr (kMask) {
-        if (!((allow >> (2 * k)) & 3u)) { pv[k] = 0; continue; }  // neither mode of this step is tried
+      for (int o = 0; o < 2; o++) {
+        auto cols = [&](uint32_t r) { return (int)(o ? __byte_perm(r, 0u, 0x4341) : r & 0x00ff00ffu); };
+        const int r0 = cols(sr.x) - cols(pr.x), r1 = cols(sr.y) - cols(pr.y), sum = r0 + r1, dif = r0 - r1;
+        const int x = __shfl_xor_sync(FULL, h ? sum : dif, 1);
+        u[o] = h ? x : sum;
+        w[o] = h ? dif : x;
       }
-      uint32_t tp = taps[k], kind = tp >> 12;
-      int a0 = sm.i4q[tp & 15], a1 = sm.i4q[(tp >> 4) & 15], a2 = sm.i4q[(tp >> 8) & 15];
-      int v = kind == 0 ? a0 : (kind == 1 ? (a0 + a1 + 1) >> 1 : (a0 + 2 * a1 + a2 + 2) >> 2);
-      pv[k] = v;
-      int d = srcp - v;
-#pragma unroll
-      for (int b = 1; b < 16; b <<= 1) {
-        int o = __shfl_xor_sync(FULL, d, b);
-        d = (lane & b) ? o - d : d + o;
-      }
-      uint32_t sums = __reduce_add_sync(FULL, (uint32_t)(d < 0 ? -d : d) << (16 * (lane >> 4)));
-#pragma unroll
-      for (int h = 0; h < 2; h++) {
-        int m = 2 * k + h;
-        if (m > 8) continue;
-        bool av = (m == 0 || m == 3 || m == 7) ? ht : ((m == 1 || m == 8) ? hl : (m == 2 ? true : (ht && hl)));
-        if constexpr (kMask) av = av && ((allow >> m) & 1u);
-        uint32_t cost = (((sums >> (16 * h)) & 0xffffu) >> 1) + lambda * (m == pm ? 1u : 4u);
-        if (av) key = min(key, (cost << 4) | (uint32_t)m);
-      }
+      auto satd_row = [](int e, int o) {
+        const int r0 = (int16_t)e, r2 = (e + 0x8000) >> 16, r1 = (int16_t)o, r3 = (o + 0x8000) >> 16;
+        const int s03 = r0 + r3, s12 = r1 + r2, d03 = r0 - r3, d12 = r1 - r2;
+        return (uint32_t)(max(abs(s03), abs(s12)) + max(abs(d03), abs(d12)));
+      };
+      cost = satd_row(u[0] + w[0], u[1] + w[1]) + satd_row(u[0] - w[0], u[1] - w[1]);
+      auto fwd_row = [](int e, int o, int (&r)[4]) {
+        const int r0 = (int16_t)e, r2 = (e + 0x8000) >> 16, r1 = (int16_t)o, r3 = (o + 0x8000) >> 16;
+        const int s03 = r0 + r3, s12 = r1 + r2, d03 = r0 - r3, d12 = r1 - r2;
+        r[0] = s03 + s12; r[1] = 2 * d03 + d12; r[2] = s03 - s12; r[3] = d03 - 2 * d12;
+      };
+      const int k = 1 + h;
+      fwd_row(u[0] * k + w[0], u[1] * k + w[1], v.a);
+      fwd_row(u[0] - w[0] * k, u[1] - w[1] * k, v.b);
     }
-    int bm = (int)(key & 15);
+    cost += __shfl_xor_sync(FULL, cost, 1);
+    cost += lambda * (m == pm ? 1u : 4u);
+    const uint32_t key = __reduce_min_sync(FULL, m < 9 && ((allow >> m) & 1u) ? (cost << 4) | (uint32_t)m : UMAX);
+    const int bm = (int)(key & 15u);
     total += key >> 4;
     if (total >= budget) return -1;
-    if (lane == 0) sm.i4m[b] = (uint8_t)bm;
-    // residual transform and quantisation, lane p -> coefficient p (raster); the chosen mode's
-    // sample p is in lane 16 (bm & 1) + p
-    int kb = bm >> 1, mine = pv[0];
+    // residual of every mode
+    uint32_t any = 0;
+    Half4 r;
 #pragma unroll
-    for (int k = 1; k < 5; k++)
-      if (kb == k) mine = pv[k];
-    int pred = __shfl_sync(FULL, mine, (bm & 1) * 16 + p);
-    int acc = fwd4_pass(fwd4_pass(srcp - pred, 1, xl), 4, yl);
-    acc = (int16_t)acc;
-    uint32_t aa = (uint32_t)(acc < 0 ? -acc : acc);
-    int l = (int)((aa * mf + bias) >> shift);
-    int lvl = acc < 0 ? -l : l;
-    if (lane < 16) sm.coef[b * 16 + p] = (int16_t)lvl;
-    bool nz = __ballot_sync(FULL, lane < 16 && lvl != 0) != 0;
-    if (nz) cbpl |= (1 << (b >> 2)) | (16 << b);
-    // inverse transform (rows then columns) and reconstruction
-    int rec = pred;
-    if (nz) {
-      int dq = clamp_i16(lvl * dqs);
-      int r = (int16_t)((inv4_pass(inv4_pass(dq, 1, xl), 4, yl) + 32) >> 6);
-      rec = clip255(pred + r);
+    for (int k = 0; k < 8; k++) {
+      int& x = k < 4 ? v.a[k & 3] : v.b[k & 3];
+      const uint32_t l = ((uint32_t)abs(x) * mf[k & 1] + bias) >> shift;
+      any |= l;
+      x = x < 0 ? -(int)l : (int)l;
+      (k < 4 ? r.a[k & 3] : r.b[k & 3]) = clamp_i16(x * dq[k & 1]);
     }
-    if (lane < 16) sm.tmp_y[(py + yl) * 16 + px + xl] = (uint8_t)rec;
+    half_inv(r, h);
+    const uint32_t nz = __ballot_sync(FULL, any != 0);
+    if (m == bm) {
+      *(uint2*)&sm.coef[b * 16 + h * 4] = pack_half(v.a);
+      *(uint2*)&sm.coef[b * 16 + h * 4 + 8] = pack_half(v.b);
+      *(uint32_t*)(tile + 24 * h) = add_clip4(pr.x, r.a);
+      *(uint32_t*)(tile + 24 * (3 - h)) = add_clip4(pr.y, r.b);
+      if (!h) sm.i4m[b] = (uint8_t)bm;
+    }
+    if ((nz >> (2 * bm)) & 3u) luma |= (1 << (b >> 2)) | (16 << b);
     __syncwarp();
   }
-  return cbpl;
+  const uint32_t* t = (const uint32_t*)&sm.win[24 * ((lane >> 1) + 1) + 4 + (lane & 1) * 8];
+  *(uint2*)&sm.tmp_y[lane * 8] = make_uint2(t[0], t[1]);
+  __syncwarp();
+  return luma;
 }
 
 // `luma`: what analyse_i4 returned.
@@ -1430,7 +1406,7 @@ __device__ __noinline__ void analyse_intra_mb(const Ctx c) {
   uint32_t lambda = sm.qt[0].lambda;
   const I16Fit fit16 = analyse_i16(ht, hl, k0.y);
   if (fit16.cost > 40 * lambda) {
-    const int cbpl = analyse_i4<false>(c, fit16.cost + lambda * 4, ht, hl, k0.y, nullptr);
+    const int cbpl = analyse_i4(c, fit16.cost + lambda * 4, ht, hl, k0.y, 0x1ffu);
     if (cbpl >= 0) {
       code_i4(c, cbpl, ht, hl, k0);
       return;
@@ -1803,211 +1779,165 @@ __device__ __noinline__ bool analyse_p_mb(const Ctx c, const PipeWait pw) {
 #include "search_form.cuh"
 
 // ---------------------------------------------------------------------------------------------
-// Deblocking of one macroblock (enc.rs:3776 deblock, h264_deblock.rs:71,187): vertical edges
-// then horizontal ones, on a shared-memory tile with 4 samples of the left / top neighbours.
-struct EdgeParams {
-  int alpha, beta, tc0[4];
-  bool strong, on;
-};
-__device__ __forceinline__ EdgeParams edge_params(int qp, const int* bs) {
-  EdgeParams e;
-  int ia = qp < 0 ? 0 : (qp > 51 ? 51 : qp);
-  e.alpha = c_alpha[ia];
-  e.beta = c_beta[ia];
-  e.on = e.alpha != 0 && e.beta != 0;
-  for (int k = 0; k < 4; k++) {
-    int b = bs[k] > 4 ? 4 : bs[k];
-    e.tc0[k] = b == 0 ? -1 : (b == 4 ? 0 : c_tc0[ia][b - 1]);
-  }
-  e.strong = bs[0] == 4;
-  return e;
+// Deblocking of one macroblock (enc.rs:3776 deblock, h264_deblock.rs:71,187): vertical edges, then
+// horizontal ones, on tiles in shared memory with 4 samples of the left / top neighbours. Lanes 0..15
+// own a luma line across the edges (row, then column), lanes 16..31 a chroma line of either plane;
+// a lane's edges in one direction follow one another without a barrier, and one rolled copy of the
+// filter serves every edge, both directions, luma and chroma, both strengths. (Every lane computing
+// every edge's parameters, the filters unrolled: 12.2 k cycles a macroblock on an idle SM.)
+constexpr int kDbY = 24, kDbC = 12;       // tile strides: luma rows from x = -4 at byte 4, chroma rows from x = -4
+constexpr int kDbPlane = 12 * kDbC;       // a chroma tile
+// nz16 (decoding order) as a raster mask: bit 4 y + x.
+__device__ __forceinline__ uint32_t raster_nz(uint32_t nz) {
+  const uint32_t t = (nz ^ (nz >> 2)) & 0x0c0cu;
+  return (nz ^ t ^ (t << 2)) & 0xffffu;
 }
-__device__ __forceinline__ void luma_line(uint8_t* o, int xs, const EdgeParams& e, int tc0) {
-  if (!e.strong && tc0 < 0) return;
-  int p0 = o[-xs], q0 = o[0], p1 = o[-2 * xs], q1 = o[xs];
-  if (abs(p0 - q0) >= e.alpha || abs(p1 - p0) >= e.beta || abs(q1 - q0) >= e.beta) return;
-  int p2 = o[-3 * xs], q2 = o[2 * xs];
-  bool ap = abs(p2 - p0) < e.beta, aq = abs(q2 - q0) < e.beta;
-  if (!e.strong) {
-    int tc = tc0 + ap + aq;
-    int d = min(max((((q0 - p0) << 2) + (p1 - q1) + 4) >> 3, -tc), tc);
-    o[-xs] = (uint8_t)clip255(p0 + d);
-    o[0] = (uint8_t)clip255(q0 - d);
-    if (ap) o[-2 * xs] = (uint8_t)(p1 + min(max((p2 + ((p0 + q0 + 1) >> 1) - (p1 << 1)) >> 1, -tc0), tc0));
-    if (aq) o[xs] = (uint8_t)(q1 + min(max((q2 + ((p0 + q0 + 1) >> 1) - (q1 << 1)) >> 1, -tc0), tc0));
-  } else {
-    int p3 = o[-4 * xs], q3 = o[3 * xs];
-    bool small = abs(p0 - q0) < ((e.alpha >> 2) + 2);
-    if (ap && small) {
-      o[-xs] = (uint8_t)((p2 + 2 * p1 + 2 * p0 + 2 * q0 + q1 + 4) >> 3);
-      o[-2 * xs] = (uint8_t)((p2 + p1 + p0 + q0 + 2) >> 2);
-      o[-3 * xs] = (uint8_t)((2 * p3 + 3 * p2 + p1 + p0 + q0 + 4) >> 3);
-    } else {
-      o[-xs] = (uint8_t)((2 * p1 + p0 + q1 + 2) >> 2);
-    }
-    if (aq && small) {
-      o[0] = (uint8_t)((p1 + 2 * p0 + 2 * q0 + 2 * q1 + q2 + 4) >> 3);
-      o[xs] = (uint8_t)((p0 + q0 + q1 + q2 + 2) >> 2);
-      o[2 * xs] = (uint8_t)((2 * q3 + 3 * q2 + q1 + q0 + p0 + 4) >> 3);
-    } else {
-      o[0] = (uint8_t)((2 * q1 + q0 + p1 + 2) >> 2);
-    }
-  }
+__device__ __forceinline__ bool far_mv(uint32_t a, uint32_t b) {
+  return abs(lo16((int)a) - lo16((int)b)) >= 4 || abs(((int)a >> 16) - ((int)b >> 16)) >= 4;
 }
-__device__ __forceinline__ void chroma_line(uint8_t* o, int xs, const EdgeParams& e, int tc0) {
-  if (!e.strong && tc0 < 0) return;
-  int p1 = o[-2 * xs], p0 = o[-xs], q0 = o[0], q1 = o[xs];
-  if (abs(p0 - q0) >= e.alpha || abs(p1 - p0) >= e.beta || abs(q1 - q0) >= e.beta) return;
-  if (e.strong) {
-    o[-xs] = (uint8_t)((2 * p1 + p0 + q1 + 2) >> 2);
-    o[0] = (uint8_t)((2 * q1 + q0 + p1 + 2) >> 2);
-  } else {
-    int tc = tc0 + 1;
-    int d = min(max((((q0 - p0) << 2) + (p1 - q1) + 4) >> 3, -tc), tc);
-    o[-xs] = (uint8_t)clip255(p0 + d);
-    o[0] = (uint8_t)clip255(q0 - d);
-  }
-}
-__device__ __forceinline__ int nz_at(uint16_t nz, int bx, int by) {
-  int b = ((by >> 1) << 3) | ((bx >> 1) << 2) | ((by & 1) << 1) | (bx & 1);
-  return (nz >> b) & 1;
-}
-// Boundary strengths of edge e in direction dir (0 vertical); returns false to skip the edge.
-// kMv4 (search forms): the motion term compares the quadrant vectors on either side of each
-// 4-sample segment (qm: this macroblock's, pm4: the neighbour's across edge 0), so the internal
-// edge between partitions gets strength 1 where their vectors differ by 4 quarter samples.
-template <bool kMv4>
-__device__ bool edge_bs(const MbInfo& q, const MbInfo* p, int dir, int e, int* bs, const MbMv4* qm, const MbMv4* pm4) {
-  bool qi = q.flags & kFlagIntra;
-  bool pi = p ? (p->flags & kFlagIntra) : qi;
-  if (qi || pi) {
-    for (int k = 0; k < 4; k++) bs[k] = e == 0 ? 4 : 3;
-    return true;
-  }
-  int coded[4];
-  for (int k = 0; k < 4; k++) {
-    if (dir == 0) coded[k] = nz_at(q.nz16, e, k) | (e == 0 ? nz_at(p->nz16, 3, k) : nz_at(q.nz16, e - 1, k));
-    else coded[k] = nz_at(q.nz16, k, e) | (e == 0 ? nz_at(p->nz16, k, 3) : nz_at(q.nz16, k, e - 1));
-  }
-  if constexpr (!kMv4) {
-    bool motion = false;
-    if (e == 0) motion = q.ref != p->ref || abs(q.mv[0] - p->mv[0]) >= 4 || abs(q.mv[1] - p->mv[1]) >= 4;
-    if (!coded[0] && !coded[1] && !coded[2] && !coded[3] && !motion) return false;
-    for (int k = 0; k < 4; k++) bs[k] = coded[k] ? 2 : (motion ? 1 : 0);
-    return true;
-  } else {
-    bool any = false;
-    for (int k = 0; k < 4; k++) {
-      int qq = dir == 0 ? (k >> 1) * 2 + (e >> 1) : (e >> 1) * 2 + (k >> 1);
-      int pq = e == 0 ? (dir == 0 ? (k >> 1) * 2 + 1 : 2 + (k >> 1))
-                      : (dir == 0 ? (k >> 1) * 2 + ((e - 1) >> 1) : ((e - 1) >> 1) * 2 + (k >> 1));
-      const MbMv4* pmm = e == 0 ? pm4 : qm;
-      bool motion = (e == 0 && q.ref != p->ref) || abs(qm->mv[qq][0] - pmm->mv[pq][0]) >= 4 ||
-                    abs(qm->mv[qq][1] - pmm->mv[pq][1]) >= 4;
-      bs[k] = coded[k] ? 2 : (motion ? 1 : 0);
-      any |= bs[k] != 0;
-    }
-    return any;
-  }
-}
-// Whether a search-form macroblock's quadrants share one vector.
-__device__ __forceinline__ bool one_vector(const MbMv4& m) {
-  const uint32_t* w = (const uint32_t*)&m;
-  return w[0] == w[1] && w[0] == w[2] && w[0] == w[3];
-}
-
+// kMv4 (search forms): the motion term of the strengths compares the quadrant vectors on either side of
+// each 4-sample segment, so the internal edge between partitions gets strength 1 where their vectors
+// differ by 4 quarter samples.
 template <bool kMv4>
 __device__ __noinline__ void deblock_mb(int mbx, int mby) {
   const FrameParams& fp = sm.fp;
   const StreamDev& sd = sm.sd;
-  int lane = lane_id();
-  int m = mby * fp.mb_w + mbx;
-  MbInfo q = ld_info(&sd.info[m]);
-  MbInfo lf, tp;
-  bool hasl = mbx > 0, hast = mby > 0;
-  if (hasl) lf = ld_info(&sd.info[m - 1]);
-  if (hast) tp = ld_info(&sd.info[m - fp.mb_w]);
-  auto quiet = [](const MbInfo& i) { return !(i.flags & kFlagIntra) && i.cbp_luma == 0; };
-  MbMv4 qm, lm, tm;
+  const int lane = lane_id(), m = mby * fp.mb_w + mbx;
+  const bool hasl = mbx > 0, hast = mby > 0;
+  // the macroblocks' state: words mv, ref | flags << 8 | cbp << 16 | qp << 24, nz | ..
+  const uint4 q = *(const uint4*)&sd.info[m];
+  const uint4 l = hasl ? *(const uint4*)&sd.info[m - 1] : q, t = hast ? *(const uint4*)&sd.info[m - fp.mb_w] : q;
+  // the tiles: lane = luma row (20 from y = -4), and chroma row (12 of either plane from y = -4)
+  uint8_t* gy = sd.cur_y + (long)(mby * 16 - 4 + lane) * fp.stride_y + mbx * 16;
+  const int cp = lane >= 12, cr = lane - 12 * cp;
+  uint8_t* gc = (cp ? sd.cur_v : sd.cur_u) + (long)(mby * 8 - 4 + cr) * fp.stride_c + mbx * 8;
+  const bool ly = lane < 20 && (lane >= 4 || hast), lc = lane < 24 && (cr >= 4 || hast);
+  const bool ly4 = ly && lane >= 4 && hasl, lc4 = lc && cr >= 4 && hasl;  // with the left neighbour's samples
+  uint4 wy = make_uint4(0u, 0u, 0u, 0u);
+  uint2 wc = make_uint2(0u, 0u);
+  uint32_t wy4 = 0, wc4 = 0;
+  if (ly) wy = *(const uint4*)gy;
+  if (ly4) wy4 = *(const uint32_t*)(gy - 4);
+  if (lc) wc = *(const uint2*)gc;
+  if (lc4) wc4 = *(const uint32_t*)(gc - 4);
+  auto intra = [](const uint4& i) { return (i.y >> 8) & kFlagIntra; };
+  auto quiet = [](const uint4& i) { return ((i.y >> 8) & kFlagIntra) == 0 && ((i.y >> 16) & 255u) == 0; };
   bool split = false;
   if constexpr (kMv4) {
-    qm = sd.mv4[m];
-    if (hasl) lm = sd.mv4[m - 1];
-    if (hast) tm = sd.mv4[m - fp.mb_w];
-    split = !one_vector(qm);
-    const uint32_t qv = *(const uint32_t*)&qm;
-    if (quiet(q) && !split && (!hasl || (quiet(lf) && one_vector(lm) && *(const uint32_t*)&lm == qv)) &&
-        (!hast || (quiet(tp) && one_vector(tm) && *(const uint32_t*)&tm == qv)))
-      return;
+    const uint4 qm = *(const uint4*)&sd.mv4[m];
+    const uint4 lm = hasl ? *(const uint4*)&sd.mv4[m - 1] : qm, tm = hast ? *(const uint4*)&sd.mv4[m - fp.mb_w] : qm;
+    auto same = [&](const uint4& v) { return v.x == qm.x && v.y == qm.x && v.z == qm.x && v.w == qm.x; };
+    split = !same(qm);
+    if (quiet(q) && !split && quiet(l) && same(lm) && quiet(t) && same(tm)) return;
+    __syncwarp();
+    if (lane < 3) *(uint4*)&sm.dbmv[4 * lane] = lane == 0 ? qm : (lane == 1 ? lm : tm);
   } else {
-    if (quiet(q) && (!hasl || (quiet(lf) && lf.mv[0] == q.mv[0] && lf.mv[1] == q.mv[1])) &&
-        (!hast || (quiet(tp) && tp.mv[0] == q.mv[0] && tp.mv[1] == q.mv[1])))
-      return;
+    if (quiet(q) && quiet(l) && l.x == q.x && quiet(t) && t.x == q.x) return;
   }
-  // tiles: luma 20x20 at (x0-4, y0-4) stride 20 in win; chroma 12x12 each in two half-sample planes
-  uint8_t* ty = sm.win;
-  auto tc = [](int p) { return sm.hp[p]; };
-  const int x0 = mbx * 16, y0 = mby * 16, cx0 = mbx * 8, cy0 = mby * 8;
-  for (int w = lane; w < 100; w += 32) {  // 20 rows x 5 words
-    int r = w / 5, k = w % 5;
-    if ((r < 4 && !hast) || (k == 0 && !hasl)) continue;
-    *(uint32_t*)&ty[r * 20 + 4 * k] = ldcg_u32(sd.cur_y + (long)(y0 - 4 + r) * fp.stride_y + x0 - 4 + 4 * k);
+  uint8_t* const ty = sm.win;
+  uint8_t* const tc = sm.hp[0];
+  if (ly) {
+    *(uint32_t*)&ty[lane * kDbY + 4] = wy4;
+    *(uint2*)&ty[lane * kDbY + 8] = make_uint2(wy.x, wy.y);
+    *(uint2*)&ty[lane * kDbY + 16] = make_uint2(wy.z, wy.w);
   }
-  for (int w = lane; w < 72; w += 32) {  // 2 planes x 12 rows x 3 words
-    int p = w / 36, rem = w % 36, r = rem / 3, k = rem % 3;
-    if ((r < 4 && !hast) || (k == 0 && !hasl)) continue;
-    const uint8_t* P = p ? sd.cur_v : sd.cur_u;
-    *(uint32_t*)&tc(p)[r * 12 + 4 * k] = ldcg_u32(P + (long)(cy0 - 4 + r) * fp.stride_c + cx0 - 4 + 4 * k);
+  if (lc) {
+    uint32_t* r = (uint32_t*)&tc[lane * kDbC];
+    r[0] = wc4;
+    r[1] = wc.x;
+    r[2] = wc.y;
   }
   __syncwarp();
-  bool intra = q.flags & kFlagIntra;
-  bool internal = intra || q.cbp_luma != 0 || split;
-  bool skip_odd = q.flags & kFlagT8;
-  int qpq = q.qp, qpcq = chroma_qp(qpq);
+  // this lane's line: luma line lane, or line lane & 7 of chroma plane (lane >> 3) & 1; segment k of four
+  const bool luma = lane < 16;
+  const int line = luma ? lane : lane & 7, k = luma ? lane >> 2 : line >> 1;
+  const int xy = luma ? kDbY : kDbC;  // row stride of its tile
+  uint8_t* const origin = luma ? ty + 4 * kDbY + 8 : tc + ((lane >> 3) & 1) * kDbPlane + 4 * kDbC + 4;
+  const int qp = (int)(q.y >> 24), qpc = chroma_qp(qp);
+  auto thresholds = [&](const uint4& p) {  // of an edge between q and p
+    const int pq = (int)(p.y >> 24);
+    return c_deblock[luma ? (qp + pq + 1) >> 1 : (qpc + chroma_qp(pq) + 1) >> 1];
+  };
+  const uint2 th_in = thresholds(q);
+  const uint32_t qz = raster_nz(q.z);
+  const bool internal = intra(q) || ((q.y >> 16) & 255u) != 0 || split;
+  const int step = !internal ? 4 : (((q.y >> 8) & kFlagT8) ? 2 : 1);
+#pragma unroll 1
   for (int dir = 0; dir < 2; dir++) {
-    for (int e = 0; e < 4; e++) {
-      const MbInfo* pm;
-      if (e == 0) {
-        if (dir == 0 ? !hasl : !hast) continue;
-        pm = dir == 0 ? &lf : &tp;
+    const uint4& p = dir ? t : l;
+    const bool has = dir ? hast : hasl;
+    const uint2 th_p = thresholds(p);
+    const uint32_t pz = raster_nz(p.z);
+    const int along = dir ? 1 : xy, xs = dir ? xy : 1;
+    uint8_t* const base = origin + line * along;
+#pragma unroll 1
+    for (int e = has ? 0 : step; e < 4; e += step) {
+      const bool edge = e == 0;  // between macroblocks
+      int bs;
+      if (intra(q) || (edge && intra(p))) {
+        bs = edge ? 4 : 3;
       } else {
-        if (!internal || ((e & 1) && skip_odd)) continue;
-        pm = nullptr;
+        const int qb = dir ? 4 * e + k : 4 * k + e;  // the block on either side
+        const uint32_t coded = (qz >> qb) | (edge ? pz >> (dir ? 12 + k : 4 * k + 3) : qz >> (dir ? qb - 4 : qb - 1));
+        bool motion;
+        if constexpr (kMv4) {
+          const int qq = dir ? (e >> 1) * 2 + (k >> 1) : (k >> 1) * 2 + (e >> 1), e1 = (e - 1) >> 1;
+          const int pq = edge ? (dir ? 8 + 2 + (k >> 1) : 4 + (k >> 1) * 2 + 1) : (dir ? e1 * 2 + (k >> 1) : (k >> 1) * 2 + e1);
+          motion = (edge && ((q.y ^ p.y) & 255u)) || far_mv(sm.dbmv[qq], sm.dbmv[pq]);
+        } else {
+          motion = edge && (((q.y ^ p.y) & 255u) || far_mv(q.x, p.x));
+        }
+        bs = (coded & 1u) ? 2 : (motion ? 1 : 0);
       }
-      int bs[4];
-      if (!edge_bs<kMv4>(q, pm ? pm : &q, dir, e, bs, &qm, dir == 0 ? &lm : &tm)) continue;
-      int qpl, qpc;
-      if (!pm) { qpl = qpq; qpc = qpcq; }
-      else { qpl = (qpq + pm->qp + 1) >> 1; qpc = (qpcq + chroma_qp(pm->qp) + 1) >> 1; }
-      EdgeParams el = edge_params(qpl, bs);
-      if (lane < 16 && el.on) {
-        if (dir == 0) luma_line(&ty[(4 + lane) * 20 + 4 + e * 4], 1, el, el.tc0[lane >> 2]);
-        else luma_line(&ty[(4 + e * 4) * 20 + 4 + lane], 20, el, el.tc0[lane >> 2]);
-      }
-      if (!(e & 1) && lane >= 16) {
-        EdgeParams ec = edge_params(qpc, bs);
-        if (ec.on) {
-          int j = lane - 16, p = j >> 3, k = j & 7;
-          if (dir == 0) chroma_line(&tc(p)[(4 + k) * 12 + 4 + e * 2], 1, ec, ec.tc0[k >> 1]);
-          else chroma_line(&tc(p)[(4 + e * 2) * 12 + 4 + k], 12, ec, ec.tc0[k >> 1]);
+      if (!luma && (e & 1)) bs = 0;
+      if (bs) {
+        const uint2 th = edge ? th_p : th_in;
+        const int alpha = (int)(th.x & 255u), beta = (int)(th.x >> 8);
+        uint8_t* const o = base + (luma ? 4 * e : 2 * e) * xs;
+        const int p0 = o[-xs], q0 = o[0], p1 = o[-2 * xs], q1 = o[xs], p2 = o[-3 * xs], q2 = o[2 * xs];
+        if (abs(p0 - q0) < alpha && abs(p1 - p0) < beta && abs(q1 - q0) < beta) {
+          const bool ap = luma && abs(p2 - p0) < beta, aq = luma && abs(q2 - q0) < beta;
+          if (bs < 4) {
+            const int tc0 = (int)((th.y >> (8 * (bs - 1))) & 255u), tcc = tc0 + (luma ? (int)ap + (int)aq : 1);
+            const int d = min(max((((q0 - p0) << 2) + (p1 - q1) + 4) >> 3, -tcc), tcc), a = (p0 + q0 + 1) >> 1;
+            o[-xs] = (uint8_t)clip255(p0 + d);
+            o[0] = (uint8_t)clip255(q0 - d);
+            if (ap) o[-2 * xs] = (uint8_t)(p1 + min(max((p2 + a - (p1 << 1)) >> 1, -tc0), tc0));
+            if (aq) o[xs] = (uint8_t)(q1 + min(max((q2 + a - (q1 << 1)) >> 1, -tc0), tc0));
+          } else {
+            const bool small = abs(p0 - q0) < ((alpha >> 2) + 2);
+            const int p3 = o[-4 * xs], q3 = o[3 * xs];
+            if (ap && small) {
+              o[-xs] = (uint8_t)((p2 + 2 * p1 + 2 * p0 + 2 * q0 + q1 + 4) >> 3);
+              o[-2 * xs] = (uint8_t)((p2 + p1 + p0 + q0 + 2) >> 2);
+              o[-3 * xs] = (uint8_t)((2 * p3 + 3 * p2 + p1 + p0 + q0 + 4) >> 3);
+            } else {
+              o[-xs] = (uint8_t)((2 * p1 + p0 + q1 + 2) >> 2);
+            }
+            if (aq && small) {
+              o[0] = (uint8_t)((p1 + 2 * p0 + 2 * q0 + 2 * q1 + q2 + 4) >> 3);
+              o[xs] = (uint8_t)((p0 + q0 + q1 + q2 + 2) >> 2);
+              o[2 * xs] = (uint8_t)((2 * q3 + 3 * q2 + q1 + q0 + p0 + 4) >> 3);
+            } else {
+              o[0] = (uint8_t)((2 * q1 + q0 + p1 + 2) >> 2);
+            }
+          }
         }
       }
       __syncwarp();
     }
+    __syncwarp();
   }
   // write back the samples this macroblock filters (rows 0..15 x cols -4..15, rows -4..-1 x cols 0..15)
-  for (int w = lane; w < 100; w += 32) {
-    int r = w / 5, k = w % 5;
-    if (r < 4 && k == 0) continue;
-    if ((r < 4 && !hast) || (k == 0 && !hasl)) continue;
-    *(uint32_t*)(sd.cur_y + (long)(y0 - 4 + r) * fp.stride_y + x0 - 4 + 4 * k) = *(const uint32_t*)&ty[r * 20 + 4 * k];
+  if (ly) {
+    const uint2 a = *(const uint2*)&ty[lane * kDbY + 8], b = *(const uint2*)&ty[lane * kDbY + 16];
+    *(uint4*)gy = make_uint4(a.x, a.y, b.x, b.y);
+    if (ly4) *(uint32_t*)(gy - 4) = *(const uint32_t*)&ty[lane * kDbY + 4];
   }
-  for (int w = lane; w < 72; w += 32) {
-    int p = w / 36, rem = w % 36, r = rem / 3, k = rem % 3;
-    if (r < 4 && k == 0) continue;
-    if ((r < 4 && !hast) || (k == 0 && !hasl)) continue;
-    uint8_t* P = p ? sd.cur_v : sd.cur_u;
-    *(uint32_t*)(P + (long)(cy0 - 4 + r) * fp.stride_c + cx0 - 4 + 4 * k) = *(const uint32_t*)&tc(p)[r * 12 + 4 * k];
+  if (lc) {
+    const uint32_t* r = (const uint32_t*)&tc[lane * kDbC];
+    *(uint2*)gc = make_uint2(r[1], r[2]);
+    if (lc4) *(uint32_t*)(gc - 4) = r[0];
   }
 }
 
@@ -2413,14 +2343,20 @@ void upload_tables() {
   }
   cudaMemcpyToSymbol(g_qtab, qt, sizeof(qt));
   cudaMemcpyToSymbol(c_cqp, kChromaQp, sizeof(kChromaQp));
-  cudaMemcpyToSymbol(c_alpha, kAlpha, sizeof(kAlpha));
-  cudaMemcpyToSymbol(c_beta, kBeta, sizeof(kBeta));
-  cudaMemcpyToSymbol(c_tc0, kTc0, sizeof(kTc0));
-  uint16_t taps[9 * 16];
+  uint2 db[52];
+  for (int qp = 0; qp < 52; qp++)
+    db[qp] = make_uint2(kAlpha[qp] | (kBeta[qp] << 8), kTc0[qp][0] | (kTc0[qp][1] << 8) | (kTc0[qp][2] << 16));
+  cudaMemcpyToSymbol(c_deblock, db, sizeof(db));
+  uint2 taps[18];
   for (int m = 0; m < 9; m++)
-    for (int q = 0; q < 16; q++) {
-      int t = i4_tap(m, q & 3, q >> 2), i = t & 0xff;
-      taps[m * 16 + q] = (uint16_t)(i | (i + 1 < 15 ? i + 1 : 15) << 4 | (i + 2 < 15 ? i + 2 : 15) << 8 | (t >> 8) << 12);
+    for (int h = 0; h < 2; h++) {
+      uint32_t w[2] = {0u, 0u};
+      for (int r = 0; r < 2; r++)
+        for (int x = 0; x < 4; x++) {
+          const int v = i4_tap(m, x, r ? 3 - h : h);
+          w[r] |= (uint32_t)((v >> 8) * 16 + (v & 255)) << (8 * x);
+        }
+      taps[2 * m + h] = make_uint2(w[0], w[1]);
     }
   cudaMemcpyToSymbol(g_i4tap, taps, sizeof(taps));
 }

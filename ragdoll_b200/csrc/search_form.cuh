@@ -703,9 +703,9 @@ __device__ __noinline__ void analyse_intra_mb_search(const Ctx c) {
   uint32_t lambda = sm.qt[0].lambda;
   const I16Fit fit16 = analyse_i16(ht, hl, k0.y);
   if (fit16.cost > 40 * lambda) {
-    const uint16_t* masks = sm.sd.hint ? sm.sd.hint[c.mb].i4_mask : nullptr;
-    const int cbpl = masks ? analyse_i4<true>(c, fit16.cost + lambda * 4, ht, hl, k0.y, masks)
-                           : analyse_i4<false>(c, fit16.cost + lambda * 4, ht, hl, k0.y, nullptr);
+    const rg_mb_hint* hint = sm.sd.hint;
+    const uint32_t masks = hint ? hint[c.mb].i4_mask[lane_id() & 15] : 0x1ffu;
+    const int cbpl = analyse_i4(c, fit16.cost + lambda * 4, ht, hl, k0.y, masks);
     if (cbpl >= 0) {
       code_i4(c, cbpl, ht, hl, k0);
       search_tail(c, 255, false, 0, 0);
