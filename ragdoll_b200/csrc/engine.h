@@ -113,12 +113,14 @@ struct FrameGroups {
   FrameParams g[kMaxGroups];
   int32_t n;
 };
-int pipeline_grid(int device, int form = 0);
+int pipeline_grid(int device);
 int pipeline_sms(int device);
 size_t pipeline_counter_ints(const FrameParams& fp, int frames);
 // Work list: every analysis / deblocking segment of `seg` macroblocks, in expected-ready order
 // with `lag` macroblock-times between consecutive pictures of a stream.
 size_t pipeline_task_count(const FrameParams& fp, int frames, int seg);
+// The range of its keys (macroblock-times from the first segment to the last).
+int pipeline_key_span(const FrameParams& fp, int frames, int lag, int seg);
 // Queues: 0 analysis, 1 deblocking (split), 2 analysis of IDR pictures (kinds != null; [f][s]).
 constexpr int kPipeQueues = 3;
 // keys (or null): each task's key, ascending within each queue.
@@ -140,7 +142,7 @@ struct CompactOut {
   int* row_bytes;    // device address of mapped host memory: [row]
 };
 void launch_pipeline(const FrameGroups& fg, const StreamDev* d_streams, int n_desc, int total_rows, int* counters,
-                     const int2* d_tasks, size_t n_tasks, const int qbeg[3], const int qend[3], int deblock_sms,
+                     const int2* d_tasks, size_t n_tasks, int key_span, const int qbeg[3], const int qend[3], int deblock_sms,
                      int intra_sms, int sms, int seg, int grid, unsigned long long timeout_ns, int* ready, int seq,
                      int* host_err, int* host_reach, cudaStream_t st, int form = 0, const CompactOut* co = nullptr);
 void launch_error_to_host(const int* counters, int n_desc, int total_rows, int* host_err, int* host_reach,

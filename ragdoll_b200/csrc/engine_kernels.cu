@@ -110,11 +110,13 @@ static_assert(offsetof(Smem, coef) % 8 == 0 && offsetof(Smem, ccoef) % 8 == 0 &&
 static_assert(20 * 24 <= kWinPlane && 24 * 12 <= kWinPlane, "the deblocking tiles fit the window's planes");
 static_assert(offsetof(Smem, pred_y) % 8 == 0 && offsetof(Smem, tmp_y) % 8 == 0, "16x16 predictions written 8 bytes per lane");
 
-// Every kernel of this file runs one warp per block, and its shared memory has this one name: the
-// functions below address it directly (shared-memory loads at constant offsets) instead of through
-// a reference, which a call turns into a generic address -- a 64-bit pointer in registers and loads
+// The warps of a block each work on a macroblock of their own; sm is the calling warp's shared memory.
+// The functions below address it directly (shared-memory loads from one offset) instead of through a
+// reference, which a call turns into a generic address -- a 64-bit pointer in registers and loads
 // that resolve their memory space as they run.
-__shared__ Smem sm;
+// Blocks are 32 x warps threads.
+extern __shared__ __align__(16) uint8_t smw[];
+#define sm (((Smem*)smw)[threadIdx.y])
 __device__ __forceinline__ uint8_t* sm_at(int off) { return (uint8_t*)&sm + off; }
 
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
@@ -2038,6 +2040,8 @@ struct PipeParams {
   int qbeg[3], qend[3];  // queue q = tasks[qbeg[q], qend[q]): 0 analysis, 1 deblocking, 2 IDR analysis
   int deblock_sms;    // SMs whose warps take queue 1 first
   int intra_sms;      // the next SMs, whose warps take queue 2 first
+  int grid;           // warps that take segments
+  int meet_ns;        // limit of a meeting of a block's warps (meet), 0: they do not wait for each other
   int role_by_sm;     // 0: by block index instead (a grid too small to reach every SM)
   int seg;
   unsigned long long timeout_ns;
@@ -2154,10 +2158,36 @@ __device__ __noinline__ void compact_row(const rg_mb_out* rec, uint32_t* dst, in
   __syncwarp();
 }
 
-// At least 16 warps per SM: up to 128 registers a thread, so nothing spills (4.5 % faster than 20,
-// which held it to 96 registers with spills).
+// Sixteen warps per SM, one block: up to 128 registers a thread, so nothing spills.
+constexpr int kBlockWarps = 16;
+
+// The warps of an SM run the same code on different macroblocks, and the code is several times the
+// SM's instruction cache: with every warp somewhere else in it, the cache that the SMs of a group
+// share behind theirs was busy all the time (0.44 lines a cycle), and a macroblock took three times as
+// long as on an idle SM. So the warps of a block (one block an SM) start their macroblocks together:
+// most of what one of them fetches is then still there for the other fifteen. A warp that has finished
+// its segment waits here until the others have finished theirs, for at most `limit` ns (a long
+// macroblock's time): one that waits for another SM's macroblock holds nobody for long, and no wait
+// of the schedule depends on a meeting. 1080p 8 x 15 launch: 34.9 ms without, 21.7 with 60 us, 24.5 with
+// 30, 21.5 with 200; learned 1080p (macroblocks three times as long) 92 without, 65.9 with 300 us, 64.5
+// with 1 ms. round: the arrivals that complete this warp's round.
+constexpr int kMeetNs = 60000, kMeetNsSearch = 400000;
+__device__ __forceinline__ void meet(int* arrived, int round, int limit) {
+  if (lane_id() == 0) {
+    int n = atomicAdd(arrived, 1) + 1;
+    if (n < round && limit) {
+      const unsigned long long t0 = global_ns();
+      do {
+        __nanosleep(200);
+        n = *(volatile int*)arrived;
+      } while (n < round && global_ns() - t0 < limit);
+    }
+  }
+  __syncwarp();
+}
+
 template <int kForm>
-__global__ void __launch_bounds__(32, 16) pipeline_kernel(const __grid_constant__ FrameGroups fg, const StreamDev* __restrict__ sds, PipeParams pp) {
+__global__ void __launch_bounds__(32 * kBlockWarps, 1) pipeline_kernel(const __grid_constant__ FrameGroups fg, const StreamDev* __restrict__ sds, PipeParams pp) {
   const int lane = lane_id();
   // Warps on the first deblock_sms SMs take deblocking segments first, on the next intra_sms SMs
   // segments of IDR pictures (the critical path of a GOP), and the others the remaining analysis
@@ -2171,17 +2201,22 @@ __global__ void __launch_bounds__(32, 16) pipeline_kernel(const __grid_constant_
     role = k == 0 ? 1 : (k == 1 ? 2 : 0);
   }
   init_tables();
-  bool empty[3] = {pp.qbeg[0] >= pp.qend[0], pp.qbeg[1] >= pp.qend[1], pp.qbeg[2] >= pp.qend[2]};
+  uint32_t empty = (pp.qbeg[0] >= pp.qend[0] ? 1u : 0u) | (pp.qbeg[1] >= pp.qend[1] ? 2u : 0u) | (pp.qbeg[2] >= pp.qend[2] ? 4u : 0u);
+  __shared__ int arrived;  // warps that have finished a segment, all rounds together
+  int round = 0;
+  if (threadIdx.y == 0 && lane == 0) arrived = 0;
   if (lane == 0) sm.reach_y = sm.reach_x = 0;  // this warp's, published once as it exits
   int group = -1;                              // whose parameters sm.fp holds
-  while (true) {
+  __syncthreads();
+  bool failed = (int)(blockIdx.x * blockDim.y + threadIdx.y) >= pp.grid;  // a warp past the grid takes nothing
+  while (!failed) {
     int t = -1;
     if (lane == 0) {
       for (int k = 0; k < 3 && t < 0; k++) {
-        int q = role + k >= 3 ? role + k - 3 : role + k;
-        if (empty[q]) continue;
-        int v = pp.qbeg[q] + atomicAdd(pp.ticket + (q ? q + 1 : 0), 1);
-        if (v < pp.qend[q]) t = v; else empty[q] = true;
+        const int q = role + k >= 3 ? role + k - 3 : role + k;
+        if ((empty >> q) & 1u) continue;
+        const int v = pp.qbeg[q] + atomicAdd(pp.ticket + (q ? q + 1 : 0), 1);
+        if (v < pp.qend[q]) t = v; else empty |= 1u << q;
       }
     }
     t = __shfl_sync(FULL, t, 0);
@@ -2200,7 +2235,6 @@ __global__ void __launch_bounds__(32, 16) pipeline_kernel(const __grid_constant_
     const bool ana = (task.y & 1) == 0;
     int* ana_rows = pp.ana + sd.rows_base;
     int* db_rows = pp.db + sd.rows_base;
-    bool failed = false;
     int seen = 0;  // of this lane's counter (wait_all)
     if (ana) {
       const bool has_prev = sd.prev_rows >= 0 && sd.kind == RG_FRAME_P;
@@ -2267,8 +2301,11 @@ __global__ void __launch_bounds__(32, 16) pipeline_kernel(const __grid_constant_
         if (rdy) picture_row_done(pp.rows_done + ps, rdy, pp.seq, H);
       }
     }
-    if (failed) break;
+    round += blockDim.y;
+    meet(&arrived, round, pp.meet_ns);
   }
+  // whoever is left need not wait for this warp any more
+  if (lane == 0) atomicAdd(&arrived, 1 << 26);
   if (lane == 0 && sm.reach_y) {
     atomicMax(pp.reach, sm.reach_y);
     atomicMax(pp.reach + 1, sm.reach_x);
@@ -2377,10 +2414,13 @@ static int max_diag_len(const FrameParams& fp) {
   return best;
 }
 
+// Shared memory of a warp of the analysis kernels.
+static size_t warp_smem(int form) { return sizeof(Smem) + (form ? sizeof(SearchSmem) : 0); }
+
 void launch_wavefront_step(const FrameParams& fp, const StreamDev* d_streams, int step, cudaStream_t st, int form) {
   dim3 grid(2 * max_diag_len(fp), fp.n_streams);
-  if (form) wavefront_step_kernel<1><<<grid, 32, 0, st>>>(fp, d_streams, step);
-  else wavefront_step_kernel<0><<<grid, 32, 0, st>>>(fp, d_streams, step);
+  if (form) wavefront_step_kernel<1><<<grid, 32, warp_smem(1), st>>>(fp, d_streams, step);
+  else wavefront_step_kernel<0><<<grid, 32, warp_smem(0), st>>>(fp, d_streams, step);
 }
 
 int pipeline_sms(int device) {
@@ -2389,16 +2429,9 @@ int pipeline_sms(int device) {
   return sms;
 }
 
-// Resident warps of the pipelined mode: sixteen per SM (fewer when they do not fit). More warps
-// overlap more of each other's waits, until the SM's front end saturates and every macroblock on
-// the critical path slows (measured on B200, 1080p 8 x 15 pictures, launch time: 7 per SM
-// 62.9 ms, 8 61.0, 10 59.1, 12 57.4, 14 56.0, 16 55.8, 18 56.2, 20-21 56.3).
-int pipeline_grid(int device, int form) {
-  int per_sm = 0;
-  if (form) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pipeline_kernel<1>, 32, 0);
-  else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pipeline_kernel<0>, 32, 0);
-  return (per_sm < 16 ? per_sm : 16) * pipeline_sms(device);
-}
+// Resident warps of the pipelined mode: a block of sixteen on every SM (launch time of 1080p 8 x 15
+// pictures by the warps an SM, before they met: 6 45.1 ms, 8 40.8, 10 38.7, 12 36.9, 14 35.6, 16 34.9).
+int pipeline_grid(int device) { return kBlockWarps * pipeline_sms(device); }
 
 // Work list of the pipelined mode, written to `tasks` (pipeline_task_count entries): every
 // analysis and deblocking segment of every picture and stream, ordered by a key of the
@@ -2416,6 +2449,11 @@ int pipeline_grid(int device, int form) {
 size_t pipeline_task_count(const FrameParams& fp, int frames, int seg) {
   size_t segs = (size_t)(fp.mb_w + seg - 1) / seg;
   return 2 * (size_t)frames * fp.n_streams * fp.mb_h * segs;
+}
+
+int pipeline_key_span(const FrameParams& fp, int frames, int lag, int seg) {
+  const int a = seg > 2 ? seg : 2;
+  return a * fp.mb_h + fp.mb_w + lag * (frames - 1);
 }
 
 size_t pipeline_task_list(const FrameParams& fp, int frames, int lag, int seg, bool split, const int32_t* kinds,
@@ -2459,7 +2497,7 @@ size_t pipeline_task_list(const FrameParams& fp, int frames, int lag, int seg, b
 }
 
 void launch_pipeline(const FrameGroups& fg, const StreamDev* d_streams, int n_desc, int total_rows, int* counters,
-                     const int2* d_tasks, size_t n_tasks, const int qbeg[3], const int qend[3], int deblock_sms,
+                     const int2* d_tasks, size_t n_tasks, int key_span, const int qbeg[3], const int qend[3], int deblock_sms,
                      int intra_sms, int sms, int seg, int grid, unsigned long long timeout_ns, int* ready, int seq,
                      int* host_err, int* host_reach, cudaStream_t st, int form, const CompactOut* co) {
   PipeParams pp;
@@ -2475,7 +2513,20 @@ void launch_pipeline(const FrameGroups& fg, const StreamDev* d_streams, int n_de
   }
   pp.deblock_sms = deblock_sms;
   pp.intra_sms = intra_sms;
-  pp.role_by_sm = grid >= sms;
+  // Meetings pay where there is work for most warps, and cost a little where the launch is one chain
+  // of macroblocks and they wait anyway: on average at least a quarter as many segments ready as there
+  // are warps (segments over the span of their keys, both roles). 8 x 15 pictures of 1080p have 1742
+  // (34.9 -> 21.7 ms), 8 x 8 learned 1238 (92 -> 65.5), four mixed sizes 1148 (17.3 -> 13.1), 4 x 3
+  // learned 4K 672 (80.9 -> 77.2), 8 x 3 full search 720p 310 (50.9 -> 52.3), one 720p stream 179 (11.8 ->
+  // 12.2).
+  const bool meet = n_tasks / 2 * 4 >= (size_t)grid * (size_t)key_span;
+  pp.meet_ns = meet ? (form ? kMeetNsSearch : kMeetNs) : 0;
+  // spread over the SMs, then up to a block's warps on each
+  pp.grid = grid < pp.n_tasks ? grid : pp.n_tasks;
+  int warps = (pp.grid + sms - 1) / sms;
+  if (warps > kBlockWarps) warps = kBlockWarps;
+  const int g = (pp.grid + warps - 1) / warps;
+  pp.role_by_sm = g >= sms;
   pp.seg = seg;
   pp.timeout_ns = timeout_ns;
   pp.rows_done = pp.db + total_rows;
@@ -2486,9 +2537,15 @@ void launch_pipeline(const FrameGroups& fg, const StreamDev* d_streams, int n_de
   pp.cwords = co ? co->words : nullptr;
   pp.crow = co ? co->row_words : 0;
   pp.cbytes = co ? co->row_bytes : nullptr;
-  int g = grid < pp.n_tasks ? grid : pp.n_tasks;
-  if (form) pipeline_kernel<1><<<g, 32, 0, st>>>(fg, d_streams, pp);
-  else pipeline_kernel<0><<<g, 32, 0, st>>>(fg, d_streams, pp);
+  const dim3 block(32, warps);
+  const size_t smem = warps * warp_smem(form);
+  if (form) {
+    cudaFuncSetAttribute(pipeline_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    pipeline_kernel<1><<<g, block, smem, st>>>(fg, d_streams, pp);
+  } else {
+    cudaFuncSetAttribute(pipeline_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    pipeline_kernel<0><<<g, block, smem, st>>>(fg, d_streams, pp);
+  }
   if (host_err) error_to_host_kernel<<<1, 1, 0, st>>>(pp.error, pp.reach, host_err, host_reach);
 }
 

@@ -691,8 +691,8 @@ static int enqueue_gops(rg_ctx* c, const uint8_t* const* dev_planes, size_t stri
   FrameGroups fg{};
   fg.g[0] = fp;
   fg.n = 1;
-  launch_pipeline(fg, c->d_streams[slot], frames * S, frames * S * fp.mb_h, c->counters, c->d_tasks, c->n_tasks, c->qbeg,
-                  c->qend, c->deblock_sms, c->intra_sms, c->sms, c->seg, c->grid, c->timeout_ns, ready, seq,
+  launch_pipeline(fg, c->d_streams[slot], frames * S, frames * S * fp.mb_h, c->counters, c->d_tasks, c->n_tasks,
+                  pipeline_key_span(fp, frames, lag, c->seg), c->qbeg, c->qend, c->deblock_sms, c->intra_sms, c->sms, c->seg, c->grid, c->timeout_ns, ready, seq,
                   c->d_err + pslot, c->d_err + 2 + 2 * pslot, c->stream, c->form != RG_FORM_PLAIN, co);
   CK(cudaGetLastError());
   CK(cudaEventRecord(p.done, c->stream));
@@ -834,6 +834,12 @@ static int group_launch(rg_ctx* const* ctxs, int32_t n, const uint8_t* const* co
     shape.insert(shape.end(), {c->cfg.width, c->cfg.height, c->S, lag});
     if (intra_q) shape.insert(shape.end(), kinds[i], kinds[i] + (size_t)frames * c->S);
   }
+  int key_span = 1;
+  for (int i = 0; i < n; i++) {
+    const rg_ctx* c = ctxs[i];
+    const int lag = c->lag > 0 ? c->lag : a * (4 + c->reach_y) + seg + c->reach_x + 3;
+    key_span = std::max(key_span, pipeline_key_span(c->fp, frames, lag, seg));
+  }
   if (shape != L->g_shape) {
     std::vector<std::vector<int2>> lists(n);
     std::vector<std::vector<uint32_t>> keys(n);
@@ -930,7 +936,7 @@ static int group_launch(rg_ctx* const* ctxs, int32_t n, const uint8_t* const* co
     if (e == cudaSuccess) e = cudaEventRecordWithFlags(L->g_done, L->stream, cudaEventRecordExternal);
     if (e == cudaSuccess) e = cudaMemsetAsync(L->g_counters, 0, sizeof(int) * n_counters, L->stream);
     if (e == cudaSuccess) {
-      launch_pipeline(fg, L->g_dstreams, n_desc, total_rows, L->g_counters, L->g_dtasks, L->g_ntasks, L->g_qbeg,
+      launch_pipeline(fg, L->g_dstreams, n_desc, total_rows, L->g_counters, L->g_dtasks, L->g_ntasks, key_span, L->g_qbeg,
                       L->g_qend, T->deblock_sms, T->intra_sms, L->sms, seg, grid, T->timeout_ns, nullptr, seq, nullptr,
                       nullptr, L->stream, L->form != RG_FORM_PLAIN);
       for (int i = 0; i < n; i++)
@@ -1112,7 +1118,7 @@ int rg_set_pipeline_tuning(rg_ctx* c, const rg_pipeline_tuning* t) {
   c->intra_sms = intra_sms < 0 ? 0 : (intra_sms > 0 ? intra_sms : default_intra_sms(c->sms));
   c->tasks_frames = -1;
   if (grid > 0) c->grid = grid;
-  else c->grid = pipeline_grid(c->cfg.device, c->form != RG_FORM_PLAIN);
+  else c->grid = pipeline_grid(c->cfg.device);
   c->timeout_ns = timeout_ms > 0 ? (unsigned long long)timeout_ms * 1000000ull : 2000000000ull;
   return RG_OK;
 }
@@ -1274,10 +1280,8 @@ int rg_set_analysis_form(rg_ctx* c, int32_t form, int32_t search_range) {
     if (cudaMalloc((void**)&c->mv4s, n) != cudaSuccess) return fail(RG_ERR_OOM, "rg_set_analysis_form: %zu bytes", n);
     CK(cudaMemset(c->mv4s, 0, n));
   }
-  bool default_grid = c->grid == pipeline_grid(c->cfg.device, c->form != RG_FORM_PLAIN);
   c->form = form;
   if (form != RG_FORM_PLAIN) c->search_range = search_range;
-  if (default_grid) c->grid = pipeline_grid(c->cfg.device, form != RG_FORM_PLAIN);
   c->hints.clear();
   return RG_OK;
 }

@@ -57,7 +57,9 @@ struct SearchSmem {
   int ccx[8], ccy[8];  // the learned form's centre candidates (ok: cok)
   bool cok[8];
 };
-__shared__ SearchSmem ss;
+// Behind every warp's Smem.
+static_assert(sizeof(Smem) % 16 == 0, "SearchSmem follows aligned");
+#define ss (((SearchSmem*)(smw + blockDim.y * sizeof(Smem)))[threadIdx.y])
 __device__ __forceinline__ void ld_q(const MbMv4* m, int q, int* v) {
   uint32_t w = ((const uint32_t*)m)[q];
   v[0] = (int16_t)(w & 0xffffu);
