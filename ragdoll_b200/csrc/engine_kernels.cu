@@ -2221,9 +2221,9 @@ __global__ void __launch_bounds__(32 * kBlockWarps, 1) pipeline_kernel(const __g
     }
     t = __shfl_sync(FULL, t, 0);
     if (t < 0) break;
-    if (__shfl_sync(FULL, lane == 0 ? ld_relaxed(pp.error) : 0, 0)) break;
-    int2 task = __ldg(pp.tasks + t);
-    int ps = task.x;
+    const int2 task = __ldg(pp.tasks + t);
+    if (__shfl_sync(FULL, ld_relaxed(pp.error), 0)) break;  // (both loads in flight together)
+    const int ps = task.x;
     load_desc(sds + ps);
     const StreamDev& sd = sm.sd;
     if (sd.group != group) {  // the descriptor's picture size
@@ -2302,7 +2302,7 @@ __global__ void __launch_bounds__(32 * kBlockWarps, 1) pipeline_kernel(const __g
       }
     }
     round += blockDim.y;
-    meet(&arrived, round, pp.meet_ns);
+    meet(&arrived, round, ana ? pp.meet_ns : 0);  // (the deblocking code fits the cache by itself)
   }
   // whoever is left need not wait for this warp any more
   if (lane == 0) atomicAdd(&arrived, 1 << 26);
