@@ -16,7 +16,7 @@
 // one descriptor of the map -- no im2col copy. The epilogue adds the bias, applies the ReLU and
 // stores the next layer's BF16 operand over its input; the heads run on the CUDA cores and write
 // the hints. While one CTA's epilogue runs, the other's MMAs can.
-// Training (cnn_train_*): the same network in f32 on the CUDA cores -- forward, the losses, the
+// Training: the same network in f32 on the CUDA cores -- forward, the losses, the
 // backward pass and Adam -- on per-macroblock crops.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -490,267 +490,436 @@ __global__ void __launch_bounds__(32 * kCoarseWarps) coarse_motion_kernel(Coarse
 // ---------------------------------------------------------------------------------------------
 // Training on the CUDA cores (f32), per-macroblock crops: 2 x 24 x 24 bytes per sample.
 // Maps: A1 [N][32][22][22], A2 [N][32][20][20], A3 [N][32][18][18] (after the ReLU).
+// The pass is about 22 M multiply-adds a sample; its kernels are bound by the FMA pipes and keep a
+// register tile per thread, so that a shared-memory load feeds about ten of them. A batch of 256:
+// 6.1 ms with a position or a weight per thread (the weight gradients in 32 blocks), 0.5 ms as below.
 constexpr int kIn = 2 * 24 * 24, kA1 = C * 22 * 22, kA2 = C * 20 * 20, kA3 = C * 18 * 18;
+constexpr int kW = C * C * 9;                  // weights of a 32 -> 32 layer
+constexpr int kHeadParams = kParams - kWp;
+// Transposed weights (train_prep_kernel): [ci][tap][co] for the forward passes, [co][8 - tap][ci] for the
+// input gradients -- the layout a convolution block loads.
+constexpr int kT1 = 0, kT2 = kT1 + 2 * 9 * C, kT3 = kT2 + kW, kTb3 = kT3 + kW, kTb2 = kTb3 + kW, kTrans = kTb2 + kW;
 
-// conv 3x3 valid of one sample per block: in [cin][hin][hin] (bytes normalised when u8 != null),
-// out [32][hin-2][hin-2] = ReLU(W x + b).
-__global__ void conv_fwd_kernel(const uint8_t* __restrict__ u8, const float* __restrict__ in, int cin, int hin,
-                                const float* __restrict__ P, int woff, int boff, float* __restrict__ out) {
-  extern __shared__ float4 sh4[];
-  float* sh = (float*)sh4;
-  float* w = sh;                       // [cin][9][32]
-  float* x = sh + C * cin * 9;         // cin * hin * hin
-  const int n = blockIdx.x, hout = hin - 2, npos = hout * hout, nin = cin * hin * hin;
-  for (int i = threadIdx.x; i < nin; i += blockDim.x)
-    x[i] = u8 ? pix_norm(u8[(size_t)n * nin + i]) : in[(size_t)n * nin + i];
-  for (int i = threadIdx.x; i < C * cin * 9; i += blockDim.x) {
-    const int o = i / (cin * 9), ci = (i / 9) % cin, t = i % 9;
-    w[(ci * 9 + t) * C + o] = P[woff + i];
+// The transposed weights; the last block counts the labels and writes 1 / count of each loss (0 for
+// none) to scales: partition, intra 4x4, offset.
+__global__ void train_prep_kernel(const float* __restrict__ P, float* __restrict__ T, const int* __restrict__ part,
+                                  const int* __restrict__ i4, const int* __restrict__ mvv, int n, float* __restrict__ scales) {
+  if (blockIdx.x + 1 < gridDim.x) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= kTrans) return;
+    if (i < kT2) {
+      const int ci = i / (9 * C), t = (i / C) % 9, co = i % C;
+      T[i] = P[kW1 + (co * 2 + ci) * 9 + t];
+    } else {
+      const int l = (i - kT2) / kW, k = (i - kT2) % kW, a = k / (9 * C), t = (k / C) % 9, b = k % C;
+      // forward: a = ci, b = co; input gradient: a = co, b = ci, taps reversed
+      T[i] = l < 2 ? P[(l == 0 ? kW2 : kW3) + (b * C + a) * 9 + t] : P[(l == 2 ? kW3 : kW2) + (a * C + b) * 9 + 8 - t];
+    }
+    return;
+  }
+  __shared__ int cnt[3];
+  if (threadIdx.x < 3) cnt[threadIdx.x] = 0;
+  __syncthreads();
+  int np = 0, ni = 0, nm = 0;
+  for (int k = threadIdx.x; k < n; k += blockDim.x) { np += part[k] >= 0; nm += mvv[k] != 0; }
+  for (int k = threadIdx.x; k < n * 16; k += blockDim.x) ni += i4[k] >= 0;
+  np = __reduce_add_sync(0xffffffffu, np);
+  ni = __reduce_add_sync(0xffffffffu, ni);
+  nm = __reduce_add_sync(0xffffffffu, nm);
+  if ((threadIdx.x & 31) == 0) {
+    atomicAdd(&cnt[0], np);
+    atomicAdd(&cnt[1], ni);
+    atomicAdd(&cnt[2], nm);
   }
   __syncthreads();
-  for (int p = threadIdx.x; p < npos; p += blockDim.x) {
-    const int y = p / hout, xx = p % hout;
-    float acc[C];
-#pragma unroll
-    for (int o = 0; o < C; o++) acc[o] = P[boff + o];
-    for (int ci = 0; ci < cin; ci++)
-#pragma unroll
-      for (int t = 0; t < 9; t++) {
-        const float v = x[(ci * hin + y + t / 3) * hin + xx + t % 3];
-        const float4* wv = (const float4*)&w[(ci * 9 + t) * C];
-#pragma unroll
-        for (int o4 = 0; o4 < C / 4; o4++) {
-          const float4 q = wv[o4];
-          acc[4 * o4] += q.x * v; acc[4 * o4 + 1] += q.y * v; acc[4 * o4 + 2] += q.z * v; acc[4 * o4 + 3] += q.w * v;
-        }
-      }
-#pragma unroll
-    for (int o = 0; o < C; o++) out[(size_t)n * C * npos + o * npos + p] = fmaxf(acc[o], 0.0f);
-  }
+  if (threadIdx.x < 3) scales[threadIdx.x] = cnt[threadIdx.x] ? 1.0f / (float)cnt[threadIdx.x] : 0.0f;
 }
 
-// Heads, losses and their gradient (one block of 32 threads per sample): labels part [N] (-1 none),
-// i4 [N][16] (raster 4x4 blocks, -1 none), mv [N][2] with mvv [N] (0 none); scale: 1 / the count of
-// each loss's labels in the batch. Writes the logits (optional), the pooled features (feat [N][17][32]:
-// the 18 x 18 mean, then the block means), the logit gradients (dlog [N][kLogits]) and dA3 (the
-// gradient at the conv3 map, masked by its ReLU); the loss is added atomically.
-__global__ void heads_kernel(const float* __restrict__ A3, const float* __restrict__ P, const int* __restrict__ part,
-                             const int* __restrict__ i4, const float* __restrict__ mv, const int* __restrict__ mvv,
-                             float sp, float si, float sm, float mv_weight, float* __restrict__ logits,
-                             float* __restrict__ feat, float* __restrict__ dlog, float* __restrict__ dA3,
-                             float* __restrict__ loss) {
-  __shared__ float f[17][C], dg[C], df[16][C], dl[kLogits], lsum[17];
-  const int n = blockIdx.x, c = threadIdx.x;
-  const float* a = A3 + (size_t)n * kA3 + c * 324;
-  float all = 0.0f, blk[16];
-  for (int b = 0; b < 16; b++) blk[b] = 0.0f;
-  for (int r = 0; r < 18; r++)
-    for (int i = 0; i < 18; i++) {
-      float x = a[r * 18 + i];
-      all += x;
-      if (r >= 1 && r <= 16 && i >= 1 && i <= 16) blk[((r - 1) >> 2) * 4 + ((i - 1) >> 2)] += x;
+// A 3x3 convolution of one sample per block (blockIdx.y: a part of its output channels, for batches
+// that do not fill the GPU): kHin x kHin input of kCin channels in shared memory, 16 channels at a
+// time (two blocks an SM). A thread computes 4 positions of a row x 8 channels: per input channel
+// three rows of six samples and 72 weights (the same for the whole warp, but at group borders) for 288
+// multiply-adds. kU8: the input are crops (bytes, normalised); kBwd: the input is an output
+// gradient, surrounded by zeros (the full correlation with the reversed taps is the input's
+// gradient), and the result is masked by the ReLU of the map `act`; otherwise bias and ReLU.
+constexpr int kConvChunk = 16;
+template <int kHin>
+struct ConvShape {
+  static constexpr int hout = kHin - 2, groups = (hout + 3) / 4, row = (4 * groups + 2 + 3) / 4 * 4;
+  static constexpr int threads = hout * groups;  // of one group of 8 channels
+};
+template <int kHin, int kCin, bool kU8, bool kBwd>
+__global__ void __launch_bounds__(kHin == 24 ? 544 : 416, kHin == 24 ? 1 : 2)
+    conv_kernel(const void* __restrict__ in, const float* __restrict__ wt, const float* __restrict__ bias,
+                const float* __restrict__ act, float* __restrict__ out, int cgs) {
+  using S = ConvShape<kHin>;
+  constexpr int kCh = kCin < kConvChunk ? kCin : kConvChunk, kMap = kHin * S::row, npos = S::hout * S::hout;
+  extern __shared__ float4 sh4[];
+  float* w = (float*)sh4;           // [kCh][9][32]
+  float* x = w + kCh * 9 * C;       // [kCh][kHin][row]
+  const int n = blockIdx.x, tid = threadIdx.x;
+  const int cg = tid / S::threads, pos = tid - cg * S::threads, y = pos / S::groups, x0 = (pos - y * S::groups) * 4;
+  const bool on = cg < cgs;
+  const int co = (blockIdx.y * cgs + (on ? cg : 0)) * 8;
+  float acc[8][4];
+#pragma unroll
+  for (int o = 0; o < 8; o++)
+#pragma unroll
+    for (int k = 0; k < 4; k++) acc[o][k] = 0.0f;
+  for (int c0 = 0; c0 < kCin; c0 += kCh) {
+    if (c0) __syncthreads();
+    for (int i = tid; i < kCh * 9 * C / 4; i += blockDim.x) ((float4*)w)[i] = ((const float4*)(wt + c0 * 9 * C))[i];
+    for (int i = tid; i < kCh * kMap; i += blockDim.x) {
+      const int ci = i / kMap, r = (i - ci * kMap) / S::row, c = i - ci * kMap - r * S::row;
+      float v = 0.0f;
+      if constexpr (kBwd) {  // the gradient map is kHin - 4 wide
+        constexpr int h = kHin - 4;
+        if (r >= 2 && r < kHin - 2 && c >= 2 && c < kHin - 2) v = ((const float*)in)[((size_t)n * kCin + c0 + ci) * h * h + (r - 2) * h + c - 2];
+      } else if (c < kHin) {
+        const size_t at = ((size_t)n * kCin + c0 + ci) * kHin * kHin + r * kHin + c;
+        v = kU8 ? pix_norm(((const uint8_t*)in)[at]) : ((const float*)in)[at];
+      }
+      x[i] = v;
     }
-  f[0][c] = all / 324.0f;
-  for (int b = 0; b < 16; b++) f[1 + b][c] = blk[b] / 16.0f;
-  __syncthreads();
-  for (int k = 0; k < 17; k++) feat[((size_t)n * 17 + k) * C + c] = f[k][c];
-  // thread 0: partition and offset; threads 1..16: block c - 1's intra 4x4 logits
-  if (c <= 16) {
-    float L = 0.0f;
-    if (c == 0) {
-      float lp[4], lm[2];
-      for (int o = 0; o < 4; o++) {
-        float s = P[kBp + o];
-        for (int k = 0; k < C; k++) s += P[kWp + o * C + k] * f[0][k];
-        lp[o] = s;
-      }
-      for (int o = 0; o < 2; o++) {
-        float s = P[kBm + o];
-        for (int k = 0; k < C; k++) s += P[kWm + o * C + k] * f[0][k];
-        lm[o] = s;
-      }
-      for (int o = 0; o < 6; o++) dl[o] = 0.0f;
-      if (part[n] >= 0) {
-        float mx = fmaxf(fmaxf(lp[0], lp[1]), fmaxf(lp[2], lp[3])), se = 0.0f;
-        for (int o = 0; o < 4; o++) se += expf(lp[o] - mx);
-        for (int o = 0; o < 4; o++) dl[o] = sp * (expf(lp[o] - mx) / se - (o == part[n] ? 1.0f : 0.0f));
-        L += sp * (logf(se) + mx - lp[part[n]]);
-      }
-      if (mvv[n]) {
-        for (int o = 0; o < 2; o++) {  // Huber (delta 1) on the offset in units of 16 quarter samples
-          float d = lm[o] - mv[2 * n + o];
-          float ad = fabsf(d);
-          L += sm * mv_weight * (ad <= 1.0f ? 0.5f * d * d : ad - 0.5f);
-          dl[4 + o] = sm * mv_weight * (ad <= 1.0f ? d : (d > 0 ? 1.0f : -1.0f));
+    __syncthreads();
+    if (on) {
+#pragma unroll 1
+      for (int ci = 0; ci < kCh; ci++) {
+        const float* xp = x + ci * kMap + y * S::row + x0;
+        const float* wp = w + ci * 9 * C + co;
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
+          const float4 a = *(const float4*)(xp + r * S::row);
+          const float2 b = *(const float2*)(xp + r * S::row + 4);
+          const float v[6] = {a.x, a.y, a.z, a.w, b.x, b.y};
+#pragma unroll
+          for (int t = 0; t < 3; t++) {
+            const float4 w0 = *(const float4*)(wp + (r * 3 + t) * C), w1 = *(const float4*)(wp + (r * 3 + t) * C + 4);
+            const float q[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+            for (int o = 0; o < 8; o++)
+#pragma unroll
+              for (int k = 0; k < 4; k++) acc[o][k] = fmaf(q[o], v[t + k], acc[o][k]);
+          }
         }
       }
-      if (logits) {
-        for (int o = 0; o < 4; o++) logits[(size_t)n * kLogits + o] = lp[o];
-        logits[(size_t)n * kLogits + 4] = lm[0];
-        logits[(size_t)n * kLogits + 5] = lm[1];
-      }
-    } else {
-      const int b = c - 1;
-      float li[9];
-      for (int o = 0; o < 9; o++) {
-        float s = P[kBi + o];
-        for (int k = 0; k < C; k++) s += P[kWi + o * C + k] * f[1 + b][k];
-        li[o] = s;
-        dl[6 + b * 9 + o] = 0.0f;
-      }
-      if (logits)
-        for (int o = 0; o < 9; o++) logits[(size_t)n * kLogits + 6 + b * 9 + o] = li[o];
-      const int lab = i4[n * 16 + b];
-      if (lab >= 0) {
-        float mx = li[0], se = 0.0f;
-        for (int o = 1; o < 9; o++) mx = fmaxf(mx, li[o]);
-        for (int o = 0; o < 9; o++) se += expf(li[o] - mx);
-        for (int o = 0; o < 9; o++) dl[6 + b * 9 + o] = si * (expf(li[o] - mx) / se - (o == lab ? 1.0f : 0.0f));
-        L += si * (logf(se) + mx - li[lab]);
-      }
     }
-    lsum[c] = L;
+  }
+  if (!on) return;
+#pragma unroll
+  for (int o = 0; o < 8; o++) {
+    const size_t base = ((size_t)n * C + co + o) * npos + y * S::hout + x0;
+    const float bo = kBwd ? 0.0f : bias[co + o];
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if (x0 + k < S::hout) out[base + k] = kBwd ? (act[base + k] > 0.0f ? acc[o][k] : 0.0f) : fmaxf(acc[o][k] + bo, 0.0f);
+  }
+}
+template <int kHin, int kCin>
+constexpr int conv_smem() {
+  return ((kCin < kConvChunk ? kCin : kConvChunk) * (9 * C + kHin * ConvShape<kHin>::row)) * 4;
+}
+
+// Heads, losses and their gradient (a block per sample): labels part [N] (-1 none), i4 [N][16] (raster
+// 4x4 blocks, -1 none), mv [N][2] with mvv [N] (0 none); scales: train_prep_kernel's. Writes the logits
+// (optional), the sample's part of the loss and of the head parameters' gradients (loss_part [N],
+// head_part [N][kHeadParams]) and dA3 (the gradient at the conv3 map, masked by its ReLU).
+constexpr int kHeadThreads = 256, kHeadRow = 325;
+__global__ void __launch_bounds__(kHeadThreads) heads_kernel(const float* __restrict__ A3, const float* __restrict__ P, const int* __restrict__ part,
+                             const int* __restrict__ i4, const float* __restrict__ mv, const int* __restrict__ mvv,
+                             const float* __restrict__ scales, float mv_weight, float* __restrict__ logits,
+                             float* __restrict__ head_part, float* __restrict__ dA3, float* __restrict__ loss_part) {
+  extern __shared__ float4 sh4[];
+  float* a = (float*)sh4;  // [32][kHeadRow]
+  __shared__ float H[kHeadParams], f[17][C], rows[8][C], lg[kLogits], dl[kLogits], dg[C], df[16][C], lsum[18];
+  const int n = blockIdx.x, t = threadIdx.x, c = t & 31, q = t >> 5;
+  const float* src = A3 + (size_t)n * kA3;
+  for (int i = t; i < kA3; i += kHeadThreads) a[(i / 324) * kHeadRow + i % 324] = src[i];
+  for (int i = t; i < kHeadParams; i += kHeadThreads) H[i] = P[kWp + i];
+  for (int i = t; i < kLogits; i += kHeadThreads) dl[i] = 0.0f;
+  if (t < 18) lsum[t] = 0.0f;
+  __syncthreads();
+  // pooling: warp q sums blocks 2q and 2q + 1, and the rows q, q + 8, q + 16 of the whole map
+  const float* m = a + c * kHeadRow;
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    const int b = 2 * q + k;
+    float s = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 16; i++) s += m[((b >> 2) * 4 + 1 + (i >> 2)) * 18 + (b & 3) * 4 + 1 + (i & 3)];
+    f[1 + b][c] = s / 16.0f;
+  }
+  float s = 0.0f;
+  for (int r = q; r < 18; r += 8)
+#pragma unroll
+    for (int i = 0; i < 18; i++) s += m[r * 18 + i];
+  rows[q][c] = s;
+  __syncthreads();
+  if (t < C) {
+    float all = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 8; k++) all += rows[k][t];
+    f[0][t] = all / 324.0f;
   }
   __syncthreads();
-  if (c == 0) {
-    float L = 0.0f;
-    for (int k = 0; k < 17; k++) L += lsum[k];
-    atomicAdd(loss, L);
+  if (t < kLogits) {  // partition 4, offset 2, intra 4x4 9 per block
+    const int b = t < 6 ? 0 : 1 + (t - 6) / 9, o = t < 4 ? t : (t < 6 ? t - 4 : (t - 6) % 9);
+    const int wo = t < 4 ? 0 : (t < 6 ? kWm - kWp : kWi - kWp), bo = t < 4 ? kBp - kWp : (t < 6 ? kBm - kWp : kBi - kWp);
+    float v = H[bo + o];
+#pragma unroll
+    for (int k = 0; k < C; k++) v += H[wo + o * C + k] * f[b][k];
+    lg[t] = v;
+    if (logits) logits[(size_t)n * kLogits + t] = v;
   }
-  for (int o = c; o < kLogits; o += C) dlog[(size_t)n * kLogits + o] = dl[o];
+  __syncthreads();
+  const float sp = scales[0], si = scales[1], sm = scales[2];
+  if (t == 0 && part[n] >= 0) {
+    const float mx = fmaxf(fmaxf(lg[0], lg[1]), fmaxf(lg[2], lg[3]));
+    float se = 0.0f;
+    for (int o = 0; o < 4; o++) se += expf(lg[o] - mx);
+    for (int o = 0; o < 4; o++) dl[o] = sp * (expf(lg[o] - mx) / se - (o == part[n] ? 1.0f : 0.0f));
+    lsum[16] = sp * (logf(se) + mx - lg[part[n]]);
+  }
+  if (t == 32 && mvv[n]) {  // Huber (delta 1) on the offset in units of 16 quarter samples
+    float L = 0.0f;
+    for (int o = 0; o < 2; o++) {
+      const float d = lg[4 + o] - mv[2 * n + o], ad = fabsf(d);
+      L += sm * mv_weight * (ad <= 1.0f ? 0.5f * d * d : ad - 0.5f);
+      dl[4 + o] = sm * mv_weight * (ad <= 1.0f ? d : (d > 0 ? 1.0f : -1.0f));
+    }
+    lsum[17] = L;
+  }
+  if (t >= 64 && t < 80) {
+    const int b = t - 64, lab = i4[n * 16 + b];
+    if (lab >= 0) {
+      const float* li = lg + 6 + b * 9;
+      float mx = li[0], se = 0.0f;
+      for (int o = 1; o < 9; o++) mx = fmaxf(mx, li[o]);
+      for (int o = 0; o < 9; o++) se += expf(li[o] - mx);
+      for (int o = 0; o < 9; o++) dl[6 + b * 9 + o] = si * (expf(li[o] - mx) / se - (o == lab ? 1.0f : 0.0f));
+      lsum[b] = si * (logf(se) + mx - li[lab]);
+    }
+  }
+  __syncthreads();
+  if (t == 0) {
+    float L = 0.0f;
+    for (int k = 0; k < 18; k++) L += lsum[k];
+    loss_part[n] = L;
+  }
+  // this sample's part of the head parameters' gradients
+  for (int e = t; e < kHeadParams; e += kHeadThreads) {
+    const int p = kWp + e;
+    float g = 0.0f;
+    if (p < kBp) g = dl[e / C] * f[0][e % C];
+    else if (p < kWm) g = dl[p - kBp];
+    else if (p < kBm) g = dl[4 + (p - kWm) / C] * f[0][(p - kWm) % C];
+    else if (p < kWi) g = dl[4 + p - kBm];
+    else if (p < kBi)
+      for (int b = 0; b < 16; b++) g += dl[6 + b * 9 + (p - kWi) / C] * f[1 + b][(p - kWi) % C];
+    else
+      for (int b = 0; b < 16; b++) g += dl[6 + b * 9 + p - kBi];
+    head_part[(size_t)n * kHeadParams + e] = g;
+  }
   // the gradient at the pooled features
-  float dgc = 0.0f;
-  for (int o = 0; o < 4; o++) dgc += P[kWp + o * C + c] * dl[o];
-  for (int o = 0; o < 2; o++) dgc += P[kWm + o * C + c] * dl[4 + o];
-  dg[c] = dgc;
-  for (int b = 0; b < 16; b++) {
-    float d = 0.0f;
-    for (int o = 0; o < 9; o++) d += P[kWi + o * C + c] * dl[6 + b * 9 + o];
-    df[b][c] = d;
+  if (t < C) {
+    float g = 0.0f;
+    for (int o = 0; o < 4; o++) g += H[o * C + t] * dl[o];
+    for (int o = 0; o < 2; o++) g += H[kWm - kWp + o * C + t] * dl[4 + o];
+    dg[t] = g / 324.0f;
+  }
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    const int b = 2 * q + k;
+    float g = 0.0f;
+    for (int o = 0; o < 9; o++) g += H[kWi - kWp + o * C + c] * dl[6 + b * 9 + o];
+    df[b][c] = g / 16.0f;
   }
   __syncthreads();
   // dA3 = pooled gradients spread over the map, masked by the ReLU
-  float* d = dA3 + (size_t)n * kA3 + c * 324;
-  for (int r = 0; r < 18; r++)
-    for (int i = 0; i < 18; i++) {
-      float v = dg[c] / 324.0f;
-      if (r >= 1 && r <= 16 && i >= 1 && i <= 16) v += df[((r - 1) >> 2) * 4 + ((i - 1) >> 2)][c] / 16.0f;
-      d[r * 18 + i] = a[r * 18 + i] > 0.0f ? v : 0.0f;
-    }
+  float* d = dA3 + (size_t)n * kA3;
+  for (int i = t; i < kA3; i += kHeadThreads) {
+    const int ch = i / 324, p = i % 324, r = p / 18, x = p % 18;
+    float v = dg[ch];
+    if (r >= 1 && r <= 16 && x >= 1 && x <= 16) v += df[((r - 1) >> 2) * 4 + ((x - 1) >> 2)][ch];
+    d[i] = a[ch * kHeadRow + p] > 0.0f ? v : 0.0f;
+  }
 }
 
-// Head parameter gradients: one block per parameter of the heads (kParams - kWp of them), a
-// reduction over the samples (and the 16 blocks for the intra 4x4 head).
-__global__ void head_grad_kernel(const float* __restrict__ feat, const float* __restrict__ dlog, int n,
-                                 float* __restrict__ G) {
-  __shared__ float red[256];
-  const int e = blockIdx.x;  // index into the head parameters
-  float s = 0.0f;
-  for (int k = threadIdx.x; k < n * 16; k += blockDim.x) {
-    const int i = k / 16, b = k % 16;
-    const float* fi = feat + (size_t)i * 17 * C;
-    const float* di = dlog + (size_t)i * kLogits;
-    const int q = kWp + e;
-    if (q < kBp) { if (b == 0) s += di[(q - kWp) / C] * fi[(q - kWp) % C]; }
-    else if (q < kWm) { if (b == 0) s += di[q - kBp]; }
-    else if (q < kBm) { if (b == 0) s += di[4 + (q - kWm) / C] * fi[(q - kWm) % C]; }
-    else if (q < kWi) { if (b == 0) s += di[4 + q - kBm]; }
-    else if (q < kBi) s += di[6 + b * 9 + (q - kWi) / C] * fi[(1 + b) * C + (q - kWi) % C];
-    else s += di[6 + b * 9 + q - kBi];
-  }
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) G[kWp + e] = red[0];
-}
-
-// Gradient of a conv's input (one sample per block): din[ci][y][x] = sum over co, taps of
-// dout[co][y - dy][x - dx] W[co][ci][dy][dx], masked by the ReLU of the input map (act > 0).
-__global__ void conv_bwd_data_kernel(const float* __restrict__ dout, int hin, const float* __restrict__ P, int woff,
-                                     const float* __restrict__ act, float* __restrict__ din) {
+// Weight gradients of a 32 -> 32 layer, dW[co][ci][t] = sum over samples, positions of dout[co][p]
+// in[ci][p + t]: a block takes `per` samples one after the other, a thread 4 output channels x 9
+// taps of one input channel (its lane) over half of the rows: per 4 positions of a row three rows of
+// six samples and 4 x 4 gradients (the same for the whole warp) for 144 multiply-adds. Channel maps are
+// 20 banks apart (mod 32), which spreads the lanes' 16-byte loads over all banks. Partial sums, a row of
+// kWgRow per (block, half), added up by train_reduce_kernel; the bias gradients behind the weights of
+// half 0.
+constexpr int kWgRow = kW + C, kWgThreads = 512;
+template <int kHin>
+struct WgShape {
+  static constexpr int hout = kHin - 2, row = 24, map = kHin * row + (kHin * row % 32 == 16 ? 4 : 20), drow = 20, dmap = hout * drow;
+  static_assert(map % 32 == 20 || map % 32 == 12 || map % 32 == 4, "the lanes' maps fall into different banks");
+  static constexpr int smem = C * (map + dmap) * 4;
+};
+template <int kHin>
+__global__ void __launch_bounds__(kWgThreads, 1) wgrad_kernel(const float* __restrict__ dout, const float* __restrict__ in, int n_samples,
+                                                              int per, float* __restrict__ part) {
+  using S = WgShape<kHin>;
+  constexpr int hout = S::hout;
   extern __shared__ float4 sh4[];
-  float* sh = (float*)sh4;
-  const int n = blockIdx.x, hout = hin - 2, nout = C * hout * hout;
-  float* w = sh;              // [9][co][ci]
-  float* d = sh + C * C * 9;  // 32 * hout * hout
-  for (int i = threadIdx.x; i < nout; i += blockDim.x) d[i] = dout[(size_t)n * nout + i];
-  for (int i = threadIdx.x; i < C * C * 9; i += blockDim.x) {
-    const int co = i / (C * 9), ci = (i / 9) % C, t = i % 9;
-    w[(t * C + co) * C + ci] = P[woff + i];
+  float* x = (float*)sh4;        // [32][map]: rows of 24
+  float* d = x + C * S::map;     // [32][hout][20], columns past hout zero
+  const int tid = threadIdx.x, lane = tid & 31, cg = (tid >> 5) & 7, half = tid >> 8;
+  const int y0 = half ? hout / 2 : 0, y1 = half ? hout : hout / 2;
+  float acc[4][9];
+#pragma unroll
+  for (int o = 0; o < 4; o++)
+#pragma unroll
+    for (int t = 0; t < 9; t++) acc[o][t] = 0.0f;
+  float bsum = 0.0f;
+  for (int s = 0; s < per; s++) {
+    const int n = blockIdx.x * per + s;
+    if (n >= n_samples) break;
+    __syncthreads();
+    for (int i = tid; i < C * kHin * kHin; i += kWgThreads) {
+      const int ci = i / (kHin * kHin), p = i - ci * kHin * kHin, r = p / kHin;
+      x[ci * S::map + r * S::row + p - r * kHin] = in[(size_t)n * C * kHin * kHin + i];
+    }
+    for (int i = tid; i < C * S::dmap; i += kWgThreads) {
+      const int r = i / S::drow, c = i - r * S::drow;
+      d[i] = c < hout ? dout[((size_t)n * C * hout + r) * hout + c] : 0.0f;
+    }
+    if (kHin < 24)  // the columns past the map, multiplied with zero gradients
+      for (int i = tid; i < C * kHin * (24 - kHin); i += kWgThreads) {
+        const int r = i / (24 - kHin);
+        x[(r / kHin) * S::map + (r % kHin) * S::row + kHin + i % (24 - kHin)] = 0.0f;
+      }
+    __syncthreads();
+    const float* xc = x + lane * S::map;
+    const float* dc = d + cg * 4 * S::dmap;
+#pragma unroll 1
+    for (int y = y0; y < y1; y++)
+#pragma unroll 1
+      for (int g = 0; g < 5; g++) {
+        float4 dv[4];
+#pragma unroll
+        for (int o = 0; o < 4; o++) dv[o] = *(const float4*)(dc + o * S::dmap + y * S::drow + 4 * g);
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
+          const float4 a = *(const float4*)(xc + (y + r) * S::row + 4 * g);
+          const float2 b = *(const float2*)(xc + (y + r) * S::row + 4 * g + 4);
+          const float v[6] = {a.x, a.y, a.z, a.w, b.x, b.y};
+#pragma unroll
+          for (int t = 0; t < 3; t++)
+#pragma unroll
+            for (int o = 0; o < 4; o++) {
+              acc[o][r * 3 + t] = fmaf(dv[o].x, v[t], acc[o][r * 3 + t]);
+              acc[o][r * 3 + t] = fmaf(dv[o].y, v[t + 1], acc[o][r * 3 + t]);
+              acc[o][r * 3 + t] = fmaf(dv[o].z, v[t + 2], acc[o][r * 3 + t]);
+              acc[o][r * 3 + t] = fmaf(dv[o].w, v[t + 3], acc[o][r * 3 + t]);
+            }
+        }
+      }
+    // bias: sixteen threads a channel
+    for (int i = tid & 15; i < S::dmap; i += 16) bsum += d[(tid >> 4) * S::dmap + i];
   }
-  __syncthreads();
-  const int npos = hin * hin;
-  for (int p = threadIdx.x; p < npos; p += blockDim.x) {
-    const int y = p / hin, x = p % hin;
-    float acc[C];
+  float* row = part + ((size_t)blockIdx.x * 2 + half) * kWgRow;
 #pragma unroll
-    for (int ci = 0; ci < C; ci++) acc[ci] = 0.0f;
-    for (int t = 0; t < 9; t++) {
-      const int oy = y - t / 3, ox = x - t % 3;
-      if (oy < 0 || oy >= hout || ox < 0 || ox >= hout) continue;
-      for (int co = 0; co < C; co++) {
-        const float g = d[(co * hout + oy) * hout + ox];
-        const float4* wv = (const float4*)&w[(t * C + co) * C];
+  for (int o = 0; o < 4; o++)
 #pragma unroll
-        for (int c4 = 0; c4 < C / 4; c4++) {
-          const float4 q = wv[c4];
-          acc[4 * c4] += q.x * g; acc[4 * c4 + 1] += q.y * g; acc[4 * c4 + 2] += q.z * g; acc[4 * c4 + 3] += q.w * g;
+    for (int t = 0; t < 9; t++) row[((cg * 4 + o) * C + lane) * 9 + t] = acc[o][t];
+#pragma unroll
+  for (int o = 1; o < 16; o <<= 1) bsum += __shfl_xor_sync(0xffffffffu, bsum, o);
+  float* row0 = part + (size_t)blockIdx.x * 2 * kWgRow;
+  if ((tid & 15) == 0) {
+    row0[kW + (tid >> 4)] = bsum;
+    row0[kWgRow + kW + (tid >> 4)] = 0.0f;
+  }
+}
+// The first layer's: warp = (4 output channels, input channel), lane = row of the map, its sums over
+// the row's positions, then over the lanes. A row of kWg1Row per block: the weights, then the biases.
+constexpr int kWg1Row = 2 * 9 * C + C, kWg1D = 23, kWg1X = 25;
+constexpr int kWg1Smem = (C * 22 * kWg1D + 2 * 24 * kWg1X) * 4;
+__global__ void __launch_bounds__(kWgThreads, 1) wgrad1_kernel(const float* __restrict__ dout, const uint8_t* __restrict__ crops, int n_samples,
+                                                               int per, float* __restrict__ part) {
+  extern __shared__ float4 sh4[];
+  float* d = (float*)sh4;          // [32][22][23]
+  float* x = d + C * 22 * kWg1D;   // [2][24][25]
+  const int tid = threadIdx.x, lane = tid & 31, cg = (tid >> 5) & 7, ci = tid >> 8;
+  float acc[4][9], bacc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+  for (int o = 0; o < 4; o++)
+#pragma unroll
+    for (int t = 0; t < 9; t++) acc[o][t] = 0.0f;
+  for (int s = 0; s < per; s++) {
+    const int n = blockIdx.x * per + s;
+    if (n >= n_samples) break;
+    __syncthreads();
+    for (int i = tid; i < kA1; i += kWgThreads) d[(i / 22) * kWg1D + i % 22] = dout[(size_t)n * kA1 + i];
+    for (int i = tid; i < kIn; i += kWgThreads) x[(i / 24) * kWg1X + i % 24] = pix_norm(crops[(size_t)n * kIn + i]);
+    __syncthreads();
+    if (lane < 22) {
+      const float* xr = x + (ci * 24 + lane) * kWg1X;
+      const float* dr = d + (cg * 4 * 22 + lane) * kWg1D;
+#pragma unroll 2
+      for (int p = 0; p < 22; p++) {
+        float v[9];
+#pragma unroll
+        for (int t = 0; t < 9; t++) v[t] = xr[(t / 3) * kWg1X + p + t % 3];
+#pragma unroll
+        for (int o = 0; o < 4; o++) {
+          const float g = dr[o * 22 * kWg1D + p];
+          bacc[o] += g;
+#pragma unroll
+          for (int t = 0; t < 9; t++) acc[o][t] = fmaf(g, v[t], acc[o][t]);
         }
       }
     }
+  }
+  float* row = part + (size_t)blockIdx.x * kWg1Row;
 #pragma unroll
-    for (int ci = 0; ci < C; ci++) {
-      const size_t i = (size_t)n * C * npos + ci * npos + p;
-      din[i] = act[i] > 0.0f ? acc[ci] : 0.0f;
+  for (int o = 0; o < 4; o++) {
+#pragma unroll
+    for (int t = 0; t < 9; t++) {
+      float v = acc[o][t];
+#pragma unroll
+      for (int k = 16; k > 0; k >>= 1) v += __shfl_xor_sync(0xffffffffu, v, k);
+      if (lane == 0) row[((cg * 4 + o) * 2 + ci) * 9 + t] = v;
     }
+    float v = bacc[o];
+#pragma unroll
+    for (int k = 16; k > 0; k >>= 1) v += __shfl_xor_sync(0xffffffffu, v, k);
+    if (lane == 0 && ci == 0) row[2 * 9 * C + cg * 4 + o] = v;
   }
 }
-
-// Gradient of a conv's weights and bias over a group of samples per block (atomic into G):
-// dW[co][ci][t] = sum over samples, positions of dout[co][p] in[ci][p + t].
-__global__ void conv_bwd_weight_kernel(const float* __restrict__ dout, const uint8_t* __restrict__ u8,
-                                       const float* __restrict__ in, int cin, int hin, int n_samples, int per_block,
-                                       int woff, int boff, float* __restrict__ G) {
-  extern __shared__ float sh[];
-  const int hout = hin - 2, nout = C * hout * hout, nin = cin * hin * hin, nw = C * cin * 9;
-  float* d = sh;
-  float* x = sh + nout;
-  float acc[36];  // nw / blockDim.x entries per thread (blockDim.x = 256: up to 9216 / 256)
-  const int per = (nw + blockDim.x - 1) / blockDim.x;
-  for (int k = 0; k < 36; k++) acc[k] = 0.0f;
-  float bacc = 0.0f;
-  for (int s = 0; s < per_block; s++) {
-    const int n = blockIdx.x * per_block + s;
-    if (n >= n_samples) break;
-    __syncthreads();
-    for (int i = threadIdx.x; i < nout; i += blockDim.x) d[i] = dout[(size_t)n * nout + i];
-    for (int i = threadIdx.x; i < nin; i += blockDim.x) x[i] = u8 ? pix_norm(u8[(size_t)n * nin + i]) : in[(size_t)n * nin + i];
-    __syncthreads();
-    for (int k = 0; k < per; k++) {
-      const int e = threadIdx.x + k * blockDim.x;
-      if (e >= nw) break;
-      const int co = e / (cin * 9), ci = (e / 9) % cin, t = e % 9;
-      const float* dp = d + co * hout * hout;
-      const float* xp = x + ci * hin * hin + (t / 3) * hin + t % 3;
-      float s2 = 0.0f;
-      for (int y = 0; y < hout; y++)
-        for (int xx = 0; xx < hout; xx++) s2 += dp[y * hout + xx] * xp[y * hin + xx];
-      acc[k] += s2;
-    }
-    if (threadIdx.x < C) {
-      const float* dp = d + threadIdx.x * hout * hout;
-      for (int i = 0; i < hout * hout; i++) bacc += dp[i];
-    }
+// The gradients: parameter e's partial sums over the blocks (or samples) that made them; the last one
+// is the loss. 32 parameters a block, eight strided parts of the rows each.
+struct TrainParts {
+  const float *w1, *w2, *w3, *head, *loss;
+  int n1, n2, n;  // rows of w1, of w2 and w3, of head and loss
+};
+__global__ void __launch_bounds__(256) train_reduce_kernel(TrainParts tp, float* __restrict__ G, float* __restrict__ loss) {
+  __shared__ float red[8][32];
+  const int e = blockIdx.x * 32 + (threadIdx.x & 31), q = threadIdx.x >> 5;
+  const float* p = nullptr;
+  int rows = 0, stride = 0;
+  if (e < kW2) { p = tp.w1 + e; rows = tp.n1; stride = kWg1Row; }
+  else if (e < kW3) { p = tp.w2 + e - kW2; rows = tp.n2; stride = kWgRow; }
+  else if (e < kWp) { p = tp.w3 + e - kW3; rows = tp.n2; stride = kWgRow; }
+  else if (e < kParams) { p = tp.head + e - kWp; rows = tp.n; stride = kHeadParams; }
+  else if (e == kParams) { p = tp.loss; rows = tp.n; stride = 1; }
+  float s = 0.0f;
+#pragma unroll 4
+  for (int r = q; r < rows; r += 8) s += p[(size_t)r * stride];
+  red[q][threadIdx.x & 31] = s;
+  __syncthreads();
+  if (q == 0) {
+    s = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 8; k++) s += red[k][threadIdx.x];
+    if (e < kParams) G[e] = s;
+    else if (e == kParams) *loss = s;
   }
-  for (int k = 0; k < per; k++) {
-    const int e = threadIdx.x + k * blockDim.x;
-    if (e < nw) atomicAdd(&G[woff + e], acc[k]);
-  }
-  if (threadIdx.x < C) atomicAdd(&G[boff + threadIdx.x], bacc);
 }
+static_assert(kW2 - kW1 == kWg1Row && kW3 - kW2 == kWgRow && kWp - kW3 == kWgRow && kW1 == 0, "partial rows in the parameters' order");
 
 __global__ void adam_kernel(float* P, const float* G, float* m, float* v, int n, float lr, float b1, float b2,
                             float eps, float c1, float c2) {
@@ -796,7 +965,7 @@ struct rg_net {
   int* counter = nullptr;  // [0] strip ticket, [1] error word
   // training scratch
   float *a1 = nullptr, *a2 = nullptr, *a3 = nullptr, *d3 = nullptr, *d2 = nullptr, *d1 = nullptr, *loss = nullptr;
-  float *feat = nullptr, *dlog = nullptr;
+  float *trans = nullptr, *parts = nullptr;  // transposed weights and scales; partial sums of the gradients
   int cap = 0;
   InferJob* jobs = nullptr;
   int jobs_cap = 0;
@@ -847,20 +1016,41 @@ int ensure_bops(rg_net* net) {
   net->bops_stale = false;
   return RG_OK;
 }
+// Samples of one block of the weight-gradient kernels: the batch spread over the SMs.
+int wgrad_per(int n, int sms) { return (n + sms - 1) / sms; }
+// Floats of the partial sums of n samples (at most n blocks of the weight-gradient kernels).
+size_t parts_floats(size_t n) { return n * (kWg1Row + 2 * 2 * (size_t)kWgRow + kHeadParams + 1); }
 int ensure_train(rg_net* net, int n) {
   if (n <= net->cap) return RG_OK;
   cudaFree(net->a1); cudaFree(net->a2); cudaFree(net->a3); cudaFree(net->d3); cudaFree(net->d2); cudaFree(net->d1);
-  cudaFree(net->feat); cudaFree(net->dlog);
+  cudaFree(net->parts);
+  net->a1 = net->a2 = net->a3 = net->d3 = net->d2 = net->d1 = net->parts = nullptr;
+  net->cap = 0;
   size_t f = sizeof(float);
-  if (cudaMalloc((void**)&net->feat, f * n * 17 * C) != cudaSuccess || cudaMalloc((void**)&net->dlog, f * n * kLogits) != cudaSuccess ||
+  if ((!net->trans && cudaMalloc((void**)&net->trans, f * (kTrans + 4)) != cudaSuccess) ||
+      cudaMalloc((void**)&net->parts, f * parts_floats(n)) != cudaSuccess ||
       cudaMalloc((void**)&net->a1, f * n * kA1) != cudaSuccess || cudaMalloc((void**)&net->a2, f * n * kA2) != cudaSuccess ||
       cudaMalloc((void**)&net->a3, f * n * kA3) != cudaSuccess || cudaMalloc((void**)&net->d3, f * n * kA3) != cudaSuccess ||
-      cudaMalloc((void**)&net->d2, f * n * kA2) != cudaSuccess || cudaMalloc((void**)&net->d1, f * n * kA1) != cudaSuccess) {
-    net->cap = 0;
+      cudaMalloc((void**)&net->d2, f * n * kA2) != cudaSuccess || cudaMalloc((void**)&net->d1, f * n * kA1) != cudaSuccess)
     return nfail(RG_ERR_OOM, "rg_net: training scratch allocation failed");
-  }
   net->cap = n;
   return RG_OK;
+}
+// One convolution layer of a training pass: a block per sample, its output channels over four blocks
+// when the samples alone do not fill the GPU.
+template <int kHin, int kCin, bool kU8, bool kBwd>
+void launch_conv(int n, int sms, const void* in, const float* wt, const float* bias, const float* act, float* out) {
+  constexpr int smem = conv_smem<kHin, kCin>();
+  cudaFuncSetAttribute(conv_kernel<kHin, kCin, kU8, kBwd>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  const int split = n >= sms ? 1 : (2 * n >= sms ? 2 : 4), cgs = 4 / split;
+  const int threads = (cgs * ConvShape<kHin>::threads + 31) / 32 * 32;
+  conv_kernel<kHin, kCin, kU8, kBwd><<<dim3(n, split), threads, smem>>>(in, wt, bias, act, out, cgs);
+}
+template <int kHin>
+void launch_wgrad(int n, int per, const float* dout, const float* in, float* part) {
+  constexpr int smem = WgShape<kHin>::smem;
+  cudaFuncSetAttribute(wgrad_kernel<kHin>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  wgrad_kernel<kHin><<<(n + per - 1) / per, kWgThreads, smem>>>(dout, in, n, per, part);
 }
 }  // namespace
 
@@ -907,7 +1097,7 @@ void rg_net_destroy(rg_net* net) {
   if (!net) return;
   cudaFree(net->P); cudaFree(net->G); cudaFree(net->M); cudaFree(net->V); cudaFree(net->bops); cudaFree(net->counter);
   cudaFree(net->a1); cudaFree(net->a2); cudaFree(net->a3); cudaFree(net->d3); cudaFree(net->d2); cudaFree(net->d1);
-  cudaFree(net->loss); cudaFree(net->jobs); cudaFree(net->feat); cudaFree(net->dlog);
+  cudaFree(net->loss); cudaFree(net->jobs); cudaFree(net->trans); cudaFree(net->parts);
   delete net;
 }
 
@@ -953,38 +1143,32 @@ int rg_net_forward_backward(rg_net* net, const uint8_t* dev_crops, int32_t n, co
   NCK(cudaSetDevice(net->device));
   int r = ensure_train(net, n);
   if (r) return r;
-  // label counts normalise each loss (host copies of the small label arrays)
-  std::vector<int32_t> part(n), i4((size_t)n * 16), mvv(n);
-  NCK(cudaMemcpy(part.data(), dev_part, sizeof(int32_t) * n, cudaMemcpyDeviceToHost));
-  NCK(cudaMemcpy(i4.data(), dev_i4, sizeof(int32_t) * n * 16, cudaMemcpyDeviceToHost));
-  NCK(cudaMemcpy(mvv.data(), dev_mvv, sizeof(int32_t) * n, cudaMemcpyDeviceToHost));
-  int np = 0, ni = 0, nm = 0;
-  for (int k = 0; k < n; k++) { np += part[k] >= 0; nm += mvv[k] != 0; }
-  for (size_t k = 0; k < i4.size(); k++) ni += i4[k] >= 0;
-  const float sp = np ? 1.0f / np : 0.0f, si = ni ? 1.0f / ni : 0.0f, sm = nm ? 1.0f / nm : 0.0f;
-  NCK(cudaMemset(net->G, 0, sizeof(float) * kParams));
-  NCK(cudaMemset(net->loss, 0, sizeof(float)));
-  const int th = 256;
-  auto attr = [](const void* k, int bytes) { cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); };
-  const int s1 = (2 * 24 * 24 + C * 2 * 9) * 4, s2 = (C * 22 * 22 + C * C * 9) * 4, s3 = (C * 20 * 20 + C * C * 9) * 4;
-  static_assert((C * 2 * 9) % 4 == 0, "input map after the weights stays 16-byte aligned");
-  attr((const void*)conv_fwd_kernel, s2);
-  conv_fwd_kernel<<<n, th, s1>>>(dev_crops, nullptr, 2, 24, net->P, kW1, kB1, net->a1);
-  conv_fwd_kernel<<<n, th, s2>>>(nullptr, net->a1, C, 22, net->P, kW2, kB2, net->a2);
-  conv_fwd_kernel<<<n, th, s3>>>(nullptr, net->a2, C, 20, net->P, kW3, kB3, net->a3);
-  heads_kernel<<<n, C>>>(net->a3, net->P, dev_part, dev_i4, dev_mv, dev_mvv, sp, si, sm, mv_weight, dev_logits,
-                         net->feat, net->dlog, net->d3, net->loss);
-  head_grad_kernel<<<kParams - kWp, 256>>>(net->feat, net->dlog, n, net->G);
-  const int sb3 = (C * 18 * 18 + C * C * 9) * 4, sb2 = (C * 20 * 20 + C * C * 9) * 4;
-  attr((const void*)conv_bwd_data_kernel, sb2);
-  conv_bwd_data_kernel<<<n, th, sb3>>>(net->d3, 20, net->P, kW3, net->a2, net->d2);
-  conv_bwd_data_kernel<<<n, th, sb2>>>(net->d2, 22, net->P, kW2, net->a1, net->d1);
-  const int per = 8, nb = (n + per - 1) / per;
-  const int w3 = (C * 18 * 18 + C * 20 * 20) * 4, w2 = (C * 20 * 20 + C * 22 * 22) * 4, w1 = (C * 22 * 22 + 2 * 24 * 24) * 4;
-  attr((const void*)conv_bwd_weight_kernel, w2);
-  conv_bwd_weight_kernel<<<nb, th, w3>>>(net->d3, nullptr, net->a2, C, 20, n, per, kW3, kB3, net->G);
-  conv_bwd_weight_kernel<<<nb, th, w2>>>(net->d2, nullptr, net->a1, C, 22, n, per, kW2, kB2, net->G);
-  conv_bwd_weight_kernel<<<nb, th, w1>>>(net->d1, dev_crops, nullptr, 2, 24, n, per, kW1, kB1, net->G);
+  int sms = 0;
+  NCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, net->device));
+  const float* P = net->P;
+  float *T = net->trans, *scales = T + kTrans;
+  // the labels' counts normalise each loss
+  train_prep_kernel<<<(kTrans + 255) / 256 + 1, 256>>>(P, T, dev_part, dev_i4, dev_mvv, n, scales);
+  launch_conv<24, 2, true, false>(n, sms, dev_crops, T + kT1, P + kB1, nullptr, net->a1);
+  launch_conv<22, C, false, false>(n, sms, net->a1, T + kT2, P + kB2, nullptr, net->a2);
+  launch_conv<20, C, false, false>(n, sms, net->a2, T + kT3, P + kB3, nullptr, net->a3);
+  const int per = wgrad_per(n, sms), nb = (n + per - 1) / per;
+  float* w1 = net->parts;
+  float* w2 = w1 + (size_t)nb * kWg1Row;
+  float* w3 = w2 + (size_t)nb * 2 * kWgRow;
+  float* head = w3 + (size_t)nb * 2 * kWgRow;
+  float* loss = head + (size_t)n * kHeadParams;
+  constexpr int hs = C * kHeadRow * 4;
+  cudaFuncSetAttribute(heads_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, hs);
+  heads_kernel<<<n, kHeadThreads, hs>>>(net->a3, P, dev_part, dev_i4, dev_mv, dev_mvv, scales, mv_weight, dev_logits, head,
+                                        net->d3, loss);
+  launch_conv<22, C, false, true>(n, sms, net->d3, T + kTb3, nullptr, net->a2, net->d2);
+  launch_conv<24, C, false, true>(n, sms, net->d2, T + kTb2, nullptr, net->a1, net->d1);
+  launch_wgrad<20>(n, per, net->d3, net->a2, w3);
+  launch_wgrad<22>(n, per, net->d2, net->a1, w2);
+  cudaFuncSetAttribute(wgrad1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWg1Smem);
+  wgrad1_kernel<<<nb, kWgThreads, kWg1Smem>>>(net->d1, dev_crops, n, per, w1);
+  train_reduce_kernel<<<(kParams + 1 + 31) / 32, 256>>>(TrainParts{w1, w2, w3, head, loss, nb, 2 * nb, n}, net->G, net->loss);
   NCK(cudaGetLastError());
   NCK(cudaDeviceSynchronize());
   if (loss_out) NCK(cudaMemcpy(loss_out, net->loss, sizeof(float), cudaMemcpyDeviceToHost));
