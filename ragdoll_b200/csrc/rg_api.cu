@@ -10,6 +10,7 @@
 #include <string>
 #include <array>
 #include <atomic>
+#include <mutex>
 #include <vector>
 
 #include "engine.h"
@@ -31,6 +32,10 @@ constexpr int kDefaultSeg = 1;
 // on the walk (-27.2 % at 0, -26.9 % at 2 and 64) while its speed does (760, 1008, 1105 frames/s).
 constexpr uint16_t kDefaultTypeBits[4] = {1, 16, 16, 40};
 constexpr int kDefaultWalk = 4;
+// The metrics' memory pool of each device (metrics_pool).
+std::mutex g_metrics_mu;
+cudaMemPool_t g_metrics_pools[64] = {};
+
 // Deblocking SMs: one in five takes the deblocking queue first (30 of 148). Measured on B200 with
 // 16 warps per SM, 1080p 8 x 15 launch: 25 SMs 52.3-53.2 ms, 30 51.4-52.3, 35-40 52.6-52.8
 // (at 7 warps per SM, before the IDR path got faster: 16 SMs 1326 frames/s, 20-30 1394-1417).
@@ -245,12 +250,6 @@ struct rg_ctx {
   std::vector<int> frames;         // frames analysed per stream
   std::vector<StreamQp> qps;       // QP of each stream (rg_set_stream_qp; default cfg.qp)
   // metrics scratch
-  float* m_rows = nullptr;
-  double* m_out = nullptr;
-  unsigned long long* m_sse = nullptr;
-  uint8_t* m_pyr = nullptr;
-  SsimJob* m_jobs = nullptr;
-  DecimateJob* m_djobs = nullptr;
   uint8_t* m_src = nullptr;
 
   uint8_t* pic_plane(int s, int slot_, int plane) const {
@@ -381,6 +380,11 @@ rg_ctx* rg_create(const rg_config* cfg) {
 void rg_destroy(rg_ctx* c) {
   if (!c) return;
   if (c->stream) cudaStreamSynchronize(c->stream);
+  {  // the metrics' idle memory goes back too
+    int dev = 0;
+    std::lock_guard<std::mutex> lock(g_metrics_mu);
+    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 && g_metrics_pools[dev]) cudaMemPoolTrimTo(g_metrics_pools[dev], 0);
+  }
   cudaFree(c->pics);
   cudaFree(c->infos);
   cudaFree(c->mv4s);
@@ -390,12 +394,6 @@ void rg_destroy(rg_ctx* c) {
   cudaFree(c->unf);
   cudaFree(c->d_streams[0]);
   cudaFree(c->d_streams[1]);
-  cudaFree(c->m_rows);
-  cudaFree(c->m_out);
-  cudaFree(c->m_sse);
-  cudaFree(c->m_pyr);
-  cudaFree(c->m_jobs);
-  cudaFree(c->m_djobs);
   cudaFree(c->m_src);
   cudaFree(c->counters);
   cudaFree(c->d_tasks);
@@ -1694,118 +1692,97 @@ struct PlanePair {
   int w, h;
 };
 
-// Evaluates SSIM of each pair, MS-SSIM of pairs with want_ms, SSE of all, on stream st.
+// The metrics' device memory, allocated and freed in stream order from a pool of the library per
+// device: it keeps at most kMetricsKeep bytes between calls (a call's scratch costs its size in page
+// mappings otherwise: six cudaMalloc / cudaFree were about 1 ms of a call), and CUDA hands a block to
+// another stream or thread only after the work that used it.
+constexpr uint64_t kMetricsKeep = 128ull << 20;
+cudaMemPool_t metrics_pool() {
+  cudaMemPool_t* const pools = g_metrics_pools;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+  std::lock_guard<std::mutex> lock(g_metrics_mu);
+  if (!pools[dev]) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    uint64_t keep = kMetricsKeep;
+    cudaMemPool_t p = nullptr;
+    if (cudaMemPoolCreate(&p, &props) != cudaSuccess) return nullptr;
+    cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
+    pools[dev] = p;
+  }
+  return pools[dev];
+}
+
+// Evaluates SSIM of each pair, MS-SSIM of pairs with want_ms, and (sse not null) the squared error of
+// all, on stream st.
 int device_metrics(const std::vector<PlanePair>& pairs, const std::vector<bool>& want_ms, cudaStream_t st,
-                   std::vector<double>& ssim, std::vector<double>& ms, std::vector<unsigned long long>& sse) {
-  int n = (int)pairs.size();
-  // pyramid levels of the MS-SSIM pairs
-  std::vector<SsimJob> jobs;
-  std::vector<DecimateJob> djobs_per_level[4];
-  std::vector<int> level_count(n, 1);
-  size_t rows_total = 0, pyr_total = 0;
-  for (int i = 0; i < n; i++) {
-    rows_total += pairs[i].h / 4 + 1;
-    if (want_ms[i]) {
-      int w = pairs[i].w, h = pairs[i].h;
-      for (int l = 1; l < 5; l++) {
-        w >>= 1; h >>= 1;
-        if (w < 8 || h < 8) break;
-        pyr_total += 2 * (size_t)w * h;
-        rows_total += h / 4 + 1;
-        level_count[i]++;
-      }
-    }
-  }
-  float* rows = nullptr;
-  double* outs = nullptr;
-  unsigned long long* sses = nullptr;
-  uint8_t* pyr = nullptr;
-  SsimJob* d_jobs = nullptr;
-  DecimateJob* d_djobs = nullptr;
-  int total_jobs = 0;
-  for (int i = 0; i < n; i++) total_jobs += want_ms[i] ? level_count[i] : 1;
-  auto cleanup = [&]() {
-    cudaFree(rows); cudaFree(outs); cudaFree(sses); cudaFree(pyr); cudaFree(d_jobs); cudaFree(d_djobs);
-  };
-  if (cudaMalloc(&rows, rows_total * sizeof(float) + 16) != cudaSuccess ||
-      cudaMalloc(&outs, total_jobs * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&sses, n * sizeof(unsigned long long)) != cudaSuccess ||
-      cudaMalloc(&pyr, pyr_total + 16) != cudaSuccess || cudaMalloc(&d_jobs, total_jobs * sizeof(SsimJob)) != cudaSuccess ||
-      cudaMalloc(&d_djobs, (4 * n + 1) * sizeof(DecimateJob)) != cudaSuccess) {
-    cleanup();
-    return fail(RG_ERR_OOM, "metrics: device allocation failed");
-  }
-  cudaMemsetAsync(sses, 0, n * sizeof(unsigned long long), st);
-  size_t rofs = 0, pofs = 0;
-  int maxw = 0, maxh = 0;
-  std::vector<int> job_of(n * 5, -1);
-  // the n full-size planes first (jobs 0..n-1: the SSE launch reads those), pyramid levels after
+                   std::vector<double>& ssim, std::vector<double>& ms, std::vector<unsigned long long>* sse) {
+  const int n = (int)pairs.size();
+  // one block of device memory: descriptors | results (f64 per level, then the squared errors) | rows |
+  // pyramids
+  const size_t pair_bytes = ssim_pair_bytes();
+  std::vector<uint8_t> host(n * (pair_bytes + sizeof(SseJob)));
+  std::vector<SsimSizes> sizes(n);
+  size_t rows = 0, pyramid = 0;
+  bool any_ms = false;
+  int maxh = 0;
   for (int i = 0; i < n; i++) {
     const PlanePair& p = pairs[i];
-    SsimJob j{p.a, p.b, p.sa, p.sb, p.w, p.h, rows + rofs, outs + jobs.size(), sses + i};
-    rofs += p.h / 4 + 1;
-    job_of[i * 5] = (int)jobs.size();
-    jobs.push_back(j);
-    maxw = std::max(maxw, p.w);
+    ssim_pair_fill(host.data() + i * pair_bytes, p.a, p.sa, p.b, p.sb, p.w, p.h, want_ms[i], nullptr, nullptr, nullptr, sizes[i]);
+    rows += sizes[i].rows;
+    pyramid += sizes[i].pyramid;
+    any_ms |= sizes[i].levels > 1;
     maxh = std::max(maxh, p.h);
   }
+  auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
+  const size_t o_out = up(host.size()), n_out = (size_t)n * 5 + n, o_rows = o_out + up(n_out * 8), o_pyr = o_rows + up(rows * 4);
+  uint8_t* d = nullptr;
+  cudaMemPool_t pool = metrics_pool();
+  if (!pool || cudaMallocFromPoolAsync((void**)&d, o_pyr + pyramid + 16, pool, st) != cudaSuccess) {
+    cudaGetLastError();
+    return fail(RG_ERR_OOM, "metrics: device allocation of %zu bytes failed", o_pyr + pyramid);
+  }
+  double* outs = (double*)(d + o_out);
+  unsigned long long* sses = (unsigned long long*)(outs + (size_t)n * 5);
+  size_t rofs = 0, pofs = 0;
+  SseJob* jobs = (SseJob*)(host.data() + n * pair_bytes);
   for (int i = 0; i < n; i++) {
     const PlanePair& p = pairs[i];
-    if (want_ms[i]) {
-      const uint8_t* sa = p.a;
-      const uint8_t* sb = p.b;
-      long ssa = p.sa, ssb = p.sb;
-      int w = p.w, h = p.h;
-      for (int l = 1; l < level_count[i]; l++) {
-        int nw = w >> 1, nh = h >> 1;
-        uint8_t* da = pyr + pofs;
-        uint8_t* db = da + (size_t)nw * nh;
-        pofs += 2 * (size_t)nw * nh;
-        djobs_per_level[l - 1].push_back(DecimateJob{sa, sb, ssa, ssb, w, h, da, db});
-        SsimJob jl{da, db, nw, nw, nw, nh, rows + rofs, outs + jobs.size(), nullptr};
-        rofs += nh / 4 + 1;
-        job_of[i * 5 + l] = (int)jobs.size();
-        jobs.push_back(jl);
-        sa = da; sb = db; ssa = nw; ssb = nw; w = nw; h = nh;
-      }
-    }
+    ssim_pair_fill(host.data() + i * pair_bytes, p.a, p.sa, p.b, p.sb, p.w, p.h, want_ms[i], (float*)(d + o_rows) + rofs,
+                   outs + (size_t)i * 5, d + o_pyr + pofs, sizes[i]);
+    rofs += sizes[i].rows;
+    pofs += sizes[i].pyramid;
+    jobs[i] = SseJob{p.a, p.b, p.sa, p.sb, p.w, p.h, sses + i};
   }
-  // decimation levels in order, then every SSIM job in one launch
-  std::vector<DecimateJob> all_d;
-  std::vector<int> dofs;
-  for (int l = 0; l < 4; l++) {
-    dofs.push_back((int)all_d.size());
-    all_d.insert(all_d.end(), djobs_per_level[l].begin(), djobs_per_level[l].end());
+  std::vector<uint64_t> res(n_out);
+  cudaError_t e = cudaMemcpyAsync(d, host.data(), host.size(), cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess && sse) e = cudaMemsetAsync(sses, 0, n * sizeof(unsigned long long), st);
+  if (e == cudaSuccess) {
+    launch_ssim(d, n, maxh, any_ms, st);
+    if (sse) launch_sse((const SseJob*)(d + n * pair_bytes), n, st);
+    e = cudaGetLastError();
   }
-  if (!all_d.empty()) CK(cudaMemcpyAsync(d_djobs, all_d.data(), all_d.size() * sizeof(DecimateJob), cudaMemcpyHostToDevice, st));
-  CK(cudaMemcpyAsync(d_jobs, jobs.data(), jobs.size() * sizeof(SsimJob), cudaMemcpyHostToDevice, st));
-  for (int l = 0; l < 4; l++) {
-    int cnt = (int)djobs_per_level[l].size();
-    if (!cnt) continue;
-    int maxpix = 0;
-    for (auto& d : djobs_per_level[l]) maxpix = std::max(maxpix, (d.src_w >> 1) * (d.src_h >> 1));
-    launch_decimate(d_djobs + dofs[l], cnt, maxpix, st);
-  }
-  launch_ssim(d_jobs, (int)jobs.size(), maxw, maxh, st);
-  launch_sse(d_jobs, n, st);
-  std::vector<double> res(jobs.size());
-  sse.assign(n, 0);
-  CK(cudaMemcpyAsync(res.data(), outs, jobs.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
-  CK(cudaMemcpyAsync(sse.data(), sses, n * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-  cudaError_t e = cudaStreamSynchronize(st);
-  cleanup();
+  if (e == cudaSuccess) e = cudaMemcpyAsync(res.data(), outs, n_out * 8, cudaMemcpyDeviceToHost, st);
+  cudaFreeAsync(d, st);
+  cudaError_t e2 = cudaStreamSynchronize(st);
+  if (e == cudaSuccess) e = e2;
   if (e != cudaSuccess) return fail(RG_ERR_CUDA, "metrics: %s", cudaGetErrorString(e));
+  const double* r = (const double*)res.data();
   ssim.assign(n, 0.0);
   ms.assign(n, 0.0);
+  if (sse) sse->assign((const unsigned long long*)res.data() + (size_t)n * 5, (const unsigned long long*)res.data() + n_out);
   for (int i = 0; i < n; i++) {
-    ssim[i] = res[job_of[i * 5]];
+    ssim[i] = r[(size_t)i * 5];
     if (!want_ms[i]) continue;
     // ms_ssim_plane_u8 (crates/ragdoll-pix/src/metrics.rs:154)
     double s0 = std::min(1.0, std::max(0.0, ssim[i]));
     if (std::fabs(1.0 - s0) < 1e-12 || (pairs[i].w >> 1) < 8 || (pairs[i].h >> 1) < 8) { ms[i] = s0; continue; }
     double scores[5] = {s0, s0, s0, s0, s0};
-    int active = level_count[i];
-    for (int l = 1; l < active; l++) scores[l] = std::min(1.0, std::max(0.0, res[job_of[i * 5 + l]]));
+    const int active = sizes[i].levels;
+    for (int l = 1; l < active; l++) scores[l] = std::min(1.0, std::max(0.0, r[(size_t)i * 5 + l]));
     double wsum = 0.0;
     for (int l = 0; l < active; l++) wsum += kMsWeights[l];
     double prod = 1.0;
@@ -1879,7 +1856,7 @@ int rg_quality_frame_prev(rg_ctx* c, int32_t s, const uint8_t* y, const uint8_t*
       {c->m_src + (size_t)w * h + (size_t)cw * ch, cw, c->pic_plane(s, par, 2), c->fp.stride_c, cw, ch}};
   std::vector<double> ss, ms;
   std::vector<unsigned long long> sse;
-  int r = device_metrics(pairs, {true, false, false}, c->stream, ss, ms, sse);
+  int r = device_metrics(pairs, {true, false, false}, c->stream, ss, ms, &sse);
   if (r) return r;
   q->ssim_y = ss[0];
   q->ssim_u = ss[1];
@@ -1951,8 +1928,7 @@ int rg_ssim_plane(int32_t device, const uint8_t* a, size_t stride_a, const uint8
     r = fail(RG_ERR_CUDA, "rg_ssim_plane: copy failed");
   } else {
     std::vector<double> ss, ms;
-    std::vector<unsigned long long> sse;
-    r = device_metrics({{d, width, d + n, width, width, height}}, {ms_ssim != nullptr}, st, ss, ms, sse);
+    r = device_metrics({{d, width, d + n, width, width, height}}, {ms_ssim != nullptr}, st, ss, ms, nullptr);
     if (!r) {
       if (ssim) *ssim = ss[0];
       if (ms_ssim) *ms_ssim = ms[0];
@@ -1977,8 +1953,7 @@ int rg_ssim_batch_device(int32_t device, const uint8_t* const* dev_a, const uint
     pairs.push_back({dev_a[i], (long)stride_a, dev_b[i], (long)stride_b, width, height});
   }
   std::vector<double> ss, ms;
-  std::vector<unsigned long long> sse;
-  int r = device_metrics(pairs, std::vector<bool>(n, ms_ssim != nullptr), (cudaStream_t)cuda_stream, ss, ms, sse);
+  int r = device_metrics(pairs, std::vector<bool>(n, ms_ssim != nullptr), (cudaStream_t)cuda_stream, ss, ms, nullptr);
   if (r) return r;
   for (int i = 0; i < n; i++) {
     if (ssim) ssim[i] = ss[i];
