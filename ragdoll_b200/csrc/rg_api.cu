@@ -11,6 +11,7 @@
 #include <array>
 #include <atomic>
 #include <mutex>
+#include <thread>
 #include <vector>
 
 #include "engine.h"
@@ -189,6 +190,7 @@ struct rg_ctx {
     int* h_reach = nullptr;              // mapped host: 1 + the reach its reference waits saw [2]
     cudaEvent_t done = nullptr;          // after the launch
     std::vector<const rg_mb_hint*> hints;  // learned form: [f][s] (empty otherwise)
+    bool flagged = false;                // the launch sets h_final as each picture's records are final
   };
   Pending pend[2];
   int pend_head = 0, pend_count = 0;
@@ -222,6 +224,11 @@ struct rg_ctx {
   GroupGraph g_graphs[2];
   int g_graph_next = 0;
   int64_t g_graph_captures = 0, g_graph_launches = 0;
+  // device-source calls (records in recs): per picture 1 once its records are final, in mapped host
+  // memory, and the stream rg_copy_records_gops copies them on meanwhile; made by the first such call
+  int* h_final = nullptr;
+  int* d_final = nullptr;
+  cudaStream_t f_out = nullptr;
   int* h_ready[2] = {nullptr, nullptr};  // mapped host memory: per picture, the launch seq once final
   int* d_ready[2] = {nullptr, nullptr};  // the same, as the device sees it
   int a_seq[2] = {0, 0}, a_frames[2] = {0, 0};
@@ -401,6 +408,8 @@ void rg_destroy(rg_ctx* c) {
   cudaFree(c->g_counters);
   cudaFree(c->g_dtasks);
   if (c->g_hstreams) cudaFreeHost(c->g_hstreams);
+  if (c->f_out) cudaStreamDestroy(c->f_out);
+  if (c->h_final) cudaFreeHost(c->h_final);
   if (c->g_done) cudaEventDestroy(c->g_done);
   for (auto& g : c->g_graphs)
     if (g.exec) cudaGraphExecDestroy(g.exec);
@@ -600,6 +609,26 @@ static void gop_desc(const rg_ctx* c, StreamDev& d, int f, int s, const uint8_t*
   d.ready = ready ? ready + f * S + s : nullptr;
 }
 
+// The context's record flags as the device sees them, cleared for the next launch (every earlier one
+// resolved); null where they cannot be had: the records are then copied after the launch.
+static int* final_flags(rg_ctx* c) {
+  const size_t n = sizeof(int) * (size_t)c->S * c->max_frames;
+  if (!c->h_final) {
+    if (!c->f_out && cudaStreamCreateWithFlags(&c->f_out, cudaStreamNonBlocking) != cudaSuccess) c->f_out = nullptr;
+    if (!c->f_out || cudaHostAlloc((void**)&c->h_final, n, cudaHostAllocMapped) != cudaSuccess) c->h_final = nullptr;
+    if (c->h_final && cudaHostGetDevicePointer((void**)&c->d_final, c->h_final, 0) != cudaSuccess) {
+      cudaFreeHost(c->h_final);
+      c->h_final = nullptr;
+    }
+    if (!c->h_final) {
+      cudaGetLastError();
+      return nullptr;
+    }
+  }
+  memset((void*)c->h_final, 0, n);
+  return c->d_final;
+}
+
 static int enqueue_gops(rg_ctx* c, const uint8_t* const* dev_planes, size_t stride_y, size_t stride_uv,
                         const int32_t* kinds, int32_t frames, rg_mb_out* rec_base, int* ready = nullptr, int seq = 0,
                         bool resolved = false, const CompactOut* co = nullptr) {
@@ -610,9 +639,12 @@ static int enqueue_gops(rg_ctx* c, const uint8_t* const* dev_planes, size_t stri
   if (stride_y < (size_t)c->cfg.width || stride_uv < (size_t)(c->cfg.width + 1) / 2)
     return fail(RG_ERR_INVALID, "rg_analyse_gops_device: stride too small");
   int S = c->S;
+  const bool flagged = !resolved;  // a call into recs: rg_copy_records_gops may copy while it runs
   if (!resolved) {
     int r = resolve_pending(c, false);
     if (r) return r;
+    ready = final_flags(c);
+    seq = 1;
   }
   for (int f = 0; f < frames; f++)
     for (int s = 0; s < S; s++) {
@@ -704,6 +736,7 @@ static int enqueue_gops(rg_ctx* c, const uint8_t* const* dev_planes, size_t stri
   p.out = nullptr;
   p.out_bytes = 0;
   p.hints = hv;
+  p.flagged = flagged && ready;
   c->pend_count++;
   for (int s = 0; s < S; s++) c->frames[s] += frames;
   return RG_OK;
@@ -741,10 +774,12 @@ static int group_launch(rg_ctx* const* ctxs, int32_t n, const uint8_t* const* co
     if (stride_y[i] < (size_t)c->cfg.width || stride_uv[i] < (size_t)(c->cfg.width + 1) / 2)
       return fail(RG_ERR_INVALID, "%s: stride too small (context %d)", who, i);
   }
+  std::vector<int*> finals(n, nullptr);  // calls into each context's recs: its record flags
   for (int i = 0; i < n; i++) {
     rg_ctx* c = ctxs[i];
     int r = resolved ? RG_OK : resolve_pending(c, false);
     if (r) return r;
+    if (!resolved) finals[i] = final_flags(c);
     for (int f = 0; f < frames; f++)
       for (int s = 0; s < c->S; s++) {
         const int k = kinds[i][f * c->S + s];
@@ -759,6 +794,10 @@ static int group_launch(rg_ctx* const* ctxs, int32_t n, const uint8_t* const* co
     c->hints.clear();
   }
   CK(cudaSetDevice(L->cfg.device));
+  if (!resolved) {
+    readies = finals.data();
+    seq = 1;
+  }
   // descriptors and rows of every context, one after the other, the contexts with more macroblocks
   // first whatever the argument order (64 streams of four sizes: 263 ms against 364 ms with the
   // smallest size's descriptors first)
@@ -974,6 +1013,7 @@ static int group_launch(rg_ctx* const* ctxs, int32_t n, const uint8_t* const* co
     p.out = nullptr;
     p.out_bytes = 0;
     p.hints.clear();
+    p.flagged = finals[i] != nullptr;
     c->pend_count++;
     for (int s = 0; s < c->S; s++) c->frames[s] += frames;
   }
@@ -1079,10 +1119,42 @@ int rg_group_graph_counts(const rg_ctx* c, int64_t* captures, int64_t* launches)
 int rg_copy_records_gops(rg_ctx* c, int32_t frames, rg_mb_out* out) {
   if (!c || !out) return fail(RG_ERR_INVALID, "rg_copy_records_gops: null argument");
   if (frames < 1 || frames > c->max_frames) return fail(RG_ERR_INVALID, "rg_copy_records_gops: frames %d", frames);
+  // A device-source call still running flags each picture as its records are final: those are copied
+  // while it goes on (1080p, 8 x 15, 870 MB: 38.6 ms for launch and copy one after the other, 25.7 so).
+  // copied: the leading pictures already in out; a call that had to be re-run leaves none.
+  int copied = 0;
+  if (c->pend_count == 1 && c->pend[c->pend_head].flagged) {
+    const rg_ctx::Pending& p = c->pend[c->pend_head];
+    const int n = std::min(frames, p.frames) * c->S;
+    cudaError_t e = cudaSuccess;
+    while (copied < n && e == cudaSuccess) {
+      const bool ended = cudaEventQuery(p.done) != cudaErrorNotReady;
+      int to = copied;  // a run of final pictures in order
+      while (to < n && *(volatile int*)(c->h_final + to) == 1) to++;
+      if (to > copied) {
+        std::atomic_thread_fence(std::memory_order_acquire);
+        e = cudaMemcpyAsync(out + (size_t)copied * c->n_mb, c->recs + (size_t)copied * c->n_mb,
+                            sizeof(rg_mb_out) * c->n_mb * (to - copied), cudaMemcpyDeviceToHost, c->f_out);
+        copied = to;
+      } else if (ended) {
+        break;
+      } else {
+        std::this_thread::yield();
+      }
+    }
+    const cudaError_t e2 = cudaStreamSynchronize(c->f_out);
+    if (e == cudaSuccess) e = e2;
+    if (e != cudaSuccess) return fail(RG_ERR_CUDA, "rg_copy_records_gops: %s", cudaGetErrorString(e));
+    CK(cudaEventSynchronize(p.done));
+    if (*(volatile int*)p.h_err) copied = 0;
+  }
   int r = rg_sync(c);  // completes (or re-runs) the pending call first
   if (r) return r;
-  CK(cudaMemcpyAsync(out, c->recs, sizeof(rg_mb_out) * c->n_mb * c->S * frames, cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
+  const size_t from = (size_t)copied * c->n_mb, to = (size_t)frames * c->S * c->n_mb;
+  if (from < to) {
+    CK(cudaMemcpyAsync(out + from, c->recs + from, sizeof(rg_mb_out) * (to - from), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+  }
   return RG_OK;
 }
 
