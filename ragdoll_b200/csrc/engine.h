@@ -75,6 +75,10 @@ struct StreamDev {
   // pipelined launches: this picture's ready flag in mapped host memory (null: the launch's
   // ready array at the descriptor's index, if any)
   int32_t* ready;
+  // pipelined launches of few pictures, plain form: per macroblock of this picture {vector, ref | 0x100}
+  // as soon as it is decided (null: none), and the previous picture's when it is of the same launch
+  uint2* dec;
+  const uint2* prev_dec;
 };
 static_assert(sizeof(StreamDev) % 8 == 0, "descriptors are copied by 8-byte words");
 
@@ -113,6 +117,9 @@ struct FrameGroups {
   FrameParams g[kMaxGroups];
   int32_t n;
 };
+// Whether the warps of an SM meet between their segments in a launch of n_tasks segments over key_span
+// macroblock-times (pipeline_kernel).
+bool pipeline_meets(size_t n_tasks, int grid, int key_span);
 int pipeline_grid(int device);
 int pipeline_sms(int device);
 size_t pipeline_counter_ints(const FrameParams& fp, int frames);
@@ -129,6 +136,7 @@ size_t pipeline_task_list(const FrameParams& fp, int frames, int lag, int seg, b
 // One launch over n_desc descriptors of up to kMaxGroups picture sizes (descriptor d: group
 // d.group, rows d.rows_base .. + its mb_h in the row counters, total_rows in all). host_err null:
 // no error hand-off kernel (launch_error_to_host queues one per caller instead).
+// early: every descriptor has its decisions (dec), zeroed (plain form).
 // Compact records (co != null): the warp deblocking a row's last segment also writes that row's
 // records, word-sparse (kCompactMaskWords mask words per record, then its nonzero words in order),
 // into the row's slot (row r of the launch, counted as the row counters are: row_words words at
@@ -144,7 +152,7 @@ struct CompactOut {
 void launch_pipeline(const FrameGroups& fg, const StreamDev* d_streams, int n_desc, int total_rows, int* counters,
                      const int2* d_tasks, size_t n_tasks, int key_span, const int qbeg[3], const int qend[3], int deblock_sms,
                      int intra_sms, int sms, int seg, int grid, unsigned long long timeout_ns, int* ready, int seq,
-                     int* host_err, int* host_reach, cudaStream_t st, int form = 0, const CompactOut* co = nullptr);
+                     int* host_err, int* host_reach, cudaStream_t st, int form = 0, const CompactOut* co = nullptr, bool early = false);
 void launch_error_to_host(const int* counters, int n_desc, int total_rows, int* host_err, int* host_reach,
                           cudaStream_t st);
 size_t pipeline_counter_ints(int total_rows, int n_desc);

@@ -94,6 +94,7 @@ struct __align__(16) Smem {
   uint32_t qpt[16];               // quarter-sample phases: the two planes averaged (init_tables)
   alignas(16) uint32_t dbmv[12];  // deblocking, search forms: quadrant vectors of the macroblock, its left and top neighbours
   int win_x, win_y, win_have;     // ensure_window: the position held (kNoWin: none), its planes built (bits 0..2)
+  int recon_seen;                 // this macroblock's neighbours are reconstructed (wait_recon)
   int db_row, seen_db;            // last acquired progress db_prev[db_row] of the reference picture
   int reach_y, reach_x;           // 1 + the largest reach waited for beyond zero motion, in macroblocks
   alignas(16) uint8_t i4m[16];    // Intra4x4PredMode of this macroblock (decoding order)
@@ -405,15 +406,19 @@ __device__ __noinline__ void mc_luma16(int x0, int y0, int mvx, int mvy) {
 __device__ __noinline__ void mc_chroma8(const uint8_t* ru, const uint8_t* rv, int stride, int mbx, int mby, int mvx, int mvy) {
   int lane = lane_id();
   int cx = mbx * 8 + (mvx >> 3), cy = mby * 8 + (mvy >> 3), fx = mvx & 7, fy = mvy & 7;
-  int wa = (8 - fx) * (8 - fy), wb = fx * (8 - fy), wc = (8 - fx) * fy, wd = fx * fy;
-  int plane = lane >> 4, idx = (lane & 15) * 4, r = idx >> 3, c0 = idx & 7;
+  // bilinear weights of the samples (0, 0), (1, 0), (0, 1), (1, 1), a byte each; a lane's four samples
+  // come from five of either row
+  const uint32_t w = (uint32_t)((8 - fx) * (8 - fy) | (fx * (8 - fy)) << 8 | ((8 - fx) * fy) << 16 | (fx * fy) << 24);
+  const int plane = lane >> 4, idx = (lane & 15) * 4, r = idx >> 3, c0 = idx & 7;
   const uint8_t* src = (plane ? rv : ru) + (long)(cy + r) * stride + cx + c0;
-  uint8_t* out = (plane ? sm.pred_v : sm.pred_u) + r * 8 + c0;
+  const uint2 a = ldg8(src), b = ldg8(src + stride);
+  uint32_t v = 0;
 #pragma unroll
   for (int k = 0; k < 4; k++) {
-    int a = ldcg_u8(src + k), b = ldcg_u8(src + k + 1), cc = ldcg_u8(src + stride + k), d = ldcg_u8(src + stride + k + 1);
-    out[k] = (uint8_t)((wa * a + wb * b + wc * cc + wd * d + 32) >> 6);
+    const uint32_t ra = __funnelshift_r(a.x, a.y, 8 * k), rb = __funnelshift_r(b.x, b.y, 8 * k);
+    v |= (__dp4a(__byte_perm(ra, rb, 0x5410), w, 32u) >> 6) << (8 * k);
   }
+  *(uint32_t*)((plane ? sm.pred_v : sm.pred_u) + r * 8 + c0) = v;
   __syncwarp();
 }
 
@@ -1089,26 +1094,34 @@ __device__ __noinline__ void load_source(const Ctx c) {
 // memory; returns the samples at the corner.
 __device__ __noinline__ Corner load_edges(const Ctx c, bool want_topright) {
   const FrameParams& fp = sm.fp;
-  int lane = lane_id();
-  const uint8_t* Y = sm.sd.cur_y;
-  int x0 = c.mbx * 16, y0 = c.mby * 16;
-  bool ht = c.mby > 0, hl = c.mbx > 0;
-  if (ht && lane < 24) {
-    bool ok = lane < 16 || (want_topright && c.mbx + 1 < fp.mb_w);
-    sm.top[lane] = ok ? ldcg_u8(Y + (long)(y0 - 1) * fp.stride_y + x0 + lane) : 0;
+  const StreamDev& sd = sm.sd;
+  const int lane = lane_id(), x0 = c.mbx * 16, y0 = c.mby * 16;
+  const bool ht = c.mby > 0, hl = c.mbx > 0;
+  // two loads a lane, both in flight together: a word of the rows above -- lanes 0..5 luma (the last two
+  // its top-right neighbour's), 6 / 7 U, 8 / 9 V, 10..12 the words that end in the corners -- and a
+  // sample of the columns to the left -- lanes 0..15 luma, 16..23 U, 24..31 V. (Byte by byte, plane by
+  // plane: 4 round trips to L2, 4 k cycles.)
+  const int tp = lane < 6 ? 0 : (lane < 10 ? 1 + ((lane - 6) >> 1) : lane - 10), lp = lane < 16 ? 0 : (lane < 24 ? 1 : 2);
+  auto plane = [&](int p) -> const uint8_t* { return p == 0 ? sd.cur_y : (p == 1 ? sd.cur_u : sd.cur_v); };
+  const bool corner = lane >= 10;
+  const bool tl = ht && lane < 13 && (corner ? hl : (lane < 4 || lane >= 6 || (want_topright && c.mbx + 1 < fp.mb_w)));
+  const int tx = corner ? -4 : 4 * (lane < 6 ? lane : (lane - 6) & 1);
+  uint32_t t = 0, l = 0;
+  if (tl) t = __ldcg((const uint32_t*)(plane(tp) + (long)((tp ? y0 >> 1 : y0) - 1) * (tp ? fp.stride_c : fp.stride_y) + (tp ? x0 >> 1 : x0) + tx));
+  if (hl)
+    l = __ldcg(plane(lp) + (long)(lp ? (y0 >> 1) + (lane & 7) : y0 + lane) * (lp ? fp.stride_c : fp.stride_y) + (lp ? x0 >> 1 : x0) - 1);
+  if (ht) {
+    if (lane < 6) *(uint32_t*)&sm.top[4 * lane] = t;
+    else if (lane < 10) *(uint32_t*)&sm.ctop[tp - 1][tx] = t;
   }
-  if (hl && lane < 16) sm.left[lane] = ldcg_u8(Y + (long)(y0 + lane) * fp.stride_y + x0 - 1);
-  int cx0 = c.mbx * 8, cy0 = c.mby * 8;
-  if (lane < 16) {
-    int p = lane >> 3, k = lane & 7;
-    const uint8_t* P = p ? sm.sd.cur_v : sm.sd.cur_u;
-    if (ht) sm.ctop[p][k] = ldcg_u8(P + (long)(cy0 - 1) * fp.stride_c + cx0 + k);
-    if (hl) sm.cleft[p][k] = ldcg_u8(P + (long)(cy0 + k) * fp.stride_c + cx0 - 1);
+  if (hl) {
+    if (lane < 16) sm.left[lane] = (uint8_t)l;
+    else sm.cleft[lp - 1][lane & 7] = (uint8_t)l;
   }
   Corner k;
-  k.y = (ht && hl) ? ldcg_u8(Y + (long)(y0 - 1) * fp.stride_y + x0 - 1) : 128;
-  k.u = (ht && hl) ? ldcg_u8(sm.sd.cur_u + (long)(cy0 - 1) * fp.stride_c + cx0 - 1) : 128;
-  k.v = (ht && hl) ? ldcg_u8(sm.sd.cur_v + (long)(cy0 - 1) * fp.stride_c + cx0 - 1) : 128;
+  k.y = ht && hl ? (int)(__shfl_sync(FULL, t, 10) >> 24) : 128;
+  k.u = ht && hl ? (int)(__shfl_sync(FULL, t, 11) >> 24) : 128;
+  k.v = ht && hl ? (int)(__shfl_sync(FULL, t, 12) >> 24) : 128;
   __syncwarp();
   return k;
 }
@@ -1559,6 +1572,8 @@ __device__ __forceinline__ void publish(int* p, int v) {
 // addresses; the state is in shared memory).
 struct PipeWait {
   const int* db_prev;    // deblocking progress per row of the reference picture (padding included); null: no wait
+  const int* ana;        // analysis progress per row of this picture, where macroblocks start before their
+                         // neighbours are reconstructed; null: those are
   int* error;
   unsigned long long timeout_ns;
 };
@@ -1580,6 +1595,54 @@ __device__ __noinline__ bool wait_reference(const Ctx c, const PipeWait pw, int 
     sm.db_row = row;
     sm.seen_db = seen;
   }
+  __syncwarp();
+  return ok;
+}
+
+// A launch of few pictures is one chain of macroblocks, each waiting for its neighbours. What the next one
+// needs first is only their vectors: its own reconstructed neighbours it reads after its motion search.
+// So there a macroblock publishes its decision before its residual is coded, and one starts on its
+// neighbours' decisions and waits for their reconstruction before the intra check. One 720p stream, 30
+// pictures: 11.86 -> 10.2 ms.
+//
+// A macroblock's decision (vector and ref) for the neighbours that wait for it alone (StreamDev.dec): one
+// 64-bit word that is its own flag, so neither side needs a fence.
+__device__ __forceinline__ void decide(const Ctx c, int mv0, int mv1, int ref) {
+  if (lane_id() == 0)
+    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(sm.sd.dec + c.mb), "l"((unsigned long long)(0x100u | (ref & 255)) << 32 | pack16(mv0, mv1)) : "memory");
+}
+// Waits until every lane's decision (p null: none) is there and returns it in w. False as wait_all.
+__device__ __noinline__ bool wait_decided(const uint2* p, uint2& w, int* error, unsigned long long timeout_ns) {
+  unsigned long long t0 = 0;
+  bool ok = !p;
+  while (true) {
+    const int failed = lane_id() == 0 ? ld_relaxed(error) : 0;  // (in flight beside the decisions)
+    if (!ok) {
+      unsigned long long v;
+      asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+      ok = (v >> 40) & 1u;
+      w = make_uint2((uint32_t)v, (uint32_t)(v >> 32));
+    }
+    if (__all_sync(FULL, ok)) return true;
+    if (!t0) t0 = global_ns();
+    const bool late = lane_id() == 0 && global_ns() - t0 > timeout_ns;
+    if (__any_sync(FULL, failed)) return false;
+    if (__any_sync(FULL, late)) {
+      if (lane_id() == 0) atomicCAS(error, 0, 1);
+      return false;
+    }
+    __nanosleep(100);
+  }
+}
+// Waits until the left and top neighbours (and the top-right one) are reconstructed, where the
+// macroblock started before they were.
+__device__ __noinline__ bool wait_recon(const Ctx c, const PipeWait pw) {
+  if (sm.recon_seen) return true;
+  const int* flag = lane_id() == 0 && c.mbx > 0 ? pw.ana + c.mby : nullptr;
+  if (lane_id() == 1 && c.mby > 0) flag = pw.ana + c.mby - 1;
+  int seen = -1;
+  const bool ok = wait_all(flag, lane_id() == 0 ? c.mbx : min(c.mbx + 2, sm.fp.mb_w), seen, pw.error, pw.timeout_ns);
+  if (lane_id() == 0) sm.recon_seen = 1;
   __syncwarp();
   return ok;
 }
@@ -1631,6 +1694,8 @@ __device__ __forceinline__ uint32_t qpel_sad2(uint2 sv, int dx0, int dy0, int dx
 // One macroblock of a P slice (enc.rs:3011 code_p_mb). In the pipelined mode (pw.db_prev) it first
 // waits for the reference frame to be final over every sample its search can read; when a wait
 // gives up it returns false and writes nothing.
+// kEarly: it starts on its neighbours' decisions, and publishes its own before the residual.
+template <bool kEarly>
 __device__ __noinline__ bool analyse_p_mb(const Ctx c, const PipeWait pw) {
   const FrameParams& fp = sm.fp;
   const StreamDev& sd = sm.sd;
@@ -1639,13 +1704,26 @@ __device__ __noinline__ bool analyse_p_mb(const Ctx c, const PipeWait pw) {
   const Bounds bd = mv_bounds(x0, y0);
   // neighbours (this picture) and the co-located macroblock of the previous one, a lane each: left,
   // top, top-right (top-left where that is absent), co-located; ref -2 when absent
-  const MbInfo* nb = nullptr;
-  if (lane == 0 && mbx > 0) nb = &sd.info[c.mb - 1];
-  if (lane == 1 && mby > 0) nb = &sd.info[c.mb - fp.mb_w];
-  if (lane == 2 && mby > 0 && fp.mb_w > 1) nb = &sd.info[c.mb - fp.mb_w + (mbx + 1 < fp.mb_w ? 1 : -1)];
-  if (lane == 3) nb = &sd.prev_info[c.mb];
-  const uint2 nw = nb ? *(const uint2*)nb : make_uint2(0u, 0xfeu);
+  int nb = -1;
+  if (lane == 0 && mbx > 0) nb = c.mb - 1;
+  if (lane == 1 && mby > 0) nb = c.mb - fp.mb_w;
+  if (lane == 2 && mby > 0 && fp.mb_w > 1) nb = c.mb - fp.mb_w + (mbx + 1 < fp.mb_w ? 1 : -1);
+  if (lane == 3) nb = c.mb;
+  uint2 nw = make_uint2(0u, 0xfeu);
   load_source(c);
+  // While the neighbours decide: what zero motion reads of the reference picture, which is waited for
+  // in any case, and its lines into the L1.
+  if (kEarly && pw.db_prev) {
+    if (!wait_reference(c, pw, (x0 + 44) >> 4, (y0 + 40) >> 4)) return false;
+    if (lane < 26) {
+      const uint8_t* p = sd.ref_y + (long)(y0 - 5 + lane) * fp.stride_y + x0 - 8;
+      asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
+      if (((uintptr_t)p ^ (uintptr_t)(p + 31)) & 128) asm volatile("prefetch.global.L1 [%0];" ::"l"(p + 31));
+    }
+  }
+  const uint2* const dec = !kEarly ? nullptr : (lane == 3 ? sd.prev_dec : sd.dec);
+  if (kEarly && !wait_decided(nb >= 0 && dec ? dec + nb : nullptr, nw, pw.error, pw.timeout_ns)) return false;
+  if (nb >= 0 && !dec) nw = *(const uint2*)&(lane == 3 ? sd.prev_info : sd.info)[nb];
   const int va = __shfl_sync(FULL, (int)nw.x, 0), vb = __shfl_sync(FULL, (int)nw.x, 1), vc = __shfl_sync(FULL, (int)nw.x, 2),
             vp = __shfl_sync(FULL, (int)nw.x, 3);
   const int ref = (int8_t)(nw.y & 255u);
@@ -1684,6 +1762,7 @@ __device__ __noinline__ bool analyse_p_mb(const Ctx c, const PipeWait pw) {
 
   // 1. skip probe
   if (in_bounds(bd, ps0, ps1) && skip_probe(c, ps0, ps1)) {
+    if (kEarly) decide(c, ps0, ps1, 0);
     code_skip(c, ps0, ps1);
     return true;
   }
@@ -1761,16 +1840,19 @@ __device__ __noinline__ bool analyse_p_mb(const Ctx c, const PipeWait pw) {
   // 3. intra 16x16 when the inter prediction is poor (enc.rs:3121-3156)
   const uint32_t inter_satd = satd16((int)offsetof(Smem, pred_y));
   if (inter_satd > 24 * lambda) {
+    if (kEarly && !wait_recon(c, pw)) return false;
     const Corner k0 = load_edges(c, false);
     const bool ht = mby > 0, hl = mbx > 0;
     const I16Fit fit16 = analyse_i16(ht, hl, k0.y);
     if (fit16.cost + lambda * 8 < inter_satd + lambda * (se_bits(mv0 - mvp0) + se_bits(mv1 - mvp1) + 1)) {
+      if (kEarly) decide(c, 0, 0, -1);
       code_i16(c, fit16.mode, ht, hl, k0);
       return true;
     }
   }
 
   // 4. P_L0_16x16 residual, record and reconstruction
+  if (kEarly) decide(c, mv0, mv1, 0);
   mc_chroma8(sd.ref_u, sd.ref_v, fp.stride_c, mbx, mby, mv0, mv1);
   code_inter(c, RG_MB_P_L0_16X16, mv0 == ps0 && mv1 == ps1, mv0, mv1, mv0 - mvp0, mv1 - mvp1);
   return true;
@@ -1973,7 +2055,7 @@ __global__ void __launch_bounds__(32) wavefront_step_kernel(const __grid_constan
       else analyse_intra_mb(c);
     } else {
       if constexpr (kForm != 0) analyse_p_mb_search(c, none);
-      else analyse_p_mb(c, none);
+      else analyse_p_mb<false>(c, none);
     }
   } else if (k - na < nd) {
     int d = step - 3;
@@ -2186,7 +2268,7 @@ __device__ __forceinline__ void meet(int* arrived, int round, int limit) {
   __syncwarp();
 }
 
-template <int kForm>
+template <int kForm, bool kEarly>
 __global__ void __launch_bounds__(32 * kBlockWarps, 1) pipeline_kernel(const __grid_constant__ FrameGroups fg, const StreamDev* __restrict__ sds, PipeParams pp) {
   const int lane = lane_id();
   // Warps on the first deblock_sms SMs take deblocking segments first, on the next intra_sms SMs
@@ -2238,13 +2320,16 @@ __global__ void __launch_bounds__(32 * kBlockWarps, 1) pipeline_kernel(const __g
     int seen = 0;  // of this lane's counter (wait_all)
     if (ana) {
       const bool has_prev = sd.prev_rows >= 0 && sd.kind == RG_FRAME_P;
-      const PipeWait pw{has_prev ? pp.db + sd.prev_rows : nullptr, pp.error, pp.timeout_ns};
+      const bool early = kEarly && sd.kind == RG_FRAME_P;
+      const PipeWait pw{has_prev ? pp.db + sd.prev_rows : nullptr, early ? ana_rows : nullptr, pp.error, pp.timeout_ns};
       if (lane == 0) sm.db_row = -1;
       // lane 0: the previous segment of this row; lane 1: the row above two macroblocks ahead; lane 2
       // (plain form): the co-located macroblock of the previous picture, whose vector is a candidate
+      // (early: analyse_p_mb waits for their decisions instead)
       const int* flag = lane == 0 && x0 > 0 ? ana_rows + y : nullptr;
       if (lane == 1 && y > 0) flag = ana_rows + y - 1;
       if (kForm == 0 && lane == 2 && has_prev) flag = pp.ana + sd.prev_rows + y;
+      if (early) flag = nullptr;
       for (int x = x0; x < x1; x++) {
         if (!wait_all(flag, lane == 0 ? x0 : (lane == 1 ? min(x + 2, Wm) : x + 1), seen, pp.error, pp.timeout_ns)) {
           failed = true;
@@ -2255,9 +2340,11 @@ __global__ void __launch_bounds__(32 * kBlockWarps, 1) pipeline_kernel(const __g
           load_source(c);
           if constexpr (kForm != 0) analyse_intra_mb_search(c);
           else analyse_intra_mb(c);
+          if constexpr (kEarly) decide(c, 0, 0, -1);
         } else {
+          if (kEarly && lane == 0) sm.recon_seen = 0;
           if constexpr (kForm != 0) failed = !analyse_p_mb_search(c, pw);
-          else failed = !analyse_p_mb(c, pw);
+          else failed = !analyse_p_mb<kEarly>(c, pw) || (kEarly && !wait_recon(c, pw));  // (the row's progress counts the left one)
           if (failed) break;
         }
         publish(ana_rows + y, x + 1);
@@ -2496,10 +2583,18 @@ size_t pipeline_task_list(const FrameParams& fp, int frames, int lag, int seg, b
   return pipeline_task_count(fp, frames, seg);
 }
 
+// Meetings pay where there is work for most warps, and cost a little where the launch is one chain
+// of macroblocks and they wait anyway: on average at least a quarter as many segments ready as there
+// are warps (segments over the span of their keys, both roles). 8 x 15 pictures of 1080p have 1742
+// (34.9 -> 21.7 ms), 8 x 8 learned 1238 (92 -> 65.5), four mixed sizes 1148 (17.3 -> 13.1), 4 x 3
+// learned 4K 672 (80.9 -> 77.2), 8 x 3 full search 720p 310 (50.9 -> 52.3), one 720p stream 179 (11.8 ->
+// 12.2).
+bool pipeline_meets(size_t n_tasks, int grid, int key_span) { return n_tasks / 2 * 4 >= (size_t)grid * (size_t)key_span; }
+
 void launch_pipeline(const FrameGroups& fg, const StreamDev* d_streams, int n_desc, int total_rows, int* counters,
                      const int2* d_tasks, size_t n_tasks, int key_span, const int qbeg[3], const int qend[3], int deblock_sms,
                      int intra_sms, int sms, int seg, int grid, unsigned long long timeout_ns, int* ready, int seq,
-                     int* host_err, int* host_reach, cudaStream_t st, int form, const CompactOut* co) {
+                     int* host_err, int* host_reach, cudaStream_t st, int form, const CompactOut* co, bool early) {
   PipeParams pp;
   pp.ticket = counters;
   pp.error = counters + 1;
@@ -2513,13 +2608,7 @@ void launch_pipeline(const FrameGroups& fg, const StreamDev* d_streams, int n_de
   }
   pp.deblock_sms = deblock_sms;
   pp.intra_sms = intra_sms;
-  // Meetings pay where there is work for most warps, and cost a little where the launch is one chain
-  // of macroblocks and they wait anyway: on average at least a quarter as many segments ready as there
-  // are warps (segments over the span of their keys, both roles). 8 x 15 pictures of 1080p have 1742
-  // (34.9 -> 21.7 ms), 8 x 8 learned 1238 (92 -> 65.5), four mixed sizes 1148 (17.3 -> 13.1), 4 x 3
-  // learned 4K 672 (80.9 -> 77.2), 8 x 3 full search 720p 310 (50.9 -> 52.3), one 720p stream 179 (11.8 ->
-  // 12.2).
-  const bool meet = n_tasks / 2 * 4 >= (size_t)grid * (size_t)key_span;
+  const bool meet = pipeline_meets(n_tasks, grid, key_span);
   pp.meet_ns = meet ? (form ? kMeetNsSearch : kMeetNs) : 0;
   // spread over the SMs, then up to a block's warps on each
   pp.grid = grid < pp.n_tasks ? grid : pp.n_tasks;
@@ -2539,13 +2628,9 @@ void launch_pipeline(const FrameGroups& fg, const StreamDev* d_streams, int n_de
   pp.cbytes = co ? co->row_bytes : nullptr;
   const dim3 block(32, warps);
   const size_t smem = warps * warp_smem(form);
-  if (form) {
-    cudaFuncSetAttribute(pipeline_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    pipeline_kernel<1><<<g, block, smem, st>>>(fg, d_streams, pp);
-  } else {
-    cudaFuncSetAttribute(pipeline_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    pipeline_kernel<0><<<g, block, smem, st>>>(fg, d_streams, pp);
-  }
+  const auto kernel = form ? pipeline_kernel<1, false> : (early ? pipeline_kernel<0, true> : pipeline_kernel<0, false>);
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  kernel<<<g, block, smem, st>>>(fg, d_streams, pp);
   if (host_err) error_to_host_kernel<<<1, 1, 0, st>>>(pp.error, pp.reach, host_err, host_reach);
 }
 

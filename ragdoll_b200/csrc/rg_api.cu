@@ -154,6 +154,7 @@ struct rg_ctx {
   int slot = 0;
   int max_frames = 1, nslots = 2;  // pictures per pipelined call; picture ring per stream
   int* counters = nullptr;         // pipelined-mode progress counters
+  uint2* decs = nullptr;           // [max_frames][S][n_mb] decisions (StreamDev.dec; on first use)
   size_t n_counters = 0;
   int* h_err = nullptr;            // mapped host memory: each pending launch's error word
   int* d_err = nullptr;            // the same, as the device sees it
@@ -396,6 +397,7 @@ void rg_destroy(rg_ctx* c) {
   cudaFree(c->infos);
   cudaFree(c->mv4s);
   cudaFree(c->d_hints);
+  cudaFree(c->decs);
   cudaFree(c->recs);
   cudaFree(c->srcs);
   cudaFree(c->unf);
@@ -548,6 +550,8 @@ static int enqueue_wavefront(rg_ctx* c, const uint8_t* const* dev_planes, size_t
     d.group = 0;
     d.rows_base = 0;
     d.prev_rows = -1;
+    d.dec = nullptr;
+    d.prev_dec = nullptr;
     d.mv4 = c->mv4s ? c->mv4s + ((size_t)s * c->nslots + par) * c->n_mb : nullptr;
     d.hint = hints ? hints[i] : nullptr;
     d.search_range = c->search_range;
@@ -580,7 +584,7 @@ static int enqueue_wavefront(rg_ctx* c, const uint8_t* const* dev_planes, size_t
 // group `group`.
 static void gop_desc(const rg_ctx* c, StreamDev& d, int f, int s, const uint8_t* const* dev_planes,
                      const int32_t* kinds, rg_mb_out* rec_base, const rg_mb_hint* hint, int group, int rows_base,
-                     int* ready = nullptr) {
+                     int* ready = nullptr, uint2* dec = nullptr) {
   const int S = c->S, g = c->frames[s] + f;
   const int cur = g % c->nslots, prv = (g + c->nslots - 1) % c->nslots;
   d.src_y = dev_planes[(f * S + s) * 3];
@@ -601,6 +605,8 @@ static void gop_desc(const rg_ctx* c, StreamDev& d, int f, int s, const uint8_t*
   d.group = group;
   d.rows_base = rows_base + (f * S + s) * c->fp.mb_h;
   d.prev_rows = f > 0 ? d.rows_base - S * c->fp.mb_h : -1;
+  d.dec = dec ? dec + ((size_t)f * S + s) * c->n_mb : nullptr;
+  d.prev_dec = dec && f > 0 ? d.dec - (size_t)S * c->n_mb : nullptr;
   d.mv4 = c->mv4s ? c->mv4s + ((size_t)s * c->nslots + cur) * c->n_mb : nullptr;
   d.hint = hint;
   d.search_range = c->search_range;
@@ -680,13 +686,26 @@ static int enqueue_gops(rg_ctx* c, const uint8_t* const* dev_planes, size_t stri
     int r = take_hints(c, frames * S, "rg_analyse_gops_device", hv);
     if (r) return r;
   }
+  // A launch too small for meetings is one chain of macroblocks: each starts on its neighbours' decisions
+  // there, before they are reconstructed.
+  const int lag = c->lag > 0 ? c->lag : auto_lag(c), key_span = pipeline_key_span(c->fp, frames, lag, c->seg);
+  uint2* dec = nullptr;
+  const size_t dec_bytes = sizeof(uint2) * (size_t)c->n_mb * S;
+  if (c->form == RG_FORM_PLAIN && !pipeline_meets(pipeline_task_count(c->fp, frames, c->seg), c->grid, key_span)) {
+    if (!c->decs && cudaMalloc((void**)&c->decs, dec_bytes * c->max_frames) != cudaSuccess) {
+      c->decs = nullptr;  // without them macroblocks wait for reconstructed neighbours
+      cudaGetLastError();
+    }
+    dec = c->decs;
+    if (dec) CK(cudaMemsetAsync(dec, 0, dec_bytes * frames, c->stream));
+  }
   int slot = c->slot;
   c->slot ^= 1;
   CK(cudaEventSynchronize(c->slot_done[slot]));
   StreamDev* h = c->h_streams[slot];
   for (int f = 0; f < frames; f++)
     for (int s = 0; s < S; s++)
-      gop_desc(c, h[f * S + s], f, s, dev_planes, kinds, rec_base, hv.empty() ? nullptr : hv[f * S + s], 0, 0);
+      gop_desc(c, h[f * S + s], f, s, dev_planes, kinds, rec_base, hv.empty() ? nullptr : hv[f * S + s], 0, 0, nullptr, dec);
   FrameParams fp = c->fp;
   fp.src_stride_y = (int)stride_y;
   fp.src_stride_uv = (int)stride_uv;
@@ -697,7 +716,6 @@ static int enqueue_gops(rg_ctx* c, const uint8_t* const* dev_planes, size_t stri
   // IDR pictures get their own queue when SMs are set aside for them
   std::vector<int32_t> kinds_key;
   if (c->intra_sms > 0 && c->grid >= 3) kinds_key.assign(kinds, kinds + (size_t)frames * S);
-  const int lag = c->lag > 0 ? c->lag : auto_lag(c);
   if (frames != c->tasks_frames || lag != c->tasks_lag || c->seg != c->tasks_seg || split != c->tasks_split ||
       kinds_key != c->tasks_kinds) {
     // rebuilt only when the call's shape, its picture kinds or the tuning change; the copy is
@@ -722,8 +740,8 @@ static int enqueue_gops(rg_ctx* c, const uint8_t* const* dev_planes, size_t stri
   fg.g[0] = fp;
   fg.n = 1;
   launch_pipeline(fg, c->d_streams[slot], frames * S, frames * S * fp.mb_h, c->counters, c->d_tasks, c->n_tasks,
-                  pipeline_key_span(fp, frames, lag, c->seg), c->qbeg, c->qend, c->deblock_sms, c->intra_sms, c->sms, c->seg, c->grid, c->timeout_ns, ready, seq,
-                  c->d_err + pslot, c->d_err + 2 + 2 * pslot, c->stream, c->form != RG_FORM_PLAIN, co);
+                  key_span, c->qbeg, c->qend, c->deblock_sms, c->intra_sms, c->sms, c->seg, c->grid, c->timeout_ns, ready, seq,
+                  c->d_err + pslot, c->d_err + 2 + 2 * pslot, c->stream, c->form != RG_FORM_PLAIN, co, dec != nullptr);
   CK(cudaGetLastError());
   CK(cudaEventRecord(p.done, c->stream));
   p.planes.assign(dev_planes, dev_planes + (size_t)frames * S * 3);
