@@ -122,12 +122,6 @@ __device__ __forceinline__ uint8_t* sm_at(int off) { return (uint8_t*)&sm + off;
 
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 __device__ __forceinline__ uint32_t pack16(int lo, int hi) { return __byte_perm((uint32_t)lo, (uint32_t)hi, 0x5410); }
-__device__ __forceinline__ MbInfo ld_info(const MbInfo* p) {
-  int4 v = *(const int4*)p;
-  MbInfo m;
-  *(int4*)&m = v;
-  return m;
-}
 __device__ __forceinline__ uint32_t wsum(uint32_t v) { return __reduce_add_sync(FULL, v); }
 __device__ __forceinline__ int clip255(int v) { return v < 0 ? 0 : (v > 255 ? 255 : v); }
 __device__ __forceinline__ int16_t clamp_i16(int v) { return (int16_t)(v < -32768 ? -32768 : (v > 32767 ? 32767 : v)); }
@@ -358,12 +352,6 @@ __device__ __noinline__ uint2 qpel8(int dx, int dy) {
   const uint2 a = lds8(&sm.win[0] + at + (e & 0xffffu)), b = lds8(&sm.win[0] + at + (e >> 16));
   return make_uint2(__vavgu4(a.x, b.x), __vavgu4(a.y, b.y));
 }
-// Cost of a full-pel position (mx, my): the warp's SAD of the 16x16 block (this lane's 8 source
-// samples sv against its 8 reference samples r) plus lambda * bits of the vector difference to
-// the predictor (enc.rs:1207 cost).
-__device__ __noinline__ uint32_t fullpel_cost(uint2 sv, uint2 r, int mx, int my, int mvp0, int mvp1, uint32_t lambda) {
-  return wsum(vsad8(sv, r)) + mvd_cost(mx * 4 - mvp0, lambda) + mvd_cost(my * 4 - mvp1, lambda);
-}
 // The cheapest of the four neighbours of (x, y) at distance st (quarter samples) inside the bounds:
 // up, left, right, down, the first on ties. s01, s23: this lane's share of their SADs, two to a word
 // (a 16x16 SAD fits 16 bits). Lane k costs neighbour k. Returns cost << 2 | k, all ones when none is
@@ -402,15 +390,10 @@ __device__ __noinline__ void mc_luma16(int x0, int y0, int mvx, int mvy) {
   *(uint2*)&sm.pred_y[(lane >> 1) * 16 + (lane & 1) * 8] = v;
   __syncwarp();
 }
-// Chroma prediction of both planes (h264_enc.rs:1279 chroma_mc_8x8_x2_scalar; enc.rs:1082).
-__device__ __noinline__ void mc_chroma8(const uint8_t* ru, const uint8_t* rv, int stride, int mbx, int mby, int mvx, int mvy) {
-  int lane = lane_id();
-  int cx = mbx * 8 + (mvx >> 3), cy = mby * 8 + (mvy >> 3), fx = mvx & 7, fy = mvy & 7;
-  // bilinear weights of the samples (0, 0), (1, 0), (0, 1), (1, 1), a byte each; a lane's four samples
-  // come from five of either row
+// Four chroma samples (the bilinear 1/8-sample filter), the first at src for phase (0, 0): weights of the
+// samples (0, 0), (1, 0), (0, 1), (1, 1) a byte each, a dot product a sample.
+__device__ __forceinline__ uint32_t chroma4(const uint8_t* src, int stride, int fx, int fy) {
   const uint32_t w = (uint32_t)((8 - fx) * (8 - fy) | (fx * (8 - fy)) << 8 | ((8 - fx) * fy) << 16 | (fx * fy) << 24);
-  const int plane = lane >> 4, idx = (lane & 15) * 4, r = idx >> 3, c0 = idx & 7;
-  const uint8_t* src = (plane ? rv : ru) + (long)(cy + r) * stride + cx + c0;
   const uint2 a = ldg8(src), b = ldg8(src + stride);
   uint32_t v = 0;
 #pragma unroll
@@ -418,7 +401,14 @@ __device__ __noinline__ void mc_chroma8(const uint8_t* ru, const uint8_t* rv, in
     const uint32_t ra = __funnelshift_r(a.x, a.y, 8 * k), rb = __funnelshift_r(b.x, b.y, 8 * k);
     v |= (__dp4a(__byte_perm(ra, rb, 0x5410), w, 32u) >> 6) << (8 * k);
   }
-  *(uint32_t*)((plane ? sm.pred_v : sm.pred_u) + r * 8 + c0) = v;
+  return v;
+}
+// Chroma prediction of both planes (h264_enc.rs:1279 chroma_mc_8x8_x2_scalar; enc.rs:1082).
+__device__ __noinline__ void mc_chroma8(const uint8_t* ru, const uint8_t* rv, int stride, int mbx, int mby, int mvx, int mvy) {
+  int lane = lane_id();
+  int cx = mbx * 8 + (mvx >> 3), cy = mby * 8 + (mvy >> 3), fx = mvx & 7, fy = mvy & 7;
+  const int plane = lane >> 4, idx = (lane & 15) * 4, r = idx >> 3, c0 = idx & 7;
+  *(uint32_t*)((plane ? sm.pred_v : sm.pred_u) + r * 8 + c0) = chroma4((plane ? rv : ru) + (long)(cy + r) * stride + cx + c0, stride, fx, fy);
   __syncwarp();
 }
 

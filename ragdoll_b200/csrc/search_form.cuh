@@ -60,36 +60,33 @@ struct SearchSmem {
 // Behind every warp's Smem.
 static_assert(sizeof(Smem) % 16 == 0, "SearchSmem follows aligned");
 #define ss (((SearchSmem*)(smw + blockDim.y * sizeof(Smem)))[threadIdx.y])
-__device__ __forceinline__ void ld_q(const MbMv4* m, int q, int* v) {
-  uint32_t w = ((const uint32_t*)m)[q];
-  v[0] = (int16_t)(w & 0xffffu);
-  v[1] = (int16_t)(w >> 16);
-}
-__device__ __noinline__ MbNb load_nb(const Ctx c) {
+// The neighbours into ss.nb, all loads in flight together: lanes 0..3 the refs of the left, top,
+// top-right and top-left macroblocks, lanes 4..9 the six vectors (a[0], a[1], b[0], b[1], cc, d).
+__device__ __forceinline__ uint32_t load_nb(const Ctx c) {
   const StreamDev& sd = sm.sd;
-  const int mb_w = sm.fp.mb_w, mb = c.mb;
-  MbNb n;
-  n.refA = n.refB = n.refC = n.refD = -2;
-  n.a[0][0] = n.a[0][1] = n.a[1][0] = n.a[1][1] = 0;
-  n.b[0][0] = n.b[0][1] = n.b[1][0] = n.b[1][1] = 0;
-  n.cc[0] = n.cc[1] = n.d[0] = n.d[1] = 0;
-  if (c.mbx > 0) {
-    n.refA = ld_info(&sd.info[mb - 1]).ref;
-    if (n.refA == 0) { ld_q(&sd.mv4[mb - 1], 1, n.a[0]); ld_q(&sd.mv4[mb - 1], 3, n.a[1]); }
+  const int lane = lane_id(), mb_w = sm.fp.mb_w;
+  const int k = lane < 4 ? lane : (lane < 8 ? (lane - 4) >> 1 : lane - 6);  // which macroblock
+  const bool have = k == 0 ? c.mbx > 0 : (c.mby > 0 && (k == 1 || (k == 2 ? c.mbx + 1 < mb_w : c.mbx > 0)));
+  const int mb = c.mb + (k == 0 ? -1 : (k == 1 ? 0 : (k == 2 ? 1 : -1)) - mb_w);
+  uint32_t w = lane < 4 ? 0xfeu : 0u;
+  if (lane < 10 && have) {
+    const int quad = lane == 4 ? 1 : (lane == 6 || lane == 8 ? 2 : 3);
+    w = lane < 4 ? ((const uint32_t*)&sd.info[mb])[1] : ((const uint32_t*)&sd.mv4[mb])[quad];
   }
-  if (c.mby > 0) {
-    n.refB = ld_info(&sd.info[mb - mb_w]).ref;
-    if (n.refB == 0) { ld_q(&sd.mv4[mb - mb_w], 2, n.b[0]); ld_q(&sd.mv4[mb - mb_w], 3, n.b[1]); }
-    if (c.mbx + 1 < mb_w) {
-      n.refC = ld_info(&sd.info[mb - mb_w + 1]).ref;
-      if (n.refC == 0) ld_q(&sd.mv4[mb - mb_w + 1], 2, n.cc);
-    }
-    if (c.mbx > 0) {
-      n.refD = ld_info(&sd.info[mb - mb_w - 1]).ref;
-      if (n.refD == 0) ld_q(&sd.mv4[mb - mb_w - 1], 3, n.d);
-    }
+  return w;
+}
+__device__ __forceinline__ void store_nb(uint32_t w) {
+  const int lane = lane_id();
+  const int ref = (int8_t)(w & 255u);
+  const int r = __shfl_sync(FULL, ref, lane < 8 ? max(lane - 4, 0) >> 1 : min(lane - 6, 3));  // the vector's macroblock
+  static_assert(sizeof(MbNb) == 16 * 4, "four refs, then six vectors");
+  int* n = (int*)&ss.nb;
+  if (lane < 4) n[lane] = ref;
+  else if (lane < 10) {
+    n[4 + 2 * (lane - 4)] = r == 0 ? lo16((int)w) : 0;
+    n[5 + 2 * (lane - 4)] = r == 0 ? (int)w >> 16 : 0;
   }
-  return n;
+  __syncwarp();
 }
 // The 4x4 block at (bx, by) in 4x4 units relative to the macroblock (-1..4); own[q] / done bit q:
 // this macroblock's quadrants already decided in the current partition type.
@@ -137,144 +134,156 @@ __device__ __forceinline__ uint32_t vec_cost(int dx, int dy, uint32_t lambda) {
 // Integer search over [xlo, xhi] x [ylo, yhi]. Lanes take columns xlo + lane + 32 j; the reference
 // rows of 8 vector rows (band) are staged in shared memory, and each lane slides its column's
 // 16 x 16 comparison down the band, a reference row at a time against the source rows it pairs
-// with. best_x / best_y / best_c: the nine parts' results (identical in every lane).
+// with. Up to four columns past the last whole group (a window of 2 R + 1 vectors has one) go a vector
+// to a lane instead of a group of their own. Costs and raster indices share a word (cost <= 65280 +
+// 91 * 66 < 2^17, index < 129^2 < 2^15), so the first least one is a minimum. ss.ib: the nine parts'
+// results. (A group for the odd column, a compare of cost and index, source and reference by single
+// words: 284 k cycles a macroblock at range 32.)
 __device__ __forceinline__ uint32_t lds4u(const uint8_t* p) {
   uintptr_t a = (uintptr_t)p;
   const uint32_t* b = (const uint32_t*)(a & ~(uintptr_t)3);
   return __funnelshift_r(b[0], b[1], (uint32_t)(a & 3) * 8u);
 }
-// A window of at most 32 vectors (the learned form's): lane v takes vector v in raster order and
-// sums its four quadrant SADs over the staged band; the same costs and ties as the wide search.
-__device__ __noinline__ void int_search_small(const Ctx c, int xlo, int xhi, int ylo,
-                                              int yhi, int mvp0, int mvp1, uint32_t lambda) {
-  IntBest& ib = ss.ib;
-  const int lane = lane_id();
-  const int x0 = c.mbx * 16, y0 = c.mby * 16, stride = sm.fp.stride_y;
-  const uint8_t* ref = sm.sd.ref_y;
-  const int xs = (x0 + xlo) & ~3;
-  const int bw = ((x0 + xhi + 20 - xs) + 3) & ~3;
-  const int nwx = xhi - xlo + 1, nwy = yhi - ylo + 1, wpr = bw >> 2;
+constexpr int kKeyBits = 15;  // of the raster index
+static_assert((2 * kMaxSearchRange + 1) * (2 * kMaxSearchRange + 1) <= 1 << kKeyBits, "raster index");
+constexpr int kPitch = 36;    // bytes of a staged row of stage_rows: consecutive rows in different banks
+// The 32 bytes from column xs (a multiple of 4) of n picture rows from row y into the band.
+__device__ __forceinline__ void stage_rows(int xs, int y, int n) {
+  const int lane = lane_id(), k = lane & 7;
+  const uint8_t* p = sm.sd.ref_y + (long)y * sm.fp.stride_y + xs + 4 * k;
   __syncwarp();
-  for (int w = lane; w < (nwy + 15) * wpr; w += 32) {
-    const int r = w / wpr, k = w - r * wpr;
-    ((uint32_t*)ss.band)[r * wpr + k] = ldw32(ref + (long)(y0 + ylo + r) * stride + xs + 4 * k);
-  }
+#pragma unroll 6
+  for (int r = lane >> 3; r < n; r += 4) *(uint32_t*)(ss.band + r * kPitch + 4 * k) = ldw32(p + (long)r * sm.fp.stride_y);
   __syncwarp();
-  const bool act = lane < nwx * nwy;
-  const int vx = act ? lane % nwx : 0, vy = act ? lane / nwx : 0;
-  const int dx = xlo + vx, dy = ylo + vy;
-  const uint8_t* rp = ss.band + vy * bw + (x0 + dx - xs);
+}
+// Keys of the nine parts (minimum kept) at the vector whose quadrant SADs are q; mci: its vector cost
+// and index.
+__device__ __forceinline__ void part_keys(uint32_t (&key)[9], uint32_t q0, uint32_t q1, uint32_t q2, uint32_t q3, uint32_t mci) {
+  const uint32_t t = q0 + q1, b = q2 + q3;
+  const uint32_t part[9] = {t + b, t, b, q0 + q2, q1 + q3, q0, q1, q2, q3};
+#pragma unroll
+  for (int k = 0; k < 9; k++) key[k] = min(key[k], (part[k] << kKeyBits) + mci);
+}
+// The same for a lane's own vector over the rows of stage_rows: its 16 x 16 block starts at byte `at`.
+__device__ __noinline__ uint4 quad_sads(int at) {
+  const uint32_t* p = (const uint32_t*)(ss.band + (at & ~3));
+  const uint32_t sh = (uint32_t)(at & 3) * 8u;
   uint32_t q[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
-  for (int r = 0; r < 16; r++) {
-    const uint32_t* sp = (const uint32_t*)&sm.src_y[r * 16];
-    const uint8_t* rr = rp + r * bw;
-    const int h = (r >> 3) * 2;
-    q[h] = __vsadu4(lds4u(rr), sp[0]) + __vsadu4(lds4u(rr + 4), sp[1]) + q[h];
-    q[h + 1] = __vsadu4(lds4u(rr + 8), sp[2]) + __vsadu4(lds4u(rr + 12), sp[3]) + q[h + 1];
-  }
-  const uint32_t mc = lambda * se_bits(4 * dx - mvp0) + lambda * se_bits(4 * dy - mvp1);
-  const uint32_t part[9] = {q[0] + q[1] + q[2] + q[3], q[0] + q[1], q[2] + q[3], q[0] + q[2], q[1] + q[3],
-                            q[0], q[1], q[2], q[3]};
-#pragma unroll
-  for (int k = 0; k < 9; k++) {
-    const uint32_t cost = act ? part[k] + mc : UMAX;
-    const uint32_t m = __reduce_min_sync(FULL, cost);
-    const uint32_t i = __reduce_min_sync(FULL, act && cost == m ? (uint32_t)lane : 0xffffffffu);
-    ib.c[k] = m;
-    ib.x[k] = xlo + (int)(i % (uint32_t)nwx);
-    ib.y[k] = ylo + (int)(i / (uint32_t)nwx);
-  }
+  for (int h = 0; h < 2; h++)
+#pragma unroll 4
+    for (int r = 8 * h; r < 8 * h + 8; r++) {
+      const uint4 s = *(const uint4*)&sm.src_y[r * 16];
+      const uint32_t* w = p + r * (kPitch / 4);
+      const uint32_t w0 = w[0], w1 = w[1], w2 = w[2], w3 = w[3], w4 = w[4];
+      q[2 * h] = __vsadu4(__funnelshift_r(w0, w1, sh), s.x) + __vsadu4(__funnelshift_r(w1, w2, sh), s.y) + q[2 * h];
+      q[2 * h + 1] = __vsadu4(__funnelshift_r(w2, w3, sh), s.z) + __vsadu4(__funnelshift_r(w3, w4, sh), s.w) + q[2 * h + 1];
+    }
+  return make_uint4(q[0], q[1], q[2], q[3]);
 }
-
 __device__ __noinline__ void int_search(const Ctx c, int xlo, int xhi, int ylo, int yhi,
                                         int mvp0, int mvp1, uint32_t lambda) {
-  IntBest& ib = ss.ib;
-  if ((xhi - xlo + 1) * (yhi - ylo + 1) <= 32) {
-    int_search_small(c, xlo, xhi, ylo, yhi, mvp0, mvp1, lambda);
-    return;
-  }
-  const FrameParams& fp = sm.fp;
   const int lane = lane_id();
-  const int x0 = c.mbx * 16, y0 = c.mby * 16, stride = fp.stride_y;
-  const uint8_t* ref = sm.sd.ref_y;
-  const int xs = (x0 + xlo) & ~3;                        // picture column of band column 0
-  const int bw = ((x0 + xhi + 20 - xs) + 3) & ~3;        // band row bytes
-  const int nwx = xhi - xlo + 1;
-  uint32_t bc[9];
-  int bi[9];
+  const int x0 = c.mbx * 16, y0 = c.mby * 16;
+  const int nwx = xhi - xlo + 1, nwy = yhi - ylo + 1;
+  uint32_t key[9];
 #pragma unroll
-  for (int k = 0; k < 9; k++) { bc[k] = UMAX; bi[k] = 0x7fffffff; }
-  for (int dy0 = ylo; dy0 <= yhi; dy0 += kBandRows) {
-    const int rows = min(kBandRows, yhi - dy0 + 1) + 15;
-    // stage reference rows y0 + dy0 .. + rows - 1, columns xs .. xs + bw - 1 (4-byte loads)
-    __syncwarp();
-    const int wpr = bw >> 2;
-    for (int w = lane; w < rows * wpr; w += 32) {
-      int r = w / wpr, k = w - r * wpr;
-      ((uint32_t*)ss.band)[r * wpr + k] = ldw32(ref + (long)(y0 + dy0 + r) * stride + xs + 4 * k);
-    }
-    __syncwarp();
-    for (int j = 0; j * 32 < nwx; j++) {
-      const int dx = xlo + lane + 32 * j;
-      const bool act = lane + 32 * j < nwx;
-      const int co = act ? x0 + dx - xs : 0;
-      uint32_t top[kBandRows][2];
+  for (int k = 0; k < 9; k++) key[k] = UMAX;
+  // a window of at most 32 vectors (the learned form's), or the columns past the last whole group: `cols`
+  // columns from xt, a lane a vector, as many rows at a time as fit
+  const bool small = nwx <= 8 && nwx * nwy <= 32;
+  const int rem = nwx & 31, cols = small ? nwx : (rem <= 4 ? rem : 0), xt = xhi - cols + 1, groups = (nwx - cols + 31) >> 5;
+  if (groups) {
+    const int stride = sm.fp.stride_y;
+    const uint8_t* ref = sm.sd.ref_y;
+    const int xs = (x0 + xlo) & ~3;                          // picture column of band column 0
+    const int bw = ((x0 + xhi - cols + 20 - xs) + 3) & ~3;   // band row bytes
+#pragma unroll 1
+    for (int dy0 = ylo; dy0 <= yhi; dy0 += kBandRows) {
+      const int rows = min(kBandRows, yhi - dy0 + 1) + 15;
+      // stage reference rows y0 + dy0 .. + rows - 1, columns xs .. xs + bw - 1 (4-byte loads)
+      __syncwarp();
+      const int wpr = bw >> 2;
+#pragma unroll 4
+      for (int w = lane; w < rows * wpr; w += 32) {
+        int r = w / wpr, k = w - r * wpr;
+        ((uint32_t*)ss.band)[r * wpr + k] = ldw32(ref + (long)(y0 + dy0 + r) * stride + xs + 4 * k);
+      }
+      __syncwarp();
+#pragma unroll 1
+      for (int j = 0; j < groups; j++) {
+        const int dx = xlo + lane + 32 * j;
+        const bool act = dx < xt;
+        const int co = act ? x0 + dx - xs : 0;
+        const uint32_t sh = (uint32_t)(co & 3) * 8u;
+        uint32_t top[kBandRows][2], acc[kBandRows][2] = {};
+#pragma unroll 1
+        for (int half = 0; half < 2; half++) {
+          uint4 s[8];
 #pragma unroll
-      for (int half = 0; half < 2; half++) {
-        uint32_t s[8][4];
-#pragma unroll
-        for (int r = 0; r < 8; r++)
-#pragma unroll
-          for (int k = 0; k < 4; k++) s[r][k] = *(const uint32_t*)&sm.src_y[(half * 8 + r) * 16 + 4 * k];
-        uint32_t acc[kBandRows][2];
-#pragma unroll
-        for (int d = 0; d < kBandRows; d++) acc[d][0] = acc[d][1] = 0;
-#pragma unroll
-        for (int i = 0; i < kBandRows + 7; i++) {
-          // reference row half * 8 + i of the band pairs with source row r = i - d for d = 0..7
-          const uint8_t* rp = ss.band + (half * 8 + i) * bw + co;
-          uint32_t R0 = lds4u(rp), R1 = lds4u(rp + 4), R2 = lds4u(rp + 8), R3 = lds4u(rp + 12);
+          for (int r = 0; r < 8; r++) s[r] = *(const uint4*)&sm.src_y[(half * 8 + r) * 16];
 #pragma unroll
           for (int d = 0; d < kBandRows; d++) {
-            const int r = i - d;
-            if (r < 0 || r > 7) continue;
-            acc[d][0] = __vsadu4(R0, s[r][0]) + __vsadu4(R1, s[r][1]) + acc[d][0];
-            acc[d][1] = __vsadu4(R2, s[r][2]) + __vsadu4(R3, s[r][3]) + acc[d][1];
+            top[d][0] = acc[d][0];
+            top[d][1] = acc[d][1];
+            acc[d][0] = acc[d][1] = 0;
           }
-        }
-        if (half == 0) {
+          const uint32_t* rp = (const uint32_t*)(ss.band + half * 8 * bw + (co & ~3));
 #pragma unroll
-          for (int d = 0; d < kBandRows; d++) { top[d][0] = acc[d][0]; top[d][1] = acc[d][1]; }
-        } else {
-          const uint32_t cx = lambda * se_bits(4 * dx - mvp0);
+          for (int i = 0; i < kBandRows + 7; i++) {
+            // reference row half * 8 + i of the band pairs with source row r = i - d for d = 0..7
+            const uint32_t w0 = rp[0], w1 = rp[1], w2 = rp[2], w3 = rp[3], w4 = rp[4];
+            rp += wpr;
+            const uint32_t R0 = __funnelshift_r(w0, w1, sh), R1 = __funnelshift_r(w1, w2, sh), R2 = __funnelshift_r(w2, w3, sh),
+                           R3 = __funnelshift_r(w3, w4, sh);
 #pragma unroll
-          for (int d = 0; d < kBandRows; d++) {
-            const int dy = dy0 + d;
-            if (!act || dy > yhi) continue;
-            const uint32_t mc = cx + lambda * se_bits(4 * dy - mvp1);
-            const uint32_t q0 = top[d][0], q1 = top[d][1], q2 = acc[d][0], q3 = acc[d][1];
-            const uint32_t part[9] = {q0 + q1 + q2 + q3, q0 + q1, q2 + q3, q0 + q2, q1 + q3, q0, q1, q2, q3};
-            const int idx = (dy - ylo) * nwx + (dx - xlo);
-#pragma unroll
-            for (int k = 0; k < 9; k++) {
-              const uint32_t cost = part[k] + mc;
-              if (cost < bc[k] || (cost == bc[k] && idx < bi[k])) { bc[k] = cost; bi[k] = idx; }
+            for (int d = 0; d < kBandRows; d++) {
+              const int r = i - d;
+              if (r < 0 || r > 7) continue;
+              acc[d][0] = __vsadu4(R0, s[r].x) + __vsadu4(R1, s[r].y) + acc[d][0];
+              acc[d][1] = __vsadu4(R2, s[r].z) + __vsadu4(R3, s[r].w) + acc[d][1];
             }
           }
         }
+        const uint32_t cx = lambda * se_bits(4 * dx - mvp0);
+        uint32_t idx = (uint32_t)((dy0 - ylo) * nwx + (dx - xlo));
+#pragma unroll
+        for (int d = 0; d < kBandRows; d++, idx += nwx)
+          if (act && dy0 + d <= yhi)
+            part_keys(key, top[d][0], top[d][1], acc[d][0], acc[d][1],
+                      ((cx + lambda * se_bits(4 * (dy0 + d) - mvp1)) << kKeyBits) + idx);
       }
     }
   }
-  // first minimum in raster order across the warp
+  if (cols) {
+    const int vrows = 32 / cols, vy = lane / cols, vx = lane - vy * cols;
+    const int xs = (x0 + xt) & ~3, dx = xt + vx;
+    const uint32_t cx = lambda * se_bits(4 * dx - mvp0);
+#pragma unroll 1
+    for (int dy0 = ylo; dy0 <= yhi; dy0 += vrows) {
+      const int n = min(vrows, yhi - dy0 + 1), dy = dy0 + vy;
+      stage_rows(xs, y0 + dy0, n + 15);
+      const bool act = vy < n;
+      const uint4 q = quad_sads(act ? vy * kPitch + (x0 + dx - xs) : 0);
+      if (act)
+        part_keys(key, q.x, q.y, q.z, q.w, ((cx + lambda * se_bits(4 * dy - mvp1)) << kKeyBits) + (uint32_t)((dy - ylo) * nwx + (dx - xlo)));
+    }
+  }
+  // the least across the warp; lane k < 9 writes part k's
+  uint32_t mine = 0;
 #pragma unroll
   for (int k = 0; k < 9; k++) {
-    uint32_t m = __reduce_min_sync(FULL, bc[k]);
-    uint32_t i = __reduce_min_sync(FULL, bc[k] == m ? (uint32_t)bi[k] : 0xffffffffu);
-    ib.c[k] = m;
-    ib.x[k] = xlo + (int)(i % (uint32_t)nwx);
-    ib.y[k] = ylo + (int)(i / (uint32_t)nwx);
+    const uint32_t m = __reduce_min_sync(FULL, key[k]);
+    if (lane == k) mine = m;
   }
+  __syncwarp();
+  if (lane < 9) {
+    const int i = (int)(mine & ((1u << kKeyBits) - 1u)), y = i / nwx;
+    ss.ib.c[lane] = mine >> kKeyBits;
+    ss.ib.x[lane] = xlo + i - y * nwx;
+    ss.ib.y[lane] = ylo + y;
+  }
+  __syncwarp();
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -369,48 +378,55 @@ __device__ __noinline__ PartFit refine_part(const Ctx c, int px, int py, int pw,
   return PartFit{best_key >> 4, cx, cy};
 }
 
-// Learned form: refinement of one part from its integer best (bx, by) by SAD -- the half-sample
-// diamond (up, left, right, down at distance 2, one step), then the quarter-sample diamond (the
-// same at distance 1, up to two steps, each from the step's start), cost SAD + lambda * vector bits
-// against the part's predictor, the first strict minimum in that order; lanes take the part's
-// 4-sample words.
-// This lane's share of the part's SAD at the vector (dx, dy) from the window's position: the part's
-// 4-sample words lane, lane + 32 (shift: log2 of the words per row).
-__device__ __noinline__ uint32_t part_sad(int at, int src, int shift, int nw, int dx, int dy) {
-  const int lane = lane_id();
-  const uint32_t e = sm.qpt[(dx & 3) | ((dy & 3) << 2)];
-  const uint8_t* p = &sm.win[0] + qpel_pos(dx, dy) + at;
-  uint32_t s = 0;
-  for (int w = lane; w < nw; w += 32) {
-    const int r = w >> shift, x = (w - (r << shift)) * 4;
-    const uint8_t* q = p + r * 24 + x;
-    s = __vsadu4(__vavgu4(lds4u(q + (e & 0xffffu)), lds4u(q + (e >> 16))), *(const uint32_t*)&sm.src_y[src + r * 16 + x]) + s;
-  }
-  return s;
-}
+// Learned form: refinement of one part from its integer best (bx, by), whose SAD is sad0, by SAD -- the
+// half-sample diamond (up, left, right, down at distance 2, one step), then the quarter-sample diamond
+// (the same at distance 1, up to two steps, each from the step's start), cost SAD + lambda * vector bits
+// against the part's predictor, the first strict minimum in that order. Eight lanes a neighbour, each
+// every eighth of the part's 4-sample words, and planes built when a step reads them. (The neighbours one
+// after the other over the whole warp, every plane for every part: 86 k cycles for the refinement of a
+// macroblock.)
 __device__ __noinline__ PartFit refine_part_sad(const Ctx c, int px, int py, int pw, int ph,
-                                                int bx, int by, int2 mvp, uint32_t lambda, Bounds bd) {
-  ensure_mb_window(c, bx, by);
-  const int at = py * 24 + px, src = py * 16 + px, shift = pw == 16 ? 2 : 1, nw = (pw * ph) >> 2;
+                                                int bx, int by, int2 mvp, uint32_t lambda, Bounds bd, uint32_t sad0) {
+  const int lane = lane_id(), k = lane >> 3, shift = pw == 16 ? 2 : 1, nw = (pw * ph) >> 2;
   const int m0x = 4 * bx, m0y = 4 * by;
-  uint32_t best = wsum(part_sad(at, src, shift, nw, 0, 0)) + vec_cost(m0x - mvp.x, m0y - mvp.y, lambda);
+  uint32_t best = sad0 + vec_cost(m0x - mvp.x, m0y - mvp.y, lambda);
   const Box box{max(bd.min0, m0x - 3), min(bd.max0, m0x + 3), max(bd.min1, m0y - 3), min(bd.max1, m0y + 3)};
+  // the lane's words: rows r0, r0 + dr, .. (8 words are two rows of a 16-sample part, four of an 8-sample one)
+  const int r0 = (lane & 7) >> shift, x = ((lane & 7) & ((1 << shift) - 1)) * 4, dr = 8 >> shift;
+  const int at = (py + r0) * 24 + px + x;
+  const uint8_t* const sp = &sm.src_y[(py + r0) * 16 + px + x];
   int q0 = 0, q1 = 0;
 #pragma unroll 1
   for (int it = 0; it < 3; it++) {
+    // the half-sample step reads planes b and h; so do quarter-sample steps from the integer position
+    // itself; those around another read j too
+    if (it < 2) ensure_window(c.mbx * 16 + bx, c.mby * 16 + by, q0 | q1 ? 7 : 3);
     const int st = it == 0 ? 2 : 1;
-    uint32_t sums = 0, s01 = 0;  // neighbours k = 3, 2 (right, down), then 1, 0
+    const int dx = q0 + (k == 1 ? -st : (k == 2 ? st : 0)), dy = q1 + (k == 0 ? -st : (k == 3 ? st : 0));
+    const uint32_t e = sm.qpt[(dx & 3) | ((dy & 3) << 2)];
+    const uint8_t* const p = &sm.win[0] + qpel_pos(dx, dy) + at;
+    const uint8_t *pa = p + (e & 0xffffu), *pb = p + (e >> 16), *s = sp;
+    uint32_t sad = 0;
 #pragma unroll 1
-    for (int k = 3; k >= 0; k--) {
-      if (k == 1) { s01 = sums; sums = 0; }
-      sums = (sums << 16) | part_sad(at, src, shift, nw, q0 + (k == 1 ? -st : (k == 2 ? st : 0)), q1 + (k == 0 ? -st : (k == 3 ? st : 0)));
+    for (int w = 0; w < nw; w += 16) {
+#pragma unroll
+      for (int u = 0; u < 2; u++)
+        sad = __vsadu4(__vavgu4(lds4u(pa + u * dr * 24), lds4u(pb + u * dr * 24)), *(const uint32_t*)(s + u * dr * 16)) + sad;
+      pa += 48 * dr;
+      pb += 48 * dr;
+      s += 32 * dr;
     }
-    const uint32_t key = best4(sums, s01, m0x + q0, m0y + q1, st, box, mvp.x, mvp.y, lambda, true);
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) sad += __shfl_xor_sync(FULL, sad, o);
+    const int vx = m0x + dx, vy = m0y + dy;
+    const bool ok = vx >= box.lo0 && vx <= box.hi0 && vy >= box.lo1 && vy <= box.hi1;
+    const uint32_t cost = sad + vec_cost(vx - mvp.x, vy - mvp.y, lambda);
+    const uint32_t key = __reduce_min_sync(FULL, ok ? (cost << 2) | (uint32_t)k : UMAX);
     if ((key >> 2) < best) {
       best = key >> 2;
-      const int k = (int)(key & 3u);
-      q0 += k == 1 ? -st : (k == 2 ? st : 0);
-      q1 += k == 0 ? -st : (k == 3 ? st : 0);
+      const int b = (int)(key & 3u);
+      q0 += b == 1 ? -st : (b == 2 ? st : 0);
+      q1 += b == 0 ? -st : (b == 3 ? st : 0);
     } else if (it) {
       break;
     }
@@ -444,14 +460,8 @@ __device__ __noinline__ void mc_chroma_q(const Ctx c) {
   const int q = (r >> 2) * 2 + (c0 >> 2);
   const int mvx = ss.qmv[q][0], mvy = ss.qmv[q][1];
   const int cx = c.mbx * 8 + c0 + (mvx >> 3), cy = c.mby * 8 + r + (mvy >> 3), fx = mvx & 7, fy = mvy & 7;
-  const int wa = (8 - fx) * (8 - fy), wb = fx * (8 - fy), wc = (8 - fx) * fy, wd = fx * fy;
-  const uint8_t* src = (plane ? sd.ref_v : sd.ref_u) + (long)cy * fp.stride_c + cx;
-  uint8_t* out = (plane ? sm.pred_v : sm.pred_u) + r * 8 + c0;
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    int a = ldcg_u8(src + k), b = ldcg_u8(src + k + 1), cc = ldcg_u8(src + fp.stride_c + k), d = ldcg_u8(src + fp.stride_c + k + 1);
-    out[k] = (uint8_t)((wa * a + wb * b + wc * cc + wd * d + 32) >> 6);
-  }
+  *(uint32_t*)((plane ? sm.pred_v : sm.pred_u) + r * 8 + c0) =
+      chroma4((plane ? sd.ref_v : sd.ref_u) + (long)cy * fp.stride_c + cx, fp.stride_c, fx, fy);
   __syncwarp();
 }
 
@@ -500,15 +510,19 @@ __device__ __noinline__ int2 learned_centre(const Ctx c, int mvp0, int mvp1, uin
   uint2 r[kCentreCands];
 #pragma unroll
   for (int k = 0; k < kCentreCands; k++) r[k] = k < n && ok[k] ? ldg8(base + (long)cy[k] * stride + cx[k]) : make_uint2(0u, 0u);
-  uint32_t best = UMAX;
-  bx = cx[0];
-  by = cy[0];
+  // two SADs to a word (each fits 16 bits); lane k costs candidate k
+  uint32_t sad = 0;
 #pragma unroll
-  for (int k = 0; k < kCentreCands; k++) {
-    if (k >= n || !ok[k]) continue;  // uniform across the warp
-    const uint32_t cost = fullpel_cost(sv, r[k], cx[k], cy[k], mvp0, mvp1, lambda);
-    if (cost < best) { best = cost; bx = cx[k]; by = cy[k]; }
+  for (int k = 0; k < kCentreCands; k += 2) {
+    const uint32_t w = wsum(vsad8(sv, r[k]) | (k + 1 < kCentreCands ? vsad8(sv, r[min(k + 1, kCentreCands - 1)]) << 16 : 0u));
+    if ((lane >> 1) == (k >> 1)) sad = (w >> (16 * (lane & 1))) & 0xffffu;
   }
+  const int k = min(lane, kCentreCands - 1);
+  const uint32_t cost = sad + mvd_cost(cx[k] * 4 - mvp0, lambda) + mvd_cost(cy[k] * 4 - mvp1, lambda);
+  const uint32_t key = __reduce_min_sync(FULL, lane < n && ok[k] ? (cost << 3) | (uint32_t)lane : UMAX);
+  const int b = key == UMAX ? 0 : (int)(key & 7u);
+  bx = cx[b];
+  by = cy[b];
   return make_int2(bx, by);
 }
 
@@ -538,9 +552,10 @@ __device__ __noinline__ bool analyse_p_mb_search(const Ctx c, const PipeWait pw)
   // Warp-uniform state (every lane computes the same values) is held once per warp in shared memory
   // (SearchSmem) instead of once per lane on the stack; every lane writes the same value, and a
   // __syncwarp before each rewrite keeps a lane from overwriting what a slower lane still reads.
-  MbNb& nb = ss.nb;
   __syncwarp();
-  nb = load_nb(c);
+  const uint32_t nw = load_nb(c);
+  load_source(c);
+  store_nb(nw);
   const int2 p16 = mv_pred(0, 0, 4, 0, 0);
   const int mvp16[2] = {p16.x, p16.y};
   int ps0 = mvp16[0], ps1 = mvp16[1];
@@ -551,7 +566,6 @@ __device__ __noinline__ bool analyse_p_mb_search(const Ctx c, const PipeWait pw)
       ps1 = 0;
     }
   }
-  load_source(c);
   const rg_mb_hint* hint = sd.hint ? sd.hint + c.mb : nullptr;
   // integer window: full search, or the learned seed's small window
   const int R = sd.search_range;
@@ -643,7 +657,8 @@ __device__ __noinline__ bool analyse_p_mb_search(const Ctx c, const PipeWait pw)
     for (int k = 0; k < np; k++) {
       const int8_t* g = c_parts[first + k];
       const int2 mvp = mv_pred(g[4], g[5], g[6], g[7], done);
-      const PartFit fit = hint ? refine_part_sad(c, g[0], g[1], g[2], g[3], ib.x[g[8]], ib.y[g[8]], mvp, lambda, bd)
+      const PartFit fit = hint ? refine_part_sad(c, g[0], g[1], g[2], g[3], ib.x[g[8]], ib.y[g[8]], mvp, lambda, bd,
+                                                 ib.c[g[8]] - vec_cost(4 * ib.x[g[8]] - mvp16[0], 4 * ib.y[g[8]] - mvp16[1], lambda))
                                : refine_part(c, g[0], g[1], g[2], g[3], ib.x[g[8]], ib.y[g[8]], mvp, lambda, bd);
       const int mv[2] = {fit.x, fit.y};
       J += fit.cost;
