@@ -28,22 +28,19 @@
 // (those of them available at the block, DC when none is).
 
 constexpr int kBandRows = 8;               // integer vectors per band row
-constexpr int kBandBytes = (kBandRows + 15) * (2 * kMaxSearchRange + 28);
+constexpr int kBandBytes = 4 * kBandRows * (2 * kMaxSearchRange + 24);  // four chunks of kBandRows rows
 constexpr int kLearnedRange = 2;           // learned form: integer window around the seed
 constexpr int kCentreCands = 7;            // learned form: candidates of the window's centre
 
 
-// A neighbouring 4x4 block for motion prediction: ref -2 not available, -1 intra, 0 inter.
+// The quadrants around and in the current macroblock that motion prediction reads, by index 4 (row + 1) +
+// column + 1 (columns -1 .. 2, rows -1 .. 1): D B0 B1 C / A0 0 1 - / A1 2 3 -. ref -2 not available (or not
+// yet decided), -1 intra, 0 inter; mv packed, 0 unless inter.
 struct NbMv {
-  int ref, x, y;
-};
-// The neighbours of the current macroblock in the quadrant grid.
-struct MbNb {
-  int refA, refB, refC, refD;
-  int a[2][2];   // left macroblock: quadrants 1 (rows 0-1) and 3 (rows 2-3)
-  int b[2][2];   // top macroblock: quadrants 2 (columns 0-1) and 3 (columns 2-3)
-  int cc[2];     // top-right macroblock: quadrant 2
-  int d[2];      // top-left macroblock: quadrant 3
+  uint32_t mv;
+  int ref;
+  __device__ __forceinline__ int x() const { return lo16((int)mv); }
+  __device__ __forceinline__ int y() const { return (int)mv >> 16; }
 };
 struct IntBest {
   int x[9], y[9];
@@ -52,8 +49,9 @@ struct IntBest {
 struct SearchSmem {
   uint8_t band[kBandBytes];
   IntBest ib;
-  MbNb nb;
-  int bmv[4][2], bmvd[4][2], own[4][2], pm[4][2], pd[4][2], qmv[4][2];
+  alignas(8) NbMv nb[12];
+  int qmv[4][2];
+  uint32_t pmvd[4];    // the chosen type's parts' vector differences
   int ccx[8], ccy[8];  // the learned form's centre candidates (ok: cok)
   bool cok[8];
 };
@@ -61,7 +59,7 @@ struct SearchSmem {
 static_assert(sizeof(Smem) % 16 == 0, "SearchSmem follows aligned");
 #define ss (((SearchSmem*)(smw + blockDim.y * sizeof(Smem)))[threadIdx.y])
 // The neighbours into ss.nb, all loads in flight together: lanes 0..3 the refs of the left, top,
-// top-right and top-left macroblocks, lanes 4..9 the six vectors (a[0], a[1], b[0], b[1], cc, d).
+// top-right and top-left macroblocks, lanes 4..9 the vectors A0, A1, B0, B1, C, D.
 __device__ __forceinline__ uint32_t load_nb(const Ctx c) {
   const StreamDev& sd = sm.sd;
   const int lane = lane_id(), mb_w = sm.fp.mb_w;
@@ -79,46 +77,34 @@ __device__ __forceinline__ void store_nb(uint32_t w) {
   const int lane = lane_id();
   const int ref = (int8_t)(w & 255u);
   const int r = __shfl_sync(FULL, ref, lane < 8 ? max(lane - 4, 0) >> 1 : min(lane - 6, 3));  // the vector's macroblock
-  static_assert(sizeof(MbNb) == 16 * 4, "four refs, then six vectors");
-  int* n = (int*)&ss.nb;
-  if (lane < 4) n[lane] = ref;
-  else if (lane < 10) {
-    n[4 + 2 * (lane - 4)] = r == 0 ? lo16((int)w) : 0;
-    n[5 + 2 * (lane - 4)] = r == 0 ? (int)w >> 16 : 0;
-  }
+  if (lane >= 4 && lane < 10) ss.nb[(int)((0x032184u >> (4 * (lane - 4))) & 15u)] = NbMv{r == 0 ? w : 0u, r};
+  if (lane == 10 || lane == 11) ss.nb[lane == 10 ? 7 : 11] = NbMv{0u, -2};
   __syncwarp();
 }
-// The 4x4 block at (bx, by) in 4x4 units relative to the macroblock (-1..4); own[q] / done bit q:
-// this macroblock's quadrants already decided in the current partition type.
-__device__ __forceinline__ NbMv nb4(int bx, int by, int done) {
-  const MbNb& n = ss.nb;
-  if (bx >= 0 && bx < 4 && by >= 0 && by < 4) {
-    int q = (by >> 1) * 2 + (bx >> 1);
-    if ((done >> q) & 1) return {0, ss.own[q][0], ss.own[q][1]};
-    return {-2, 0, 0};
-  }
-  if (bx == -1 && by == -1) return {n.refD, n.d[0], n.d[1]};
-  if (bx == -1 && by >= 0 && by < 4) return {n.refA, n.a[by >> 1][0], n.a[by >> 1][1]};
-  if (by == -1 && bx >= 0 && bx < 4) return {n.refB, n.b[bx >> 1][0], n.b[bx >> 1][1]};
-  if (by == -1 && bx == 4) return {n.refC, n.cc[0], n.cc[1]};
-  return {-2, 0, 0};  // right of or below the macroblock: not decoded yet
-}
-// Motion vector predictor of the partition whose top-left 4x4 block is (bx, by) and width pw (4x4
-// units), H.264 8.4.1.3; dir 1 16x8 top, 2 16x8 bottom, 3 8x16 left, 4 8x16 right, 0 median only.
-__device__ __noinline__ int2 mv_pred(int bx, int by, int pw, int dir, int done) {
-  NbMv A = nb4(bx - 1, by, done), B = nb4(bx, by - 1, done), C = nb4(bx + pw, by - 1, done);
-  if (C.ref == -2) C = nb4(bx - 1, by - 1, done);
-  if (dir == 1 && B.ref == 0) return make_int2(B.x, B.y);
-  if ((dir == 2 || dir == 3) && A.ref == 0) return make_int2(A.x, A.y);
-  if (dir == 4 && C.ref == 0) return make_int2(C.x, C.y);
-  if (B.ref == -2 && C.ref == -2 && A.ref != -2) return make_int2(A.x, A.y);
-  int m = (A.ref == 0) + (B.ref == 0) + (C.ref == 0);
-  if (m == 1) {
-    const NbMv& o = A.ref == 0 ? A : (B.ref == 0 ? B : C);
-    return make_int2(o.x, o.y);
-  }
+// Partition parts 0..8 in coding order: 16x16 | 16x8 top, bottom | 8x16 left, right | 8x8. Their neighbours A,
+// B, C, D as indices into ss.nb (4 bits each, A lowest), then the quadrants covered (bits 16..19), the
+// directional rule (bits 20..21: 1 B, 2 A, 3 C), and x / 8, y / 8, width 8, height 8 (bits 24..27).
+__device__ __constant__ uint32_t c_part[9] = {
+    0x00000314u | 15u << 16,
+    0x00000314u | 3u << 16 | 1u << 20 | 8u << 24, 0x00004758u | 12u << 16 | 2u << 20 | (2u | 8u) << 24,
+    0x00000214u | 5u << 16 | 2u << 20 | 4u << 24, 0x00001325u | 10u << 16 | 3u << 20 | (1u | 4u) << 24,
+    0x00000214u | 1u << 16 | 12u << 24, 0x00001325u | 2u << 16 | (1u | 12u) << 24,
+    0x00004658u | 4u << 16 | (2u | 12u) << 24, 0x00005769u | 8u << 16 | 15u << 24};
+__device__ __forceinline__ int type_first(int t) { return (0x5310 >> (4 * t)) & 15; }
+__device__ __forceinline__ int type_parts(int t) { return (0x4221 >> (4 * t)) & 15; }
+// Motion vector predictor of a part (H.264 8.4.1.3), packed.
+__device__ __noinline__ uint32_t mv_pred(uint32_t part) {
+  const NbMv A = ss.nb[part & 15u], B = ss.nb[(part >> 4) & 15u], D = ss.nb[(part >> 12) & 15u];
+  NbMv C = ss.nb[(part >> 8) & 15u];
+  if (C.ref == -2) C = D;
+  const int dir = (int)((part >> 20) & 3u);
+  if (dir == 1 && B.ref == 0) return B.mv;
+  if (dir == 2 && A.ref == 0) return A.mv;
+  if (dir == 3 && C.ref == 0) return C.mv;
+  if (B.ref == -2 && C.ref == -2 && A.ref != -2) return A.mv;
+  if ((A.ref == 0) + (B.ref == 0) + (C.ref == 0) == 1) return A.ref == 0 ? A.mv : (B.ref == 0 ? B.mv : C.mv);
   auto med = [](int x, int y, int z) { return min(max(x, y), max(min(x, y), z)); };
-  return make_int2(med(A.x, B.x, C.x), med(A.y, B.y, C.y));
+  return pack16(med(A.x(), B.x(), C.x()), med(A.y(), B.y(), C.y()));
 }
 // A refined part: its cost and quarter-sample vector.
 struct PartFit {
@@ -132,8 +118,8 @@ __device__ __forceinline__ uint32_t vec_cost(int dx, int dy, uint32_t lambda) {
 
 // ---------------------------------------------------------------------------------------------
 // Integer search over [xlo, xhi] x [ylo, yhi]. Lanes take columns xlo + lane + 32 j; the reference
-// rows of 8 vector rows (band) are staged in shared memory, and each lane slides its column's
-// 16 x 16 comparison down the band, a reference row at a time against the source rows it pairs
+// rows of 8 vector rows (band) are staged in shared memory -- four chunks of 8 rows, three of a band and
+// the next band's last one on its way -- and each lane slides its column's 16 x 16 comparison down the band, a reference row at a time against the source rows it pairs
 // with. Up to four columns past the last whole group (a window of 2 R + 1 vectors has one) go a vector
 // to a lane instead of a group of their own. Costs and raster indices share a word (cost <= 65280 +
 // 91 * 66 < 2^17, index < 129^2 < 2^15), so the first least one is a minimum. ss.ib: the nine parts'
@@ -194,21 +180,35 @@ __device__ __noinline__ void int_search(const Ctx c, int xlo, int xhi, int ylo, 
   const bool small = nwx <= 8 && nwx * nwy <= 32;
   const int rem = nwx & 31, cols = small ? nwx : (rem <= 4 ? rem : 0), xt = xhi - cols + 1, groups = (nwx - cols + 31) >> 5;
   if (groups) {
-    const int stride = sm.fp.stride_y;
-    const uint8_t* ref = sm.sd.ref_y;
     const int xs = (x0 + xlo) & ~3;                          // picture column of band column 0
-    const int bw = ((x0 + xhi - cols + 20 - xs) + 3) & ~3;   // band row bytes
+    const int wpr = (x0 + xhi - cols + 23 - xs) >> 2;        // words of a band row
+    // chunk q holds the reference rows y0 + ylo + 8 q ..; its copy in words, lane by lane
+    const int dr = 32 / wpr, dk = 32 - dr * wpr, lr = lane / wpr, lk = lane - lr * wpr;
+    const uint32_t band = (uint32_t)__cvta_generic_to_shared(ss.band);
+    auto stage = [&](int q) {
+      const int n = min(kBandRows, nwy + 15 - kBandRows * q);
+      const uint8_t* src = sm.sd.ref_y + (long)(y0 + ylo + kBandRows * q) * sm.fp.stride_y + xs;
+      const uint32_t dst = band + (uint32_t)((q & 3) * kBandRows * wpr) * 4u;
 #pragma unroll 1
-    for (int dy0 = ylo; dy0 <= yhi; dy0 += kBandRows) {
-      const int rows = min(kBandRows, yhi - dy0 + 1) + 15;
-      // stage reference rows y0 + dy0 .. + rows - 1, columns xs .. xs + bw - 1 (4-byte loads)
-      __syncwarp();
-      const int wpr = bw >> 2;
-#pragma unroll 4
-      for (int w = lane; w < rows * wpr; w += 32) {
-        int r = w / wpr, k = w - r * wpr;
-        ((uint32_t*)ss.band)[r * wpr + k] = ldw32(ref + (long)(y0 + dy0 + r) * stride + xs + 4 * k);
+      for (int r = lr, k = lk; r < n; r += dr) {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + (uint32_t)(r * wpr + k) * 4u),
+                     "l"(src + (long)r * sm.fp.stride_y + 4 * k) : "memory");
+        k += dk;
+        if (k >= wpr) {
+          k -= wpr;
+          r++;
+        }
       }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    __syncwarp();
+    stage(0);
+    stage(1);
+    stage(2);
+#pragma unroll 1
+    for (int dy0 = ylo, b = 0; dy0 <= yhi; dy0 += kBandRows, b++) {
+      stage(b + 3);  // (nothing past the last row)
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
       __syncwarp();
 #pragma unroll 1
       for (int j = 0; j < groups; j++) {
@@ -228,10 +228,12 @@ __device__ __noinline__ void int_search(const Ctx c, int xlo, int xhi, int ylo, 
             top[d][1] = acc[d][1];
             acc[d][0] = acc[d][1] = 0;
           }
-          const uint32_t* rp = (const uint32_t*)(ss.band + half * 8 * bw + (co & ~3));
+          const uint32_t *rp = (const uint32_t*)ss.band + ((b + half) & 3) * kBandRows * wpr + (co >> 2),
+                         *rn = (const uint32_t*)ss.band + ((b + half + 1) & 3) * kBandRows * wpr + (co >> 2);
 #pragma unroll
           for (int i = 0; i < kBandRows + 7; i++) {
             // reference row half * 8 + i of the band pairs with source row r = i - d for d = 0..7
+            if (i == kBandRows) rp = rn;
             const uint32_t w0 = rp[0], w1 = rp[1], w2 = rp[2], w3 = rp[3], w4 = rp[4];
             rp += wpr;
             const uint32_t R0 = __funnelshift_r(w0, w1, sh), R1 = __funnelshift_r(w1, w2, sh), R2 = __funnelshift_r(w2, w3, sh),
@@ -253,7 +255,9 @@ __device__ __noinline__ void int_search(const Ctx c, int xlo, int xhi, int ylo, 
             part_keys(key, top[d][0], top[d][1], acc[d][0], acc[d][1],
                       ((cx + lambda * se_bits(4 * (dy0 + d) - mvp1)) << kKeyBits) + idx);
       }
+      __syncwarp();  // every lane is done with the chunk that is overwritten next
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
   }
   if (cols) {
     const int vrows = 32 / cols, vy = lane / cols, vx = lane - vy * cols;
@@ -291,21 +295,27 @@ __device__ __noinline__ void int_search(const Ctx c, int xlo, int xhi, int ylo, 
 // integer best (bx, by) with predictor mvp. Candidates of one step are evaluated in parallel: slot
 // = candidate * blocks + 4x4 block, each lane the SATD of one block's prediction (from the
 // half-sample planes of a window around the integer best) against the source.
-__device__ __forceinline__ uint32_t satd4_regs(const uint32_t* sa, const uint32_t* pa) {
-  int t[4][4];
+// Half the SATD of a 4x4 block of byte rows (an even number before the halving): columns 0, 2 and 1, 3 packed as
+// hi * 65536 + lo through the column butterflies, |x + y| + |x - y| = 2 max(|x|, |y|) for the last one.
+__device__ __forceinline__ uint32_t half_satd4(const uint32_t* sa, const uint32_t* pa) {
+  int e[4], o[4];
 #pragma unroll
   for (int y = 0; y < 4; y++) {
-    int d[4];
-#pragma unroll
-    for (int x = 0; x < 4; x++) d[x] = (int)((sa[y] >> (8 * x)) & 255) - (int)((pa[y] >> (8 * x)) & 255);
-    int s03 = d[0] + d[3], s12 = d[1] + d[2], d03 = d[0] - d[3], d12 = d[1] - d[2];
-    t[y][0] = s03 + s12; t[y][1] = d03 + d12; t[y][2] = s03 - s12; t[y][3] = d03 - d12;
+    e[y] = (int)(sa[y] & 0x00ff00ffu) - (int)(pa[y] & 0x00ff00ffu);
+    o[y] = (int)__byte_perm(sa[y], 0u, 0x4341) - (int)__byte_perm(pa[y], 0u, 0x4341);
   }
+  auto cols = [](int (&v)[4]) {
+    const int s03 = v[0] + v[3], s12 = v[1] + v[2], d03 = v[0] - v[3], d12 = v[1] - v[2];
+    v[0] = s03 + s12; v[1] = d03 + d12; v[2] = s03 - s12; v[3] = d03 - d12;
+  };
+  cols(e);
+  cols(o);
   uint32_t s = 0;
 #pragma unroll
-  for (int x = 0; x < 4; x++) {
-    int s03 = t[0][x] + t[3][x], s12 = t[1][x] + t[2][x], d03 = t[0][x] - t[3][x], d12 = t[1][x] - t[2][x];
-    s += abs(s03 + s12) + abs(d03 + d12) + abs(s03 - s12) + abs(d03 - d12);
+  for (int y = 0; y < 4; y++) {
+    const int r0 = (int16_t)e[y], r2 = (e[y] + 0x8000) >> 16, r1 = (int16_t)o[y], r3 = (o[y] + 0x8000) >> 16;
+    const int s03 = r0 + r3, s12 = r1 + r2, d03 = r0 - r3, d12 = r1 - r2;
+    s += (uint32_t)(max(abs(s03), abs(s12)) + max(abs(d03), abs(d12)));
   }
   return s;
 }
@@ -354,13 +364,13 @@ __device__ __noinline__ PartFit refine_part(const Ctx c, int px, int py, int pw,
         qpel4(px + ox, py + oy, vx - m0x, vy - m0y, pa);
 #pragma unroll
         for (int r = 0; r < 4; r++) sa[r] = *(const uint32_t*)&sm.src_y[(py + oy + r) * 16 + px + ox];
-        s = satd4_regs(sa, pa);
+        s = half_satd4(sa, pa);
       }
       // sum over the candidate's blocks (consecutive lanes; nblk divides 32)
       for (int o = 1; o < nblk; o <<= 1) s += __shfl_xor_sync(FULL, s, o);
       uint32_t k = UMAX;
       if (ok && blk == 0) {
-        uint32_t cost = (s >> 1) + vec_cost(vx - mvp.x, vy - mvp.y, lambda);
+        uint32_t cost = s + vec_cost(vx - mvp.x, vy - mvp.y, lambda);
         k = (cost << 4) | (uint32_t)(step == 0 ? cand : cand + 1);
       }
       key = min(key, __reduce_min_sync(FULL, k));
@@ -467,7 +477,7 @@ __device__ __noinline__ void mc_chroma_q(const Ctx c) {
 
 // Search-form side state of a coded macroblock: the record's partition fields and the quadrant
 // vectors later macroblocks and the deblocking filter read (lane 0 writes). parts: the quadrants'
-// vectors ss.qmv and the partitions' differences ss.bmvd; otherwise (mvx, mvy) everywhere and no
+// vectors ss.qmv and the partitions' differences ss.pmvd; otherwise (mvx, mvy) everywhere and no
 // differences.
 __device__ __noinline__ void search_tail(const Ctx c, int ptype, bool parts, int mvx, int mvy) {
   if (lane_id() != 0) return;
@@ -479,8 +489,8 @@ __device__ __noinline__ void search_tail(const Ctx c, int ptype, bool parts, int
     m.mv[q][1] = (int16_t)(parts ? ss.qmv[q][1] : mvy);
     rec->part_mv[q][0] = m.mv[q][0];
     rec->part_mv[q][1] = m.mv[q][1];
-    rec->part_mvd[q][0] = (int16_t)(parts ? ss.bmvd[q][0] : 0);
-    rec->part_mvd[q][1] = (int16_t)(parts ? ss.bmvd[q][1] : 0);
+    rec->part_mvd[q][0] = (int16_t)(parts ? ss.pmvd[q] & 0xffffu : 0u);
+    rec->part_mvd[q][1] = (int16_t)(parts ? ss.pmvd[q] >> 16 : 0u);
   }
   rec->part_type = (uint8_t)ptype;
   rec->reserved2[0] = rec->reserved2[1] = rec->reserved2[2] = 0;
@@ -526,19 +536,6 @@ __device__ __noinline__ int2 learned_centre(const Ctx c, int mvp0, int mvp1, uin
   return make_int2(bx, by);
 }
 
-// Partition geometry in coding order: {type, first part, parts}; part k: {px, py, pw, ph, bx, by,
-// pw4, dir, integer-search index}.
-__device__ __constant__ int8_t c_parts[9][9] = {
-    {0, 0, 16, 16, 0, 0, 4, 0, 0},                                  // 16x16
-    {0, 0, 16, 8, 0, 0, 4, 1, 1}, {0, 8, 16, 8, 0, 2, 4, 2, 2},      // 16x8
-    {0, 0, 8, 16, 0, 0, 2, 3, 3}, {8, 0, 8, 16, 2, 0, 2, 4, 4},      // 8x16
-    {0, 0, 8, 8, 0, 0, 2, 0, 5}, {8, 0, 8, 8, 2, 0, 2, 0, 6},        // 8x8
-    {0, 8, 8, 8, 0, 2, 2, 0, 7}, {8, 8, 8, 8, 2, 2, 2, 0, 8}};
-__device__ __constant__ int8_t c_type_first[4] = {0, 1, 3, 5};
-__device__ __constant__ int8_t c_type_parts[4] = {1, 2, 2, 4};
-// quadrants covered by part k (bit mask)
-__device__ __constant__ uint8_t c_part_quads[9] = {15, 3, 12, 5, 10, 1, 2, 4, 8};
-
 // One macroblock of a P slice in the search forms (see the head of this file); false when a wait for
 // the reference picture gave up.
 __device__ __noinline__ bool analyse_p_mb_search(const Ctx c, const PipeWait pw) {
@@ -549,23 +546,15 @@ __device__ __noinline__ bool analyse_p_mb_search(const Ctx c, const PipeWait pw)
   const uint32_t lambda = sm.qt[0].lambda;
   const Bounds bd = mv_bounds(x0, y0);
   const int imin0 = (bd.min0 + 3) >> 2, imin1 = (bd.min1 + 3) >> 2, imax0 = bd.max0 >> 2, imax1 = bd.max1 >> 2;
-  // Warp-uniform state (every lane computes the same values) is held once per warp in shared memory
-  // (SearchSmem) instead of once per lane on the stack; every lane writes the same value, and a
-  // __syncwarp before each rewrite keeps a lane from overwriting what a slower lane still reads.
   __syncwarp();
   const uint32_t nw = load_nb(c);
   load_source(c);
   store_nb(nw);
-  const int2 p16 = mv_pred(0, 0, 4, 0, 0);
-  const int mvp16[2] = {p16.x, p16.y};
+  const uint32_t p16 = mv_pred(c_part[0]);
+  const int mvp16[2] = {lo16((int)p16), (int)p16 >> 16};
   int ps0 = mvp16[0], ps1 = mvp16[1];
-  {
-    NbMv A = nb4(-1, 0, 0), B = nb4(0, -1, 0);
-    if (mbx == 0 || mby == 0 || (A.ref == 0 && A.x == 0 && A.y == 0) || (B.ref == 0 && B.x == 0 && B.y == 0)) {
-      ps0 = 0;
-      ps1 = 0;
-    }
-  }
+  const NbMv nbA = ss.nb[4], nbB = ss.nb[1];
+  if (mbx == 0 || mby == 0 || (nbA.ref == 0 && nbA.mv == 0) || (nbB.ref == 0 && nbB.mv == 0)) ps0 = ps1 = 0;
   const rg_mb_hint* hint = sd.hint ? sd.hint + c.mb : nullptr;
   // integer window: full search, or the learned seed's small window
   const int R = sd.search_range;
@@ -577,10 +566,9 @@ __device__ __noinline__ bool analyse_p_mb_search(const Ctx c, const PipeWait pw)
   int* ccy = ss.ccy;
   bool* cok = ss.cok;
   if (hint) {
-    NbMv A = nb4(-1, 0, 0), B = nb4(0, -1, 0), C = nb4(4, -1, 0);
-    if (C.ref == -2) C = nb4(-1, -1, 0);
-    const int vx[kCentreCands] = {mvp16[0] + hint->mv_off[0], mvp16[0], hint->mv_coarse[0], A.x, B.x, C.x, 0};
-    const int vy[kCentreCands] = {mvp16[1] + hint->mv_off[1], mvp16[1], hint->mv_coarse[1], A.y, B.y, C.y, 0};
+    const NbMv A = nbA, B = nbB, C = ss.nb[3].ref == -2 ? ss.nb[0] : ss.nb[3];
+    const int vx[kCentreCands] = {mvp16[0] + hint->mv_off[0], mvp16[0], hint->mv_coarse[0], A.x(), B.x(), C.x(), 0};
+    const int vy[kCentreCands] = {mvp16[1] + hint->mv_off[1], mvp16[1], hint->mv_coarse[1], A.y(), B.y(), C.y(), 0};
     const bool use[kCentreCands] = {true, true, (hint->flags & 1) != 0, A.ref == 0, B.ref == 0, C.ref == 0, true};
     xhi = -(1 << 20);
     yhi = -(1 << 20);
@@ -642,54 +630,62 @@ __device__ __noinline__ bool analyse_p_mb_search(const Ctx c, const PipeWait pw)
   // 3-4. refinement of every tried type, the least total cost wins
   int best_t = -1;
   uint32_t best_j = UMAX;
-  int (&bmv)[4][2] = ss.bmv;  // per part (coding order) of the best type (warp-uniform, shared)
-  int (&bmvd)[4][2] = ss.bmvd;
+  // lane k < 4: part k's vector and difference of the current and of the best type; their quadrants' vectors
+  uint32_t mv_k = 0, mvd_k = 0, quad = 0, best_mv = 0, best_mvd = 0, best_quad = 0;
+#pragma unroll 1
   for (int t = 0; t < 4; t++) {
     if (!((part_mask >> t) & 1)) continue;
-    int (&own)[4][2] = ss.own;
     __syncwarp();
-    for (int q = 0; q < 4; q++) own[q][0] = own[q][1] = 0;
-    int done = 0;
+    const int own = 5 + (lane & 1) + 2 * (lane & 2);  // quadrant lane's place in ss.nb
+    if (lane < 4) ss.nb[own] = NbMv{0u, -2};
+    __syncwarp();
     uint32_t J = lambda * (uint32_t)sd.type_bits[t];
-    int (&pm)[4][2] = ss.pm;
-    int (&pd)[4][2] = ss.pd;
-    const int first = c_type_first[t], np = c_type_parts[t];
+    const int first = type_first(t), np = type_parts(t);
+    mvd_k = 0;
+#pragma unroll 1
     for (int k = 0; k < np; k++) {
-      const int8_t* g = c_parts[first + k];
-      const int2 mvp = mv_pred(g[4], g[5], g[6], g[7], done);
-      const PartFit fit = hint ? refine_part_sad(c, g[0], g[1], g[2], g[3], ib.x[g[8]], ib.y[g[8]], mvp, lambda, bd,
-                                                 ib.c[g[8]] - vec_cost(4 * ib.x[g[8]] - mvp16[0], 4 * ib.y[g[8]] - mvp16[1], lambda))
-                               : refine_part(c, g[0], g[1], g[2], g[3], ib.x[g[8]], ib.y[g[8]], mvp, lambda, bd);
-      const int mv[2] = {fit.x, fit.y};
+      const uint32_t part = c_part[first + k];
+      const uint32_t mvp = mv_pred(part);
+      const int bx = ss.ib.x[first + k], by = ss.ib.y[first + k];
+      const int2 mp = make_int2(lo16((int)mvp), (int)mvp >> 16);
+      const int px = (part >> 21) & 8u, py = (part >> 22) & 8u, pw = (part >> 26) & 1u ? 8 : 16, ph = (part >> 27) & 1u ? 8 : 16;
+      const PartFit fit = hint ? refine_part_sad(c, px, py, pw, ph, bx, by, mp, lambda, bd,
+                                                 ss.ib.c[first + k] - vec_cost(4 * bx - mvp16[0], 4 * by - mvp16[1], lambda))
+                               : refine_part(c, px, py, pw, ph, bx, by, mp, lambda, bd);
       J += fit.cost;
-      pm[k][0] = mv[0]; pm[k][1] = mv[1];
-      pd[k][0] = mv[0] - mvp.x; pd[k][1] = mv[1] - mvp.y;
-      const int qm = c_part_quads[first + k];
-      for (int q = 0; q < 4; q++)
-        if ((qm >> q) & 1) { own[q][0] = mv[0]; own[q][1] = mv[1]; }
-      done |= qm;
+      const uint32_t mv = pack16(fit.x, fit.y);
+      if (lane == k) {
+        mv_k = mv;
+        mvd_k = pack16(fit.x - mp.x, fit.y - mp.y);
+      }
+      __syncwarp();
+      if (lane < 4 && ((part >> (16 + lane)) & 1u)) {
+        ss.nb[own] = NbMv{mv, 0};
+        quad = mv;
+      }
+      __syncwarp();
     }
     if (J < best_j) {
       best_j = J;
       best_t = t;
-      for (int k = 0; k < 4; k++) {
-        bmv[k][0] = k < np ? pm[k][0] : 0; bmv[k][1] = k < np ? pm[k][1] : 0;
-        bmvd[k][0] = k < np ? pd[k][0] : 0; bmvd[k][1] = k < np ? pd[k][1] : 0;
-      }
+      best_mv = mv_k;
+      best_mvd = mvd_k;
+      best_quad = quad;
     }
   }
   // quadrant vectors of the chosen type and its prediction
-  int (&qmv)[4][2] = ss.qmv;
+  if (lane < 4) {
+    ss.qmv[lane][0] = lo16((int)best_quad);
+    ss.qmv[lane][1] = (int)best_quad >> 16;
+    ss.pmvd[lane] = best_mvd;
+  }
   __syncwarp();
-  {
-    const int first = c_type_first[best_t], np = c_type_parts[best_t];
-    for (int k = 0; k < np; k++) {
-      const int qm = c_part_quads[first + k];
-      for (int q = 0; q < 4; q++)
-        if ((qm >> q) & 1) { qmv[q][0] = bmv[k][0]; qmv[q][1] = bmv[k][1]; }
-      const int8_t* g = c_parts[first + k];
-      predict_part(c, g[0], g[1], g[2], g[3], ib.x[g[8]], ib.y[g[8]], bmv[k][0], bmv[k][1]);
-    }
+#pragma unroll 1
+  for (int k = 0; k < type_parts(best_t); k++) {
+    const int i = type_first(best_t) + k;
+    const uint32_t part = c_part[i], mv = __shfl_sync(FULL, best_mv, k);
+    predict_part(c, (part >> 21) & 8u, (part >> 22) & 8u, (part >> 26) & 1u ? 8 : 16, (part >> 27) & 1u ? 8 : 16, ss.ib.x[i], ss.ib.y[i],
+                 lo16((int)mv), (int)mv >> 16);
   }
   // 5. intra 16x16 when the inter prediction is poor (the plain form's rule, enc.rs:3121-3156)
   const uint32_t inter_satd = satd16((int)offsetof(Smem, pred_y));
@@ -706,8 +702,9 @@ __device__ __noinline__ bool analyse_p_mb_search(const Ctx c, const PipeWait pw)
   // residual, late skip (a 16x16 macroblock at the skip vector), record and reconstruction
   mc_chroma_q(c);
   const int type = best_t == 0 ? RG_MB_P_L0_16X16 : (best_t == 1 ? RG_MB_P_L0_16X8 : (best_t == 2 ? RG_MB_P_L0_8X16 : RG_MB_P_8X8));
-  const bool skipped = code_inter(c, type, best_t == 0 && bmv[0][0] == ps0 && bmv[0][1] == ps1, bmv[0][0], bmv[0][1],
-                                  bmvd[0][0], bmvd[0][1]);
+  const uint32_t mv = __shfl_sync(FULL, best_mv, 0), mvd = __shfl_sync(FULL, best_mvd, 0);
+  const bool skipped = code_inter(c, type, best_t == 0 && mv == pack16(ps0, ps1), lo16((int)mv), (int)mv >> 16, lo16((int)mvd),
+                                  (int)mvd >> 16);
   search_tail(c, best_t, !skipped, ps0, ps1);
   return true;
 }
