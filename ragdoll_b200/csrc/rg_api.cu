@@ -713,9 +713,10 @@ static int enqueue_gops(rg_ctx* c, const uint8_t* const* dev_planes, size_t stri
   CK(cudaEventRecord(c->slot_done[slot], c->stream));
   CK(cudaMemsetAsync(c->counters, 0, sizeof(int) * pipeline_counter_ints(c->fp, frames), c->stream));
   int split = c->deblock_sms > 0 && c->grid >= 2 ? 1 : 0;
-  // IDR pictures get their own queue when SMs are set aside for them
+  // IDR pictures get their own queue when SMs are set aside for them (a single picture of each stream heads
+  // nothing, and its work list then holds for either kind)
   std::vector<int32_t> kinds_key;
-  if (c->intra_sms > 0 && c->grid >= 3) kinds_key.assign(kinds, kinds + (size_t)frames * S);
+  if (c->intra_sms > 0 && c->grid >= 3 && frames > 1) kinds_key.assign(kinds, kinds + (size_t)frames * S);
   if (frames != c->tasks_frames || lag != c->tasks_lag || c->seg != c->tasks_seg || split != c->tasks_split ||
       kinds_key != c->tasks_kinds) {
     // rebuilt only when the call's shape, its picture kinds or the tuning change; the copy is
@@ -1679,7 +1680,15 @@ int rg_analyse_batch(rg_ctx* c, const uint8_t* const* planes, size_t stride_y, s
     dev[3 * s + 1] = d + (size_t)w * c->cfg.height;
     dev[3 * s + 2] = d + (size_t)w * c->cfg.height + (size_t)cw * ((c->cfg.height + 1) / 2);
   }
-  int r = rg_analyse_batch_device(c, dev.data(), w, cw, kinds);
+  // One launch for the pictures, which this call completes itself (a wait that gives up is re-run by the
+  // sync below), while they are one chain of macroblocks; the per-diagonal launches for more work than
+  // that (16 streams of 1080p: 33.5 ms either way), the search forms (640x352: 7.8 ms against 8.2), where
+  // the reconstruction before deblocking is kept, and for what they refuse. A P picture by 42 launches and
+  // by one: 320x180 0.89 -> 0.58 ms, 720p 3.9 -> 2.9, 1080p 6.2 -> 4.7, 8 x 720p 7.5 -> 6.8 (8 x 720p IDR 7.9 -> 8.3).
+  bool one = !c->keep_unfiltered && c->form == RG_FORM_PLAIN &&
+             !pipeline_meets(pipeline_task_count(c->fp, 1, c->seg), c->grid, pipeline_key_span(c->fp, 1, 0, c->seg));
+  for (int s = 0; s < c->S; s++) one = one && (kinds[s] == RG_FRAME_IDR || (kinds[s] == RG_FRAME_P && c->frames[s] > 0));
+  int r = one ? rg_analyse_gops_device(c, dev.data(), w, cw, kinds, 1) : rg_analyse_batch_device(c, dev.data(), w, cw, kinds);
   if (r) return r;
   if (out) return rg_copy_records(c, out);
   return rg_sync(c);
