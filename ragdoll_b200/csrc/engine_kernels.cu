@@ -1523,7 +1523,10 @@ __device__ __forceinline__ unsigned long long global_ns() {
 // of this warp). The first check and the final one are acquire loads; in between the lanes poll with
 // relaxed loads (which leave the L1 alone) and sleep 32 ns doubling to 512 ns. False on timeout
 // (recorded in *error) or when another warp failed.
-__device__ __noinline__ bool wait_all(const int* p, int need, int& seen, int* error, unsigned long long timeout_ns) {
+// kHelp: the warp holds nothing but its segment, and takes part in its block's searches meanwhile.
+__device__ void help_searches(unsigned* board);
+template <bool kHelp = false>
+__device__ __noinline__ bool wait_all(const int* p, int need, int& seen, int* error, unsigned long long timeout_ns, unsigned* board = nullptr) {
   bool ok = !p || seen >= need;
   if (__all_sync(FULL, ok)) return true;
   unsigned long long t0 = 0;
@@ -1547,6 +1550,11 @@ __device__ __noinline__ bool wait_all(const int* p, int need, int& seen, int* er
         if (lane_id() == 0) atomicCAS(error, 0, 1);
         return false;
       }
+      if (kHelp && __shfl_sync(FULL, *(volatile unsigned*)board, 0)) {
+        help_searches(board);
+        t0 = global_ns();  // (the time limit is of waiting)
+        continue;
+      }
       __nanosleep(sleep);
       sleep = min(sleep * 2, 512u);
     }
@@ -1566,6 +1574,7 @@ struct PipeWait {
                          // neighbours are reconstructed; null: those are
   int* error;
   unsigned long long timeout_ns;
+  unsigned* board;       // search forms: the block's open searches (help_searches); null: nobody helps
 };
 // Waits until the reference picture is final over the macroblocks left of and above (xx, rr),
 // clamped to the picture: rows above the last are final where the row below is deblocked; the last
@@ -2274,9 +2283,15 @@ __global__ void __launch_bounds__(32 * kBlockWarps, 1) pipeline_kernel(const __g
   }
   init_tables();
   uint32_t empty = (pp.qbeg[0] >= pp.qend[0] ? 1u : 0u) | (pp.qbeg[1] >= pp.qend[1] ? 2u : 0u) | (pp.qbeg[2] >= pp.qend[2] ? 4u : 0u);
+  __shared__ unsigned board;  // search forms: warps whose search others may take part in
   __shared__ int arrived;  // warps that have finished a segment, all rounds together
   int round = 0;
-  if (threadIdx.y == 0 && lane == 0) arrived = 0;
+  if (threadIdx.y == 0 && lane == 0) {
+    arrived = 0;
+    board = 0;
+  }
+  if constexpr (kForm != 0)
+    if (lane == 0) ss.job.ticket = kNoJob;
   if (lane == 0) sm.reach_y = sm.reach_x = 0;  // this warp's, published once as it exits
   int group = -1;                              // whose parameters sm.fp holds
   __syncthreads();
@@ -2311,7 +2326,7 @@ __global__ void __launch_bounds__(32 * kBlockWarps, 1) pipeline_kernel(const __g
     if (ana) {
       const bool has_prev = sd.prev_rows >= 0 && sd.kind == RG_FRAME_P;
       const bool early = kEarly && sd.kind == RG_FRAME_P;
-      const PipeWait pw{has_prev ? pp.db + sd.prev_rows : nullptr, early ? ana_rows : nullptr, pp.error, pp.timeout_ns};
+      const PipeWait pw{has_prev ? pp.db + sd.prev_rows : nullptr, early ? ana_rows : nullptr, pp.error, pp.timeout_ns, kForm != 0 ? &board : nullptr};
       if (lane == 0) sm.db_row = -1;
       // lane 0: the previous segment of this row; lane 1: the row above two macroblocks ahead; lane 2
       // (plain form): the co-located macroblock of the previous picture, whose vector is a candidate
@@ -2321,7 +2336,7 @@ __global__ void __launch_bounds__(32 * kBlockWarps, 1) pipeline_kernel(const __g
       if (kForm == 0 && lane == 2 && has_prev) flag = pp.ana + sd.prev_rows + y;
       if (early) flag = nullptr;
       for (int x = x0; x < x1; x++) {
-        if (!wait_all(flag, lane == 0 ? x0 : (lane == 1 ? min(x + 2, Wm) : x + 1), seen, pp.error, pp.timeout_ns)) {
+        if (!wait_all<kForm != 0>(flag, lane == 0 ? x0 : (lane == 1 ? min(x + 2, Wm) : x + 1), seen, pp.error, pp.timeout_ns, &board)) {
           failed = true;
           break;
         }
@@ -2350,7 +2365,7 @@ __global__ void __launch_bounds__(32 * kBlockWarps, 1) pipeline_kernel(const __g
       if (lane == 2 && y > 0) flag = db_rows + y - 1;
       if (lane == 3 && x0 > 0) flag = db_rows + y;
       for (int x = x0; x < x1; x++) {
-        if (!wait_all(flag, lane == 3 ? x0 : min(x + (lane == 1 ? 1 : 2), Wm), seen, pp.error, pp.timeout_ns)) {
+        if (!wait_all<kForm != 0>(flag, lane == 3 ? x0 : min(x + (lane == 1 ? 1 : 2), Wm), seen, pp.error, pp.timeout_ns, &board)) {
           failed = true;
           break;
         }

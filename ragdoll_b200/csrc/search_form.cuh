@@ -28,7 +28,8 @@
 // (those of them available at the block, DC when none is).
 
 constexpr int kBandRows = 8;               // integer vectors per band row
-constexpr int kBandBytes = 4 * kBandRows * (2 * kMaxSearchRange + 24);  // four chunks of kBandRows rows
+constexpr int kUnitBands = 1;  // (2: full search 8 x 3 720p 24.8 ms against 23.7)
+constexpr int kBandBytes = (kUnitBands + 2) * kBandRows * (2 * kMaxSearchRange + 24);  // the rows of a unit
 constexpr int kLearnedRange = 2;           // learned form: integer window around the seed
 constexpr int kCentreCands = 7;            // learned form: candidates of the window's centre
 
@@ -46,8 +47,19 @@ struct IntBest {
   int x[9], y[9];
   uint32_t c[9];
 };
+// The whole groups of an integer search, in units of kUnitBands bands: what a warp of the block needs to do one.
+struct SearchJob {
+  const uint8_t* ref;
+  int stride, x0, y0, xlo, xt, ylo, yhi, nwx, mvp0, mvp1;
+  uint32_t lambda;
+  uint32_t ticket;   // next unit | units << 16; kNoJob while there is none
+  int done;          // units finished
+  uint32_t key[9];   // the least so far
+};
+constexpr uint32_t kNoJob = 0x8000u;  // (a ticket past any unit)
 struct SearchSmem {
   uint8_t band[kBandBytes];
+  SearchJob job;
   IntBest ib;
   alignas(8) NbMv nb[12];
   int qmv[4][2];
@@ -118,8 +130,8 @@ __device__ __forceinline__ uint32_t vec_cost(int dx, int dy, uint32_t lambda) {
 
 // ---------------------------------------------------------------------------------------------
 // Integer search over [xlo, xhi] x [ylo, yhi]. Lanes take columns xlo + lane + 32 j; the reference
-// rows of 8 vector rows (band) are staged in shared memory -- four chunks of 8 rows, three of a band and
-// the next band's last one on its way -- and each lane slides its column's 16 x 16 comparison down the band, a reference row at a time against the source rows it pairs
+// rows of 8 vector rows (a band) are staged in shared memory, and each lane slides its column's 16 x 16
+// comparison down the band, a reference row at a time against the source rows it pairs
 // with. Up to four columns past the last whole group (a window of 2 R + 1 vectors has one) go a vector
 // to a lane instead of a group of their own. Costs and raster indices share a word (cost <= 65280 +
 // 91 * 66 < 2^17, index < 129^2 < 2^15), so the first least one is a minimum. ss.ib: the nine parts'
@@ -167,8 +179,124 @@ __device__ __noinline__ uint4 quad_sads(int at) {
     }
   return make_uint4(q[0], q[1], q[2], q[3]);
 }
+// Unit u (kUnitBands bands) of warp `owner`'s search, over this warp's band; the least keys into the job's.
+__device__ __noinline__ void search_unit(int owner, int u) {
+  SearchSmem& os = ((SearchSmem*)(smw + blockDim.y * sizeof(Smem)))[owner];
+  const SearchJob& jb = os.job;
+  const uint8_t* const src = ((const Smem*)smw)[owner].src_y;
+  const int lane = lane_id(), yhi = jb.yhi, nwx = jb.nwx, ylo = jb.ylo + kUnitBands * kBandRows * u;
+  const uint32_t lambda = jb.lambda;
+  uint32_t key[9];
+#pragma unroll
+  for (int k = 0; k < 9; k++) key[k] = UMAX;
+  const int xs = (jb.x0 + jb.xlo) & ~3;              // picture column of band column 0
+  const int wpr = (jb.x0 + jb.xt + 22 - xs) >> 2;    // words of a band row
+  {
+    // its reference rows from y0 + ylo, in words, lane by lane
+    const int dr = 32 / wpr, dk = 32 - dr * wpr, n = min((kUnitBands + 2) * kBandRows, yhi - ylo + 16);
+    const uint8_t* p = jb.ref + (long)(jb.y0 + ylo) * jb.stride + xs;
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(ss.band);
+    __syncwarp();
+    int r = lane / wpr, k = lane - r * wpr;
+#pragma unroll 1
+    for (; r < n; r += dr) {
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + (uint32_t)(r * wpr + k) * 4u),
+                   "l"(p + (long)r * jb.stride + 4 * k) : "memory");
+      k += dk;
+      if (k >= wpr) {
+        k -= wpr;
+        r++;
+      }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
+  }
+#pragma unroll 1
+  for (int dy0 = ylo, b = 0; b < kUnitBands && dy0 <= yhi; dy0 += kBandRows, b++) {
+#pragma unroll 1
+    for (int d0 = jb.xlo; d0 < jb.xt; d0 += 32) {
+      const int dx = d0 + lane;
+      const bool act = dx < jb.xt;
+      const int co = act ? jb.x0 + dx - xs : 0;
+      const uint32_t sh = (uint32_t)(co & 3) * 8u;
+      uint32_t top[kBandRows][2], acc[kBandRows][2] = {};
+#pragma unroll 1
+      for (int half = 0; half < 2; half++) {
+        uint4 s[8];
+#pragma unroll
+        for (int r = 0; r < 8; r++) s[r] = *(const uint4*)(src + (half * 8 + r) * 16);
+#pragma unroll
+        for (int d = 0; d < kBandRows; d++) {
+          top[d][0] = acc[d][0];
+          top[d][1] = acc[d][1];
+          acc[d][0] = acc[d][1] = 0;
+        }
+        const uint32_t* rp = (const uint32_t*)ss.band + (b + half) * kBandRows * wpr + (co >> 2);
+#pragma unroll
+        for (int i = 0; i < kBandRows + 7; i++) {
+          // reference row half * 8 + i of the band pairs with source row r = i - d for d = 0..7
+          const uint32_t w0 = rp[0], w1 = rp[1], w2 = rp[2], w3 = rp[3], w4 = rp[4];
+          rp += wpr;
+          const uint32_t R0 = __funnelshift_r(w0, w1, sh), R1 = __funnelshift_r(w1, w2, sh), R2 = __funnelshift_r(w2, w3, sh),
+                         R3 = __funnelshift_r(w3, w4, sh);
+#pragma unroll
+          for (int d = 0; d < kBandRows; d++) {
+            const int r = i - d;
+            if (r < 0 || r > 7) continue;
+            acc[d][0] = __vsadu4(R0, s[r].x) + __vsadu4(R1, s[r].y) + acc[d][0];
+            acc[d][1] = __vsadu4(R2, s[r].z) + __vsadu4(R3, s[r].w) + acc[d][1];
+          }
+        }
+      }
+      const uint32_t cx = lambda * se_bits(4 * dx - jb.mvp0);
+      uint32_t idx = (uint32_t)((dy0 - jb.ylo) * nwx + (dx - jb.xlo));
+#pragma unroll
+      for (int d = 0; d < kBandRows; d++, idx += nwx)
+        if (act && dy0 + d <= yhi)
+          part_keys(key, top[d][0], top[d][1], acc[d][0], acc[d][1],
+                    ((cx + lambda * se_bits(4 * (dy0 + d) - jb.mvp1)) << kKeyBits) + idx);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 9; k++) {
+    const uint32_t m = __reduce_min_sync(FULL, key[k]);
+    if (lane == k) atomicMin(&os.job.key[k], m);
+  }
+  // the keys before the count
+  __threadfence_block();
+  __syncwarp();
+  if (lane == 0) atomicAdd(&os.job.done, 1);
+}
+// Takes units of `owner`'s search until none is left.
+__device__ __forceinline__ void search_units(int owner) {
+  SearchJob& jb = ((SearchSmem*)(smw + blockDim.y * sizeof(Smem)))[owner].job;
+  while (true) {
+    uint32_t t = 0;
+    if (lane_id() == 0) t = atomicAdd(&jb.ticket, 1u);
+    t = __shfl_sync(FULL, t, 0);
+    if ((t & 0xffffu) >= (t >> 16)) break;
+    __threadfence_block();  // the job was written before its ticket
+    search_unit(owner, (int)(t & 0xffffu));
+  }
+}
+// A warp that waits for its segment meanwhile takes part in the searches open in its block (board: a bit per
+// warp with one).
+__device__ __noinline__ void help_searches(unsigned* board) {
+  unsigned open = __shfl_sync(FULL, *(volatile unsigned*)board, 0);
+  while (open) {
+    search_units(__ffs(open) - 1);
+    if (lane_id() == 0) atomicAnd(board, ~(open & -open));  // no unit left (a search opened since goes without help)
+    open &= open - 1;
+  }
+}
+
+// board (or null): the block's warps that wait take part. A macroblock's search is then a few units long
+// instead of nine bands: at range 32 a macroblock's search took 105 k cycles of the chain that a launch of
+// few pictures is (full search 8 x 3 720p: 28.6 ms without help, 23.6 so; learned 1080p 8 x 8, whose walk
+// falls back to it, 50.2 and 46.7, 4K 4 x 3 48.7 and 46.6). Sharing the partition types' refinement the same
+// way gave the full search 6 % more and cost the learned form 3 %.
 __device__ __noinline__ void int_search(const Ctx c, int xlo, int xhi, int ylo, int yhi,
-                                        int mvp0, int mvp1, uint32_t lambda) {
+                                        int mvp0, int mvp1, uint32_t lambda, unsigned* board) {
   const int lane = lane_id();
   const int x0 = c.mbx * 16, y0 = c.mby * 16;
   const int nwx = xhi - xlo + 1, nwy = yhi - ylo + 1;
@@ -178,86 +306,35 @@ __device__ __noinline__ void int_search(const Ctx c, int xlo, int xhi, int ylo, 
   // a window of at most 32 vectors (the learned form's), or the columns past the last whole group: `cols`
   // columns from xt, a lane a vector, as many rows at a time as fit
   const bool small = nwx <= 8 && nwx * nwy <= 32;
-  const int rem = nwx & 31, cols = small ? nwx : (rem <= 4 ? rem : 0), xt = xhi - cols + 1, groups = (nwx - cols + 31) >> 5;
-  if (groups) {
-    const int xs = (x0 + xlo) & ~3;                          // picture column of band column 0
-    const int wpr = (x0 + xhi - cols + 23 - xs) >> 2;        // words of a band row
-    // chunk q holds the reference rows y0 + ylo + 8 q ..; its copy in words, lane by lane
-    const int dr = 32 / wpr, dk = 32 - dr * wpr, lr = lane / wpr, lk = lane - lr * wpr;
-    const uint32_t band = (uint32_t)__cvta_generic_to_shared(ss.band);
-    auto stage = [&](int q) {
-      const int n = min(kBandRows, nwy + 15 - kBandRows * q);
-      const uint8_t* src = sm.sd.ref_y + (long)(y0 + ylo + kBandRows * q) * sm.fp.stride_y + xs;
-      const uint32_t dst = band + (uint32_t)((q & 3) * kBandRows * wpr) * 4u;
-#pragma unroll 1
-      for (int r = lr, k = lk; r < n; r += dr) {
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + (uint32_t)(r * wpr + k) * 4u),
-                     "l"(src + (long)r * sm.fp.stride_y + 4 * k) : "memory");
-        k += dk;
-        if (k >= wpr) {
-          k -= wpr;
-          r++;
-        }
-      }
-      asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    __syncwarp();
-    stage(0);
-    stage(1);
-    stage(2);
-#pragma unroll 1
-    for (int dy0 = ylo, b = 0; dy0 <= yhi; dy0 += kBandRows, b++) {
-      stage(b + 3);  // (nothing past the last row)
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
-      __syncwarp();
-#pragma unroll 1
-      for (int j = 0; j < groups; j++) {
-        const int dx = xlo + lane + 32 * j;
-        const bool act = dx < xt;
-        const int co = act ? x0 + dx - xs : 0;
-        const uint32_t sh = (uint32_t)(co & 3) * 8u;
-        uint32_t top[kBandRows][2], acc[kBandRows][2] = {};
-#pragma unroll 1
-        for (int half = 0; half < 2; half++) {
-          uint4 s[8];
-#pragma unroll
-          for (int r = 0; r < 8; r++) s[r] = *(const uint4*)&sm.src_y[(half * 8 + r) * 16];
-#pragma unroll
-          for (int d = 0; d < kBandRows; d++) {
-            top[d][0] = acc[d][0];
-            top[d][1] = acc[d][1];
-            acc[d][0] = acc[d][1] = 0;
-          }
-          const uint32_t *rp = (const uint32_t*)ss.band + ((b + half) & 3) * kBandRows * wpr + (co >> 2),
-                         *rn = (const uint32_t*)ss.band + ((b + half + 1) & 3) * kBandRows * wpr + (co >> 2);
-#pragma unroll
-          for (int i = 0; i < kBandRows + 7; i++) {
-            // reference row half * 8 + i of the band pairs with source row r = i - d for d = 0..7
-            if (i == kBandRows) rp = rn;
-            const uint32_t w0 = rp[0], w1 = rp[1], w2 = rp[2], w3 = rp[3], w4 = rp[4];
-            rp += wpr;
-            const uint32_t R0 = __funnelshift_r(w0, w1, sh), R1 = __funnelshift_r(w1, w2, sh), R2 = __funnelshift_r(w2, w3, sh),
-                           R3 = __funnelshift_r(w3, w4, sh);
-#pragma unroll
-            for (int d = 0; d < kBandRows; d++) {
-              const int r = i - d;
-              if (r < 0 || r > 7) continue;
-              acc[d][0] = __vsadu4(R0, s[r].x) + __vsadu4(R1, s[r].y) + acc[d][0];
-              acc[d][1] = __vsadu4(R2, s[r].z) + __vsadu4(R3, s[r].w) + acc[d][1];
-            }
-          }
-        }
-        const uint32_t cx = lambda * se_bits(4 * dx - mvp0);
-        uint32_t idx = (uint32_t)((dy0 - ylo) * nwx + (dx - xlo));
-#pragma unroll
-        for (int d = 0; d < kBandRows; d++, idx += nwx)
-          if (act && dy0 + d <= yhi)
-            part_keys(key, top[d][0], top[d][1], acc[d][0], acc[d][1],
-                      ((cx + lambda * se_bits(4 * (dy0 + d) - mvp1)) << kKeyBits) + idx);
-      }
-      __syncwarp();  // every lane is done with the chunk that is overwritten next
+  const int rem = nwx & 31, cols = small ? nwx : (rem <= 4 ? rem : 0), xt = xhi - cols + 1;
+  const int units = xt > xlo ? (nwy + kUnitBands * kBandRows - 1) / (kUnitBands * kBandRows) : 0;
+  if (units) {
+    SearchJob& jb = ss.job;
+    if (lane == 0) {
+      jb.ref = sm.sd.ref_y;
+      jb.stride = sm.fp.stride_y;
+      jb.x0 = x0; jb.y0 = y0; jb.xlo = xlo; jb.xt = xt; jb.ylo = ylo; jb.yhi = yhi; jb.nwx = nwx;
+      jb.mvp0 = mvp0; jb.mvp1 = mvp1; jb.lambda = lambda;
+      jb.done = 0;
     }
-    asm volatile("cp.async.wait_all;" ::: "memory");
+    if (lane < 9) jb.key[lane] = UMAX;
+    __threadfence_block();  // the job (and this warp's source) before its ticket
+    __syncwarp();
+    if (lane == 0) {
+      atomicExch(&jb.ticket, (uint32_t)units << 16);
+      if (board) atomicOr(board, 1u << threadIdx.y);
+    }
+    __syncwarp();
+    search_units(threadIdx.y);
+    if (lane == 0) {
+      if (board) atomicAnd(board, ~(1u << threadIdx.y));
+      atomicExch(&jb.ticket, kNoJob);
+      while (*(volatile int*)&jb.done < units) __nanosleep(50);  // units others still have, each of bounded work
+    }
+    __threadfence_block();
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 9; k++) key[k] = ((volatile uint32_t*)jb.key)[k];
   }
   if (cols) {
     const int vrows = 32 / cols, vy = lane / cols, vx = lane - vy * cols;
@@ -605,7 +682,7 @@ __device__ __noinline__ bool analyse_p_mb_search(const Ctx c, const PipeWait pw)
     yhi = min(lcy + kLearnedRange, imax1);
   }
   IntBest& ib = ss.ib;  // warp-uniform: once per warp in shared memory
-  int_search(c, xlo, xhi, ylo, yhi, mvp16[0], mvp16[1], lambda);
+  int_search(c, xlo, xhi, ylo, yhi, mvp16[0], mvp16[1], lambda, pw.board);
   if (hint) {
     bool edge = (ib.x[0] == xlo && xlo > imin0) || (ib.x[0] == xhi && xhi < imax0) ||
                 (ib.y[0] == ylo && ylo > imin1) || (ib.y[0] == yhi && yhi < imax1);
@@ -616,7 +693,7 @@ __device__ __noinline__ bool analyse_p_mb_search(const Ctx c, const PipeWait pw)
       ylo = max(cy - kLearnedRange, imin1);
       yhi = min(cy + kLearnedRange, imax1);
       if (!wait_window(c, pw, xhi, yhi)) return false;
-      int_search(c, xlo, xhi, ylo, yhi, mvp16[0], mvp16[1], lambda);
+      int_search(c, xlo, xhi, ylo, yhi, mvp16[0], mvp16[1], lambda, pw.board);
       edge = (ib.x[0] == xlo && xlo > imin0) || (ib.x[0] == xhi && xhi < imax0) ||
              (ib.y[0] == ylo && ylo > imin1) || (ib.y[0] == yhi && yhi < imax1);
     }
@@ -624,7 +701,7 @@ __device__ __noinline__ bool analyse_p_mb_search(const Ctx c, const PipeWait pw)
       xlo = max(fcx - R, imin0); xhi = min(fcx + R, imax0);
       ylo = max(fcy - R, imin1); yhi = min(fcy + R, imax1);
       if (!wait_window(c, pw, xhi, yhi)) return false;
-      int_search(c, xlo, xhi, ylo, yhi, mvp16[0], mvp16[1], lambda);
+      int_search(c, xlo, xhi, ylo, yhi, mvp16[0], mvp16[1], lambda, pw.board);
     }
   }
   // 3-4. refinement of every tried type, the least total cost wins
