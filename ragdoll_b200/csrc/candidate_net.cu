@@ -48,7 +48,7 @@ __device__ __forceinline__ float pix_norm(uint8_t v) { return ((float)v - 128.0f
 // activation buffer per CTA holds every map of its strip in turn (the input in plane 0, then each
 // layer's output over its input: a layer's epilogue starts once all its MMAs have completed).
 constexpr int kStripMbs = 2;
-constexpr int kThreads = 256;  // 8 warps; warps w and w + 4 share TMEM lanes 32 (w % 4)..
+constexpr int kThreads = 256;  // 8 warps; warps w and w + 4 share TMEM lanes 32 (w % 4)..; a ninth issues the MMAs
 constexpr int kCtasPerSm = 2;
 constexpr int kRow = 16 * kStripMbs + 8;  // row stride (positions) of every map of a strip: 40
 constexpr int kTiles1 = (22 * kRow + 127) / 128, kTiles2 = (20 * kRow + 127) / 128, kTiles3 = (18 * kRow + 127) / 128;
@@ -58,7 +58,7 @@ constexpr int kPosBuf = ((kTiles1 * 128 + kTap > kTiles2 * 128 + kTap ? kTiles1 
 static_assert(kPosBuf >= kTiles1 * 128 + kTap + 1 && kPosBuf >= kTiles3 * 128 + kTap,
               "tap reach (conv1's last pair one position further) and outputs fit the buffer");
 static_assert(kPosBuf >= 24 * kRow, "the input map fits plane 0");
-static_assert(kTap < 128 && kTiles1 <= kThreads / 32 && kTiles2 <= kTiles1 && kTiles3 <= kTiles1, "a warp a tile, read by it and the one before");
+static_assert(kTap < 128 && kTiles2 == kTiles1 && kTiles3 <= kTiles1, "a tile reads its positions and the next tile's; layers 0 and 1 store every tile");
 static_assert(kTiles1 * 32 <= 256, "accumulators of one layer fit the CTA's 256 tensor-memory columns");
 static_assert(kStripMbs * 4 <= kThreads / 32, "pooling: a warp per (macroblock, 8-channel plane)");
 // shared memory (bytes): the buffer (4 planes of 8 channels) | B operands | the rest
@@ -72,7 +72,7 @@ struct InferMisc {
   float head[15][kHeadPitch];    // weights, then the bias: partition (4), offset (2), intra 4x4 (9)
   float pool[kStripMbs][17][kHeadPitch];  // per macroblock: the 18 x 18 mean, then the 16 block means
   float logit[kStripMbs * 16 * 9 + kStripMbs * 6];
-  alignas(8) uint64_t mbar[kTiles1];  // per accumulator tile: its MMAs have completed
+  alignas(8) uint64_t mbar[kTiles1], ready[kTiles1];  // per tile: its MMAs have completed; its map is stored
   uint32_t tmem;
   int strip;
 };
@@ -174,7 +174,7 @@ __device__ __forceinline__ uint32_t topk_mask(const float (&l)[N], int k, float 
   return m;
 }
 
-__global__ void __launch_bounds__(kThreads, kCtasPerSm) cnn_infer_kernel(InferParams ip) {
+__global__ void __launch_bounds__(kThreads + 32, kCtasPerSm) cnn_infer_kernel(InferParams ip) {
   extern __shared__ __align__(1024) uint8_t smem[];
   InferMisc& ms = *reinterpret_cast<InferMisc*>(smem + kOffMisc);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -190,7 +190,10 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) cnn_infer_kernel(InferPa
   }
   if (tid == 0) {
 #pragma unroll
-    for (int t = 0; t < kTiles1; t++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&ms.mbar[t])));
+    for (int t = 0; t < kTiles1; t++) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&ms.mbar[t])));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(smem_u32(&ms.ready[t])));
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
@@ -228,7 +231,8 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) cnn_infer_kernel(InferPa
   if (tid == 0) ms.strip = atomicAdd(ip.counter, 1);
   __syncthreads();
   int strip = ms.strip;
-  if (strip < total) load_input(strip);
+  __syncthreads();  // every thread has it before the next one is written
+  if (strip < total && warp < 8) load_input(strip);
   // shared-memory descriptors: conv1's five tap pairs on plane 0, the two channel halves of the
   // buffer for conv2 and conv3, the B operands; a tile / tap adds its offset in 16-byte units
   const uint64_t bufd0 = umma_desc(sBuf, kPlane, 128), bufd1 = umma_desc(sBuf + 2 * kPlane, kPlane, 128);
@@ -237,29 +241,29 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) cnn_infer_kernel(InferPa
     const int job = strip / (ip.mb_h * ip.strips_per_row), rem = strip % (ip.mb_h * ip.strips_per_row);
     const int mby = rem / ip.strips_per_row, mbx0 = (rem % ip.strips_per_row) * kStripMbs;
     const InferJob jb = ip.jobs[job];
+    if (warp < 8)
 #pragma unroll
     for (int k = 0; k < kPer; k++) {
       __nv_bfloat162 two = __floats2bfloat162_rn(pix_norm(ca[k]), pix_norm(pa[k]));
       ((uint4*)buf)[tid + kThreads * k] = make_uint4(*(uint32_t*)&two, 0u, 0u, 0u);
     }
     if (tid == 0) ms.strip = atomicAdd(ip.counter, 1);  // read after the first layer's barrier
-    int next = total;
-    for (int layer = 0; layer < 3; layer++) {
-      fence_async_smem();
-      fence_before_sync();
-      __syncthreads();
-      fence_after_sync();
-      // Warp t issues tile t's MMAs, and each tile completes on its own barrier: its epilogue runs while other
-      // tiles' MMAs do. It writes positions 128 t .. 128 t + 127 over the layer's input, which tiles t and
-      // t - 1 read (from 128 t and 128 (t - 1), over fewer than 256 positions). The MMAs bound the kernel:
-      // 269 a strip at 67 cycles (M = 128, N = 32: 16 cycles of the tensor pipe; one CTA an SM alone has one
-      // every 76). One thread issuing all tiles in order: 2.44 ms for eight 1080p pictures with the coarse
-      // pass, 2.39 so.
-      const int tiles = layer == 0 ? kTiles1 : (layer == 1 ? kTiles2 : kTiles3);
-      if (warp < kTiles1 && lane == 0) {
-        const int t = warp;
-        const uint32_t d = tmem + (uint32_t)(t * 32);
-        if (layer == 0) {
+    fence_async_smem();
+    fence_before_sync();
+    __syncthreads();
+    fence_after_sync();
+    const int next = ms.strip;
+    // The ninth warp issues the MMAs of all three layers, tile by tile; each tile completes on its own
+    // barrier, and its epilogue, which stores the tile's positions 128 t .. 128 t + 127 over the layer's
+    // input, runs while other tiles' MMAs do. A tile reads the positions of tiles t and t + 1 of its input:
+    // its MMAs start once both are stored, and tile t is stored once tiles t - 1 and t have completed. The
+    // MMAs bound the kernel: 269 a strip, each 46 cycles (M = 128, N = 32: 16 of the tensor pipe; measured
+    // alone, whatever the layout of A). Layers one after the other for the whole strip left the tensor
+    // cores 67 cycles a MMA: 2.39 ms for eight 1080p pictures with the coarse pass, 2.15 so.
+    if (warp == 8) {
+      if (lane == 0) {
+#pragma unroll 1
+        for (int t = 0; t < kTiles1; t++) {
 #pragma unroll
           for (int k = 0; k < kB1Mmas; k++) {
             // taps 2k and 2k + 1 (tap 9: a zero-weight partner one position on) as the two
@@ -267,28 +271,45 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) cnn_infer_kernel(InferPa
             const int ta = 2 * k, tb = 2 * k + 1;
             const int oa = (ta / 3) * kRow + ta % 3, ob = tb < 9 ? (tb / 3) * kRow + tb % 3 : oa + 1;
             const uint64_t a = umma_desc(sBuf + (uint32_t)((t * 128 + oa) * 16), (uint32_t)((ob - oa) * 16), 128);
-            umma_bf16(d, a, b1d + (uint64_t)(k * 64), k > 0);
+            umma_bf16(tmem + (uint32_t)(t * 32), a, b1d + (uint64_t)(k * 64), k > 0);
           }
-        } else if (t < tiles) {
-          const uint64_t bd = layer == 1 ? b2d : b3d;
-#pragma unroll
-          for (int tap = 0; tap < 9; tap++)
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-              const uint64_t off = (uint64_t)(t * 128 + (tap / 3) * kRow + tap % 3);
-              umma_bf16(d, (h ? bufd1 : bufd0) + off, bd + (uint64_t)((tap * 2 + h) * 64), tap > 0 || h > 0);
-            }
+          umma_commit(&ms.mbar[t]);
         }
-        umma_commit(&ms.mbar[t]);  // (also without a tile: every barrier's phase turns every layer)
+#pragma unroll 1
+        for (int layer = 1; layer < 3; layer++) {
+          const int tiles = layer == 1 ? kTiles2 : kTiles3, before = layer == 1 ? kTiles1 : kTiles2;
+          const uint64_t bd = layer == 1 ? b2d : b3d;
+          if (ok) ok = mbar_wait(&ms.ready[0], (uint32_t)(layer - 1));
+#pragma unroll 1
+          for (int t = 0; t < kTiles1; t++) {
+            if (ok && t + 1 < before) ok = mbar_wait(&ms.ready[t + 1], (uint32_t)(layer - 1));
+            if (!ok) break;
+            fence_after_sync();
+            if (t < tiles) {
+              const uint32_t d = tmem + (uint32_t)(t * 32);
+#pragma unroll
+              for (int tap = 0; tap < 9; tap++)
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                  const uint64_t off = (uint64_t)(t * 128 + (tap / 3) * kRow + tap % 3);
+                  umma_bf16(d, (h ? bufd1 : bufd0) + off, bd + (uint64_t)((tap * 2 + h) * 64), tap > 0 || h > 0);
+                }
+            }
+            umma_commit(&ms.mbar[t]);  // (also without a tile: every barrier's phase turns every layer)
+          }
+        }
       }
+      phase ^= 1;  // three layers
       __syncwarp();
-      if (layer == 0) {  // the next strip's bytes, in flight while the tensor cores work
-        next = ms.strip;
-        if (next < total) load_input(next);
-      }
+    } else if (next < total) {
+      load_input(next);  // the next strip's bytes, in flight while the tensor cores work
+    }
+    for (int layer = 0; layer < 3 && warp < 8; layer++, phase ^= 1) {
+      const int tiles = layer == 0 ? kTiles1 : (layer == 1 ? kTiles2 : kTiles3);
       // epilogue: warp w reads rows 32 (w % 4) .. + 31 of tiles w / 4, + 2, ..; bias, ReLU, BF16 into the
       // buffer's four planes
       const int wl = warp & 3;
+#pragma unroll 1
       for (int t = warp >> 2; t < kTiles1; t += 2) {
         if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&ms.mbar[max(t - 1, 0)], phase) && mbar_wait(&ms.mbar[t], phase));
         if (!ok || t >= tiles) continue;
@@ -310,13 +331,17 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) cnn_infer_kernel(InferPa
           }
           *(uint4*)(buf + q * kPlane + p * 16) = make_uint4(w[0], w[1], w[2], w[3]);
         }
+        if (layer < 2) {  // the tile's map to the MMAs of the next layer
+          fence_async_smem();
+          fence_before_sync();
+          __syncwarp();
+          if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&ms.ready[t])) : "memory");
+        }
       }
-      // a wait that gave up is made uniform before anyone acts on it (this also completes conv3's map)
-      phase ^= 1;
-      ok = __syncthreads_and(ok ? 1 : 0) != 0;
-      if (!ok && tid == 0) atomicExch(ip.error, 1);
-      if (!ok) break;
     }
+    // a wait that gave up is made uniform before anyone acts on it (this also completes conv3's map)
+    ok = __syncthreads_and(ok ? 1 : 0) != 0;
+    if (!ok && tid == 0) atomicExch(ip.error, 1);
     if (!ok) break;
     // pooling of the conv3 map (map column 16 j + i is sample x 16 (mbx0 + j) - 1 + i): warp w
     // takes macroblock j = w / 4 and 8-channel plane q = w % 4; lane l < 16 sums map column l + 1
@@ -372,7 +397,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) cnn_infer_kernel(InferPa
     __syncthreads();
     // logits, one a thread at a time: of (block, intra 4x4 mode), then of (macroblock, partition or offset)
     constexpr int kBlockLogits = kStripMbs * 16 * 9;
-    for (int i = tid; i < kBlockLogits + kStripMbs * 6; i += kThreads) {
+    for (int i = tid; i < kBlockLogits + kStripMbs * 6 && tid < kThreads; i += kThreads) {
       const bool block = i < kBlockLogits;
       const int n = block ? i / 9 : (i - kBlockLogits) / 6, o = block ? 6 + i - n * 9 : i - kBlockLogits - n * 6;
       const float* f = block ? ms.pool[n >> 4][1 + (n & 15)] : ms.pool[n][0];
@@ -1291,7 +1316,7 @@ int rg_net_predict_hints(rg_net* net, const uint8_t* const* dev_cur, const uint8
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, net->device);
   const int strips = n_pictures * ip.mb_h * ip.strips_per_row;
   const int ctas = kCtasPerSm * sms < strips ? kCtasPerSm * sms : strips;
-  cnn_infer_kernel<<<ctas, kThreads, kSmemInfer, st>>>(ip);
+  cnn_infer_kernel<<<ctas, kThreads + 32, kSmemInfer, st>>>(ip);
   NCK(cudaGetLastError());
   if (net->coarse_range > 0) {
     CoarseParams cp{net->jobs, n_pictures, width, height, (int)stride, ip.mb_w, ip.mb_h, net->coarse_range / 2};
