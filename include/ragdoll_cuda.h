@@ -229,7 +229,9 @@ int rg_group_graph_counts(const rg_ctx* ctx, int64_t* captures, int64_t* launche
 int rg_analyse_gops(rg_ctx* ctx, const uint8_t* const* planes, size_t stride_y, size_t stride_uv,
                     const int32_t* kinds, int32_t frames, rg_mb_out* out);
 
-/* Copies the records of the last `frames` pictures of an rg_analyse_gops / _device call. */
+/* Copies the records of the last `frames` pictures of an rg_analyse_gops / _device / _group call, as the
+ * launch finishes them. Returns once the context's own pictures are analysed, deblocked and copied (the
+ * other contexts of a group launch may still be running). */
 int rg_copy_records_gops(rg_ctx* ctx, int32_t frames, rg_mb_out* out);
 
 /*

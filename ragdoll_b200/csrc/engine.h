@@ -75,6 +75,7 @@ struct StreamDev {
   // pipelined launches: this picture's ready flag in mapped host memory (null: the launch's
   // ready array at the descriptor's index, if any)
   int32_t* ready;
+  int32_t* done;  // the same once the picture is deblocked as well (or null)
   // pipelined launches of few pictures, plain form: per macroblock of this picture {vector, ref | 0x100}
   // as soon as it is decided (null: none), and the previous picture's when it is of the same launch
   uint2* dec;

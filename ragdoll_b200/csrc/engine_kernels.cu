@@ -2380,6 +2380,8 @@ __global__ void __launch_bounds__(32 * kBlockWarps, 1) pipeline_kernel(const __g
         }
         publish(db_rows + y, x + 1);
       }
+      // the last row's last macroblock comes after every other of the picture
+      if (!failed && y == H - 1 && x1 == Wm && sd.done && lane == 0) st_release_sys(sd.done, pp.seq);
       // Compact records of the row, by the warp that deblocked its last segment: on the deblocking
       // SMs and after the row's deblocking progress was published, so neither the analysis
       // wavefront nor the deblocking chain waits for it (done at the end of the row's analysis it

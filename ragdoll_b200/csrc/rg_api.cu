@@ -191,6 +191,8 @@ struct rg_ctx {
     int* h_reach = nullptr;              // mapped host: 1 + the reach its reference waits saw [2]
     cudaEvent_t done = nullptr;          // after the launch
     std::vector<const rg_mb_hint*> hints;  // learned form: [f][s] (empty otherwise)
+    bool group = false;                  // part of a group launch
+    bool complete = false;               // every picture known to be done: never re-run
     bool flagged = false;                // the launch sets h_final as each picture's records are final
   };
   Pending pend[2];
@@ -558,6 +560,7 @@ static int enqueue_wavefront(rg_ctx* c, const uint8_t* const* dev_planes, size_t
     d.walk = c->walk;
     for (int k = 0; k < 4; k++) { d.type_bits[k] = c->type_bits[k]; d.pad3_[k] = 0; }
     d.ready = nullptr;
+    d.done = nullptr;
   }
   FrameParams fp = c->fp;
   fp.src_stride_y = (int)stride_y;
@@ -584,7 +587,7 @@ static int enqueue_wavefront(rg_ctx* c, const uint8_t* const* dev_planes, size_t
 // group `group`.
 static void gop_desc(const rg_ctx* c, StreamDev& d, int f, int s, const uint8_t* const* dev_planes,
                      const int32_t* kinds, rg_mb_out* rec_base, const rg_mb_hint* hint, int group, int rows_base,
-                     int* ready = nullptr, uint2* dec = nullptr) {
+                     int* ready = nullptr, uint2* dec = nullptr, int* done = nullptr) {
   const int S = c->S, g = c->frames[s] + f;
   const int cur = g % c->nslots, prv = (g + c->nslots - 1) % c->nslots;
   d.src_y = dev_planes[(f * S + s) * 3];
@@ -613,12 +616,14 @@ static void gop_desc(const rg_ctx* c, StreamDev& d, int f, int s, const uint8_t*
   d.walk = c->walk;
   for (int k = 0; k < 4; k++) { d.type_bits[k] = c->type_bits[k]; d.pad3_[k] = 0; }
   d.ready = ready ? ready + f * S + s : nullptr;
+  d.done = done ? done + f * S + s : nullptr;
 }
 
-// The context's record flags as the device sees them, cleared for the next launch (every earlier one
+// The context's flags as the device sees them -- per picture of a call: records final, then (group
+// launches) per picture: deblocked -- cleared for the next launch (every earlier one
 // resolved); null where they cannot be had: the records are then copied after the launch.
 static int* final_flags(rg_ctx* c) {
-  const size_t n = sizeof(int) * (size_t)c->S * c->max_frames;
+  const size_t n = sizeof(int) * 2 * (size_t)c->S * c->max_frames;
   if (!c->h_final) {
     if (!c->f_out && cudaStreamCreateWithFlags(&c->f_out, cudaStreamNonBlocking) != cudaSuccess) c->f_out = nullptr;
     if (!c->f_out || cudaHostAlloc((void**)&c->h_final, n, cudaHostAllocMapped) != cudaSuccess) c->h_final = nullptr;
@@ -756,6 +761,7 @@ static int enqueue_gops(rg_ctx* c, const uint8_t* const* dev_planes, size_t stri
   p.out_bytes = 0;
   p.hints = hv;
   p.flagged = flagged && ready;
+  p.group = p.complete = false;
   c->pend_count++;
   for (int s = 0; s < S; s++) c->frames[s] += frames;
   return RG_OK;
@@ -867,7 +873,7 @@ static int group_launch(rg_ctx* const* ctxs, int32_t n, const uint8_t* const* co
       for (int s = 0; s < c->S; s++)
         gop_desc(c, L->g_hstreams[desc_base[i] + f * c->S + s], f, s, dev_planes[i], kinds[i],
                  rec_bases && rec_bases[i] ? rec_bases[i] : c->recs, nullptr, i, rows_base[i],
-                 readies ? readies[i] : nullptr);
+                 readies ? readies[i] : nullptr, nullptr, finals[i] ? finals[i] + c->S * c->max_frames : nullptr);
   }
   // launch shape: the segment length and SM roles of the context with the most macroblocks (its
   // tuning suits the bulk of the work), the largest grid of any
@@ -1033,6 +1039,8 @@ static int group_launch(rg_ctx* const* ctxs, int32_t n, const uint8_t* const* co
     p.out_bytes = 0;
     p.hints.clear();
     p.flagged = finals[i] != nullptr;
+    p.group = true;
+    p.complete = false;
     c->pend_count++;
     for (int s = 0; s < c->S; s++) c->frames[s] += frames;
   }
@@ -1143,8 +1151,8 @@ int rg_copy_records_gops(rg_ctx* c, int32_t frames, rg_mb_out* out) {
   // copied: the leading pictures already in out; a call that had to be re-run leaves none.
   int copied = 0;
   if (c->pend_count == 1 && c->pend[c->pend_head].flagged) {
-    const rg_ctx::Pending& p = c->pend[c->pend_head];
-    const int n = std::min(frames, p.frames) * c->S;
+    rg_ctx::Pending& p = c->pend[c->pend_head];
+    const int n = std::min(frames, p.frames) * c->S, all = p.frames * c->S;
     cudaError_t e = cudaSuccess;
     while (copied < n && e == cudaSuccess) {
       const bool ended = cudaEventQuery(p.done) != cudaErrorNotReady;
@@ -1164,6 +1172,24 @@ int rg_copy_records_gops(rg_ctx* c, int32_t frames, rg_mb_out* out) {
     const cudaError_t e2 = cudaStreamSynchronize(c->f_out);
     if (e == cudaSuccess) e = e2;
     if (e != cudaSuccess) return fail(RG_ERR_CUDA, "rg_copy_records_gops: %s", cudaGetErrorString(e));
+    // Of a group launch this context waits for its own pictures only -- analysed, copied and deblocked --
+    // while the other contexts' go on: their records are then copied during the launch too (four sizes, 4
+    // streams x 10, fetched one after the other, smallest first: 19.7 ms when each waited for the launch, 15.6 so).
+    if (p.group && frames <= p.frames && copied == n) {
+      const volatile int* done = c->h_final + c->S * c->max_frames;
+      for (int k = 0; k < all;) {
+        if (done[k] == 1) k++;
+        else if (cudaEventQuery(p.done) != cudaErrorNotReady) break;
+        else std::this_thread::yield();
+      }
+      std::atomic_thread_fence(std::memory_order_acquire);
+      p.complete = true;
+      for (int k = 0; k < all; k++) p.complete = p.complete && done[k] == 1;
+      if (p.complete) {
+        if (c->a_out) CK(cudaStreamSynchronize(c->a_out));
+        return RG_OK;
+      }
+    }
     CK(cudaEventSynchronize(p.done));
     if (*(volatile int*)p.h_err) copied = 0;
   }
@@ -1311,7 +1337,7 @@ static int resolve_oldest(rg_ctx* c) {
   rg_ctx::Pending& p = c->pend[c->pend_head];
   CK(cudaEventSynchronize(p.done));
   const int oy = ((volatile int*)p.h_reach)[0], ox = ((volatile int*)p.h_reach)[1];
-  if (*(volatile int*)p.h_err == 0) {
+  if (*(volatile int*)p.h_err == 0 || p.complete) {
     observe_reach(c, oy, ox);
     c->pend_head ^= 1;
     c->pend_count--;

@@ -61,3 +61,32 @@ def test_copy_of_a_group_while_running():
             e.sync()
         for a, b in zip(*sets):
             assert a.records_gops(F).tobytes() == b.records_gops(F).tobytes()
+
+
+@pytest.mark.parametrize("order", [(0, 1, 2), (2, 1, 0)])
+def test_group_contexts_fetched_before_the_launch_ends_go_on(order):
+    """A context's records fetched while other contexts of the launch still run: its reconstruction, its
+    next group call and one of its own equal those of contexts synchronised after each launch."""
+    from ragdoll_b200.engine import Engine
+    sizes = [(96, 80), (176, 144), (1280, 720)]
+    calls = [_device_call(w, h, 70 + w) for w, h in sizes]
+    sets = [[Engine(w, h, 30, profile=2, num_streams=S, max_frames=F) for w, h in sizes] for _ in range(2)]
+    args = ([c[1] for c in calls], [w for w, _ in sizes], [(w + 1) // 2 for w, _ in sizes])
+    for call in range(2):
+        got = {}
+        Engine.analyse_gops_group(sets[0], *args, [_kinds(call == 0)] * 3, F)
+        for i in order:
+            got[i] = sets[0][i].records_gops(F)
+        Engine.analyse_gops_group(sets[1], *args, [_kinds(call == 0)] * 3, F)
+        for e in sets[1]:
+            e.sync()
+        for i in order:
+            assert got[i].tobytes() == sets[1][i].records_gops(F).tobytes()
+    w, h = sizes[0]
+    for s in sets:
+        s[0].analyse_gops_device(calls[0][1], w, (w + 1) // 2, _kinds(False), F)
+    assert sets[0][0].records_gops(F).tobytes() == sets[1][0].records_gops(F).tobytes()
+    for a, b in zip(*sets):
+        for k in range(S):
+            for p, q in zip(a.recon_coded(k), b.recon_coded(k)):
+                assert np.array_equal(p, q)
