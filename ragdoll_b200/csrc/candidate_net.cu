@@ -237,21 +237,77 @@ __global__ void __launch_bounds__(kThreads + 32, kCtasPerSm) cnn_infer_kernel(In
   // buffer for conv2 and conv3, the B operands; a tile / tap adds its offset in 16-byte units
   const uint64_t bufd0 = umma_desc(sBuf, kPlane, 128), bufd1 = umma_desc(sBuf + 2 * kPlane, kPlane, 128);
   const uint64_t b1d = umma_desc(sB1, 512, 128), b2d = umma_desc(sB2, 512, 128), b3d = umma_desc(sB3, 512, 128);
-  while (strip < total && ok) {
-    const int job = strip / (ip.mb_h * ip.strips_per_row), rem = strip % (ip.mb_h * ip.strips_per_row);
-    const int mby = rem / ip.strips_per_row, mbx0 = (rem % ip.strips_per_row) * kStripMbs;
-    const InferJob jb = ip.jobs[job];
+  // The loaded bytes into the input map, and the ticket of the strip after (read behind the barrier).
+  auto store_input = [&]() {
     if (warp < 8)
 #pragma unroll
-    for (int k = 0; k < kPer; k++) {
-      __nv_bfloat162 two = __floats2bfloat162_rn(pix_norm(ca[k]), pix_norm(pa[k]));
-      ((uint4*)buf)[tid + kThreads * k] = make_uint4(*(uint32_t*)&two, 0u, 0u, 0u);
-    }
-    if (tid == 0) ms.strip = atomicAdd(ip.counter, 1);  // read after the first layer's barrier
+      for (int k = 0; k < kPer; k++) {
+        __nv_bfloat162 two = __floats2bfloat162_rn(pix_norm(ca[k]), pix_norm(pa[k]));
+        ((uint4*)buf)[tid + kThreads * k] = make_uint4(*(uint32_t*)&two, 0u, 0u, 0u);
+      }
+    if (tid == 0) ms.strip = atomicAdd(ip.counter, 1);
     fence_async_smem();
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
+  };
+  // Logits and hints of strip st from its pooled map (warps 0 .. 7, beside the next strip's first MMAs).
+  auto finish = [&](int st) {
+    const int job = st / (ip.mb_h * ip.strips_per_row), rem = st % (ip.mb_h * ip.strips_per_row);
+    const int mby = rem / ip.strips_per_row, mbx0 = (rem % ip.strips_per_row) * kStripMbs;
+    const InferJob jb = ip.jobs[job];
+    // logits, one a thread at a time: of (block, intra 4x4 mode), then of (macroblock, partition or offset)
+    constexpr int kBlockLogits = kStripMbs * 16 * 9;
+    for (int i = tid; i < kBlockLogits + kStripMbs * 6; i += kThreads) {
+      const bool block = i < kBlockLogits;
+      const int n = block ? i / 9 : (i - kBlockLogits) / 6, o = block ? 6 + i - n * 9 : i - kBlockLogits - n * 6;
+      const float* f = block ? ms.pool[n >> 4][1 + (n & 15)] : ms.pool[n][0];
+      const float* W = ms.head[o];
+      float s = W[C];
+#pragma unroll
+      for (int c = 0; c < C; c++) s += W[c] * f[c];
+      ms.logit[i] = s;
+    }
+    asm volatile("bar.sync 1, 256;" ::: "memory");  // warps 0 .. 7
+    // heads and hints: threads 0 .. 16 kStripMbs - 1 the intra 4x4 heads of (macroblock tid / 16,
+    // block tid % 16), the next kStripMbs threads the partition and offset heads of their macroblock
+    if (tid < 16 * kStripMbs + kStripMbs) {
+      const bool blockhead = tid < 16 * kStripMbs;
+      const int j = blockhead ? tid / 16 : tid - 16 * kStripMbs, mbx = mbx0 + j;
+      if (mbx < ip.mb_w) {
+        const int m = mby * ip.mb_w + mbx;
+        float* lg = jb.logits ? jb.logits + (size_t)m * kLogits : nullptr;
+        if (blockhead) {
+          const int b = tid % 16;
+          float li[9];
+#pragma unroll
+          for (int o = 0; o < 9; o++) li[o] = ms.logit[tid * 9 + o];
+          // 4x4 block b in raster order; the hint holds decoding order
+          const int bx = b & 3, by = b >> 2;
+          const int dec = ((by >> 1) << 3) | ((bx >> 1) << 2) | ((by & 1) << 1) | (bx & 1);
+          jb.hints[m].i4_mask[dec] = (uint16_t)topk_mask(li, ip.i4_k, ip.i4_margin);
+          if (lg)
+            for (int o = 0; o < 9; o++) lg[6 + b * 9 + o] = li[o];
+        } else {
+          const float* l = &ms.logit[kBlockLogits + 6 * j];
+          const float lp[4] = {l[0], l[1], l[2], l[3]}, lm[2] = {l[4], l[5]};
+          rg_mb_hint& hh = jb.hints[m];
+          hh.part_mask = (uint8_t)topk_mask(lp, ip.part_k, ip.part_margin);
+          hh.flags = 0;  // the coarse motion pass, when on, follows
+          hh.mv_coarse[0] = hh.mv_coarse[1] = 0;
+          for (int o = 0; o < 2; o++) hh.mv_off[o] = (int8_t)max(-127, min(127, __float2int_rn(16.0f * lm[o])));
+          if (lg) {
+            for (int o = 0; o < 4; o++) lg[o] = lp[o];
+            lg[4] = lm[0];
+            lg[5] = lm[1];
+          }
+        }
+      }
+    }
+  };
+  if (strip < total) store_input();
+  int pooled = -1;  // the strip whose hints are still to be written
+  while (strip < total && ok) {
     const int next = ms.strip;
     // The ninth warp issues the MMAs of all three layers, tile by tile; each tile completes on its own
     // barrier, and its epilogue, which stores the tile's positions 128 t .. 128 t + 127 over the layer's
@@ -259,7 +315,8 @@ __global__ void __launch_bounds__(kThreads + 32, kCtasPerSm) cnn_infer_kernel(In
     // its MMAs start once both are stored, and tile t is stored once tiles t - 1 and t have completed. The
     // MMAs bound the kernel: 269 a strip, each 46 cycles (M = 128, N = 32: 16 of the tensor pipe; measured
     // alone, whatever the layout of A). Layers one after the other for the whole strip left the tensor
-    // cores 67 cycles a MMA: 2.39 ms for eight 1080p pictures with the coarse pass, 2.15 so.
+    // cores 67 cycles a MMA: 2.39 ms for eight 1080p pictures with the coarse pass, 2.15 so, and 2.12 with a strip's logits
+    // beside the next strip's first MMAs.
     if (warp == 8) {
       if (lane == 0) {
 #pragma unroll 1
@@ -301,8 +358,9 @@ __global__ void __launch_bounds__(kThreads + 32, kCtasPerSm) cnn_infer_kernel(In
       }
       phase ^= 1;  // three layers
       __syncwarp();
-    } else if (next < total) {
-      load_input(next);  // the next strip's bytes, in flight while the tensor cores work
+    } else {
+      if (next < total) load_input(next);  // the next strip's bytes, in flight while the tensor cores work
+      if (pooled >= 0) finish(pooled);
     }
     for (int layer = 0; layer < 3 && warp < 8; layer++, phase ^= 1) {
       const int tiles = layer == 0 ? kTiles1 : (layer == 1 ? kTiles2 : kTiles3);
@@ -395,56 +453,11 @@ __global__ void __launch_bounds__(kThreads + 32, kCtasPerSm) cnn_infer_kernel(In
         for (int k = 0; k < 8; k++) ms.pool[j][0][8 * q + k] = tot[k] * (1.0f / 324.0f);
     }
     __syncthreads();
-    // logits, one a thread at a time: of (block, intra 4x4 mode), then of (macroblock, partition or offset)
-    constexpr int kBlockLogits = kStripMbs * 16 * 9;
-    for (int i = tid; i < kBlockLogits + kStripMbs * 6 && tid < kThreads; i += kThreads) {
-      const bool block = i < kBlockLogits;
-      const int n = block ? i / 9 : (i - kBlockLogits) / 6, o = block ? 6 + i - n * 9 : i - kBlockLogits - n * 6;
-      const float* f = block ? ms.pool[n >> 4][1 + (n & 15)] : ms.pool[n][0];
-      const float* W = ms.head[o];
-      float s = W[C];
-#pragma unroll
-      for (int c = 0; c < C; c++) s += W[c] * f[c];
-      ms.logit[i] = s;
-    }
-    __syncthreads();
-    // heads and hints: threads 0 .. 16 kStripMbs - 1 the intra 4x4 heads of (macroblock tid / 16,
-    // block tid % 16), the next kStripMbs threads the partition and offset heads of their macroblock
-    if (tid < 16 * kStripMbs + kStripMbs) {
-      const bool blockhead = tid < 16 * kStripMbs;
-      const int j = blockhead ? tid / 16 : tid - 16 * kStripMbs, mbx = mbx0 + j;
-      if (mbx < ip.mb_w) {
-        const int m = mby * ip.mb_w + mbx;
-        float* lg = jb.logits ? jb.logits + (size_t)m * kLogits : nullptr;
-        if (blockhead) {
-          const int b = tid % 16;
-          float li[9];
-#pragma unroll
-          for (int o = 0; o < 9; o++) li[o] = ms.logit[tid * 9 + o];
-          // 4x4 block b in raster order; the hint holds decoding order
-          const int bx = b & 3, by = b >> 2;
-          const int dec = ((by >> 1) << 3) | ((bx >> 1) << 2) | ((by & 1) << 1) | (bx & 1);
-          jb.hints[m].i4_mask[dec] = (uint16_t)topk_mask(li, ip.i4_k, ip.i4_margin);
-          if (lg)
-            for (int o = 0; o < 9; o++) lg[6 + b * 9 + o] = li[o];
-        } else {
-          const float* l = &ms.logit[kBlockLogits + 6 * j];
-          const float lp[4] = {l[0], l[1], l[2], l[3]}, lm[2] = {l[4], l[5]};
-          rg_mb_hint& hh = jb.hints[m];
-          hh.part_mask = (uint8_t)topk_mask(lp, ip.part_k, ip.part_margin);
-          hh.flags = 0;  // the coarse motion pass, when on, follows
-          hh.mv_coarse[0] = hh.mv_coarse[1] = 0;
-          for (int o = 0; o < 2; o++) hh.mv_off[o] = (int8_t)max(-127, min(127, __float2int_rn(16.0f * lm[o])));
-          if (lg) {
-            for (int o = 0; o < 4; o++) lg[o] = lp[o];
-            lg[4] = lm[0];
-            lg[5] = lm[1];
-          }
-        }
-      }
-    }
+    if (next < total) store_input();  // over the map that has been pooled
+    pooled = strip;
     strip = next;
   }
+  if (ok && pooled >= 0 && warp < 8) finish(pooled);
   fence_before_sync();
   __syncthreads();
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" ::"r"(tmem));

@@ -38,12 +38,12 @@ std::mutex g_metrics_mu;
 cudaMemPool_t g_metrics_pools[64] = {};
 
 // Deblocking SMs: one in five takes the deblocking queue first (30 of 148). Measured on B200 with
-// 16 warps per SM, 1080p 8 x 15 launch: 25 SMs 52.3-53.2 ms, 30 51.4-52.3, 35-40 52.6-52.8
-// (at 7 warps per SM, before the IDR path got faster: 16 SMs 1326 frames/s, 20-30 1394-1417).
+// 16 warps per SM, 1080p 8 x 15 launch: 16 SMs 24.9 ms, 20 21.8, 25 21.6, 30 21.4, 36 21.9; the other
+// forms and a single stream within 1 % from 12 to 36.
 int default_deblock_sms(int sms) { return sms >= 5 ? (sms + 4) / 5 : 0; }
 // The analysis of IDR pictures heads every GOP (each P picture trails it): the next one SM in
-// seven takes it first (21 of 148; with 30 deblocking SMs: 20 IDR SMs 51.6 ms, 30 51.8, 49 52.3;
-// at 7 warps per SM one in three was best). Those warps continue with P pictures once the IDR
+// seven takes it first (21 of 148; with 30 deblocking SMs: 8 IDR SMs 28.2 ms, 14 22.9, 21 21.4, 30 21.4).
+// Those warps continue with P pictures once the IDR
 // queue is empty.
 int default_intra_sms(int sms) { return sms >= 7 ? sms / 7 : 0; }
 
