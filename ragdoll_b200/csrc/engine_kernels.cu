@@ -2249,10 +2249,10 @@ constexpr int kBlockWarps = 16;
 // most of what one of them fetches is then still there for the other fifteen. A warp that has finished
 // its segment waits here until the others have finished theirs, for at most `limit` ns (a long
 // macroblock's time): one that waits for another SM's macroblock holds nobody for long, and no wait
-// of the schedule depends on a meeting. 1080p 8 x 15 launch: 34.9 ms without, 21.7 with 60 us, 24.5 with
-// 30, 21.5 with 200; learned 1080p (macroblocks three times as long) 92 without, 65.9 with 300 us, 64.5
+// of the schedule depends on a meeting. 1080p 8 x 15 launch: 34.9 ms without, 24.1 with 30 us, 21.5 with
+// 60, 21.2 with 120; learned 1080p 8 x 8 (macroblocks three times as long) 53 with 100 us, 44.6 with 400 and
 // with 1 ms. round: the arrivals that complete this warp's round.
-constexpr int kMeetNs = 60000, kMeetNsSearch = 400000;
+constexpr int kMeetNs = 120000, kMeetNsSearch = 400000;
 __device__ __forceinline__ void meet(int* arrived, int round, int limit) {
   if (lane_id() == 0) {
     int n = atomicAdd(arrived, 1) + 1;
