@@ -54,6 +54,7 @@ struct SearchJob {
   uint32_t lambda;
   uint32_t ticket;   // next unit | units << 16; kNoJob while there is none
   int done;          // units finished
+  bool dead;         // the wait for them gave up: the launch fails, and no other job is opened
   uint32_t key[9];   // the least so far
 };
 constexpr uint32_t kNoJob = 0x8000u;  // (a ticket past any unit)
@@ -290,13 +291,13 @@ __device__ __noinline__ void help_searches(unsigned* board) {
   }
 }
 
-// board (or null): the block's warps that wait take part. A macroblock's search is then a few units long
+// pw.board (or null): the block's warps that wait take part. A macroblock's search is then a few units long
 // instead of nine bands: at range 32 a macroblock's search took 105 k cycles of the chain that a launch of
 // few pictures is (full search 8 x 3 720p: 28.6 ms without help, 23.6 so; learned 1080p 8 x 8, whose walk
 // falls back to it, 50.2 and 46.7, 4K 4 x 3 48.7 and 46.6). Sharing the partition types' refinement the same
 // way gave the full search 6 % more and cost the learned form 3 %.
 __device__ __noinline__ void int_search(const Ctx c, int xlo, int xhi, int ylo, int yhi,
-                                        int mvp0, int mvp1, uint32_t lambda, unsigned* board) {
+                                        int mvp0, int mvp1, uint32_t lambda, const PipeWait pw) {
   const int lane = lane_id();
   const int x0 = c.mbx * 16, y0 = c.mby * 16;
   const int nwx = xhi - xlo + 1, nwy = yhi - ylo + 1;
@@ -308,7 +309,7 @@ __device__ __noinline__ void int_search(const Ctx c, int xlo, int xhi, int ylo, 
   const bool small = nwx <= 8 && nwx * nwy <= 32;
   const int rem = nwx & 31, cols = small ? nwx : (rem <= 4 ? rem : 0), xt = xhi - cols + 1;
   const int units = xt > xlo ? (nwy + kUnitBands * kBandRows - 1) / (kUnitBands * kBandRows) : 0;
-  if (units) {
+  if (units && !(pw.board && ss.job.dead)) {
     SearchJob& jb = ss.job;
     if (lane == 0) {
       jb.ref = sm.sd.ref_y;
@@ -322,14 +323,25 @@ __device__ __noinline__ void int_search(const Ctx c, int xlo, int xhi, int ylo, 
     __syncwarp();
     if (lane == 0) {
       atomicExch(&jb.ticket, (uint32_t)units << 16);
-      if (board) atomicOr(board, 1u << threadIdx.y);
+      if (pw.board) atomicOr(pw.board, 1u << threadIdx.y);
     }
     __syncwarp();
     search_units(threadIdx.y);
     if (lane == 0) {
-      if (board) atomicAnd(board, ~(1u << threadIdx.y));
+      if (pw.board) atomicAnd(pw.board, ~(1u << threadIdx.y));
       atomicExch(&jb.ticket, kNoJob);
-      while (*(volatile int*)&jb.done < units) __nanosleep(50);  // units others still have, each of bounded work
+      // units others still have, each of bounded work; past the limit the launch fails as for any wait, and
+      // this warp opens no other job (whoever is at work on this one still reads it)
+      unsigned long long t0 = 0;
+      while (*(volatile int*)&jb.done < units) {
+        if (!t0) t0 = global_ns();
+        else if (global_ns() - t0 > pw.timeout_ns) {
+          if (pw.error) atomicCAS(pw.error, 0, 1);
+          jb.dead = true;
+          break;
+        }
+        __nanosleep(50);
+      }
     }
     __threadfence_block();
     __syncwarp();
@@ -682,7 +694,7 @@ __device__ __noinline__ bool analyse_p_mb_search(const Ctx c, const PipeWait pw)
     yhi = min(lcy + kLearnedRange, imax1);
   }
   IntBest& ib = ss.ib;  // warp-uniform: once per warp in shared memory
-  int_search(c, xlo, xhi, ylo, yhi, mvp16[0], mvp16[1], lambda, pw.board);
+  int_search(c, xlo, xhi, ylo, yhi, mvp16[0], mvp16[1], lambda, pw);
   if (hint) {
     bool edge = (ib.x[0] == xlo && xlo > imin0) || (ib.x[0] == xhi && xhi < imax0) ||
                 (ib.y[0] == ylo && ylo > imin1) || (ib.y[0] == yhi && yhi < imax1);
@@ -693,7 +705,7 @@ __device__ __noinline__ bool analyse_p_mb_search(const Ctx c, const PipeWait pw)
       ylo = max(cy - kLearnedRange, imin1);
       yhi = min(cy + kLearnedRange, imax1);
       if (!wait_window(c, pw, xhi, yhi)) return false;
-      int_search(c, xlo, xhi, ylo, yhi, mvp16[0], mvp16[1], lambda, pw.board);
+      int_search(c, xlo, xhi, ylo, yhi, mvp16[0], mvp16[1], lambda, pw);
       edge = (ib.x[0] == xlo && xlo > imin0) || (ib.x[0] == xhi && xhi < imax0) ||
              (ib.y[0] == ylo && ylo > imin1) || (ib.y[0] == yhi && yhi < imax1);
     }
@@ -701,7 +713,7 @@ __device__ __noinline__ bool analyse_p_mb_search(const Ctx c, const PipeWait pw)
       xlo = max(fcx - R, imin0); xhi = min(fcx + R, imax0);
       ylo = max(fcy - R, imin1); yhi = min(fcy + R, imax1);
       if (!wait_window(c, pw, xhi, yhi)) return false;
-      int_search(c, xlo, xhi, ylo, yhi, mvp16[0], mvp16[1], lambda, pw.board);
+      int_search(c, xlo, xhi, ylo, yhi, mvp16[0], mvp16[1], lambda, pw);
     }
   }
   // 3-4. refinement of every tried type, the least total cost wins
