@@ -2291,10 +2291,7 @@ __global__ void __launch_bounds__(32 * kBlockWarps, 1) pipeline_kernel(const __g
     board = 0;
   }
   if constexpr (kForm != 0)
-    if (lane == 0) {
-      ss.job.ticket = kNoJob;
-      ss.job.dead = false;
-    }
+    if (lane == 0) ss.job.ticket = kNoJob;
   if (lane == 0) sm.reach_y = sm.reach_x = 0;  // this warp's, published once as it exits
   int group = -1;                              // whose parameters sm.fp holds
   __syncthreads();

@@ -54,7 +54,6 @@ struct SearchJob {
   uint32_t lambda;
   uint32_t ticket;   // next unit | units << 16; kNoJob while there is none
   int done;          // units finished
-  bool dead;         // the wait for them gave up: the launch fails, and no other job is opened
   uint32_t key[9];   // the least so far
 };
 constexpr uint32_t kNoJob = 0x8000u;  // (a ticket past any unit)
@@ -296,8 +295,11 @@ __device__ __noinline__ void help_searches(unsigned* board) {
 // few pictures is (full search 8 x 3 720p: 28.6 ms without help, 23.6 so; learned 1080p 8 x 8, whose walk
 // falls back to it, 50.2 and 46.7, 4K 4 x 3 48.7 and 46.6). Sharing the partition types' refinement the same
 // way gave the full search 6 % more and cost the learned form 3 %.
-__device__ __noinline__ void int_search(const Ctx c, int xlo, int xhi, int ylo, int yhi,
-                                        int mvp0, int mvp1, uint32_t lambda, const PipeWait pw) {
+//
+// False when the wait for units others took gave up: ss.ib then holds nothing, and the caller has to leave as
+// after any wait that did -- the warp takes no other segment, so the job that others may still read stays as it is.
+[[nodiscard]] __device__ __noinline__ bool int_search(const Ctx c, int xlo, int xhi, int ylo, int yhi, int mvp0, int mvp1,
+                                                      uint32_t lambda, const PipeWait pw) {
   const int lane = lane_id();
   const int x0 = c.mbx * 16, y0 = c.mby * 16;
   const int nwx = xhi - xlo + 1, nwy = yhi - ylo + 1;
@@ -309,7 +311,7 @@ __device__ __noinline__ void int_search(const Ctx c, int xlo, int xhi, int ylo, 
   const bool small = nwx <= 8 && nwx * nwy <= 32;
   const int rem = nwx & 31, cols = small ? nwx : (rem <= 4 ? rem : 0), xt = xhi - cols + 1;
   const int units = xt > xlo ? (nwy + kUnitBands * kBandRows - 1) / (kUnitBands * kBandRows) : 0;
-  if (units && !(pw.board && ss.job.dead)) {
+  if (units) {
     SearchJob& jb = ss.job;
     if (lane == 0) {
       jb.ref = sm.sd.ref_y;
@@ -327,22 +329,23 @@ __device__ __noinline__ void int_search(const Ctx c, int xlo, int xhi, int ylo, 
     }
     __syncwarp();
     search_units(threadIdx.y);
+    bool ok = true;
     if (lane == 0) {
       if (pw.board) atomicAnd(pw.board, ~(1u << threadIdx.y));
       atomicExch(&jb.ticket, kNoJob);
-      // units others still have, each of bounded work; past the limit the launch fails as for any wait, and
-      // this warp opens no other job (whoever is at work on this one still reads it)
+      // units others still have, each of bounded work; past the limit the launch fails as for any wait
       unsigned long long t0 = 0;
       while (*(volatile int*)&jb.done < units) {
         if (!t0) t0 = global_ns();
         else if (global_ns() - t0 > pw.timeout_ns) {
           if (pw.error) atomicCAS(pw.error, 0, 1);
-          jb.dead = true;
+          ok = false;
           break;
         }
         __nanosleep(50);
       }
     }
+    if (!__shfl_sync(FULL, ok, 0)) return false;
     __threadfence_block();
     __syncwarp();
 #pragma unroll
@@ -377,6 +380,7 @@ __device__ __noinline__ void int_search(const Ctx c, int xlo, int xhi, int ylo, 
     ss.ib.y[lane] = ylo + y;
   }
   __syncwarp();
+  return true;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -625,8 +629,8 @@ __device__ __noinline__ int2 learned_centre(const Ctx c, int mvp0, int mvp1, uin
   return make_int2(bx, by);
 }
 
-// One macroblock of a P slice in the search forms (see the head of this file); false when a wait for
-// the reference picture gave up.
+// One macroblock of a P slice in the search forms (see the head of this file); false, with nothing
+// written, when a wait for the reference picture or for shared search units gave up.
 __device__ __noinline__ bool analyse_p_mb_search(const Ctx c, const PipeWait pw) {
   const StreamDev& sd = sm.sd;
   const int lane = lane_id();
@@ -694,7 +698,7 @@ __device__ __noinline__ bool analyse_p_mb_search(const Ctx c, const PipeWait pw)
     yhi = min(lcy + kLearnedRange, imax1);
   }
   IntBest& ib = ss.ib;  // warp-uniform: once per warp in shared memory
-  int_search(c, xlo, xhi, ylo, yhi, mvp16[0], mvp16[1], lambda, pw);
+  if (!int_search(c, xlo, xhi, ylo, yhi, mvp16[0], mvp16[1], lambda, pw)) return false;
   if (hint) {
     bool edge = (ib.x[0] == xlo && xlo > imin0) || (ib.x[0] == xhi && xhi < imax0) ||
                 (ib.y[0] == ylo && ylo > imin1) || (ib.y[0] == yhi && yhi < imax1);
@@ -705,7 +709,7 @@ __device__ __noinline__ bool analyse_p_mb_search(const Ctx c, const PipeWait pw)
       ylo = max(cy - kLearnedRange, imin1);
       yhi = min(cy + kLearnedRange, imax1);
       if (!wait_window(c, pw, xhi, yhi)) return false;
-      int_search(c, xlo, xhi, ylo, yhi, mvp16[0], mvp16[1], lambda, pw);
+      if (!int_search(c, xlo, xhi, ylo, yhi, mvp16[0], mvp16[1], lambda, pw)) return false;
       edge = (ib.x[0] == xlo && xlo > imin0) || (ib.x[0] == xhi && xhi < imax0) ||
              (ib.y[0] == ylo && ylo > imin1) || (ib.y[0] == yhi && yhi < imax1);
     }
@@ -713,7 +717,7 @@ __device__ __noinline__ bool analyse_p_mb_search(const Ctx c, const PipeWait pw)
       xlo = max(fcx - R, imin0); xhi = min(fcx + R, imax0);
       ylo = max(fcy - R, imin1); yhi = min(fcy + R, imax1);
       if (!wait_window(c, pw, xhi, yhi)) return false;
-      int_search(c, xlo, xhi, ylo, yhi, mvp16[0], mvp16[1], lambda, pw);
+      if (!int_search(c, xlo, xhi, ylo, yhi, mvp16[0], mvp16[1], lambda, pw)) return false;
     }
   }
   // 3-4. refinement of every tried type, the least total cost wins
