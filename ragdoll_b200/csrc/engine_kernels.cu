@@ -2636,7 +2636,8 @@ void launch_pipeline(const FrameGroups& fg, const StreamDev* d_streams, int n_de
   const dim3 block(32, warps);
   const size_t smem = warps * warp_smem(form);
   const auto kernel = form ? pipeline_kernel<1, false> : (early ? pipeline_kernel<0, true> : pipeline_kernel<0, false>);
-  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // (a whole block's, whatever this launch takes: contexts of other threads launch the same kernel)
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kBlockWarps * warp_smem(form)));
   kernel<<<g, block, smem, st>>>(fg, d_streams, pp);
   if (host_err) error_to_host_kernel<<<1, 1, 0, st>>>(pp.error, pp.reach, host_err, host_reach);
 }
