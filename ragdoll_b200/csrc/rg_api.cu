@@ -619,12 +619,24 @@ static void gop_desc(const rg_ctx* c, StreamDev& d, int f, int s, const uint8_t*
   d.done = done ? done + f * S + s : nullptr;
 }
 
+// The context's device for what a call makes on its first use, whichever one is current.
+struct OnDevice {
+  int was = -1;
+  explicit OnDevice(int device) {
+    if (cudaGetDevice(&was) != cudaSuccess || was == device || cudaSetDevice(device) != cudaSuccess) was = -1;
+  }
+  ~OnDevice() {
+    if (was >= 0) cudaSetDevice(was);
+  }
+};
+
 // The context's flags as the device sees them -- per picture of a call: records final, then (group
 // launches) per picture: deblocked -- cleared for the next launch (every earlier one
 // resolved); null where they cannot be had: the records are then copied after the launch.
 static int* final_flags(rg_ctx* c) {
   const size_t n = sizeof(int) * 2 * (size_t)c->S * c->max_frames;
   if (!c->h_final) {
+    OnDevice on(c->cfg.device);
     if (!c->f_out && cudaStreamCreateWithFlags(&c->f_out, cudaStreamNonBlocking) != cudaSuccess) c->f_out = nullptr;
     if (!c->f_out || cudaHostAlloc((void**)&c->h_final, n, cudaHostAllocMapped) != cudaSuccess) c->h_final = nullptr;
     if (c->h_final && cudaHostGetDevicePointer((void**)&c->d_final, c->h_final, 0) != cudaSuccess) {
@@ -697,9 +709,12 @@ static int enqueue_gops(rg_ctx* c, const uint8_t* const* dev_planes, size_t stri
   uint2* dec = nullptr;
   const size_t dec_bytes = sizeof(uint2) * (size_t)c->n_mb * S;
   if (c->form == RG_FORM_PLAIN && !pipeline_meets(pipeline_task_count(c->fp, frames, c->seg), c->grid, key_span)) {
-    if (!c->decs && cudaMalloc((void**)&c->decs, dec_bytes * c->max_frames) != cudaSuccess) {
-      c->decs = nullptr;  // without them macroblocks wait for reconstructed neighbours
-      cudaGetLastError();
+    if (!c->decs) {
+      OnDevice on(c->cfg.device);
+      if (cudaMalloc((void**)&c->decs, dec_bytes * c->max_frames) != cudaSuccess) {
+        c->decs = nullptr;  // without them macroblocks wait for reconstructed neighbours
+        cudaGetLastError();
+      }
     }
     dec = c->decs;
     if (dec) CK(cudaMemsetAsync(dec, 0, dec_bytes * frames, c->stream));

@@ -1,0 +1,61 @@
+"""Which device the library's host code allocates on, with two devices and a current device that is not the
+context's, against a stand-in for the CUDA runtime (fake_cudart.c; no GPU)."""
+import os
+import shutil
+import subprocess
+import sys
+from pathlib import Path
+
+import pytest
+
+HERE = Path(__file__).resolve().parent
+CUDA_INCLUDE = Path(os.environ.get("CUDA_HOME", "/usr/local/cuda")) / "include"
+PRELUDE = """
+import ctypes, sys
+sys.path.insert(0, sys.argv[2])
+import numpy as np
+fake = ctypes.CDLL(sys.argv[1])
+fake.fake_log.restype = ctypes.c_char_p
+from ragdoll_b200.engine import RG_FRAME_IDR, RG_FRAME_P, Engine, RgError, lib
+log = lambda: fake.fake_log().decode().split("\\n")[:-1]
+"""
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    cc = shutil.which("gcc")
+    if not cc or not CUDA_INCLUDE.exists():
+        pytest.skip("needs gcc and the CUDA headers")
+    so = tmp_path_factory.mktemp("fake") / "libfake_cudart.so"
+    subprocess.run([cc, "-shared", "-fPIC", "-O1", f"-I{CUDA_INCLUDE}", "-o", str(so), str(HERE / "fake_cudart.c")], check=True)
+    return so
+
+
+def _run(fake, body):
+    r = subprocess.run([sys.executable, "-c", PRELUDE + body, str(fake), str(HERE.parent)], env={**os.environ, "LD_PRELOAD": str(fake)},
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_buffers_of_a_first_call_are_on_the_contexts_device(fake):
+    """A call while another device is current is refused by its launch, as ever; what it allocated on the way
+    is the context's for the calls to come, and therefore on the context's device."""
+    _run(fake, """
+w = h = 32
+eng = Engine(w, h, 30, profile=2, device=0, max_frames=2)
+planes = [np.zeros(w * h, np.uint8) for _ in range(3)] * 2
+args = ([p.ctypes.data for p in planes], w, w // 2, [RG_FRAME_IDR, RG_FRAME_P], 2)
+fake.cudaSetDevice(1)
+fake.fake_clear()
+try:
+    eng.analyse_gops_device(*args)
+    raise SystemExit("accepted")
+except RgError:
+    pass
+fake.cudaSetDevice(0)
+eng.analyse_gops_device(*args)
+eng.records_gops(2)
+made = log()
+assert any(l.startswith("malloc") for l in made) and any(l.startswith("stream") for l in made), made
+assert all(l.endswith(" 0") for l in made), made
+""")
