@@ -1115,9 +1115,12 @@ int ensure_bops(rg_net* net) {
 }
 // Samples of one block of the weight-gradient kernels: the batch spread over the SMs.
 int wgrad_per(int n, int sms) { return (n + sms - 1) / sms; }
-// Floats of the partial sums of n samples (at most n blocks of the weight-gradient kernels).
-size_t parts_floats(size_t n) { return n * (kWg1Row + 2 * 2 * (size_t)kWgRow + kHeadParams + 1); }
-int ensure_train(rg_net* net, int n) {
+// Floats of the partial sums of batches of up to n samples: a row per block of the weight-gradient kernels (one
+// an SM at most, whatever the batch), and one per sample of the heads.
+size_t parts_floats(int n, int sms) {
+  return (size_t)(n < sms ? n : sms) * (kWg1Row + 2 * 2 * kWgRow) + (size_t)n * (kHeadParams + 1);
+}
+int ensure_train(rg_net* net, int n, int sms) {
   if (n <= net->cap) return RG_OK;
   cudaFree(net->a1); cudaFree(net->a2); cudaFree(net->a3); cudaFree(net->d3); cudaFree(net->d2); cudaFree(net->d1);
   cudaFree(net->parts);
@@ -1125,7 +1128,7 @@ int ensure_train(rg_net* net, int n) {
   net->cap = 0;
   size_t f = sizeof(float);
   if ((!net->trans && cudaMalloc((void**)&net->trans, f * (kTrans + 4)) != cudaSuccess) ||
-      cudaMalloc((void**)&net->parts, f * parts_floats(n)) != cudaSuccess ||
+      cudaMalloc((void**)&net->parts, f * parts_floats(n, sms)) != cudaSuccess ||
       cudaMalloc((void**)&net->a1, f * n * kA1) != cudaSuccess || cudaMalloc((void**)&net->a2, f * n * kA2) != cudaSuccess ||
       cudaMalloc((void**)&net->a3, f * n * kA3) != cudaSuccess || cudaMalloc((void**)&net->d3, f * n * kA3) != cudaSuccess ||
       cudaMalloc((void**)&net->d2, f * n * kA2) != cudaSuccess || cudaMalloc((void**)&net->d1, f * n * kA1) != cudaSuccess)
@@ -1238,10 +1241,10 @@ int rg_net_forward_backward(rg_net* net, const uint8_t* dev_crops, int32_t n, co
   if (!net || !dev_crops || n < 1 || !dev_part || !dev_i4 || !dev_mv || !dev_mvv)
     return nfail(RG_ERR_INVALID, "rg_net_forward_backward: bad arguments");
   NCK(cudaSetDevice(net->device));
-  int r = ensure_train(net, n);
-  if (r) return r;
   int sms = 0;
   NCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, net->device));
+  int r = ensure_train(net, n, sms);
+  if (r) return r;
   const float* P = net->P;
   float *T = net->trans, *scales = T + kTrans;
   // the labels' counts normalise each loss

@@ -1,7 +1,7 @@
 /* A stand-in for the CUDA runtime's memory, stream and launch calls with two devices, preloaded in front of
  * it: device memory is host memory, launches do nothing. It keeps the current device, refuses a launch into
- * another device's stream as the runtime does, and logs every allocation and pool call with its device
- * (fake_log). Tests of the library's host code (test_device_calls.py). */
+ * another device's stream as the runtime does, and logs every allocation (device, bytes) and pool call (fake_log).
+ * Tests of the library's host code (test_device_calls.py). */
 #include <cuda_runtime_api.h>
 #include <stdarg.h>
 #include <stdio.h>
@@ -25,7 +25,7 @@ struct CUevent_st { int device; };
 struct CUmemPoolHandle_st { int device; };
 static cudaError_t take(void** p, size_t n, const char* what) {
   *p = calloc(1, n + 4096);
-  note("%s %d\n", what, cur);
+  note("%s %d %zu\n", what, cur, n);
   return cudaSuccess;
 }
 

@@ -1,4 +1,4 @@
-"""Which device the library's host code allocates on, with two devices and a current device that is not the
+"""What the library's host code allocates, and on which of two devices where the current one is not the
 context's, against a stand-in for the CUDA runtime (fake_cudart.c; no GPU)."""
 import os
 import shutil
@@ -17,7 +17,7 @@ import numpy as np
 fake = ctypes.CDLL(sys.argv[1])
 fake.fake_log.restype = ctypes.c_char_p
 from ragdoll_b200.engine import RG_FRAME_IDR, RG_FRAME_P, Engine, RgError, lib
-log = lambda: fake.fake_log().decode().split("\\n")[:-1]
+log = lambda: [l.split() for l in fake.fake_log().decode().split("\\n")[:-1]]
 """
 
 
@@ -56,6 +56,24 @@ fake.cudaSetDevice(0)
 eng.analyse_gops_device(*args)
 eng.records_gops(2)
 made = log()
-assert any(l.startswith("malloc") for l in made) and any(l.startswith("stream") for l in made), made
-assert all(l.endswith(" 0") for l in made), made
+assert {"malloc", "stream"} <= {l[0] for l in made}, made
+assert all(l[1] == "0" for l in made), made
+""")
+
+
+def test_training_scratch_grows_with_the_activations(fake):
+    """The six maps of a sample are 309,248 bytes; the partial sums are a few rows a sample and a row a block
+    of the weight gradients, of which there are no more than SMs. A smaller batch allocates nothing."""
+    _run(fake, """
+from ragdoll_b200.learned import CandidateNet
+n = 4096
+net = CandidateNet(0)
+buf = np.zeros(n * 1152, np.uint8)
+fake.fake_clear()
+for batch in (n, n, 150, 1):
+    net.forward_backward(buf.ctypes.data, batch, buf.ctypes.data, buf.ctypes.data, buf.ctypes.data, buf.ctypes.data)
+    if batch == n:
+        size = sum(int(l[2]) for l in log())
+    assert size <= 1.05 * n * 309248, size / n
+    assert size == sum(int(l[2]) for l in log())
 """)
