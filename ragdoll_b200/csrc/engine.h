@@ -118,9 +118,12 @@ struct FrameGroups {
   FrameParams g[kMaxGroups];
   int32_t n;
 };
-// Whether the warps of an SM meet between their segments in a launch of n_tasks segments over key_span
-// macroblock-times (pipeline_kernel).
-bool pipeline_meets(size_t n_tasks, int grid, int key_span);
+// A launch's pictures: IDR ones alone, single pictures of both kinds, or anything else.
+enum class PictureMix { kIdr, kSingles, kGops };
+PictureMix picture_mix(const int32_t* kinds, int streams, int frames);
+// Whether the warps of an SM meet between their segments (pipeline_kernel) in a launch of n_tasks segments
+// over key_span macroblock-times; form: RG_FORM_*.
+bool pipeline_meets(size_t n_tasks, int grid, int key_span, int form, PictureMix mix);
 int pipeline_grid(int device);
 int pipeline_sms(int device);
 size_t pipeline_counter_ints(const FrameParams& fp, int frames);
@@ -151,7 +154,7 @@ struct CompactOut {
   int* row_bytes;    // device address of mapped host memory: [row]
 };
 void launch_pipeline(const FrameGroups& fg, const StreamDev* d_streams, int n_desc, int total_rows, int* counters,
-                     const int2* d_tasks, size_t n_tasks, int key_span, const int qbeg[3], const int qend[3], int deblock_sms,
+                     const int2* d_tasks, size_t n_tasks, bool meet, const int qbeg[3], const int qend[3], int deblock_sms,
                      int intra_sms, int sms, int seg, int grid, unsigned long long timeout_ns, int* ready, int seq,
                      int* host_err, int* host_reach, cudaStream_t st, int form = 0, const CompactOut* co = nullptr, bool early = false);
 void launch_error_to_host(const int* counters, int n_desc, int total_rows, int* host_err, int* host_reach,

@@ -2590,16 +2590,34 @@ size_t pipeline_task_list(const FrameParams& fp, int frames, int lag, int seg, b
   return pipeline_task_count(fp, frames, seg);
 }
 
-// Meetings pay where there is work for most warps, and cost a little where the launch is one chain
-// of macroblocks and they wait anyway: on average at least a quarter as many segments ready as there
-// are warps (segments over the span of their keys, both roles). 8 x 15 pictures of 1080p have 1742
-// (34.9 -> 21.7 ms), 8 x 8 learned 1238 (92 -> 65.5), four mixed sizes 1148 (17.3 -> 13.1), 4 x 3
-// learned 4K 672 (80.9 -> 77.2), 8 x 3 full search 720p 310 (50.9 -> 52.3), one 720p stream 179 (11.8 ->
-// 12.2).
-bool pipeline_meets(size_t n_tasks, int grid, int key_span) { return n_tasks / 2 * 4 >= (size_t)grid * (size_t)key_span; }
+// Meetings pay where there is work for enough warps, and cost a little where the launch is one chain of
+// macroblocks and they wait anyway. The measure is the segments ready side by side (both roles: all of them
+// over the span of their keys) for each warp; launch times apart -> meeting, 2368 warps (in the plain form a
+// launch whose warps stay apart also starts macroblocks early, so both sides differ by that too):
+//   plain (720p, 1080p, 360p High, 2 to 15 pictures): 0.05 7.2 -> 9.1 ms, 0.10 8.8 -> 9.8, 0.127 8.13 -> 8.03,
+//     0.14 10.9 -> 10.5, 0.19 13.1 -> 11.5, 0.24 14.6 -> 12.0, 0.38 18.8 -> 13.8;
+//   learned (360p to 4K): 0.06 15.4 -> 15.6, 0.10 12.0 -> 12.2, 0.12 18.5 -> 17.9, 0.18 22.9 -> 20.6, 0.30 46.5 -> 38.6;
+//   IDR pictures alone: 0.12 3.7 -> 3.9, 0.18 3.90 -> 3.98, 0.215 12.1 -> 12.3, 0.233 4.14 -> 4.08, 0.36 4.7 -> 4.3;
+//   single pictures, IDR and P side by side: 0.054 3.52 -> 3.59, 0.072 2.10 -> 1.90, 0.08 11.7 -> 11.1, 0.107 13.5 -> 11.6;
+//   full search (its searches are shared by the warps that wait instead): 0.06 22.1 -> 23.3, 0.24 34.2 -> 38.9,
+//     0.37 99 -> 108, 0.44 92.6 -> 88.7, 0.48 56.2 -> 51.9.
+// So the lines lie at 1/8, at 2/9 for IDR pictures alone, at 1/14 for single pictures of both kinds (the code
+// of both is then fetched all along) and at 2/5 for the full search.
+PictureMix picture_mix(const int32_t* kinds, int streams, int frames) {
+  const int n = streams * frames;
+  int idr = 0;
+  for (int i = 0; i < n; i++) idr += kinds[i] == RG_FRAME_IDR;
+  return idr == n ? PictureMix::kIdr : (frames == 1 && idr ? PictureMix::kSingles : PictureMix::kGops);
+}
+bool pipeline_meets(size_t n_tasks, int grid, int key_span, int form, PictureMix mix) {
+  const size_t ready = n_tasks / 2, warps = (size_t)grid * (size_t)key_span;
+  if (form == RG_FORM_FULLSEARCH) return 5 * ready >= 2 * warps;
+  if (mix == PictureMix::kIdr) return 9 * ready >= 2 * warps;
+  return (mix == PictureMix::kSingles ? 14 : 8) * ready >= warps;
+}
 
 void launch_pipeline(const FrameGroups& fg, const StreamDev* d_streams, int n_desc, int total_rows, int* counters,
-                     const int2* d_tasks, size_t n_tasks, int key_span, const int qbeg[3], const int qend[3], int deblock_sms,
+                     const int2* d_tasks, size_t n_tasks, bool meet, const int qbeg[3], const int qend[3], int deblock_sms,
                      int intra_sms, int sms, int seg, int grid, unsigned long long timeout_ns, int* ready, int seq,
                      int* host_err, int* host_reach, cudaStream_t st, int form, const CompactOut* co, bool early) {
   PipeParams pp;
@@ -2615,7 +2633,6 @@ void launch_pipeline(const FrameGroups& fg, const StreamDev* d_streams, int n_de
   }
   pp.deblock_sms = deblock_sms;
   pp.intra_sms = intra_sms;
-  const bool meet = pipeline_meets(n_tasks, grid, key_span);
   pp.meet_ns = meet ? (form ? kMeetNsSearch : kMeetNs) : 0;
   // spread over the SMs, then up to a block's warps on each
   pp.grid = grid < pp.n_tasks ? grid : pp.n_tasks;

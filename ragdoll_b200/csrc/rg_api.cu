@@ -705,10 +705,12 @@ static int enqueue_gops(rg_ctx* c, const uint8_t* const* dev_planes, size_t stri
   }
   // A launch too small for meetings is one chain of macroblocks: each starts on its neighbours' decisions
   // there, before they are reconstructed.
-  const int lag = c->lag > 0 ? c->lag : auto_lag(c), key_span = pipeline_key_span(c->fp, frames, lag, c->seg);
+  const int lag = c->lag > 0 ? c->lag : auto_lag(c);
+  const bool meet = pipeline_meets(pipeline_task_count(c->fp, frames, c->seg), c->grid, pipeline_key_span(c->fp, frames, lag, c->seg),
+                                   c->form, picture_mix(kinds, S, frames));
   uint2* dec = nullptr;
   const size_t dec_bytes = sizeof(uint2) * (size_t)c->n_mb * S;
-  if (c->form == RG_FORM_PLAIN && !pipeline_meets(pipeline_task_count(c->fp, frames, c->seg), c->grid, key_span)) {
+  if (c->form == RG_FORM_PLAIN && !meet) {
     if (!c->decs) {
       OnDevice on(c->cfg.device);
       if (cudaMalloc((void**)&c->decs, dec_bytes * c->max_frames) != cudaSuccess) {
@@ -761,7 +763,7 @@ static int enqueue_gops(rg_ctx* c, const uint8_t* const* dev_planes, size_t stri
   fg.g[0] = fp;
   fg.n = 1;
   launch_pipeline(fg, c->d_streams[slot], frames * S, frames * S * fp.mb_h, c->counters, c->d_tasks, c->n_tasks,
-                  key_span, c->qbeg, c->qend, c->deblock_sms, c->intra_sms, c->sms, c->seg, c->grid, c->timeout_ns, ready, seq,
+                  meet, c->qbeg, c->qend, c->deblock_sms, c->intra_sms, c->sms, c->seg, c->grid, c->timeout_ns, ready, seq,
                   c->d_err + pslot, c->d_err + 2 + 2 * pslot, c->stream, c->form != RG_FORM_PLAIN, co, dec != nullptr);
   CK(cudaGetLastError());
   CK(cudaEventRecord(p.done, c->stream));
@@ -912,10 +914,12 @@ static int group_launch(rg_ctx* const* ctxs, int32_t n, const uint8_t* const* co
     if (intra_q) shape.insert(shape.end(), kinds[i], kinds[i] + (size_t)frames * c->S);
   }
   int key_span = 1;
+  std::vector<int32_t> all_kinds;
   for (int i = 0; i < n; i++) {
     const rg_ctx* c = ctxs[i];
     const int lag = c->lag > 0 ? c->lag : a * (4 + c->reach_y) + seg + c->reach_x + 3;
     key_span = std::max(key_span, pipeline_key_span(c->fp, frames, lag, seg));
+    all_kinds.insert(all_kinds.end(), kinds[i], kinds[i] + (size_t)frames * c->S);
   }
   if (shape != L->g_shape) {
     std::vector<std::vector<int2>> lists(n);
@@ -989,8 +993,10 @@ static int group_launch(rg_ctx* const* ctxs, int32_t n, const uint8_t* const* co
   // holds the launch as its own pending call, resolved and if a wait gave up re-run picture by
   // picture by the context itself) -- as a CUDA graph, captured for each launch shape and replayed
   // while it holds (the descriptors' contents change per call; the copy reads them as it runs).
+  const bool meet = pipeline_meets(L->g_ntasks, grid, key_span, L->form,
+                                   picture_mix(all_kinds.data(), (int)all_kinds.size() / frames, frames));
   std::vector<int64_t> key = L->g_shape;
-  key.insert(key.end(), {n_desc, total_rows, (int64_t)n_counters, (int64_t)L->g_ntasks, T->deblock_sms,
+  key.insert(key.end(), {meet, n_desc, total_rows, (int64_t)n_counters, (int64_t)L->g_ntasks, T->deblock_sms,
                          T->intra_sms, L->sms, (int64_t)T->timeout_ns, (int64_t)(uintptr_t)L->g_dstreams,
                          (int64_t)(uintptr_t)L->g_hstreams, (int64_t)(uintptr_t)L->g_counters,
                          (int64_t)(uintptr_t)L->g_dtasks, L->form, seq});
@@ -1013,7 +1019,7 @@ static int group_launch(rg_ctx* const* ctxs, int32_t n, const uint8_t* const* co
     if (e == cudaSuccess) e = cudaEventRecordWithFlags(L->g_done, L->stream, cudaEventRecordExternal);
     if (e == cudaSuccess) e = cudaMemsetAsync(L->g_counters, 0, sizeof(int) * n_counters, L->stream);
     if (e == cudaSuccess) {
-      launch_pipeline(fg, L->g_dstreams, n_desc, total_rows, L->g_counters, L->g_dtasks, L->g_ntasks, key_span, L->g_qbeg,
+      launch_pipeline(fg, L->g_dstreams, n_desc, total_rows, L->g_counters, L->g_dtasks, L->g_ntasks, meet, L->g_qbeg,
                       L->g_qend, T->deblock_sms, T->intra_sms, L->sms, seg, grid, T->timeout_ns, nullptr, seq, nullptr,
                       nullptr, L->stream, L->form != RG_FORM_PLAIN);
       for (int i = 0; i < n; i++)
@@ -1727,7 +1733,8 @@ int rg_analyse_batch(rg_ctx* c, const uint8_t* const* planes, size_t stride_y, s
   // the reconstruction before deblocking is kept, and for what they refuse. A P picture by 42 launches and
   // by one: 320x180 0.89 -> 0.58 ms, 720p 3.9 -> 2.9, 1080p 6.2 -> 4.7, 8 x 720p 7.5 -> 6.8 (8 x 720p IDR 7.9 -> 8.3).
   bool one = !c->keep_unfiltered && c->form == RG_FORM_PLAIN &&
-             !pipeline_meets(pipeline_task_count(c->fp, 1, c->seg), c->grid, pipeline_key_span(c->fp, 1, 0, c->seg));
+             !pipeline_meets(pipeline_task_count(c->fp, 1, c->seg), c->grid, pipeline_key_span(c->fp, 1, 0, c->seg),
+                             RG_FORM_PLAIN, picture_mix(kinds, c->S, 1));
   for (int s = 0; s < c->S; s++) one = one && (kinds[s] == RG_FRAME_IDR || (kinds[s] == RG_FRAME_P && c->frames[s] > 0));
   int r = one ? rg_analyse_gops_device(c, dev.data(), w, cw, kinds, 1) : rg_analyse_batch_device(c, dev.data(), w, cw, kinds);
   if (r) return r;
