@@ -1728,13 +1728,14 @@ int rg_analyse_batch(rg_ctx* c, const uint8_t* const* planes, size_t stride_y, s
     dev[3 * s + 2] = d + (size_t)w * c->cfg.height + (size_t)cw * ((c->cfg.height + 1) / 2);
   }
   // One launch for the pictures, which this call completes itself (a wait that gives up is re-run by the
-  // sync below), while they are one chain of macroblocks; the per-diagonal launches for more work than
-  // that (16 streams of 1080p: 33.5 ms either way), the search forms (640x352: 7.8 ms against 8.2), where
-  // the reconstruction before deblocking is kept, and for what they refuse. A P picture by 42 launches and
-  // by one: 320x180 0.89 -> 0.58 ms, 720p 3.9 -> 2.9, 1080p 6.2 -> 4.7, 8 x 720p 7.5 -> 6.8 (8 x 720p IDR 7.9 -> 8.3).
-  bool one = !c->keep_unfiltered && c->form == RG_FORM_PLAIN &&
-             !pipeline_meets(pipeline_task_count(c->fp, 1, c->seg), c->grid, pipeline_key_span(c->fp, 1, 0, c->seg),
-                             RG_FORM_PLAIN, picture_mix(kinds, c->S, 1));
+  // sync below); the per-diagonal launches for the search forms (640x352: 7.8 ms against 8.2), where the
+  // reconstruction before deblocking is kept, where the tuning leaves fewer warps than four a segment ready
+  // (1080p with 32 warps would wait for them), and for what they refuse. Per-diagonal -> one launch in ms, all
+  // IDR | all P | half of each, High, sources on the device: 320x180 0.95 -> 0.83 | 0.88 -> 0.55; 720p 3.81 -> 3.49 | 3.48
+  // -> 2.28; 8 x 720p 3.85 -> 3.58 | 4.07 -> 2.77 | 4.00 -> 3.67; 1080p 5.73 -> 5.34 | 5.28 -> 3.52; 16 x 1080p 7.8 -> 6.1 |
+  // 7.3 -> 6.2 | 7.6 -> 6.4; 4 x 4K 12.4 -> 11.0 | 11.5 -> 9.4 | 12.1 -> 11.5; 128 x 1080p 25.5 -> 16.6 | 28.3 -> 16.9 | 31.5 -> 18.2.
+  const size_t ready = pipeline_task_count(c->fp, 1, c->seg) / 2, warps = (size_t)c->grid * pipeline_key_span(c->fp, 1, 0, c->seg);
+  bool one = !c->keep_unfiltered && c->form == RG_FORM_PLAIN && (c->grid >= pipeline_grid(c->cfg.device) || 4 * ready <= warps);
   for (int s = 0; s < c->S; s++) one = one && (kinds[s] == RG_FRAME_IDR || (kinds[s] == RG_FRAME_P && c->frames[s] > 0));
   int r = one ? rg_analyse_gops_device(c, dev.data(), w, cw, kinds, 1) : rg_analyse_batch_device(c, dev.data(), w, cw, kinds);
   if (r) return r;
