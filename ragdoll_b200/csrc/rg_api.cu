@@ -390,10 +390,10 @@ rg_ctx* rg_create(const rg_config* cfg) {
 void rg_destroy(rg_ctx* c) {
   if (!c) return;
   if (c->stream) cudaStreamSynchronize(c->stream);
-  {  // the metrics' idle memory goes back too
-    int dev = 0;
+  {  // the metrics' idle memory of its device goes back too
+    const int dev = c->cfg.device;
     std::lock_guard<std::mutex> lock(g_metrics_mu);
-    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 && g_metrics_pools[dev]) cudaMemPoolTrimTo(g_metrics_pools[dev], 0);
+    if (dev >= 0 && dev < 64 && g_metrics_pools[dev]) cudaMemPoolTrimTo(g_metrics_pools[dev], 0);
   }
   cudaFree(c->pics);
   cudaFree(c->infos);

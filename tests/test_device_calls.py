@@ -61,6 +61,20 @@ assert all(l[1] == "0" for l in made), made
 """)
 
 
+def test_destroying_a_context_trims_its_devices_metrics_pool(fake):
+    _run(fake, """
+from ragdoll_b200.engine import ssim_batch_device
+eng = Engine(32, 32, 30, profile=2, device=0)
+plane = np.zeros(1024, np.uint8).ctypes.data
+for device in (0, 1):
+    ssim_batch_device([plane], [plane], 32, 32, 32, 32, device=device)
+fake.cudaSetDevice(1)
+fake.fake_clear()
+eng.close()
+assert [l for l in log() if l[0] == "trim"] == [["trim", "0", "to", "0"]], log()
+""")
+
+
 def test_training_scratch_grows_with_the_activations(fake):
     """The six maps of a sample are 309,248 bytes; the partial sums are a few rows a sample and a row a block
     of the weight gradients, of which there are no more than SMs. A smaller batch allocates nothing."""
