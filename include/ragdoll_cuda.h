@@ -524,15 +524,21 @@ int rg_ssim_plane(int32_t device, const uint8_t* a, size_t stride_a, const uint8
 
 /*
  * SSIM and (if ms_ssim) 5-scale MS-SSIM of n plane pairs of one size already on the device --
- * e.g. every reconstructed picture of a job against its source -- in shared launches: one 2x2
- * decimation launch per pyramid level for all pairs, then one SSIM launch over every pair and
- * level, then one for the row totals. Same arithmetic as rg_ssim_plane. dev_a[i] / dev_b[i]: device
- * planes with the given strides; ssim / ms_ssim: host arrays of n doubles (either may be NULL).
- * Synchronous on cuda_stream (NULL: legacy default stream); allocates its working memory.
+ * e.g. every reconstructed picture of a job against its source -- in three shared launches: the
+ * planes, read once, with all pyramid levels; the levels; the row totals. Same arithmetic as
+ * rg_ssim_plane. dev_a[i] / dev_b[i]: device planes with the given strides; ssim / ms_ssim: host
+ * arrays of n doubles (either may be NULL). Synchronous on cuda_stream (NULL: legacy default
+ * stream). Its working memory (two thirds of a plane's bytes per pair with MS-SSIM) comes from a pool of
+ * the library that keeps up to 128 MB per device between calls (rg_trim_metrics_memory).
  */
 int rg_ssim_batch_device(int32_t device, const uint8_t* const* dev_a, const uint8_t* const* dev_b, int32_t n,
                          int32_t width, int32_t height, size_t stride_a, size_t stride_b, double* ssim, double* ms_ssim,
                          void* cuda_stream);
+
+/* Gives back the device memory that rg_ssim_batch_device, rg_ssim_plane and rg_quality_frame keep
+ * between calls on `device`; rg_destroy does so too for its context's device. Calls that are running
+ * keep what they use, and the next call allocates again. */
+int rg_trim_metrics_memory(int32_t device);
 
 /*
  * Allocation-free SSIM / MS-SSIM of two planes already on the device. No counterpart in the
@@ -555,7 +561,7 @@ int rg_ssim_batch_device(int32_t device, const uint8_t* const* dev_a, const uint
  * (cudaGetSymbolAddress) with that device current and keeps the address for the life of the
  * process; make that first call before any stream capture begins. Resetting a device
  * (cudaDeviceReset, or any teardown of its primary context) after that first call is not
- * supported: the kept address and the kernel's shared-memory attribute would be stale.
+ * supported: the kept address would be stale.
  */
 int rg_ssim_plane_device_noalloc(const uint8_t* dev_a, size_t stride_a, const uint8_t* dev_b,
                                  size_t stride_b, int32_t width, int32_t height, double* dev_out,

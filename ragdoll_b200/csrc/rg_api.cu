@@ -390,11 +390,7 @@ rg_ctx* rg_create(const rg_config* cfg) {
 void rg_destroy(rg_ctx* c) {
   if (!c) return;
   if (c->stream) cudaStreamSynchronize(c->stream);
-  {  // the metrics' idle memory of its device goes back too
-    const int dev = c->cfg.device;
-    std::lock_guard<std::mutex> lock(g_metrics_mu);
-    if (dev >= 0 && dev < 64 && g_metrics_pools[dev]) cudaMemPoolTrimTo(g_metrics_pools[dev], 0);
-  }
+  rg_trim_metrics_memory(c->cfg.device);
   cudaFree(c->pics);
   cudaFree(c->infos);
   cudaFree(c->mv4s);
@@ -1842,8 +1838,9 @@ struct PlanePair {
 
 // The metrics' device memory, allocated and freed in stream order from a pool of the library per
 // device: it keeps at most kMetricsKeep bytes between calls (a call's scratch costs its size in page
-// mappings otherwise: six cudaMalloc / cudaFree were about 1 ms of a call), and CUDA hands a block to
-// another stream or thread only after the work that used it.
+// mappings otherwise: six cudaMalloc / cudaFree were about 1 ms of a call) until rg_trim_metrics_memory or
+// the end of a context of the device, and CUDA hands a block to another stream or thread only after the
+// work that used it.
 constexpr uint64_t kMetricsKeep = 128ull << 20;
 cudaMemPool_t metrics_pool() {
   cudaMemPool_t* const pools = g_metrics_pools;
@@ -2107,6 +2104,13 @@ int rg_ssim_batch_device(int32_t device, const uint8_t* const* dev_a, const uint
     if (ssim) ssim[i] = ss[i];
     if (ms_ssim) ms_ssim[i] = ms[i];
   }
+  return RG_OK;
+}
+
+int rg_trim_metrics_memory(int32_t device) {
+  if (device < 0 || device >= 64) return fail(RG_ERR_INVALID, "rg_trim_metrics_memory: device %d", device);
+  std::lock_guard<std::mutex> lock(g_metrics_mu);
+  if (g_metrics_pools[device]) CK(cudaMemPoolTrimTo(g_metrics_pools[device], 0));
   return RG_OK;
 }
 

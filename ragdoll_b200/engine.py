@@ -56,7 +56,7 @@ EXPORTS = [
     "rg_analyse_gops_fetch", "rg_set_analysis_form", "rg_set_hints", "rg_encoder_new_gops",
     "rg_net_param_count", "rg_net_create", "rg_net_destroy", "rg_net_set_params", "rg_net_get_params",
     "rg_net_predict_hints", "rg_net_check", "rg_net_crops", "rg_net_forward_backward", "rg_net_adam_step",
-    "rg_set_hint_net", "rg_encoder_set_form", "rg_ssim_batch_device", "rg_set_search_tuning",
+    "rg_set_hint_net", "rg_encoder_set_form", "rg_ssim_batch_device", "rg_trim_metrics_memory", "rg_set_search_tuning",
     "rg_net_set_hint_policy", "rg_net_set_coarse_range", "rg_analyse_gops_group",
     "rg_set_record_compaction", "rg_analyse_gops_fetch_compact", "rg_records_compact", "rg_records_expand",
     "rg_writer_picture_compact", "rg_encoder_record_bytes", "rg_group_graph_counts",
@@ -517,6 +517,11 @@ def ssim_batch_device(dev_a, dev_b, width: int, height: int, stride_a: int, stri
     _check(lib().rg_ssim_batch_device(device, A(*dev_a), A(*dev_b), n, width, height, stride_a, stride_b,
                                       s.ctypes.data, m.ctypes.data if ms else None, stream or None))
     return s, m
+
+
+def trim_metrics_memory(device: int = 0) -> None:
+    """Gives back the device memory the SSIM and quality calls keep between calls (up to 128 MB a device)."""
+    _check(lib().rg_trim_metrics_memory(device))
 
 
 def ssim_plane_device_noalloc(dev_a: int, stride_a: int, dev_b: int, stride_b: int, width: int, height: int,

@@ -75,6 +75,25 @@ assert [l for l in log() if l[0] == "trim"] == [["trim", "0", "to", "0"]], log()
 """)
 
 
+def test_metrics_memory_is_given_back_on_request(fake):
+    _run(fake, """
+from ragdoll_b200.engine import ssim_batch_device, trim_metrics_memory
+plane = np.zeros(1024, np.uint8).ctypes.data
+trim_metrics_memory(1)                      # nothing kept yet
+ssim_batch_device([plane], [plane], 32, 32, 32, 32, device=1)
+fake.fake_clear()
+trim_metrics_memory(0)
+trim_metrics_memory(1)
+assert log() == [["trim", "1", "to", "0"]], log()
+for device in (-1, 64):
+    try:
+        trim_metrics_memory(device)
+        raise SystemExit("accepted")
+    except RgError:
+        pass
+""")
+
+
 def test_training_scratch_grows_with_the_activations(fake):
     """The six maps of a sample are 309,248 bytes; the partial sums are a few rows a sample and a row a block
     of the weight gradients, of which there are no more than SMs. A smaller batch allocates nothing."""
