@@ -1905,8 +1905,10 @@ int device_metrics(const std::vector<PlanePair>& pairs, const std::vector<bool>&
   std::vector<uint64_t> res(n_out);
   cudaError_t e = cudaMemcpyAsync(d, host.data(), host.size(), cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess && sse) e = cudaMemsetAsync(sses, 0, n * sizeof(unsigned long long), st);
+  int dev = 0;
+  if (e == cudaSuccess) e = cudaGetDevice(&dev);
   if (e == cudaSuccess) {
-    launch_ssim(d, n, maxh, any_ms, st);
+    launch_ssim(d, n, maxh, any_ms, pipeline_sms(dev), st);
     if (sse) launch_sse((const SseJob*)(d + n * pair_bytes), n, st);
     e = cudaGetLastError();
   }

@@ -200,10 +200,10 @@ static void launch_rows(const SsimPair* p, int n, int h, bool pyramid, cudaStrea
   if (s) ssim_rows_kernel<false, kStrip, kChunk><<<dim3(s, n), kRowThreads, 0, st>>>(p);
 }
 
-void launch_ssim(const void* d_pairs, int n, int max_height, bool pyramid, cudaStream_t st) {
+void launch_ssim(const void* d_pairs, int n, int max_height, bool pyramid, int sms, cudaStream_t st) {
   const SsimPair* p = (const SsimPair*)d_pairs;
   // two blocks an SM of the tall kind: about as many as hide each other's loads
-  if (n * ssim_strips(max_height, pyramid, kTallStrip) >= 2 * 148) launch_rows<kTallStrip, kTallChunk>(p, n, max_height, pyramid, st);
+  if (n * ssim_strips(max_height, pyramid, kTallStrip) >= 2 * sms) launch_rows<kTallStrip, kTallChunk>(p, n, max_height, pyramid, st);
   else launch_rows<kFlatStrip, kFlatChunk>(p, n, max_height, pyramid, st);
   ssim_finish_kernel<<<dim3(pyramid ? 5 : 1, n), 32, 0, st>>>(p);
 }

@@ -27,8 +27,8 @@ struct SsimSizes {
 size_t ssim_pair_bytes();
 void ssim_pair_fill(void* pair, const uint8_t* a, long sa, const uint8_t* b, long sb, int w, int h, bool ms, float* rows,
                     double* out, uint8_t* pyr, SsimSizes& used);
-// SSIM of every scale of n pairs into their out (pyramid: some have more than one scale).
-void launch_ssim(const void* d_pairs, int n, int max_height, bool pyramid, cudaStream_t st);
+// SSIM of every scale of n pairs into their out (pyramid: some have more than one scale) on a device of `sms` SMs.
+void launch_ssim(const void* d_pairs, int n, int max_height, bool pyramid, int sms, cudaStream_t st);
 void launch_sse(const SseJob* d_jobs, int n_jobs, cudaStream_t st);
 
 // VMAF-Lite of one plane pair (ref a, distorted b; prev: the previous reference frame or null).

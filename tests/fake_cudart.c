@@ -1,15 +1,17 @@
 /* A stand-in for the CUDA runtime's memory, stream and launch calls with two devices, preloaded in front of
  * it: device memory is host memory, launches do nothing. It keeps the current device, refuses a launch into
- * another device's stream as the runtime does, and logs every allocation (device, bytes) and pool call (fake_log).
- * Tests of the library's host code (test_device_calls.py). */
+ * another device's stream as the runtime does, and logs every allocation (device, bytes) and pool call
+ * (fake_log) and the launches' grids (fake_launches). The devices have fake_sms SMs. For tests of the
+ * library's host code (test_device_calls.py). */
 #include <cuda_runtime_api.h>
 #include <stdarg.h>
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
 
+int fake_sms = 148;
 static int cur, last;
-static char text[1 << 16];
+static char text[1 << 16], launches[1 << 16];
 static void note(const char* fmt, ...) {
   va_list ap;
   va_start(ap, fmt);
@@ -18,7 +20,8 @@ static void note(const char* fmt, ...) {
   va_end(ap);
 }
 const char* fake_log(void) { return text; }
-void fake_clear(void) { text[0] = 0; }
+const char* fake_launches(void) { return launches; }
+void fake_clear(void) { text[0] = launches[0] = 0; }
 
 struct CUstream_st { int device; };
 struct CUevent_st { int device; };
@@ -35,13 +38,15 @@ cudaError_t cudaSetDevice(int d) {
   cur = d;
   return cudaSuccess;
 }
-cudaError_t cudaDeviceGetAttribute(int* v, enum cudaDeviceAttr a, int d) { (void)a; (void)d; *v = 148; return cudaSuccess; }
+cudaError_t cudaDeviceGetAttribute(int* v, enum cudaDeviceAttr a, int d) { (void)a; (void)d; *v = fake_sms; return cudaSuccess; }
 cudaError_t cudaDeviceSynchronize(void) { return cudaSuccess; }
 cudaError_t cudaGetLastError(void) { int e = last; last = 0; return (cudaError_t)e; }
 const char* cudaGetErrorString(cudaError_t e) { return e ? "refused" : "no error"; }
 cudaError_t cudaFuncSetAttribute(const void* f, enum cudaFuncAttribute a, int v) { (void)f; (void)a; (void)v; return cudaSuccess; }
 cudaError_t cudaLaunchKernel(const void* f, dim3 g, dim3 b, void** args, size_t sm, cudaStream_t st) {
-  (void)f; (void)g; (void)b; (void)args; (void)sm;
+  (void)f; (void)b; (void)args; (void)sm;
+  size_t n = strlen(launches);
+  snprintf(launches + n, sizeof launches - n, "%u %u\n", g.x, g.y);
   if (st && st->device != cur) return (cudaError_t)(last = cudaErrorInvalidResourceHandle);
   return cudaSuccess;
 }

@@ -15,7 +15,7 @@ import ctypes, sys
 sys.path.insert(0, sys.argv[2])
 import numpy as np
 fake = ctypes.CDLL(sys.argv[1])
-fake.fake_log.restype = ctypes.c_char_p
+fake.fake_log.restype = fake.fake_launches.restype = ctypes.c_char_p
 from ragdoll_b200.engine import RG_FRAME_IDR, RG_FRAME_P, Engine, RgError, lib
 log = lambda: [l.split() for l in fake.fake_log().decode().split("\\n")[:-1]]
 """
@@ -91,6 +91,21 @@ for device in (-1, 64):
         raise SystemExit("accepted")
     except RgError:
         pass
+""")
+
+
+def test_ssim_strips_follow_the_devices_sms(fake):
+    """Tall strips (16 window rows) once there are two blocks an SM of them, flat ones (4) before: four planes
+    of 1080 rows are 68 tall strips."""
+    _run(fake, """
+from ragdoll_b200.engine import ssim_batch_device
+plane = np.zeros(64 * 1080, np.uint8).ctypes.data
+for sms, strips in ((34, 17), (35, 68), (148, 68)):
+    ctypes.c_int.in_dll(fake, "fake_sms").value = sms
+    fake.fake_clear()
+    ssim_batch_device([plane] * 4, [plane] * 4, 64, 1080, 64, 64)
+    grids = [tuple(map(int, l.split())) for l in fake.fake_launches().decode().split("\\n")[:-1]]
+    assert grids[0] == (strips, 4), (sms, grids)
 """)
 
 
