@@ -2040,6 +2040,10 @@ __global__ void __launch_bounds__(32) wavefront_step_kernel(const __grid_constan
   init_tables();
   load_params(fp);
   load_desc(streams + blockIdx.y);
+  if constexpr (kForm != 0) {
+    if (lane_id() == 0) ss.job.failed = false;  // (nobody shares searches here)
+    __syncwarp();
+  }
   const StreamDev& sd = sm.sd;
   int na = diag_len(fp, step);
   int nd = fp.deblock ? diag_len(fp, step - 3) : 0;
@@ -2291,7 +2295,10 @@ __global__ void __launch_bounds__(32 * kBlockWarps, 1) pipeline_kernel(const __g
     board = 0;
   }
   if constexpr (kForm != 0)
-    if (lane == 0) ss.job.ticket = kNoJob;
+    if (lane == 0) {
+      ss.job.ticket = kNoJob;
+      ss.job.failed = false;
+    }
   if (lane == 0) sm.reach_y = sm.reach_x = 0;  // this warp's, published once as it exits
   int group = -1;                              // whose parameters sm.fp holds
   __syncthreads();

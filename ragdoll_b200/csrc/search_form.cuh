@@ -54,6 +54,7 @@ struct SearchJob {
   uint32_t lambda;
   uint32_t ticket;   // next unit | units << 16; kNoJob while there is none
   int done;          // units finished
+  bool failed;       // the wait for them gave up: the launch fails, and this warp leaves
   uint32_t key[9];   // the least so far
 };
 constexpr uint32_t kNoJob = 0x8000u;  // (a ticket past any unit)
@@ -296,10 +297,12 @@ __device__ __noinline__ void help_searches(unsigned* board) {
 // falls back to it, 50.2 and 46.7, 4K 4 x 3 48.7 and 46.6). Sharing the partition types' refinement the same
 // way gave the full search 6 % more and cost the learned form 3 %.
 //
-// False when the wait for units others took gave up: ss.ib then holds nothing, and the caller has to leave as
-// after any wait that did -- the warp takes no other segment, so the job that others may still read stays as it is.
-[[nodiscard]] __device__ __noinline__ bool int_search(const Ctx c, int xlo, int xhi, int ylo, int yhi, int mvp0, int mvp1,
-                                                      uint32_t lambda, const PipeWait pw) {
+// ss.job.failed once the wait for units others took gave up: ss.ib then holds nothing, and the caller has to
+// leave as after any wait that did -- the warp takes no other segment, so the job that others may still read
+// stays as it is. (As a result of this function it made the full search 6 % slower, 8 x 3 720p 24.4 -> 25.9 ms.)
+// A window of a vector a lane has no units and cannot fail.
+__device__ __noinline__ void int_search(const Ctx c, int xlo, int xhi, int ylo, int yhi,
+                                        int mvp0, int mvp1, uint32_t lambda, const PipeWait pw) {
   const int lane = lane_id();
   const int x0 = c.mbx * 16, y0 = c.mby * 16;
   const int nwx = xhi - xlo + 1, nwy = yhi - ylo + 1;
@@ -329,7 +332,6 @@ __device__ __noinline__ void help_searches(unsigned* board) {
     }
     __syncwarp();
     search_units(threadIdx.y);
-    bool ok = true;
     if (lane == 0) {
       if (pw.board) atomicAnd(pw.board, ~(1u << threadIdx.y));
       atomicExch(&jb.ticket, kNoJob);
@@ -339,13 +341,12 @@ __device__ __noinline__ void help_searches(unsigned* board) {
         if (!t0) t0 = global_ns();
         else if (global_ns() - t0 > pw.timeout_ns) {
           if (pw.error) atomicCAS(pw.error, 0, 1);
-          ok = false;
+          jb.failed = true;
           break;
         }
         __nanosleep(50);
       }
     }
-    if (!__shfl_sync(FULL, ok, 0)) return false;
     __threadfence_block();
     __syncwarp();
 #pragma unroll
@@ -380,7 +381,6 @@ __device__ __noinline__ void help_searches(unsigned* board) {
     ss.ib.y[lane] = ylo + y;
   }
   __syncwarp();
-  return true;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -698,7 +698,7 @@ __device__ __noinline__ bool analyse_p_mb_search(const Ctx c, const PipeWait pw)
     yhi = min(lcy + kLearnedRange, imax1);
   }
   IntBest& ib = ss.ib;  // warp-uniform: once per warp in shared memory
-  if (!int_search(c, xlo, xhi, ylo, yhi, mvp16[0], mvp16[1], lambda, pw)) return false;
+  int_search(c, xlo, xhi, ylo, yhi, mvp16[0], mvp16[1], lambda, pw);
   if (hint) {
     bool edge = (ib.x[0] == xlo && xlo > imin0) || (ib.x[0] == xhi && xhi < imax0) ||
                 (ib.y[0] == ylo && ylo > imin1) || (ib.y[0] == yhi && yhi < imax1);
@@ -709,7 +709,7 @@ __device__ __noinline__ bool analyse_p_mb_search(const Ctx c, const PipeWait pw)
       ylo = max(cy - kLearnedRange, imin1);
       yhi = min(cy + kLearnedRange, imax1);
       if (!wait_window(c, pw, xhi, yhi)) return false;
-      if (!int_search(c, xlo, xhi, ylo, yhi, mvp16[0], mvp16[1], lambda, pw)) return false;
+      int_search(c, xlo, xhi, ylo, yhi, mvp16[0], mvp16[1], lambda, pw);
       edge = (ib.x[0] == xlo && xlo > imin0) || (ib.x[0] == xhi && xhi < imax0) ||
              (ib.y[0] == ylo && ylo > imin1) || (ib.y[0] == yhi && yhi < imax1);
     }
@@ -717,9 +717,12 @@ __device__ __noinline__ bool analyse_p_mb_search(const Ctx c, const PipeWait pw)
       xlo = max(fcx - R, imin0); xhi = min(fcx + R, imax0);
       ylo = max(fcy - R, imin1); yhi = min(fcy + R, imax1);
       if (!wait_window(c, pw, xhi, yhi)) return false;
-      if (!int_search(c, xlo, xhi, ylo, yhi, mvp16[0], mvp16[1], lambda, pw)) return false;
+      int_search(c, xlo, xhi, ylo, yhi, mvp16[0], mvp16[1], lambda, pw);
     }
   }
+  // a wait for shared units gave up: in the full search, or in the fallback above (the small windows share nothing)
+  static_assert(2 * kLearnedRange + 1 <= 8 && (2 * kLearnedRange + 1) * (2 * kLearnedRange + 1) <= 32, "a vector a lane");
+  if (ss.job.failed) return false;
   // 3-4. refinement of every tried type, the least total cost wins
   int best_t = -1;
   uint32_t best_j = UMAX;
