@@ -2040,10 +2040,6 @@ __global__ void __launch_bounds__(32) wavefront_step_kernel(const __grid_constan
   init_tables();
   load_params(fp);
   load_desc(streams + blockIdx.y);
-  if constexpr (kForm != 0) {
-    if (lane_id() == 0) ss.job.failed = false;  // (nobody shares searches here)
-    __syncwarp();
-  }
   const StreamDev& sd = sm.sd;
   int na = diag_len(fp, step);
   int nd = fp.deblock ? diag_len(fp, step - 3) : 0;
@@ -2358,6 +2354,11 @@ __global__ void __launch_bounds__(32 * kBlockWarps, 1) pipeline_kernel(const __g
           if constexpr (kForm != 0) failed = !analyse_p_mb_search(c, pw);
           else failed = !analyse_p_mb<kEarly>(c, pw) || (kEarly && !wait_recon(c, pw));  // (the row's progress counts the left one)
           if (failed) break;
+          if constexpr (kForm != 0)
+            if (*(volatile bool*)&ss.job.failed) {  // (nothing of it is published)
+              failed = true;
+              break;
+            }
         }
         publish(ana_rows + y, x + 1);
       }

@@ -54,7 +54,7 @@ struct SearchJob {
   uint32_t lambda;
   uint32_t ticket;   // next unit | units << 16; kNoJob while there is none
   int done;          // units finished
-  bool failed;       // the wait for them gave up: the launch fails, and this warp leaves
+  bool failed;       // the wait for them gave up: the launch fails, and this warp leaves with its macroblock
   uint32_t key[9];   // the least so far
 };
 constexpr uint32_t kNoJob = 0x8000u;  // (a ticket past any unit)
@@ -297,10 +297,10 @@ __device__ __noinline__ void help_searches(unsigned* board) {
 // falls back to it, 50.2 and 46.7, 4K 4 x 3 48.7 and 46.6). Sharing the partition types' refinement the same
 // way gave the full search 6 % more and cost the learned form 3 %.
 //
-// ss.job.failed once the wait for units others took gave up: ss.ib then holds nothing, and the caller has to
-// leave as after any wait that did -- the warp takes no other segment, so the job that others may still read
-// stays as it is. (As a result of this function it made the full search 6 % slower, 8 x 3 720p 24.4 -> 25.9 ms.)
-// A window of a vector a lane has no units and cannot fail.
+// ss.job.failed once the wait for units others took gave up: the window's first vector stands for every part's
+// then, so that what follows reads what it may, and the macroblock is not published (pipeline_kernel): the warp
+// leaves, as after any wait that gave up, and the job that others may still read stays as it is. (As this
+// function's result it made the full search 6 % slower, read after it the learned form 0.7 %; so it is 1 and 0.1 %.)
 __device__ __noinline__ void int_search(const Ctx c, int xlo, int xhi, int ylo, int yhi,
                                         int mvp0, int mvp1, uint32_t lambda, const PipeWait pw) {
   const int lane = lane_id();
@@ -342,6 +342,7 @@ __device__ __noinline__ void int_search(const Ctx c, int xlo, int xhi, int ylo, 
         else if (global_ns() - t0 > pw.timeout_ns) {
           if (pw.error) atomicCAS(pw.error, 0, 1);
           jb.failed = true;
+          for (int k = 0; k < 9; k++) atomicExch(&jb.key[k], 0u);  // (below any cost: it stays)
           break;
         }
         __nanosleep(50);
@@ -629,8 +630,8 @@ __device__ __noinline__ int2 learned_centre(const Ctx c, int mvp0, int mvp1, uin
   return make_int2(bx, by);
 }
 
-// One macroblock of a P slice in the search forms (see the head of this file); false, with nothing
-// written, when a wait for the reference picture or for shared search units gave up.
+// One macroblock of a P slice in the search forms (see the head of this file); false when a wait for
+// the reference picture gave up (for shared search units: ss.job.failed).
 __device__ __noinline__ bool analyse_p_mb_search(const Ctx c, const PipeWait pw) {
   const StreamDev& sd = sm.sd;
   const int lane = lane_id();
@@ -720,9 +721,6 @@ __device__ __noinline__ bool analyse_p_mb_search(const Ctx c, const PipeWait pw)
       int_search(c, xlo, xhi, ylo, yhi, mvp16[0], mvp16[1], lambda, pw);
     }
   }
-  // a wait for shared units gave up: in the full search, or in the fallback above (the small windows share nothing)
-  static_assert(2 * kLearnedRange + 1 <= 8 && (2 * kLearnedRange + 1) * (2 * kLearnedRange + 1) <= 32, "a vector a lane");
-  if (ss.job.failed) return false;
   // 3-4. refinement of every tried type, the least total cost wins
   int best_t = -1;
   uint32_t best_j = UMAX;
