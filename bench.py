@@ -51,8 +51,8 @@ METRIC = "1080p H.264 encode frames/s: learned vs plain GPU, equal PSNR, \u22642
 UNIT = "frames/s"
 BYTES_PER_FRAME = 7.5 * W * H  # source 1.5 + reference 1.5 + recon 1.5 + deblock read/write 3.0 (x W*H)
 # DRAM bytes per picture of pipeline_kernel measured by ncu (dram__bytes_read + write) on a launch
-# of 8 streams x 4 pictures of this workload: 490.2 MB / 32 (scaled to a launch by its pictures).
-TRAFFIC_PER_FRAME = 464.1e6 / 32
+# of 8 streams x 4 pictures of this workload: 464.7 MB / 32 (scaled to a launch by its pictures).
+TRAFFIC_PER_FRAME = 464.7e6 / 32
 
 
 def dist_env():
@@ -1110,8 +1110,8 @@ def run_engine(args, rank, world, local):
 
     # SSIM and MS-SSIM of 120 luma plane pairs in one batched call (shared launches over every
     # pair and pyramid level); the pairs are pictures of the step's clip (their values do not change
-    # the work). Algorithmic bytes per 1080p pair: both planes read at the five levels, and four
-    # decimations reading one level and writing the next: ~5.98 W H.
+    # the work). Algorithmic bytes per 1080p pair: both planes read once, each of the four pyramid
+    # levels written and read once: ~3.33 W H.
     from ragdoll_b200.engine import ssim_batch_device
     qstream = torch.cuda.Stream(device=local)
     pa = [base + i * fbytes for i in range(FRAMES)]
@@ -1128,7 +1128,7 @@ def run_engine(args, rank, world, local):
     q_wall_ms = (time.perf_counter() - tq) * 1000 / q_reps
     q_ms = q0.elapsed_time(q1) / q_reps
     lv = sum(4.0 ** -k for k in range(5))
-    q_bytes = FRAMES * W * H * (2 * lv + 2 * (lv - 4.0 ** -4) + 2 * (lv - 1))
+    q_bytes = FRAMES * W * H * (2 + 4 * (lv - 1))
 
     # per-launch duration of the dominant kernel
     steps_per_frame = (eng.mb_w - 1) + 2 * (eng.mb_h - 1) + 1 + 3

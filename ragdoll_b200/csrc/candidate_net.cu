@@ -46,7 +46,8 @@ __device__ __forceinline__ float pix_norm(uint8_t v) { return ((float)v - 128.0f
 // ---------------------------------------------------------------------------------------------
 // Inference on the tensor cores. Two CTAs per SM, each a strip of two macroblocks at a time; one
 // activation buffer per CTA holds every map of its strip in turn (the input in plane 0, then each
-// layer's output over its input: a layer's epilogue starts once all its MMAs have completed).
+// layer's output over its input, tile by tile: a tile's MMAs read its positions and the next tile's, so
+// tile t is stored once the MMAs of tiles t - 1 and t have completed).
 constexpr int kStripMbs = 2;
 constexpr int kThreads = 256;  // 8 warps; warps w and w + 4 share TMEM lanes 32 (w % 4)..; a ninth issues the MMAs
 constexpr int kCtasPerSm = 2;
@@ -471,7 +472,7 @@ __global__ void __launch_bounds__(kThreads + 32, kCtasPerSm) cnn_infer_kernel(In
 // wins. Bound by instructions: the eight windows of a block overlap and are decimated once, by words
 // where they lie inside the picture, and a lane slides down a column of displacements, so that a row of
 // the window is read once for eight of them. Eight 1080p pictures at r = 16: 0.77 ms with a window per
-// macroblock and a vector at a time, 0.25 ms so.
+// macroblock and a vector at a time, 0.20 ms so (the launch alone).
 constexpr int kCoarseMaxR = 32;
 constexpr int kCoarseMbs = 8;                                             // macroblocks (warps) of a block
 constexpr int kCoarseRow = 8 * kCoarseMbs + 2 * kCoarseMaxR + 4;          // window row stride (bytes), an odd number of words
